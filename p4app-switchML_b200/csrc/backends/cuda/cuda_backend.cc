@@ -766,126 +766,4 @@ int ConvertU8OnDevice(bool widen, const void* in, void* out, unsigned long long 
   return static_cast<int>(e);
 }
 
-int EmulatedAllReduce(int nranks, void* const* in_ptrs, void* const* out_ptrs,
-                      unsigned long long numel, int elem_type, int mode, int algo, int block_numel,
-                      size_t slot_bytes, int slots_per_channel, int channels, float post_scale,
-                      int repeats, int exponent_lookahead, std::string* error) {
-  using namespace kernels;
-  auto fail = [&](const std::string& m, int code) {
-    if (error) *error = m;
-    return code;
-  };
-  if (nranks < 1 || nranks > kMaxRanks) return fail("nranks out of range", -1);
-  if (algo == ALGO_ZEROCOPY) return fail("zero-copy needs real symmetric memory", -1);
-  if (slot_bytes / 4 / block_numel * slots_per_channel > 8192)
-    return fail("slots_per_channel * slot_bytes / (4 * block_numel) exceeds 8192", -1);
-  int dev = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceProp prop;
-  if (cudaGetDeviceProperties(&prop, dev) != cudaSuccess) return fail("no CUDA device", -2);
-  int esz = elem_type == ELEM_BF16 ? 2 : 4;
-  size_t oneshot_bytes = algo == ALGO_ONESHOT ? (numel * esz + 255) / 256 * 256 : 256;
-  int max_channels = prop.multiProcessorCount / nranks;  // all virtual ranks share the GPU
-  if (max_channels < 1) max_channels = 1;
-  if (channels > 0 && channels < max_channels) max_channels = channels;
-
-  RankCtx proto;
-  memset(&proto, 0, sizeof(proto));
-  proto.nranks = nranks;
-  proto.slot_bytes = slot_bytes;
-  proto.slots_per_channel = slots_per_channel;
-  proto.sc_fence = 0;
-  proto.exp_ring = ExpRingDepth(slots_per_channel);
-  proto.exp_lookahead = ExpLookahead(slots_per_channel, exponent_lookahead < 0 ? kDefaultExpLookahead : exponent_lookahead);
-  proto.block_numel = block_numel;
-  proto.quant_base = quant::QuantBase(nranks);
-  proto.oneshot_bytes = oneshot_bytes;
-  proto.timeout_ns = 2000000000ull;  // 2 s: generous for one GPU, still bounded
-  size_t bytes = StagingBytes(slot_bytes, slots_per_channel, block_numel, max_channels,
-                              oneshot_bytes, nranks, &proto.data_offset, &proto.exp_offset,
-                              &proto.oneshot_offset);
-  proto.stage_bytes = ReportedStageBytes(bytes);
-  std::vector<char*> stage(nranks, nullptr);
-  int* status = nullptr;
-  unsigned long long* counters = nullptr;
-  RankCtx* d_ctx = nullptr;
-  JobArgs* d_job = nullptr;
-  unsigned long long* epochs = nullptr;
-  int result = 0;
-  cudaError_t e = cudaSuccess;
-  auto cleanup = [&] {
-    for (char* p : stage) if (p) cudaFree(p);
-    if (status) cudaFree(status);
-    if (counters) cudaFree(counters);
-    if (epochs) cudaFree(epochs);
-    if (d_ctx) cudaFree(d_ctx);
-    if (d_job) cudaFree(d_job);
-  };
-  for (int r = 0; r < nranks && e == cudaSuccess; r++) {
-    e = cudaMalloc(&stage[r], bytes);
-    if (e == cudaSuccess) e = cudaMemset(stage[r], 0, bytes);
-  }
-  if (e == cudaSuccess) e = cudaMalloc(&status, nranks * sizeof(int));
-  if (e == cudaSuccess) e = cudaMemset(status, 0, nranks * sizeof(int));
-  if (e == cudaSuccess) e = cudaMalloc(&counters, nranks * 16 * sizeof(unsigned long long));
-  if (e == cudaSuccess) e = cudaMemset(counters, 0, nranks * 16 * sizeof(unsigned long long));
-  if (e == cudaSuccess) e = cudaMalloc(&epochs, nranks * kMaxChannels * sizeof(unsigned long long));
-  if (e == cudaSuccess) e = cudaMemset(epochs, 0, nranks * kMaxChannels * sizeof(unsigned long long));
-  if (e == cudaSuccess) e = cudaMalloc(&d_ctx, nranks * sizeof(RankCtx));
-  if (e == cudaSuccess) e = cudaMalloc(&d_job, nranks * sizeof(JobArgs));
-  if (e != cudaSuccess) {
-    cleanup();
-    return fail(std::string("allocation failed: ") + cudaGetErrorString(e), -3);
-  }
-  if (algo == ALGO_PUSH && PushTileCapacity(proto, elem_type, mode) == 0) {
-    cleanup();
-    return fail("ALGO_PUSH needs at least two ranks and slots of about twice nranks * max(block, 128) * 4 bytes", -1);
-  }
-  std::vector<RankCtx> ctxs(nranks, proto);
-  std::vector<JobArgs> jobs(nranks);
-  unsigned long long epoch = 0;
-  for (int it = 0; it < (repeats < 1 ? 1 : repeats) && result == 0; it++) {
-    LaunchPlan plan;
-    for (int r = 0; r < nranks; r++) {
-      ctxs[r].rank = r;
-      for (int p = 0; p < nranks; p++) ctxs[r].stage_peer[p] = stage[p];
-      ctxs[r].status = status + r;
-      ctxs[r].counters = counters + r * 16;
-      ctxs[r].epoch_words = epochs + static_cast<size_t>(r) * kMaxChannels;
-      JobArgs& j = jobs[r];
-      memset(&j, 0, sizeof(j));
-      j.in = in_ptrs[r];
-      j.out = out_ptrs[r];
-      j.numel = numel;
-      j.elem_type = elem_type;
-      j.mode = mode;
-      j.algo = algo;
-      j.post_scale = post_scale;
-      j.bulk_copy = DeviceMemory(j.in) && DeviceMemory(j.out);
-      j.oneshot_parity = it & 1;
-    }
-    plan = PlanLaunch(ctxs[0], jobs[0], channels, max_channels);
-    for (int r = 0; r < nranks; r++) {
-      jobs[r].tile_elems = plan.tile_elems;
-      jobs[r].epochs = plan.epochs;
-    }
-    epoch += plan.epochs;
-    cudaMemcpy(d_ctx, ctxs.data(), nranks * sizeof(RankCtx), cudaMemcpyHostToDevice);
-    cudaMemcpy(d_job, jobs.data(), nranks * sizeof(JobArgs), cudaMemcpyHostToDevice);
-    e = LaunchAllReduceEmulated(d_ctx, d_job, jobs[0], nranks, plan, 0);
-    if (e == cudaSuccess) e = cudaDeviceSynchronize();
-    if (e != cudaSuccess) {
-      result = fail(std::string("emulated launch failed: ") + cudaGetErrorString(e), -4);
-      break;
-    }
-    std::vector<int> st(nranks);
-    cudaMemcpy(st.data(), status, nranks * sizeof(int), cudaMemcpyDeviceToHost);
-    for (int r = 0; r < nranks; r++) {
-      if (st[r] != STATUS_OK) result = fail("kernel status " + std::to_string(st[r]) + " on rank " + std::to_string(r), st[r]);
-    }
-  }
-  cleanup();
-  return result;
-}
-
 }  // namespace switchml

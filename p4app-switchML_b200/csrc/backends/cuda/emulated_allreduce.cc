@@ -1,0 +1,247 @@
+// EmulatedAllReduce (cuda_backend.h): several ranks of one aggregation played by one
+// cooperative kernel on one GPU.
+//
+// A call used to cost 5 to 25 ms around a kernel of 0.1 to 0.4 ms: cudaGetDeviceProperties
+// (2.8 ms), seven to nine cudaMalloc / cudaFree pairs (0.2 to 0.3 ms each, and every free
+// waits for the device), clears of the whole staging memory and three blocking copies. Now
+// the staging memory of a finished call is kept for the next one, and everything the kernel
+// has to know travels as a launch argument. Flags, exponent words and epochs need no clearing
+// between calls, for the same reason as between the jobs of a context: epochs only grow.
+#include <cuda_runtime.h>
+
+#include <cstdio>
+#include <cstring>
+#include <memory>
+#include <mutex>
+#include <string>
+#include <vector>
+
+#include "backends/cuda/cuda_backend.h"
+#include "kernels/allreduce_kernels.h"
+#include "switchml/quant_math.h"
+
+namespace switchml {
+
+namespace {
+
+using namespace kernels;
+
+// Staging memory of all ranks of a call, with their epochs, counters and status words.
+struct EmuWorkspace {
+  int device = -1;
+  size_t capacity = 0;              // bytes of `memory`
+  char* memory = nullptr;           // [epochs and counters][rank 0's staging region][rank 1's] ...
+  int* status = nullptr;            // kMaxRanks words of pinned host memory that the kernel writes
+  int* status_dev = nullptr;
+  std::string layout;               // geometry that the flags and exponent words in `memory` belong to
+
+  ~EmuWorkspace() {
+    int current = -1;
+    cudaGetDevice(&current);
+    if (device >= 0 && device != current) cudaSetDevice(device);
+    if (memory) cudaFree(memory);
+    if (status) cudaFreeHost(status);
+    if (device >= 0 && device != current) cudaSetDevice(current);
+  }
+};
+
+constexpr size_t kEpochBytes = size_t(kMaxRanks) * kMaxChannels * sizeof(unsigned long long);
+constexpr size_t kCounterBytes = size_t(kMaxRanks) * 16 * sizeof(unsigned long long);
+constexpr size_t kHeadBytes = (kEpochBytes + kCounterBytes + 4095) / 4096 * 4096;
+
+// Workspaces that no call is using. A call takes one out and puts it back when its kernel has
+// ended, so calls of several threads never share one. Bounded: at most kKept, together at
+// most kKeptBytes; what does not fit is freed at once, and all are given back when an
+// allocation fails or by ReleaseEmulationWorkspaces().
+class WorkspacePool {
+ public:
+  static WorkspacePool& Get() {
+    static WorkspacePool* pool = new WorkspacePool;  // never destroyed: the CUDA runtime may be gone by then
+    return *pool;
+  }
+  // The workspace of `layout` if there is one, else the smallest that is large enough.
+  std::unique_ptr<EmuWorkspace> Take(int device, size_t bytes, const std::string& layout) {
+    std::lock_guard<std::mutex> lk(mu_);
+    size_t best = free_.size();
+    for (size_t i = 0; i < free_.size(); i++) {
+      const EmuWorkspace& w = *free_[i];
+      if (w.device != device || w.capacity < bytes) continue;
+      if (w.layout == layout) {
+        best = i;
+        break;
+      }
+      if (best == free_.size() || w.capacity < free_[best]->capacity) best = i;
+    }
+    if (best == free_.size()) return nullptr;
+    std::unique_ptr<EmuWorkspace> w = std::move(free_[best]);
+    free_.erase(free_.begin() + best);
+    return w;
+  }
+  void Put(std::unique_ptr<EmuWorkspace> w) {
+    std::vector<std::unique_ptr<EmuWorkspace>> drop;  // freed after the lock is gone
+    std::lock_guard<std::mutex> lk(mu_);
+    free_.push_back(std::move(w));
+    auto kept = [&] {
+      size_t sum = 0;
+      for (const auto& f : free_) sum += f->capacity;
+      return sum;
+    };
+    while (free_.size() > kKept || (!free_.empty() && kept() > kKeptBytes)) {
+      drop.push_back(std::move(free_.front()));  // the one that has been lying here longest
+      free_.erase(free_.begin());
+    }
+  }
+  void Clear() {
+    std::vector<std::unique_ptr<EmuWorkspace>> drop;
+    std::lock_guard<std::mutex> lk(mu_);
+    drop.swap(free_);
+  }
+
+ private:
+  static constexpr size_t kKept = 4;
+  static constexpr size_t kKeptBytes = size_t(1) << 29;
+  std::mutex mu_;
+  std::vector<std::unique_ptr<EmuWorkspace>> free_;
+};
+
+std::unique_ptr<EmuWorkspace> NewWorkspace(int device, size_t bytes, cudaError_t* e) {
+  std::unique_ptr<EmuWorkspace> w(new EmuWorkspace);
+  w->device = device;
+  *e = cudaMalloc(reinterpret_cast<void**>(&w->memory), bytes);
+  if (*e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    WorkspacePool::Get().Clear();
+    *e = cudaMalloc(reinterpret_cast<void**>(&w->memory), bytes);
+  }
+  if (*e == cudaSuccess)
+    *e = cudaHostAlloc(reinterpret_cast<void**>(&w->status), kMaxRanks * sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable);
+  if (*e == cudaSuccess) *e = cudaHostGetDevicePointer(reinterpret_cast<void**>(&w->status_dev), w->status, 0);
+  w->capacity = bytes;
+  if (*e == cudaSuccess) return w;
+  cudaGetLastError();
+  return nullptr;
+}
+
+int SmCount(int device) {
+  static int count[64] = {0};
+  if (device < 0 || device >= 64) return 0;
+  if (count[device] == 0) {
+    int n = 0;
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) return 0;
+    count[device] = n;
+  }
+  return count[device];
+}
+
+}  // namespace
+
+void ReleaseEmulationWorkspaces() { WorkspacePool::Get().Clear(); }
+
+int EmulatedAllReduce(int nranks, void* const* in_ptrs, void* const* out_ptrs,
+                      unsigned long long numel, int elem_type, int mode, int algo, int block_numel,
+                      size_t slot_bytes, int slots_per_channel, int channels, float post_scale,
+                      int repeats, int exponent_lookahead, std::string* error) {
+  auto fail = [&](const std::string& m, int code) {
+    if (error) *error = m;
+    return code;
+  };
+  if (nranks < 1 || nranks > kMaxRanks) return fail("nranks out of range", -1);
+  if (algo == ALGO_ZEROCOPY) return fail("zero-copy needs real symmetric memory", -1);
+  if (slot_bytes / 4 / block_numel * slots_per_channel > 8192)
+    return fail("slots_per_channel * slot_bytes / (4 * block_numel) exceeds 8192", -1);
+  int dev = 0;
+  cudaGetDevice(&dev);
+  const int sms = SmCount(dev);
+  if (sms <= 0) return fail("no CUDA device", -2);
+  int esz = elem_type == ELEM_BF16 ? 2 : 4;
+  size_t oneshot_bytes = algo == ALGO_ONESHOT ? (numel * esz + 255) / 256 * 256 : 256;
+  int max_channels = sms / nranks;  // all virtual ranks share the GPU
+  if (max_channels < 1) max_channels = 1;
+  if (channels > 0 && channels < max_channels) max_channels = channels;
+
+  RankCtx proto;
+  memset(&proto, 0, sizeof(proto));
+  proto.nranks = nranks;
+  proto.slot_bytes = slot_bytes;
+  proto.slots_per_channel = slots_per_channel;
+  proto.sc_fence = 0;
+  proto.exp_ring = ExpRingDepth(slots_per_channel);
+  proto.exp_lookahead = ExpLookahead(slots_per_channel, exponent_lookahead < 0 ? kDefaultExpLookahead : exponent_lookahead);
+  proto.block_numel = block_numel;
+  proto.quant_base = quant::QuantBase(nranks);
+  proto.oneshot_bytes = oneshot_bytes;
+  proto.timeout_ns = 2000000000ull;  // 2 s: generous for one GPU, still bounded
+  const size_t bytes = StagingBytes(slot_bytes, slots_per_channel, block_numel, max_channels,
+                                    oneshot_bytes, nranks, &proto.data_offset, &proto.exp_offset,
+                                    &proto.oneshot_offset);
+  proto.stage_bytes = ReportedStageBytes(bytes);
+  if (algo == ALGO_PUSH && PushTileCapacity(proto, elem_type, mode) == 0)
+    return fail("ALGO_PUSH needs at least two ranks and slots of about twice nranks * max(block, 128) * 4 bytes", -1);
+
+  // Flags and exponent words of another layout are noise in this one, so they are cleared (with
+  // the epochs, which start over) when the layout changes, and only then.
+  char layout[128];
+  snprintf(layout, sizeof(layout), "%d/%zu/%d/%d/%d/%zu", nranks, slot_bytes, slots_per_channel, block_numel, max_channels, bytes);
+  const size_t need = kHeadBytes + bytes * nranks;
+  cudaError_t e = cudaSuccess;
+  std::unique_ptr<EmuWorkspace> ws = WorkspacePool::Get().Take(dev, need, layout);
+  if (!ws) ws = NewWorkspace(dev, need, &e);
+  if (!ws) return fail(std::string("allocation failed: ") + cudaGetErrorString(e), -3);
+  char* const stage0 = ws->memory + kHeadBytes;
+  if (ws->layout != layout) {
+    ws->layout.clear();
+    e = cudaMemsetAsync(ws->memory, 0, kHeadBytes, 0);
+    if (e == cudaSuccess) e = cudaMemset2DAsync(stage0, bytes, 0, proto.oneshot_offset, nranks, 0);
+    if (e != cudaSuccess) return fail(std::string("allocation failed: ") + cudaGetErrorString(e), -3);
+  }
+
+  EmuArgs args;
+  memset(&args, 0, sizeof(args));
+  LaunchPlan plan;
+  for (int it = 0; it < (repeats < 1 ? 1 : repeats); it++) {
+    for (int r = 0; r < nranks; r++) {
+      RankCtx& c = args.ctx[r];
+      c = proto;
+      c.rank = r;
+      for (int p = 0; p < nranks; p++) c.stage_peer[p] = stage0 + bytes * p;
+      c.status = ws->status_dev + r;
+      c.epoch_words = reinterpret_cast<unsigned long long*>(ws->memory) + static_cast<size_t>(r) * kMaxChannels;
+      c.counters = reinterpret_cast<unsigned long long*>(ws->memory + kEpochBytes) + r * 16;
+      JobArgs& j = args.job[r];
+      j.in = in_ptrs[r];
+      j.out = out_ptrs[r];
+      j.numel = numel;
+      j.elem_type = elem_type;
+      j.mode = mode;
+      j.algo = algo;
+      j.post_scale = post_scale;
+      if (it == 0) j.bulk_copy = DeviceMemory(j.in) && DeviceMemory(j.out);
+      j.oneshot_parity = it & 1;
+    }
+    if (it == 0) {
+      plan = PlanLaunch(args.ctx[0], args.job[0], channels, max_channels);
+      for (int r = 0; r < nranks; r++) ws->status[r] = STATUS_OK;
+    }
+    for (int r = 0; r < nranks; r++) {
+      args.job[r].tile_elems = plan.tile_elems;
+      args.job[r].epochs = plan.epochs;
+    }
+    e = LaunchAllReduceEmulated(args, nranks, plan, 0);
+    if (e != cudaSuccess) break;
+  }
+  if (e == cudaSuccess) e = cudaDeviceSynchronize();
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return fail(std::string("emulated launch failed: ") + cudaGetErrorString(e), -4);
+  }
+  for (int r = 0; r < nranks; r++) {
+    const int st = *reinterpret_cast<volatile int*>(ws->status + r);
+    if (st != STATUS_OK) return fail("kernel status " + std::to_string(st) + " on rank " + std::to_string(r), st);
+  }
+  // Only after a call that went well: the ranks' epochs are in step then.
+  ws->layout = layout;
+  WorkspacePool::Get().Put(std::move(ws));
+  return 0;
+}
+
+}  // namespace switchml

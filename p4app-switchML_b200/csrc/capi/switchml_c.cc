@@ -265,6 +265,8 @@ int sml_emu_allreduce(int nranks, void* const* in_ptrs, void* const* out_ptrs, u
   return r;
 }
 
+void sml_emu_release(void) { ReleaseEmulationWorkspaces(); }
+
 int sml_convert_u8(int widen, const void* in, void* out, uint64_t numel, void* stream) {
   std::string err;
   int r = ConvertU8OnDevice(widen != 0, in, out, numel, stream, &err);

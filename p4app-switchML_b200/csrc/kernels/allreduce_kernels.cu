@@ -1052,15 +1052,18 @@ AllReduceKernel(const RankCtx ctx, const JobArgs job, unsigned long long epc) {
 // All ranks in one grid: blockIdx.y selects the rank whose role this CTA plays.
 template <int ELEM, int MODE, int ALGO>
 __global__ void __launch_bounds__(kThreads, 1)
-AllReduceEmuKernel(const RankCtx* ctxs, const JobArgs* jobs, unsigned long long epc) {
+AllReduceEmuKernel(const __grid_constant__ EmuArgs args, unsigned long long epc) {
   __shared__ StagedShared s_state;
   __shared__ float s_sf[(MODE == MODE_QUANT && (ALGO == ALGO_STAGED || ALGO == ALGO_PUSH)) ? kMaxBlocksPerSlot : 1];
   __shared__ RankCtx s_ctx;
   __shared__ JobArgs s_job;
-  if (threadIdx.x == 0) {
-    s_ctx = ctxs[blockIdx.y];
-    s_job = jobs[blockIdx.y];
-  }
+  // This rank's arguments as whole words, side by side: one trip to the constant bank instead of
+  // one thread's walk through both structs.
+  static_assert(sizeof(RankCtx) % 4 == 0 && sizeof(JobArgs) % 4 == 0, "copied as words");
+  const unsigned* from_ctx = reinterpret_cast<const unsigned*>(&args.ctx[blockIdx.y]);
+  const unsigned* from_job = reinterpret_cast<const unsigned*>(&args.job[blockIdx.y]);
+  for (unsigned i = threadIdx.x; i < sizeof(RankCtx) / 4; i += blockDim.x) reinterpret_cast<unsigned*>(&s_ctx)[i] = from_ctx[i];
+  for (unsigned i = threadIdx.x; i < sizeof(JobArgs) / 4; i += blockDim.x) reinterpret_cast<unsigned*>(&s_job)[i] = from_job[i];
   __syncthreads();
   SML_EPOCH_PROLOGUE(s_ctx, s_job, blockIdx.x, ALGO)
   RunJob<ELEM, MODE, ALGO>(s_ctx, s_job, blockIdx.x, epc, s_base, &s_state.failed, s_sf);
@@ -1233,10 +1236,9 @@ cudaError_t LaunchOne(const RankCtx& ctx, const JobArgs& job, const LaunchPlan& 
 }
 
 template <int ELEM, int MODE, int ALGO>
-cudaError_t LaunchOneEmu(const RankCtx* ctxs, const JobArgs* jobs, int nranks,
-                         const LaunchPlan& plan, cudaStream_t stream) {
+cudaError_t LaunchOneEmu(const EmuArgs& emu, int nranks, const LaunchPlan& plan, cudaStream_t stream) {
   unsigned long long epc = plan.elems_per_channel;
-  void* args[] = {&ctxs, &jobs, &epc};
+  void* args[] = {const_cast<EmuArgs*>(&emu), &epc};
   dim3 grid(plan.channels, nranks);
   // Cooperative launch: the runtime refuses the launch unless all CTAs can be resident
   // together, which the cross-"rank" barriers need.
@@ -1426,11 +1428,10 @@ cudaError_t LaunchAllReduce(const RankCtx& ctx, const JobArgs& job, const Launch
   SML_DISPATCH(LaunchOne, job.elem_type, job.mode, job.algo, ctx, job, plan, stream);
 }
 
-cudaError_t LaunchAllReduceEmulated(const RankCtx* ctxs_dev, const JobArgs* jobs_dev,
-                                    const JobArgs& job0, int nranks, const LaunchPlan& plan,
+cudaError_t LaunchAllReduceEmulated(const EmuArgs& args, int nranks, const LaunchPlan& plan,
                                     cudaStream_t stream) {
   if (nranks < 1 || nranks > kMaxRanks || plan.channels > kMaxChannels) return cudaErrorInvalidValue;
-  SML_DISPATCH(LaunchOneEmu, job0.elem_type, job0.mode, job0.algo, ctxs_dev, jobs_dev, nranks, plan, stream);
+  SML_DISPATCH(LaunchOneEmu, args.job[0].elem_type, args.job[0].mode, args.job[0].algo, args, nranks, plan, stream);
 }
 
 cudaError_t LaunchLocalCopy(const void* in, void* out, size_t bytes, cudaStream_t stream) {

@@ -149,11 +149,13 @@ LaunchPlan PlanLaunch(const RankCtx& ctx, const JobArgs& job, int requested_chan
 cudaError_t LaunchAllReduce(const RankCtx& ctx, const JobArgs& job, const LaunchPlan& plan,
                             cudaStream_t stream);
 // Single-GPU emulation of `nranks` ranks: one cooperative launch whose blockIdx.y is the
-// rank, every "peer" region living on the same device. `ctxs`/`jobs` are device arrays
-// of length nranks. Exercises the peer-memory code path bit for bit.
-// `job0` is the host copy of jobs_dev[0] (selects the instantiation).
-cudaError_t LaunchAllReduceEmulated(const RankCtx* ctxs_dev, const JobArgs* jobs_dev,
-                                    const JobArgs& job0, int nranks, const LaunchPlan& plan,
+// rank, every "peer" region living on the same device. Exercises the peer-memory code path
+// bit for bit. The ranks' arguments travel with the launch.
+struct EmuArgs {
+  RankCtx ctx[kMaxRanks];
+  JobArgs job[kMaxRanks];
+};
+cudaError_t LaunchAllReduceEmulated(const EmuArgs& args, int nranks, const LaunchPlan& plan,
                                     cudaStream_t stream);
 // Single worker, plain sum, out of place: copy `bytes` bytes with one kernel.
 cudaError_t LaunchLocalCopy(const void* in, void* out, size_t bytes, cudaStream_t stream);

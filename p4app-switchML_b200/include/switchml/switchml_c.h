@@ -84,6 +84,8 @@ int sml_emu_allreduce(int nranks, void* const* in_ptrs, void* const* out_ptrs, u
                       int elem_type, int mode, int algo, int block_numel, uint64_t slot_bytes,
                       int slots_per_channel, int channels, float post_scale, int repeats,
                       int exponent_lookahead);
+/* Free the staging memory that sml_emu_allreduce keeps for its next call (at most 512 MiB). */
+void sml_emu_release(void);
 
 /* Stand-alone controller / software switch (what rank 0 otherwise hosts in-process). */
 void* sml_controller_start(const char* ip, int port, int udp_port);

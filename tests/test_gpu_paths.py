@@ -6,6 +6,7 @@ import numpy as np
 import pytest
 import torch
 
+import switchml_b200 as sml
 from switchml_b200 import lib
 from switchml_b200.ops.emulation import emulated_allreduce
 from switchml_b200.ops.oracle import quant_allreduce_oracle
@@ -44,3 +45,45 @@ def test_kept_staging_memory_serves_other_geometries_and_threads():
     lib().sml_emu_release()
     walk(2)
     assert not errors, errors[0]
+
+
+@pytest.fixture
+def ctx():
+    c = sml.Context.get_instance()
+    yield c
+    if c.state() == sml.ContextState.RUNNING:
+        c.stop()
+
+
+@pytest.mark.parametrize("block", [32, 64, 256, 1024])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_one_worker_exact_pass_at_its_edges(ctx, dtype, block):
+    """Every vector width (what the addresses allow), whole and partial last chunks, blocks of part of
+    a row up to all rows; values of all scales, zero blocks, infinities' neighbours."""
+    assert ctx.start(sml.make_config("cuda", packet_numel=block, mode="int32_quant", launch="inline"))
+    gen = torch.Generator(device="cuda").manual_seed(block)
+    for numel in (1, block - 1, 1023, 1024, 1025, 8192, 3 * 8192 + 1024 + block + 5):
+        for off_in, off_out in ((0, 0), (1, 1), (2, 2), (4, 4), (0, 1), (3, 8)):
+            base = torch.randn(numel + 16, device="cuda", generator=gen) * torch.logspace(-35, 35, numel + 16, device="cuda")
+            base[numel // 2: numel // 2 + 2 * block] = 0.0
+            x = base.to(dtype)[off_in:off_in + numel]
+            frame = torch.full((numel + 16,), 7.0, dtype=dtype, device="cuda")
+            y = frame[off_out:off_out + numel]
+            ctx.all_reduce(x, y)
+            want = torch.from_numpy(quant_allreduce_oracle([x.float().cpu().numpy()], block)).to(dtype)
+            assert torch.equal(y.cpu(), want), (numel, off_in, off_out)
+            assert bool((frame[:off_out] == 7).all()) and bool((frame[off_out + numel:] == 7).all())
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.int32, torch.uint8])
+def test_one_worker_sum_copies_every_alignment(ctx, dtype):
+    assert ctx.start(sml.make_config("cuda", mode="float_sum", launch="inline"))
+    for numel in (1, 7, 15, 16, 17, 8191, 65536 + 3):
+        for off_in in (0, 1, 3):
+            for off_out in (0, 1, 2, 5):
+                x = torch.randint(1, 200, (numel + 8,), device="cuda").to(dtype)[off_in:off_in + numel]
+                frame = torch.zeros(numel + 8, dtype=dtype, device="cuda")
+                ctx.all_reduce(x, frame[off_out:off_out + numel])
+                want = torch.zeros(numel + 8, dtype=dtype)
+                want[off_out:off_out + numel] = x.cpu()
+                assert torch.equal(frame.cpu(), want), (numel, off_in, off_out)

@@ -2,13 +2,10 @@
 #include "backends/cuda/cuda_backend.h"
 
 #include <cuda_runtime.h>
+#include <sys/prctl.h>
 #if __has_include(<nvtx3/nvToolsExt.h>)
 #include <nvtx3/nvToolsExt.h>
-#define SML_NVTX_PUSH(name) nvtxRangePushA(name)
-#define SML_NVTX_POP() nvtxRangePop()
-#else
-#define SML_NVTX_PUSH(name) ((void)0)
-#define SML_NVTX_POP() ((void)0)
+#define SML_NVTX 1
 #endif
 
 #include <atomic>
@@ -19,6 +16,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <deque>
+#include <functional>
 #include <mutex>
 #include <sstream>
 #include <thread>
@@ -70,14 +68,56 @@ struct EventPool {
   }
 };
 
+// Where threads that wait for jobs meet the backend that finishes them. Shared with the jobs: a
+// caller may hold one longer than the backend lives.
+struct Completions {
+  std::mutex mu;                     // held while finished jobs are taken off the queue
+  std::function<void()> reap;        // finish every job at the head of the queue whose event has fired; empty once the backend is gone
+};
+
+// Looking at events must not disturb a stream capture that goes on elsewhere in the process.
+struct RelaxedCapture {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
+// Two work items on the same stream are in order by themselves. The handle of the per-thread
+// default stream names another stream in every thread.
+inline bool SameStream(cudaStream_t a, cudaStream_t b) { return a == b && a != cudaStreamPerThread; }
+
 struct EventState : public DeviceJobState {
   cudaEvent_t done = nullptr;
+  cudaStream_t stream = nullptr;  // where the job runs
   std::shared_ptr<EventPool> pool;
+  std::shared_ptr<Completions> completions;
   ~EventState() override {
     if (pool) pool->Put(done);
   }
-  void StreamWait(void* stream) override {
-    cudaStreamWaitEvent(static_cast<cudaStream_t>(stream), done, 0);
+  void StreamWait(void* other) override {
+    if (!SameStream(stream, static_cast<cudaStream_t>(other))) cudaStreamWaitEvent(static_cast<cudaStream_t>(other), done, 0);
+  }
+  void HelpComplete(Job& job, double milliseconds) override {
+    const auto start = std::chrono::steady_clock::now();
+    RelaxedCapture relaxed;
+    for (;;) {
+      {
+        std::lock_guard<std::mutex> lk(completions->mu);
+        if (!completions->reap) return;
+        completions->reap();
+      }
+      const JobStatus s = job.GetJobStatus();
+      if (s == FINISHED || s == FAILED) return;
+      // Not fired yet. Without a limit the driver waits, which answers fastest.
+      if (milliseconds < 0) {
+        cudaEventSynchronize(done);
+      } else if (std::chrono::steady_clock::now() - start > std::chrono::duration<double, std::milli>(milliseconds)) {
+        return;
+      } else if (std::chrono::steady_clock::now() - start > std::chrono::microseconds(100)) {
+        std::this_thread::sleep_for(std::chrono::microseconds(10));
+      }
+      std::this_thread::yield();
+    }
   }
 };
 
@@ -87,12 +127,40 @@ struct InFlight {
   JobSlice slice;
   cudaEvent_t done = nullptr;
   cudaEvent_t ready = nullptr;
-  int status_slot = 0;
+  int status_slot = -1;  // -1: the job's kernel reports no status
   unsigned long long tiles = 0;
   std::string launch_error;
 };
 
 static const int kStatusSlots = 4096;
+// launch = worker: with this many jobs in flight the launcher thread takes over, which may wait for
+// room in the stream's queue (about a thousand launches) while the callers go on.
+static const size_t kDirectLaunches = 256;
+
+// One NVTX range per job for timeline tools; without one the name is not even put together.
+struct NvtxRange {
+#ifdef SML_NVTX
+  NvtxRange(const Job& job, const Tensor& t) {
+    static const bool listening = [] {
+      const bool on = nvtxRangePushA("switchml") != NVTX_NO_PUSH_POP_TRACKING;
+      if (on) nvtxRangePop();
+      return on;
+    }();
+    if (!listening) return;
+    char name[96];
+    snprintf(name, sizeof(name), "switchml job %llu: %llu x %s", static_cast<unsigned long long>(job.id_),
+             static_cast<unsigned long long>(t.numel), DataTypeName(t.data_type));
+    nvtxRangePushA(name);
+    open = true;
+  }
+  ~NvtxRange() {
+    if (open) nvtxRangePop();
+  }
+  bool open = false;
+#else
+  NvtxRange(const Job&, const Tensor&) {}
+#endif
+};
 
 class CudaBackend : public CudaBackendInterface {
  public:
@@ -123,11 +191,19 @@ class CudaBackend : public CudaBackendInterface {
  private:
   void LauncherLoop();
   void CompletionLoop();
+  void Reap();
+  void FinishInFlight(InFlight& f, cudaError_t e);
+  void PushInFlight(InFlight&& f);
+  size_t InFlightCount();
   void BindServiceThread(const char* what);
   // Enqueue the kernels of `job` on `stream`; fills `f`. Caller holds launch_mu_.
   // `capturing`: the stream is being captured into a CUDA graph; nothing that belongs to
   // this one submission (events, status slot, buffer parity) may end up in the launch.
   void LaunchJob(const std::shared_ptr<Job>& job, cudaStream_t stream, InFlight* f, bool capturing = false);
+  // The same for a single worker, whose job is one pass over the tensor (or none).
+  cudaError_t LaunchLocalJob(const Tensor& t, cudaStream_t stream, InFlight* f);
+  // What follows the kernels (`e`: how their launch went): the job's event and its ordering hooks.
+  void FinishLaunch(const std::shared_ptr<Job>& job, cudaStream_t stream, InFlight* f, cudaError_t e, bool capturing);
   cudaEvent_t GetEvent() { return events_->Get(); }
   void PutEvent(cudaEvent_t e) { events_->Put(e); }
 
@@ -154,10 +230,11 @@ class CudaBackend : public CudaBackendInterface {
   std::mutex launch_mu_;  // serialises launches: one job order on every rank
   // launch = inline: all jobs share the staging slots, the flag pad and the per-channel
   // epochs, so two jobs must never run on the GPU at the same time. A job submitted on a
-  // stream other than the previous job's is ordered after that job through this event.
-  cudaEvent_t order_event_ = nullptr;
-  cudaStream_t order_stream_ = nullptr;
-  bool order_valid_ = false;
+  // stream other than the previous job's is ordered after that job through its own event.
+  std::shared_ptr<EventState> last_job_;
+  // launch = worker: jobs handed to the scheduler that the launcher thread has not enqueued yet.
+  // While there are none a submitting thread enqueues its job itself.
+  int queued_jobs_ = 0;
   unsigned long long epoch_base_ = 0;
   int oneshot_parity_ = 0;
   unsigned long long launched_jobs_ = 0;
@@ -171,6 +248,8 @@ class CudaBackend : public CudaBackendInterface {
   std::condition_variable q_cv_;
   std::deque<InFlight> inflight_;
   bool stop_completer_ = false;
+  bool completer_asleep_ = false;
+  std::shared_ptr<Completions> completions_ = std::make_shared<Completions>();
   std::atomic<bool> failed_{false};
 };
 
@@ -268,8 +347,8 @@ void CudaBackend::SetupWorker() {
   int lo = 0, hi = 0;
   cudaDeviceGetStreamPriorityRange(&lo, &hi);
   SML_CUDA_CHECK(cudaStreamCreateWithPriority(&comm_stream_, cudaStreamNonBlocking, hi));
-  SML_CUDA_CHECK(cudaEventCreateWithFlags(&order_event_, cudaEventDisableTiming));
-  order_valid_ = false;
+  last_job_.reset();
+  queued_jobs_ = 0;
   SML_CUDA_CHECK(cudaMalloc(&dev_counters_, 16 * sizeof(unsigned long long)));
   SML_CUDA_CHECK(cudaMemset(dev_counters_, 0, 16 * sizeof(unsigned long long)));
   SML_CUDA_CHECK(cudaMalloc(&dev_epochs_, kernels::kMaxChannels * sizeof(unsigned long long)));
@@ -301,6 +380,8 @@ void CudaBackend::SetupWorker() {
               << ", staging " << (bytes >> 20) << " MiB, up to " << max_channels_ << " channels, launch "
               << c.launch;
   stop_completer_ = false;
+  completer_asleep_ = false;
+  completions_->reap = [this] { Reap(); };
   set_up_ = true;
   completer_ = std::thread(&CudaBackend::CompletionLoop, this);
   if (!inline_launch_) launcher_ = std::thread(&CudaBackend::LauncherLoop, this);
@@ -316,6 +397,10 @@ void CudaBackend::CleanupWorker() {
   }
   q_cv_.notify_all();
   if (completer_.joinable()) completer_.join();
+  {
+    std::lock_guard<std::mutex> lk(completions_->mu);
+    completions_->reap = nullptr;
+  }
   cudaSetDevice(device_);
   cudaDeviceSynchronize();
   bool peers_alive = !failed_.load();
@@ -325,9 +410,7 @@ void CudaBackend::CleanupWorker() {
   if (staging_.local) allocator_->Destroy(&staging_, peers_alive);
   if (comm_stream_) cudaStreamDestroy(comm_stream_);
   comm_stream_ = nullptr;
-  if (order_event_) cudaEventDestroy(order_event_);
-  order_event_ = nullptr;
-  order_valid_ = false;
+  last_job_.reset();
   if (dev_counters_) cudaFree(dev_counters_);
   if (dev_trace_) cudaFree(dev_trace_);
   if (dev_epochs_) cudaFree(dev_epochs_);
@@ -360,8 +443,9 @@ void CudaBackend::SymmetricReset() {
   heap_used_ = 0;
 }
 
-// nullptr if kernels may dereference `p`, else the reason why not.
-static const char* GpuCannotAccess(const void* p) {
+// nullptr if kernels may dereference `p`, else the reason why not. `device`: whether it is ordinary
+// device memory (what kernels::DeviceMemory asks).
+static const char* GpuCannotAccess(const void* p, bool* device) {
   if (p == nullptr) return "null pointer";
   cudaPointerAttributes at;
   if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
@@ -369,6 +453,7 @@ static const char* GpuCannotAccess(const void* p) {
     return "the address is unknown to CUDA";
   }
   if (at.type == cudaMemoryTypeUnregistered) return "the address is ordinary (pageable) host memory";
+  *device = at.type == cudaMemoryTypeDevice;
   return nullptr;
 }
 
@@ -379,18 +464,25 @@ void CudaBackend::LaunchJob(const std::shared_ptr<Job>& job, cudaStream_t stream
   // The kernels dereference both pointers on the GPU: refuse anything the GPU cannot be
   // trusted to reach (ordinary malloc'ed host memory) instead of launching into a fault.
   // Device, managed and pinned (cudaHostAlloc / cudaHostRegister) memory pass.
+  bool in_device = true, out_device = true;
   if (t.numel > 0) {
-    const char* why = GpuCannotAccess(t.in_ptr);
-    if (!why && t.out_ptr != t.in_ptr) why = GpuCannotAccess(t.out_ptr);
+    const char* why = GpuCannotAccess(t.in_ptr, &in_device);
+    out_device = in_device;
+    if (!why && t.out_ptr != t.in_ptr) why = GpuCannotAccess(t.out_ptr, &out_device);
     if (why) {
       f->launch_error = std::string("backend = cuda needs device, managed or pinned memory: ") + why;
       return;
     }
   }
+  NvtxRange range(*job, user);
+  if (n_ == 1) {
+    FinishLaunch(job, stream, f, LaunchLocalJob(t, stream, f), capturing);
+    return;
+  }
   // uint8: widen into int32 scratch of the stream's memory pool, reduce that in place,
   // narrow into the caller's output. With one worker the sum is the input itself.
   void* widened = nullptr;
-  if (t.data_type == UINT8 && n_ > 1 && t.numel > 0) {
+  if (t.data_type == UINT8 && t.numel > 0) {
     if (capturing) {
       f->launch_error = "uint8 jobs cannot be captured into a CUDA graph";
       return;
@@ -404,6 +496,7 @@ void CudaBackend::LaunchJob(const std::shared_ptr<Job>& job, cudaStream_t stream
       return;
     }
     t.in_ptr = t.out_ptr = widened;
+    in_device = out_device = true;
     t.data_type = INT32;
   }
   const bool integer = t.data_type == INT32 || t.data_type == UINT8;
@@ -429,7 +522,7 @@ void CudaBackend::LaunchJob(const std::shared_ptr<Job>& job, cudaStream_t stream
   a.post_scale = c.average && !integer && !broadcast ? 1.0f / static_cast<float>(n_) : 1.0f;
   size_t esz = DataTypeSize(t.data_type);
   size_t bytes = t.numel * esz;
-  a.bulk_copy = t.numel > 0 && kernels::DeviceMemory(t.in_ptr) && kernels::DeviceMemory(t.out_ptr);
+  a.bulk_copy = t.numel > 0 && in_device && out_device;
 
   // Pick the algorithm (identically on every rank: it depends on sizes and on whether the
   // pointers sit in the symmetric heap, which is allocated in lock step).
@@ -440,7 +533,7 @@ void CudaBackend::LaunchJob(const std::shared_ptr<Job>& job, cudaStream_t stream
   auto heap_usable = [&](const void* p) {
     return in_heap(p) && (reinterpret_cast<uintptr_t>(p) & 15) == 0 && (!ctx_.use_multimem || heap_.multicast);
   };
-  const bool out_in_heap = n_ > 1 && heap_usable(t.out_ptr);
+  const bool out_in_heap = heap_usable(t.out_ptr);
   const bool heap_ok = out_in_heap && heap_usable(t.in_ptr);
   auto describe_heap = [&] {
     for (int p = 0; p < n_; p++) a.user_peer[p] = static_cast<char*>(heap_.peers[p]);
@@ -450,7 +543,7 @@ void CudaBackend::LaunchJob(const std::shared_ptr<Job>& job, cudaStream_t stream
     a.out_offset = static_cast<const char*>(t.out_ptr) - static_cast<const char*>(heap_.local);
   };
   // Peer-memory transport moves large messages with posted stores only, unless told otherwise.
-  const bool push = n_ > 1 && !ctx_.use_multimem && c.p2p_algo == "push" &&
+  const bool push = !ctx_.use_multimem && c.p2p_algo == "push" &&
                     kernels::PushTileCapacity(ctx_, a.elem_type, a.mode) > 0;
   // (Tensors of the symmetric heap are reduced where they lie when the switch can do it;
   // over plain peer memory small ones are quicker through the one-barrier kernel.)
@@ -490,46 +583,59 @@ void CudaBackend::LaunchJob(const std::shared_ptr<Job>& job, cudaStream_t stream
   // Replays of a captured launch share one status word that nobody waits on; a timeout in
   // a replay still shows up in the device counters.
   f->status_slot = capturing ? kStatusSlots - 2 : static_cast<int>(launched_jobs_++ % (kStatusSlots - 2));
-  f->done = capturing ? nullptr : GetEvent();
 
   cudaError_t e = cudaSuccess;
   host_status_[f->status_slot] = kernels::STATUS_OK;  // the ring is far longer than the queue
   kernels::RankCtx job_ctx = ctx_;
   job_ctx.status = dev_status_ + f->status_slot;
-  // A single worker reducing in place has nothing to do (float_sum: the sum of one term;
-  // quantised mode still runs, because quantise/dequantise rounds the values).
-  bool nothing_to_do = n_ == 1 && t.in_ptr == t.out_ptr && a.mode == kernels::MODE_SUM && a.post_scale == 1.0f;
-  // One NVTX range per job: shows up in timeline tools, costs nothing without one.
-  char range[96];
-  snprintf(range, sizeof(range), "switchml job %llu: %llu x %s", static_cast<unsigned long long>(job->id_),
-           static_cast<unsigned long long>(t.numel), DataTypeName(user.data_type));
-  SML_NVTX_PUSH(range);
-  bool plain_copy = n_ == 1 && a.mode == kernels::MODE_SUM && a.post_scale == 1.0f && !nothing_to_do;
-  // One worker in the exact mode: one pass that rounds every value to its block's grid (a mean
-  // over one worker scales by one).
-  const bool local_quant = n_ == 1 && a.mode == kernels::MODE_QUANT && t.numel > 0;
-  if (local_quant)
-    e = kernels::LaunchLocalQuant(t.in_ptr, t.out_ptr, t.numel, a.elem_type, ctx_.block_numel, stream);
-  else if (t.numel > 0 && plain_copy) e = kernels::LaunchLocalCopy(t.in_ptr, t.out_ptr, bytes, stream);
-  else if (t.numel > 0 && !nothing_to_do) e = kernels::LaunchAllReduce(job_ctx, a, plan, stream);
-  if (t.numel > 0 && !nothing_to_do && e == cudaSuccess) kernel_launches_ += widened ? 3 : 1;
-  SML_NVTX_POP();
+  if (t.numel > 0) {
+    e = kernels::LaunchAllReduce(job_ctx, a, plan, stream);
+    if (e == cudaSuccess) kernel_launches_ += widened ? 3 : 1;
+  }
   if (widened) {
     if (e == cudaSuccess) e = kernels::LaunchNarrowI32(widened, user.out_ptr, user.numel, stream);
     cudaFreeAsync(widened, stream);
   }
+  SML_VLOG(2) << "job " << job->id_ << ": " << t.numel << " x " << DataTypeName(user.data_type)
+              << " algo " << a.algo << " mode " << a.mode << " channels " << plan.channels
+              << " epochs " << plan.epochs;
+  FinishLaunch(job, stream, f, e, capturing);
+}
+
+cudaError_t CudaBackend::LaunchLocalJob(const Tensor& t, cudaStream_t stream, InFlight* f) {
+  const size_t bytes = t.numel * DataTypeSize(t.data_type);
+  f->tiles = (bytes + ctx_.slot_bytes - 1) / ctx_.slot_bytes;
+  if (t.numel == 0) return cudaSuccess;
+  const bool integer = t.data_type == INT32 || t.data_type == UINT8;
+  cudaError_t e = cudaSuccess;
+  if (!integer && config_.backend_.cuda.mode == "int32_quant") {
+    // The exact mode rounds every value to its block's grid, also with nobody to add to. (A mean
+    // over one worker scales by one.)
+    e = kernels::LaunchLocalQuant(t.in_ptr, t.out_ptr, t.numel, t.data_type == BFLOAT16 ? kernels::ELEM_BF16 : kernels::ELEM_F32,
+                                  ctx_.block_numel, stream);
+  } else if (t.in_ptr != t.out_ptr) {
+    e = kernels::LaunchLocalCopy(t.in_ptr, t.out_ptr, bytes, stream);
+  } else {
+    return cudaSuccess;  // the sum of one term, in place: nothing to do
+  }
+  if (e == cudaSuccess) kernel_launches_++;
+  return e;
+}
+
+void CudaBackend::FinishLaunch(const std::shared_ptr<Job>& job, cudaStream_t stream, InFlight* f, cudaError_t e, bool capturing) {
+  f->done = capturing ? nullptr : GetEvent();
   if (e == cudaSuccess && f->done) e = cudaEventRecord(f->done, stream);
   if (e != cudaSuccess) {
     f->launch_error = std::string("kernel launch failed: ") + cudaGetErrorString(e);
     cudaGetLastError();
   }
-  SML_VLOG(2) << "job " << job->id_ << ": " << t.numel << " x " << DataTypeName(user.data_type)
-              << " algo " << a.algo << " mode " << a.mode << " channels " << plan.channels
-              << " epochs " << plan.epochs;
   if (f->done) {
     auto st = std::make_shared<EventState>();
     st->done = f->done;
+    st->stream = stream;
     st->pool = events_;
+    st->completions = completions_;
+    last_job_ = st;
     job->SetDeviceState(st);
   } else {
     job->SetDeviceState(nullptr);  // captured: the work is ordered by the graph itself
@@ -547,22 +653,38 @@ bool CudaBackend::OnSubmit(const std::shared_ptr<Job>& job) {
     return true;
   }
   cudaSetDevice(device_);
-  if (!inline_launch_) {
-    // Remember where the producer stream is now; the launcher orders the job after it.
-    cudaEvent_t ready = GetEvent();
-    cudaEventRecord(ready, static_cast<cudaStream_t>(job->producer_stream_));
-    job->ready_event_ = ready;
-    return false;  // goes through the scheduler
-  }
   InFlight f;
   f.job = job;
-  cudaStream_t user_stream = static_cast<cudaStream_t>(job->producer_stream_);
+  const cudaStream_t user_stream = static_cast<cudaStream_t>(job->producer_stream_);
   cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(user_stream, &capture) != cudaSuccess) {
     capture = cudaStreamCaptureStatusNone;
     cudaGetLastError();
   }
   const bool capturing = capture == cudaStreamCaptureStatusActive;
+  if (!inline_launch_) {
+    // Where the producer stream is now: the job comes after it.
+    f.ready = GetEvent();
+    cudaEventRecord(f.ready, user_stream);
+    std::lock_guard<std::mutex> lk(launch_mu_);
+    if (capturing || queued_jobs_ > 0 || InFlightCount() >= kDirectLaunches) {
+      queued_jobs_++;
+      job->ready_event_ = f.ready;
+      return false;  // goes through the scheduler, so that the caller does not wait for the stream's queue
+    }
+    // Nobody is ahead of this job: enqueueing it here costs less than waking the launcher thread
+    // (a blocking allreduce of 64 Ki elements took 38 us with the hand-over).
+    job->SetJobStatus(QUEUED);
+    job->SetJobStatus(RUNNING);
+    cudaStreamWaitEvent(comm_stream_, f.ready, 0);
+    LaunchJob(job, comm_stream_, &f);
+    PushInFlight(std::move(f));
+    return true;
+  }
+  if (InFlightCount() > kStatusSlots / 4) {  // a status word must have been read before its slot comes round again
+    std::lock_guard<std::mutex> lk(completions_->mu);
+    Reap();
+  }
   {
     std::lock_guard<std::mutex> lk(launch_mu_);
     job->SetJobStatus(QUEUED);
@@ -570,27 +692,15 @@ bool CudaBackend::OnSubmit(const std::shared_ptr<Job>& job) {
     // Not while capturing: an event recorded outside the capture cannot be waited on inside
     // it. A captured job is ordered by the graph it becomes part of; whoever replays that
     // graph next to other jobs of this context orders the two.
-    if (!capturing && order_valid_ && order_stream_ != user_stream)
-      cudaStreamWaitEvent(user_stream, order_event_, 0);
+    if (!capturing && last_job_) last_job_->StreamWait(user_stream);
     LaunchJob(job, user_stream, &f, capturing);
-    if (!capturing && cudaEventRecord(order_event_, user_stream) == cudaSuccess) {
-      order_stream_ = user_stream;
-      order_valid_ = true;
-    } else if (!capturing) {
-      cudaGetLastError();
-    }
+    if (!capturing) PushInFlight(std::move(f));
   }
   if (capturing) {
     // The kernels now live in the graph under capture and run whenever it is replayed;
     // as far as this submission goes the job is done.
     context_.NotifyJobCompletion(job, f.launch_error.empty(), f.launch_error);
-    return true;
   }
-  {
-    std::lock_guard<std::mutex> lk(q_mu_);
-    inflight_.push_back(std::move(f));
-  }
-  q_cv_.notify_all();
   return true;
 }
 
@@ -626,67 +736,120 @@ void CudaBackend::LauncherLoop() {
       std::lock_guard<std::mutex> lk(launch_mu_);
       if (f.ready) cudaStreamWaitEvent(comm_stream_, f.ready, 0);
       LaunchJob(js.job, comm_stream_, &f);
+      PushInFlight(std::move(f));
+      queued_jobs_--;
     }
-    {
-      std::lock_guard<std::mutex> lk(q_mu_);
-      inflight_.push_back(std::move(f));
-    }
-    q_cv_.notify_all();
     // The scheduler's barrier (one consumer) lets us take the next job at once: jobs are
     // queued back to back on the stream and complete in order.
   }
 }
 
+void CudaBackend::PushInFlight(InFlight&& f) {
+  bool wake;
+  {
+    std::lock_guard<std::mutex> lk(q_mu_);
+    inflight_.push_back(std::move(f));
+    wake = completer_asleep_;
+  }
+  if (wake) q_cv_.notify_all();
+}
+
+size_t CudaBackend::InFlightCount() {
+  std::lock_guard<std::mutex> lk(q_mu_);
+  return inflight_.size();
+}
+
+// Finishes jobs for those that nobody waits for (a thread that waits for a job does it itself,
+// EventState::HelpComplete). It looks at the head of the queue every few microseconds while there
+// are jobs, and for a while after the last one: a thread that sits in cudaEventSynchronize holds
+// up the launches of the others (9 us per launch instead of 3), and waking one that sleeps costs
+// every submission a system call.
 void CudaBackend::CompletionLoop() {
   cudaSetDevice(device_);
   BindServiceThread("completion");
-  Stats& stats = context_.GetStats();
+  prctl(PR_SET_TIMERSLACK, 1000ul, 0ul, 0ul, 0ul);  // of this thread: sleep 20 us, not 70
+  int quiet = 0;  // turns without a job
   for (;;) {
-    InFlight f;
     {
       std::unique_lock<std::mutex> lk(q_mu_);
-      q_cv_.wait(lk, [this] { return stop_completer_ || !inflight_.empty(); });
-      if (inflight_.empty()) return;  // stop requested and nothing left
-      f = std::move(inflight_.front());
-      inflight_.pop_front();
+      if (inflight_.empty() && !stop_completer_ && ++quiet > 100) {
+        completer_asleep_ = true;
+        q_cv_.wait(lk, [this] { return stop_completer_ || !inflight_.empty(); });
+        completer_asleep_ = false;
+      }
+      if (!inflight_.empty()) quiet = 0;
+      else if (stop_completer_) return;  // stop requested and nothing left
     }
-    bool ok = f.launch_error.empty();
-    std::string why = f.launch_error;
-    if (ok) {
-      cudaError_t e = cudaEventSynchronize(f.done);
-      if (e != cudaSuccess) {
-        ok = false;
-        why = std::string("device error: ") + cudaGetErrorString(e);
-        failed_ = true;
-      } else {
-        int st = *reinterpret_cast<volatile int*>(host_status_ + f.status_slot);
-        if (st != kernels::STATUS_OK) {
-          ok = false;
-          std::ostringstream o;
-          if ((st & 0xf) == kernels::STATUS_TIMEOUT) {
-            o << "a peer did not arrive within " << config_.backend_.cuda.wait_timeout_ms
-              << " ms (channel " << (st >> 8) << ", phase " << ((st >> 4) & 0xf) << ")";
-            stats.AddTimeouts(0, 1);
-          } else if ((st & 0xf) == kernels::STATUS_BOUNDS) {
-            o << "checked build: a tile of channel " << (st >> 8) << " would reach outside its region";
-          } else {
-            o << "kernel status " << st;
-          }
-          why = o.str();
-          failed_ = true;
-        }
+    {
+      std::unique_lock<std::mutex> lk(completions_->mu, std::try_to_lock);
+      if (lk) Reap();
+    }
+    std::this_thread::sleep_for(std::chrono::microseconds(20));
+  }
+}
+
+// Caller holds completions_->mu.
+void CudaBackend::Reap() {
+  RelaxedCapture relaxed;
+  for (;;) {
+    InFlight* head = nullptr;  // stays where it is: only this function takes jobs off the queue
+    {
+      std::lock_guard<std::mutex> lk(q_mu_);
+      if (inflight_.empty()) return;
+      head = &inflight_.front();
+    }
+    cudaError_t e = cudaSuccess;
+    if (head->launch_error.empty()) {
+      e = cudaEventQuery(head->done);
+      if (e == cudaErrorNotReady) {
+        cudaGetLastError();
+        return;
       }
     }
-    stats.AddTotalPktsSent(0, f.tiles);
-    if (ok) stats.AddCorrectPktsReceived(0, f.tiles);
-    PutEvent(f.ready);
-    // f.done belongs to the job's EventState and returns to the pool with the job.
-    if (f.via_scheduler) {
-      if (!ok) f.job->failure_reason_ = why;
-      context_.NotifyJobSliceCompletion(0, f.slice);
-    } else {
-      context_.NotifyJobCompletion(f.job, ok, why);
+    InFlight f = std::move(*head);
+    {
+      std::lock_guard<std::mutex> lk(q_mu_);
+      inflight_.pop_front();
     }
+    FinishInFlight(f, e);
+  }
+}
+
+void CudaBackend::FinishInFlight(InFlight& f, cudaError_t e) {
+  Stats& stats = context_.GetStats();
+  bool ok = f.launch_error.empty();
+  std::string why = f.launch_error;
+  if (ok && e != cudaSuccess) {
+    ok = false;
+    why = std::string("device error: ") + cudaGetErrorString(e);
+    failed_ = true;
+  } else if (ok && f.status_slot >= 0) {
+    int st = *reinterpret_cast<volatile int*>(host_status_ + f.status_slot);
+    if (st != kernels::STATUS_OK) {
+      ok = false;
+      std::ostringstream o;
+      if ((st & 0xf) == kernels::STATUS_TIMEOUT) {
+        o << "a peer did not arrive within " << config_.backend_.cuda.wait_timeout_ms
+          << " ms (channel " << (st >> 8) << ", phase " << ((st >> 4) & 0xf) << ")";
+        stats.AddTimeouts(0, 1);
+      } else if ((st & 0xf) == kernels::STATUS_BOUNDS) {
+        o << "checked build: a tile of channel " << (st >> 8) << " would reach outside its region";
+      } else {
+        o << "kernel status " << st;
+      }
+      why = o.str();
+      failed_ = true;
+    }
+  }
+  stats.AddTotalPktsSent(0, f.tiles);
+  if (ok) stats.AddCorrectPktsReceived(0, f.tiles);
+  PutEvent(f.ready);
+  // f.done belongs to the job's EventState and returns to the pool with the job.
+  if (f.via_scheduler) {
+    if (!ok) f.job->failure_reason_ = why;
+    context_.NotifyJobSliceCompletion(0, f.slice);
+  } else {
+    context_.NotifyJobCompletion(f.job, ok, why);
   }
 }
 

@@ -9,12 +9,14 @@
 //    the symmetric staging region (flags, exponent slots, one-shot buffers, data slots)
 //    and, if asked, a symmetric heap for zero-copy tensors; start the launcher and the
 //    completion threads.
-//  * launch = worker: a launcher thread pulls jobs from the FIFO scheduler and enqueues
-//    their kernels on an internal high-priority stream, ordered after the producer
-//    stream by an event. launch = inline: the submitting thread enqueues the kernels on
-//    the caller's own stream (stream-ordered like any other kernel).
-//  * A completion thread waits for each job's event, reads the kernel's status word and
-//    finishes or fails the job.
+//  * launch = worker: kernels run on an internal high-priority stream, ordered after the
+//    producer stream by an event. The submitting thread enqueues them; with many jobs in
+//    flight a launcher thread takes over, fed by the FIFO scheduler. launch = inline: the
+//    submitting thread enqueues the kernels on the caller's own stream (stream-ordered like
+//    any other kernel).
+//  * A thread that waits for a job waits for its event, reads the kernel's status word and
+//    finishes or fails the job itself; a completion thread does so for the jobs that
+//    nobody waits for.
 #ifndef SWITCHML_CUDA_BACKEND_H_
 #define SWITCHML_CUDA_BACKEND_H_
 

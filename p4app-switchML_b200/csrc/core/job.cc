@@ -27,15 +27,29 @@ Job::Job(Tensor tensor, JobType job_type, ExtraJobInfo extra_job_info)
       extra_job_info_(extra_job_info),
       job_status_(INIT) {}
 
-void Job::WaitToComplete() {
-  std::unique_lock<std::mutex> lk(access_mutex_);
-  job_event_.wait(lk, [this] { return job_status_ == FINISHED || job_status_ == FAILED; });
-}
+void Job::WaitToComplete() { WaitToCompleteFor(-1); }
 
 bool Job::WaitToCompleteFor(double milliseconds) {
+  const auto deadline = std::chrono::steady_clock::now() + std::chrono::duration<double, std::milli>(milliseconds < 0 ? 0 : milliseconds);
+  auto wait = [&](std::unique_lock<std::mutex>& lk, auto condition) {
+    if (milliseconds >= 0) return job_event_.wait_until(lk, deadline, condition);
+    job_event_.wait(lk, condition);
+    return true;
+  };
+  auto over = [this] { return job_status_ == FINISHED || job_status_ == FAILED; };
+  std::shared_ptr<DeviceJobState> st;
+  {
+    std::unique_lock<std::mutex> lk(access_mutex_);
+    if (!wait(lk, [&] { return launched_ || over(); })) return false;
+    if (over()) return true;
+    st = device_state_;
+  }
+  if (st) {
+    const std::chrono::duration<double, std::milli> left = deadline - std::chrono::steady_clock::now();
+    st->HelpComplete(*this, milliseconds < 0 ? -1 : (left.count() > 0 ? left.count() : 0));
+  }
   std::unique_lock<std::mutex> lk(access_mutex_);
-  return job_event_.wait_for(lk, std::chrono::duration<double, std::milli>(milliseconds),
-                             [this] { return job_status_ == FINISHED || job_status_ == FAILED; });
+  return wait(lk, over);
 }
 
 JobStatus Job::GetJobStatus() {

@@ -50,12 +50,18 @@ enum JobStatus {
 
 const char* JobStatusName(JobStatus s);
 
+class Job;
+
 // Device-side ordering hooks attached by the cuda backend (opaque here so that the
 // core stays free of CUDA headers).
 struct DeviceJobState {
   virtual ~DeviceJobState() {}
   // Make `stream` (a cudaStream_t) wait for the job's device work.
   virtual void StreamWait(void* stream) = 0;
+  // The calling thread waits for the device work itself and finishes `job` (and the jobs before
+  // it) without waiting for the completion thread to come by; gives up after `milliseconds`
+  // (< 0: never).
+  virtual void HelpComplete(Job& job, double milliseconds) = 0;
 };
 
 class Job {

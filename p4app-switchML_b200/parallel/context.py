@@ -23,6 +23,9 @@ class JobStatus(enum.IntEnum):
     FAILED = 4
 
 
+_STATUS = tuple(JobStatus)
+
+
 class ContextState(enum.IntEnum):
     CREATED = 0
     STARTING = 1
@@ -31,22 +34,32 @@ class ContextState(enum.IntEnum):
     STOPPED = 4
 
 
+try:
+    import torch as _torch
+    _TORCH_CODES = {_torch.float32: 0, _torch.int32: 1, _torch.bfloat16: 2, _torch.uint8: 3}
+    _raw_stream = getattr(_torch._C, "_cuda_getCurrentRawStream", None)
+except ImportError:  # numpy-only environments
+    _torch, _TORCH_CODES, _raw_stream = None, {}, None
+
+
+def _current_stream(device_index):
+    """Handle of torch's current stream. (A Stream object, as ``torch.cuda.current_stream`` makes
+    one, costs as much as the rest of a submission.)"""
+    if _raw_stream is not None:
+        return _raw_stream(device_index)
+    return _torch.cuda.current_stream(device_index).cuda_stream
+
+
 def _describe(t):
-    """(pointer, numel, dtype code, cuda stream or None) of a tensor-like object."""
-    try:
-        import torch
-    except ImportError:  # numpy-only environments
-        torch = None
-    if torch is not None and isinstance(t, torch.Tensor):
+    """(pointer, numel, dtype code, cuda stream or None, is it on a GPU) of a tensor-like object."""
+    if _torch is not None and isinstance(t, _torch.Tensor):
         if not t.is_contiguous():
             raise ValueError("tensor must be contiguous")
-        code = {torch.float32: 0, torch.int32: 1, torch.bfloat16: 2, torch.uint8: 3}.get(t.dtype)
+        code = _TORCH_CODES.get(t.dtype)
         if code is None:
             raise TypeError("unsupported dtype %s (float32, int32, bfloat16, uint8)" % t.dtype)
-        stream = None
-        if t.is_cuda:
-            stream = torch.cuda.current_stream(t.device).cuda_stream
-        return t.data_ptr(), t.numel(), code, stream, t.is_cuda
+        is_cuda = t.is_cuda
+        return t.data_ptr(), t.numel(), code, _current_stream(t.get_device()) if is_cuda else None, is_cuda
     import numpy as np
     if isinstance(t, np.ndarray):
         if not t.flags["C_CONTIGUOUS"]:
@@ -61,6 +74,8 @@ def _describe(t):
 class Job:
     """Handle of a submitted allreduce (``switchml::Job``)."""
 
+    __slots__ = ("_h", "_keep", "__weakref__")
+
     def __init__(self, handle, keepalive):
         self._h = handle
         self._keep = keepalive  # the tensors must outlive the job
@@ -68,18 +83,15 @@ class Job:
     def wait(self, timeout_ms=None):
         """Block until FINISHED or FAILED (``Job::WaitToComplete``); returns the status."""
         st = lib().sml_job_wait(self._h, -1.0 if timeout_ms is None else float(timeout_ms))
-        return JobStatus(st)
+        return _STATUS[st] if st >= 0 else JobStatus(st)
 
     def status(self):
         return JobStatus(lib().sml_job_status(self._h))
 
     def stream_wait(self, stream=None):
         """Order a CUDA stream after the job without waiting on the host (cuda backend)."""
-        if stream is None:
-            import torch
-            stream = torch.cuda.current_stream()
-        ptr = getattr(stream, "cuda_stream", stream)
-        if lib().sml_job_stream_wait(self._h, ctypes.c_void_p(ptr)) != 0:
+        ptr = _current_stream(_torch.cuda.current_device()) if stream is None else getattr(stream, "cuda_stream", stream)
+        if lib().sml_job_stream_wait(self._h, ptr) != 0:
             raise NativeError(last_error())
 
     def error(self):
@@ -98,7 +110,8 @@ class Job:
 
     def __del__(self):
         try:
-            self.release()
+            if self._h:
+                self.release()
         except Exception:
             pass
 
@@ -163,8 +176,7 @@ class Context:
                 raise ValueError("out must match the input's size and dtype")
         if stream is not None:
             cur_stream = getattr(stream, "cuda_stream", stream)
-        h = lib().sml_allreduce_async(ctypes.c_void_p(ptr), ctypes.c_void_p(optr), numel, code,
-                                      ctypes.c_void_p(cur_stream or 0))
+        h = lib().sml_allreduce_async(ptr, optr, numel, code, cur_stream)
         if h < 0:
             raise NativeError(last_error())
         return Job(h, (tensor, out))
@@ -182,7 +194,7 @@ class Context:
         ptr, numel, code, cur_stream, _ = _describe(tensor)
         if stream is not None:
             cur_stream = getattr(stream, "cuda_stream", stream)
-        h = lib().sml_broadcast_async(ctypes.c_void_p(ptr), numel, code, int(root), ctypes.c_void_p(cur_stream or 0))
+        h = lib().sml_broadcast_async(ptr, numel, code, int(root), cur_stream)
         if h < 0:
             raise NativeError(last_error())
         return Job(h, (tensor,))

@@ -87,3 +87,46 @@ def test_one_worker_sum_copies_every_alignment(ctx, dtype):
                 want = torch.zeros(numel + 8, dtype=dtype)
                 want[off_out:off_out + numel] = x.cpu()
                 assert torch.equal(frame.cpu(), want), (numel, off_in, off_out)
+
+
+@pytest.mark.parametrize("launch", ["worker", "inline"])
+def test_many_jobs_from_several_threads_and_streams(ctx, launch):
+    """More jobs in flight than are enqueued directly, waited for by several threads at once, some by
+    status alone; jobs on other streams than their predecessors."""
+    assert ctx.start(sml.make_config("cuda", packet_numel=64, mode="int32_quant", launch=launch))
+    numel, errors = 5000, []
+    want = {}
+    xs = [torch.randn(numel, device="cuda") * 2.0 ** i for i in range(4)]
+    for i, x in enumerate(xs):
+        want[i] = quant_allreduce_oracle([x.cpu().numpy()], 64)
+
+    def walk(which):
+        try:
+            stream = torch.cuda.Stream()
+            ys = [torch.zeros(numel, device="cuda") for _ in range(8)]
+            stream.wait_stream(torch.cuda.current_stream())
+            with torch.cuda.stream(stream):
+                jobs = [ctx.all_reduce_async(xs[which], ys[k % 8]) for k in range(400)]
+                jobs[-1].stream_wait()
+                total = ys[0] + ys[7]
+            stream.synchronize()
+            assert np.array_equal(total.cpu().numpy(), 2 * want[which])
+            for k, j in enumerate(jobs):
+                if k % 50 == 7:
+                    while j.status() not in (sml.JobStatus.FINISHED, sml.JobStatus.FAILED):
+                        pass
+                else:
+                    assert j.wait(20000 if k % 2 else None) == sml.JobStatus.FINISHED, j.error()
+                j.release()
+        except BaseException as e:  # noqa: B902 - handed to the main thread
+            errors.append(e)
+
+    threads = [threading.Thread(target=walk, args=(w,)) for w in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors[0]
+    ctx.wait_for_all_jobs()
+    st = ctx.get_stats()
+    assert st["jobs_finished"] == 1600 and st["jobs_failed"] == 0

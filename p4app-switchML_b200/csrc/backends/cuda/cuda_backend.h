@@ -61,6 +61,13 @@ int EmulatedAllReduce(int nranks, void* const* in_ptrs, void* const* out_ptrs,
 // Free the staging memory that EmulatedAllReduce keeps.
 void ReleaseEmulationWorkspaces();
 
+// Allreduce of `numel` elements of pinned host memory through the running context: chunks of
+// `chunk_numel` elements are copied to `device` (room for all of them), reduced in place and copied
+// back on three streams (cudaStream_t of the current device). Returns when `host_out` is
+// complete: 0, or -1 with the reason.
+int HostPipelinedAllReduce(const void* host_in, void* host_out, void* device, uint64_t numel, DataType type,
+                           uint64_t chunk_numel, void* stream_in, void* stream_comm, void* stream_out, std::string* error);
+
 // True if the kernels were compiled with -DSWITCHML_CHECKED (geometry checks before every
 // tile; a violation sets STATUS_BOUNDS instead of touching memory).
 bool KernelsCheckedBuild();

@@ -265,6 +265,20 @@ int sml_emu_allreduce(int nranks, void* const* in_ptrs, void* const* out_ptrs, u
   return r;
 }
 
+int sml_host_allreduce(const void* host_in, void* host_out, void* device, uint64_t numel, int dtype,
+                       uint64_t chunk_numel, void* stream_in, void* stream_comm, void* stream_out) {
+  try {
+    if (dtype < 0 || dtype > 3 || chunk_numel == 0) return Fail("bad argument");
+    std::string err;
+    if (HostPipelinedAllReduce(host_in, host_out, device, numel, static_cast<DataType>(dtype), chunk_numel, stream_in,
+                               stream_comm, stream_out, &err) != 0)
+      return Fail(err);
+    return 0;
+  } catch (const std::exception& e) {
+    return Fail(e.what());
+  }
+}
+
 void sml_emu_release(void) { ReleaseEmulationWorkspaces(); }
 
 int sml_convert_u8(int widen, const void* in, void* out, uint64_t numel, void* stream) {

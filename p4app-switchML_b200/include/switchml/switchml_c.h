@@ -84,6 +84,10 @@ int sml_emu_allreduce(int nranks, void* const* in_ptrs, void* const* out_ptrs, u
                       int elem_type, int mode, int algo, int block_numel, uint64_t slot_bytes,
                       int slots_per_channel, int channels, float post_scale, int repeats,
                       int exponent_lookahead);
+/* Allreduce of pinned host memory: chunks go to `device` (room for numel elements), are reduced there and
+ * come back, on three streams of the current device. Returns when host_out is complete. */
+int sml_host_allreduce(const void* host_in, void* host_out, void* device, uint64_t numel, int dtype,
+                       uint64_t chunk_numel, void* stream_in, void* stream_comm, void* stream_out);
 /* Free the staging memory that sml_emu_allreduce keeps for its next call (at most 512 MiB). */
 void sml_emu_release(void);
 

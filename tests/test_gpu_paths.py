@@ -130,3 +130,23 @@ def test_many_jobs_from_several_threads_and_streams(ctx, launch):
     ctx.wait_for_all_jobs()
     st = ctx.get_stats()
     assert st["jobs_finished"] == 1600 and st["jobs_failed"] == 0
+
+
+@pytest.mark.parametrize("mode", ["float_sum", "int32_quant"])
+@pytest.mark.parametrize("numel,chunk", [(1, 1 << 24), (3, 2), ((1 << 18) + 1, 1 << 24), ((1 << 20) + 77, 1 << 18),
+                                         (5_000_003, 1 << 24)])
+def test_host_pipeline_chunks(ctx, mode, numel, chunk):
+    """Chunks that divide the tensor and that do not; twice through the same buffers."""
+    from switchml_b200.parallel.host_pipeline import HostAllReduce
+    assert ctx.start(sml.make_config("cuda", packet_numel=64, mode=mode, launch="inline"))
+    hx, hy = torch.empty(numel, pin_memory=True), torch.zeros(numel, pin_memory=True)
+    pipe = HostAllReduce(ctx, numel, torch.float32, chunk_numel=chunk)
+    for scale in (1.0, 1e-3):
+        hx.copy_(torch.randn(numel) * scale)
+        assert pipe.run(hx, hy) is hy
+        if mode == "float_sum":
+            assert torch.equal(hx, hy)
+        else:
+            want = np.concatenate([quant_allreduce_oracle([hx[lo:hi].numpy()], 64) for lo, hi in pipe.bounds])
+            assert np.array_equal(hy.numpy(), want)
+    pipe.close()

@@ -8,7 +8,12 @@
 // brings [K_TILE x 64] boxes with the 128-byte swizzle into shared memory, which is
 // exactly the canonical MN-major operand layout of the instruction.
 //
-// One persistent CTA per SM, 128 x 256 output tiles, statically scheduled
+// Three kernels:
+//   wgrad_wide.cuh   plain GEMM, one CTA per 128 x 256 tile: short reductions
+//   wgrad_pair.cuh   plain GEMM, two CTAs per 256 x 256 or 256 x 128 tile (cta_group::2)
+//   here             the GEMM that is summed over GPUs in the same kernel
+//
+// The fused kernel: one persistent CTA per SM, 128 x 256 output tiles, statically scheduled
 // (tile = blockIdx.x, += gridDim.x). Warp roles:
 //   warp 0      TMA producer: fills a ring of kStages operand stages
 //   warp 1      MMA issuer: one elected thread issues tcgen05.mma (M128 N256 K16, fp32
@@ -17,10 +22,10 @@
 //               tile t overlaps the main loop of tile t+1)
 //   warps 4-7   epilogue: tcgen05.ld 32 columns at a time, stage through swizzled shared
 //               memory, TMA store to global
-// The fused variant additionally reduces every finished tile across GPUs (see
-// wgrad_gemm.h): warps 8-11 wait until all ranks have stored tile t, let the NVSwitch add
-// the ranks' copies (multimem.ld_reduce) and broadcast the sum (multimem.st), while the
-// tensor cores already work on later tiles; warps whose GEMM role is over join in.
+// Every finished tile is reduced across GPUs (see wgrad_gemm.h): warps 8-11 wait until all
+// ranks have stored tile t, let the NVSwitch add the ranks' copies (multimem.ld_reduce) and
+// broadcast the sum (multimem.st), while the tensor cores already work on later tiles; warps
+// whose GEMM role is over join in.
 //
 // Every wait is bounded: an mbarrier or flag wait that runs out of budget raises an abort
 // flag in shared memory, records an error code for the host, and all roles drain, free
@@ -30,6 +35,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
 #include <cstring>
 #include <mutex>
 
@@ -50,7 +56,7 @@ constexpr int kEpiCols = 32;  // fp32 columns per epilogue step = one 128-byte r
 constexpr int kEpiBytes = kTileM * kEpiCols * 4;  // 16 KiB
 constexpr int kEpiBufs = 2;
 constexpr int kTmemCols = 512;
-constexpr int kThreads = 384;  // 12 warps; warps 8-11 idle unless the reduce is fused
+constexpr int kThreads = 384;  // 12 warps
 constexpr unsigned long long kMbarBudgetNs = 2000000000ull;  // an mbarrier wait gives up after two seconds
 
 struct __align__(1024) SharedStorage {
@@ -136,12 +142,15 @@ constexpr uint32_t kInstrDesc = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) 
                                 (static_cast<uint32_t>(kTileN >> 3) << 17) |
                                 (static_cast<uint32_t>(kTileM >> 4) << 24);
 
-__device__ __forceinline__ void Mma(uint32_t tmem_d, uint64_t a_desc, uint64_t b_desc, uint32_t accumulate) {
+__device__ __forceinline__ void MmaWith(uint32_t tmem_d, uint64_t a_desc, uint64_t b_desc, uint32_t instr, uint32_t accumulate) {
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
       "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "l"(a_desc), "l"(b_desc), "r"(kInstrDesc), "r"(accumulate) : "memory");
+      ::"r"(tmem_d), "l"(a_desc), "l"(b_desc), "r"(instr), "r"(accumulate) : "memory");
+}
+__device__ __forceinline__ void Mma(uint32_t tmem_d, uint64_t a_desc, uint64_t b_desc, uint32_t accumulate) {
+  MmaWith(tmem_d, a_desc, b_desc, kInstrDesc, accumulate);
 }
 
 // Arrive on an mbarrier once every tcgen05 operation issued so far by this thread is done.
@@ -160,6 +169,32 @@ __device__ __forceinline__ void TmemLoad32(uint32_t taddr, uint32_t (&r)[32]) {
         "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
         "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
       : "r"(taddr) : "memory");
+}
+
+// One warp: 32 rows of 32 fp32 accumulator columns to global memory, through 4 KiB of shared
+// memory (1024-byte aligned, free) and a TMA store of one bulk group. Row `lane` of the box is 128
+// bytes = 8 chunks of 16 bytes, chunk index XOR-ed with (row mod 8) as the 128-byte swizzle of the
+// store's tensor map expects. Out-of-range parts are clipped.
+__device__ __forceinline__ void SwizzledRow(const uint32_t (&v)[32], uint8_t* buf, int lane) {
+  uint8_t* row = buf + lane * 128;
+#pragma unroll
+  for (int j = 0; j < 8; j++)
+    *reinterpret_cast<uint4*>(row + ((j ^ (lane & 7)) << 4)) = make_uint4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+}
+__device__ __forceinline__ void StoreBuffer(const uint8_t* buf, int lane, const CUtensorMap* map, int x, int y) {
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  __syncwarp();
+  if (lane == 0) {
+    TmaStore2D(map, buf, x, y);
+    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+  }
+}
+__device__ __forceinline__ void StoreBox32(uint32_t taddr, uint8_t* buf, int lane, const CUtensorMap* map, int x, int y) {
+  uint32_t v[32];
+  TmemLoad32(taddr, v);
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+  SwizzledRow(v, buf, lane);
+  StoreBuffer(buf, lane, map, x, y);
 }
 
 __device__ __forceinline__ void NamedBarrier(int id, int nthreads) {
@@ -343,14 +378,13 @@ __global__ void __launch_bounds__(512) WgradGatherKernel(const char* dy, const c
   }
 }
 
-// kMode 0: plain GEMM; 1: every finished tile is reduced across the ranks; 2: gather mode (owned tiles over the
+// kMode 1: every finished tile is reduced across the ranks; 2: gather mode (owned tiles over the
 // gathered operands, broadcast).
 template <int kMode>
 __global__ void __launch_bounds__(kThreads, 1)
 WgradGemmKernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                 const __grid_constant__ CUtensorMap map_d, const float* dw, int M, int N, int K, WgradFusedArgs fused,
                 int rows_per_item, int* error_flag) {
-  constexpr bool kFused = kMode != 0;
   extern __shared__ uint8_t smem_raw[];
   SharedStorage& sh = *reinterpret_cast<SharedStorage*>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -486,31 +520,27 @@ WgradGemmKernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
       // All TMEM reads of this accumulator are done: hand it back to the MMA warp.
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       MbarArrive(&sh.acc_empty[acc]);
-      if (kFused) {
-        // Publish the tile: its stores must have landed before the peers may reduce it.
-        if (epi_tid == 0) {
-          asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
-          asm volatile("fence.proxy.async.global;" ::: "memory");
-          __threadfence_system();
-          if (kMode == 2) {  // only this rank's broadcasting warps wait for it
-            StoreReleaseSys(fused.flags_peer[fused.rank] + static_cast<size_t>(tile) * 8 + fused.rank, fused.epoch);
-          } else {
-            for (int p = 0; p < fused.nranks; p++)
-              StoreReleaseSys(fused.flags_peer[p] + static_cast<size_t>(tile) * 8 + fused.rank, fused.epoch);
-          }
+      // Publish the tile: its stores must have landed before the peers may reduce it.
+      if (epi_tid == 0) {
+        asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+        asm volatile("fence.proxy.async.global;" ::: "memory");
+        __threadfence_system();
+        if (kMode == 2) {  // only this rank's broadcasting warps wait for it
+          StoreReleaseSys(fused.flags_peer[fused.rank] + static_cast<size_t>(tile) * 8 + fused.rank, fused.epoch);
+        } else {
+          for (int p = 0; p < fused.nranks; p++)
+            StoreReleaseSys(fused.flags_peer[p] + static_cast<size_t>(tile) * 8 + fused.rank, fused.epoch);
         }
       }
     }
     if (epi_tid == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
   }
 
-  if (kFused) {
-    // Every warp that has nothing (more) to do for the GEMM helps with the cross-GPU
-    // reduction: warps 8-11 and 3 from the start, the others when their role is finished.
-    __syncwarp();
-    if (kMode == 2) BroadcastWork(fused, dw, M, N, tiles_n, num_tiles, rows_per_item, &sh.abort);
-    else ReduceWork(fused, M, N, tiles_n, num_tiles, rows_per_item, &sh.abort);
-  }
+  // Every warp that has nothing (more) to do for the GEMM helps with the cross-GPU
+  // reduction: warps 8-11 and 3 from the start, the others when their role is finished.
+  __syncwarp();
+  if (kMode == 2) BroadcastWork(fused, dw, M, N, tiles_n, num_tiles, rows_per_item, &sh.abort);
+  else ReduceWork(fused, M, N, tiles_n, num_tiles, rows_per_item, &sh.abort);
 
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
@@ -518,7 +548,7 @@ WgradGemmKernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTmemCols) : "memory");
   }
-  if (kFused && warp == 0) {
+  if (warp == 0) {
     // No CTA leaves before the matching CTA of every rank has finished reducing, so when
     // the kernel has ended everywhere every tile holds the global sum on every rank.
     unsigned long long* done = fused.flags_peer[fused.rank] + static_cast<size_t>(num_tiles + blockIdx.x) * 8;
@@ -533,200 +563,10 @@ WgradGemmKernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
   if (threadIdx.x == 0 && sh.abort && error_flag) *reinterpret_cast<volatile int*>(error_flag) = 1;
 }
 
-// ---- 2-CTA variant ---------------------------------------------------------------------
-// Two CTAs of a cluster share one 256 x 256 tile: each loads its own 128 rows of A and its
-// own 128 columns of B, the leader issues tcgen05.mma.cta_group::2 (M256 N256 K16) which
-// reads B from both CTAs' shared memory, and each CTA ends up with its 128 x 256 half of
-// the accumulator in its own TMEM. Per SM this halves the shared-memory traffic for B, which
-// is what bounds the 1-CTA kernel on large shapes. Plain GEMM only (no fused reduce).
-constexpr int k2Stages = 6;
-constexpr int k2ABytes = kTileK * 128 * 2;  // 128 rows of A   : 16 KiB
-constexpr int k2BBytes = kTileK * 128 * 2;  // 128 columns of B: 16 KiB
-constexpr int k2StageBytes = k2ABytes + k2BBytes;
-constexpr int k2Threads = 256;
-constexpr uint32_t kPeerBitMask = 0xFEFFFFFFu;  // clears the CTA-rank bit of a shared::cluster address
+#include "kernels/tile_queue.cuh"
+#include "kernels/wgrad_wide.cuh"
 
-struct __align__(1024) SharedStorage2 {
-  uint8_t stage[k2Stages][k2StageBytes];
-  uint8_t epi[kEpiBufs][kEpiBytes];
-  uint64_t full[k2Stages];
-  uint64_t empty[k2Stages];
-  uint64_t acc_full[2];
-  uint64_t acc_empty[2];
-  uint32_t tmem_base;
-  volatile int abort;
-};
-
-constexpr uint32_t kInstrDesc2 = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u << 16) |
-                                 (static_cast<uint32_t>(256 >> 3) << 17) | (static_cast<uint32_t>(256 >> 4) << 24);
-
-__device__ __forceinline__ void ClusterSync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-
-// TMA load issued by either CTA of the pair; the bytes are counted on the leader's barrier.
-__device__ __forceinline__ void TmaLoad2D_2Cta(void* smem_dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-      ::"r"(SmemAddr(smem_dst)), "l"(map), "r"(x), "r"(y), "r"(SmemAddr(bar) & kPeerBitMask) : "memory");
-}
-
-__device__ __forceinline__ void Mma2(uint32_t tmem_d, uint64_t a_desc, uint64_t b_desc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "l"(a_desc), "l"(b_desc), "r"(kInstrDesc2), "r"(accumulate) : "memory");
-}
-
-// Arrive, in both CTAs of the pair, on the barrier at this shared-memory offset once all
-// MMAs issued so far are done.
-__device__ __forceinline__ void MmaCommit2(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
-               ::"r"(SmemAddr(bar)), "h"(static_cast<uint16_t>(3)) : "memory");
-}
-
-__device__ __forceinline__ void MbarArriveOnLeader(uint64_t* bar) {
-  uint32_t remote;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(remote) : "r"(SmemAddr(bar)));
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(remote) : "memory");
-}
-
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(k2Threads, 1)
-WgradGemm2CtaKernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                    const __grid_constant__ CUtensorMap map_d, int M, int N, int K, int* error_flag) {
-  extern __shared__ uint8_t smem_raw[];
-  SharedStorage2& sh = *reinterpret_cast<SharedStorage2*>(
-      (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  uint32_t cta_rank;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(cta_rank));
-  const bool leader = cta_rank == 0;
-  const int tiles_m = (M + 255) / 256, tiles_n = (N + 255) / 256;
-  const int num_tiles = tiles_m * tiles_n;
-  const int k_blocks = (K + kTileK - 1) / kTileK;
-  const int pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
-
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < k2Stages; s++) {
-      MbarInit(&sh.full[s], 1);
-      MbarInit(&sh.empty[s], 1);
-    }
-    for (int b = 0; b < 2; b++) {
-      MbarInit(&sh.acc_full[b], 1);
-      MbarInit(&sh.acc_empty[b], 256);  // the epilogue threads of both CTAs
-    }
-    sh.abort = 0;
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  if (warp == 2) {
-    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;"
-                 ::"r"(SmemAddr(&sh.tmem_base)), "r"(kTmemCols) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
-  }
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();
-  ClusterSync();  // both CTAs' barriers exist before anybody signals across the pair
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tmem_base = sh.tmem_base;
-
-  if (warp == 0) {
-    if (lane == 0) {
-      uint32_t it = 0;
-      for (int tile = pair; tile < num_tiles && !sh.abort; tile += num_pairs) {
-        const int m0 = (tile / tiles_n) * 256 + static_cast<int>(cta_rank) * 128;
-        const int n0 = (tile % tiles_n) * 256 + static_cast<int>(cta_rank) * 128;
-        for (int kb = 0; kb < k_blocks; kb++, it++) {
-          const int s = it % k2Stages;
-          const uint32_t phase = (it / k2Stages) & 1;
-          if (!MbarWait(&sh.empty[s], phase ^ 1, &sh.abort)) break;
-          if (leader) MbarExpectTx(&sh.full[s], 2 * k2StageBytes);  // both CTAs' loads
-          uint8_t* a = sh.stage[s];
-          uint8_t* b = sh.stage[s] + k2ABytes;
-          for (int j = 0; j < 2; j++) TmaLoad2D_2Cta(a + j * (kTileK * 128), &map_a, m0 + j * kAtomMN, kb * kTileK, &sh.full[s]);
-          for (int j = 0; j < 2; j++) TmaLoad2D_2Cta(b + j * (kTileK * 128), &map_b, n0 + j * kAtomMN, kb * kTileK, &sh.full[s]);
-        }
-      }
-    }
-  } else if (warp == 1) {
-    if (lane == 0 && leader) {
-      uint32_t it = 0, local_tile = 0;
-      for (int tile = pair; tile < num_tiles && !sh.abort; tile += num_pairs, local_tile++) {
-        const int acc = local_tile & 1;
-        const uint32_t acc_phase = (local_tile >> 1) & 1;
-        if (!MbarWait(&sh.acc_empty[acc], acc_phase ^ 1, &sh.abort)) break;
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t tmem_d = tmem_base + acc * kTileN;
-        bool ok = true;
-        for (int kb = 0; kb < k_blocks && ok; kb++, it++) {
-          const int s = it % k2Stages;
-          const uint32_t phase = (it / k2Stages) & 1;
-          ok = MbarWait(&sh.full[s], phase, &sh.abort);
-          if (!ok) break;
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          const uint32_t a_addr = SmemAddr(sh.stage[s]);
-          const uint32_t b_addr = a_addr + k2ABytes;
-#pragma unroll
-          for (int kk = 0; kk < kTileK / kMmaK; kk++) {
-            uint64_t da = OperandDesc(a_addr + kk * kMmaK * 128, kTileK * 128);
-            uint64_t db = OperandDesc(b_addr + kk * kMmaK * 128, kTileK * 128);
-            Mma2(tmem_d, da, db, (kb | kk) != 0);
-          }
-          MmaCommit2(&sh.empty[s]);
-        }
-        if (!ok) break;
-        MmaCommit2(&sh.acc_full[acc]);
-      }
-    }
-  } else if (warp >= 4) {
-    const int q = warp - 4;
-    const int row = q * 32 + lane;
-    const int epi_tid = threadIdx.x - 128;
-    uint32_t local_tile = 0, stores = 0;
-    for (int tile = pair; tile < num_tiles; tile += num_pairs, local_tile++) {
-      const int m0 = (tile / tiles_n) * 256 + static_cast<int>(cta_rank) * 128;
-      const int n0 = (tile % tiles_n) * 256;
-      const int acc = local_tile & 1;
-      const uint32_t acc_phase = (local_tile >> 1) & 1;
-      if (!MbarWait(&sh.acc_full[acc], acc_phase, &sh.abort)) break;
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      for (int c = 0; c < kTileN / kEpiCols; c++, stores++) {
-        const int buf = stores % kEpiBufs;
-        if (epi_tid == 0 && stores >= kEpiBufs) asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(kEpiBufs - 1) : "memory");
-        NamedBarrier(1, 128);
-        uint32_t v[32];
-        TmemLoad32(tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * kTileN + c * kEpiCols, v);
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        uint8_t* dst_row = sh.epi[buf] + row * 128;
-#pragma unroll
-        for (int j = 0; j < 8; j++) {
-          uint4 w = make_uint4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
-          *reinterpret_cast<uint4*>(dst_row + ((j ^ (row & 7)) << 4)) = w;
-        }
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        NamedBarrier(2, 128);
-        if (epi_tid == 0) {
-          TmaStore2D(&map_d, sh.epi[buf], n0 + c * kEpiCols, m0);
-          asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-        }
-      }
-      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-      if (leader) MbarArrive(&sh.acc_empty[acc]);
-      else MbarArriveOnLeader(&sh.acc_empty[acc]);
-    }
-    if (epi_tid == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
-  }
-
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();
-  ClusterSync();  // the peer may still be signalling into this CTA's shared memory
-  if (warp == 2) {
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTmemCols) : "memory");
-  }
-  if (threadIdx.x == 0 && sh.abort && error_flag) *reinterpret_cast<volatile int*>(error_flag) = 1;
-}
+#include "kernels/wgrad_pair.cuh"
 
 // ---- host side ------------------------------------------------------------------------
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -763,7 +603,43 @@ bool MakeMap(CUtensorMap* map, CUtensorMapDataType type, int esz, const void* ba
 
 int g_sm_count[64] = {0};
 
+// Lets `kernel` use `bytes` of dynamic shared memory on the current device; once per device (`done`: a
+// bit for each).
+void AllowSmem(const void* kernel, size_t bytes, std::atomic<unsigned long long>* done) {
+  int dev = 0;
+  cudaGetDevice(&dev);
+  const unsigned long long bit = 1ull << (dev & 63);
+  if (done->load(std::memory_order_acquire) & bit) return;
+  cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
+  done->fetch_or(bit, std::memory_order_release);
+}
+
 }  // namespace
+
+// The plain GEMM, one CTA per tile. fc6 (32 x 4096 x 25088): 76.1 us -> 67.2 us (6.1 TB/s of
+// output; the stores alone take 63.5), 100 x 8000 x 8000: 56 -> 47 us.
+static int LaunchWide(const void* dy, const void* x, float* dw, int M, int N, int K, int* error_flag, cudaStream_t stream) {
+  CUtensorMap map_a, map_b, map_d;
+  if (!MakeMap(&map_a, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, dy, K, M, kTileK, kAtomMN) ||
+      !MakeMap(&map_b, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, x, K, N, kTileK, kAtomMN) ||
+      !MakeMap(&map_d, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, dw, M, N, 32, kEpiCols))
+    return -3;
+  const int tiles_n = (N + kTileN - 1) / kTileN;
+  const long long tiles = static_cast<long long>((M + kTileM - 1) / kTileM) * tiles_n;
+  if (tiles > 0x7fffffffll) return -1;
+  // Short reductions want room to store, long ones to load.
+  static std::atomic<unsigned long long> allowed_store{0}, allowed_load{0};
+  if (K <= 4 * kTileK) {
+    AllowSmem(reinterpret_cast<const void*>(WgradWideKernel<3, 2>), sizeof(WideShared<3, 2>) + 1024, &allowed_store);
+    WgradWideKernel<3, 2><<<static_cast<unsigned>(tiles), kWideThreads, sizeof(WideShared<3, 2>) + 1024, stream>>>(
+        map_a, map_b, map_d, tiles_n, K, error_flag);
+  } else {
+    AllowSmem(reinterpret_cast<const void*>(WgradWideKernel<4, 1>), sizeof(WideShared<4, 1>) + 1024, &allowed_load);
+    WgradWideKernel<4, 1><<<static_cast<unsigned>(tiles), kWideThreads, sizeof(WideShared<4, 1>) + 1024, stream>>>(
+        map_a, map_b, map_d, tiles_n, K, error_flag);
+  }
+  return cudaGetLastError() == cudaSuccess ? 0 : -4;
+}
 
 extern "C" int switchml_wgrad_gemm(const void* dy, const void* x, float* dw, int M, int N, int K,
                                    const WgradFusedArgs* fused, int* error_flag, void* stream_ptr) {
@@ -772,7 +648,9 @@ extern "C" int switchml_wgrad_gemm(const void* dy, const void* x, float* dw, int
   if ((M % 8) || (N % 8)) return -2;
   if ((reinterpret_cast<uintptr_t>(dy) | reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(dw)) & 15)
     return -2;
-  const bool gather = fused && fused->nranks > 1 && fused->mode == 1;
+  if (!fused || fused->nranks <= 1)
+    return LaunchWide(dy, x, dw, M, N, K, error_flag, static_cast<cudaStream_t>(stream_ptr));
+  const bool gather = fused->mode == 1;
   if (gather && (!fused->gather_local || !fused->gather_mc || !fused->gather_counter || !fused->out_mc || !fused->work_counter ||
                  fused->nranks > 8))
     return -1;
@@ -792,54 +670,94 @@ extern "C" int switchml_wgrad_gemm(const void* dy, const void* x, float* dw, int
   int sms = (dev >= 0 && dev < 64 && g_sm_count[dev] > 0) ? g_sm_count[dev] : 148;
   if (sms > 148) sms = 148;  // the flag array has room for 148 closing flags
   int tiles = ((M + kTileM - 1) / kTileM) * ((N + kTileN - 1) / kTileN);
-  int grid = tiles < sms ? tiles : sms;
   size_t smem = sizeof(SharedStorage) + 1024;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
-  WgradFusedArgs none;
-  memset(&none, 0, sizeof(none));
-  cudaError_t e;
-  if (fused && fused->nranks > 1) {
-    if (fused->nranks > 8 || !fused->out_mc || !fused->work_counter) return -1;
-    // All CTAs take part in the closing cross-GPU barrier, so the grid must be the same on
-    // every rank and fully resident: one CTA per SM at most.
-    static bool attr_f = false;
-    if (!attr_f) {
-      cudaFuncSetAttribute(WgradGemmKernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-      cudaFuncSetAttribute(WgradGemmKernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-      attr_f = true;
-    }
-    // One CTA on every SM even when there are fewer tiles: the others only reduce (or broadcast).
-    // Work items of that: a few per warp of the grid, between 2 and 32 rows of a tile each.
-    grid = sms;
-    const long long owned_rows = static_cast<long long>((tiles + fused->nranks - 1) / fused->nranks) * kTileM;
-    const long long warps = static_cast<long long>(grid) * (kThreads / 32);
-    int rows_per_item = 32;
-    while (rows_per_item > 2 && owned_rows / rows_per_item < 2 * warps) rows_per_item >>= 1;
-    if (gather) {
-      const size_t bytes_a = static_cast<size_t>(K) * M * 2, bytes_b = static_cast<size_t>(K) * N * 2;
-      size_t vecs = (bytes_a + bytes_b) / 16;
-      int gblocks = static_cast<int>((vecs + 511) / 512);
-      if (gblocks > sms) gblocks = sms;
-      if (gblocks < 1) gblocks = 1;
-      WgradGatherKernel<<<gblocks, 512, 0, stream>>>(static_cast<const char*>(dy), static_cast<const char*>(x), *fused,
-                                                    bytes_a, bytes_b, static_cast<size_t>(tiles) + 148);
-      if (cudaGetLastError() != cudaSuccess) return -4;
-      WgradGemmKernel<2><<<grid, kThreads, smem, stream>>>(map_a, map_b, map_d, dw, M, N, k_rows, *fused, rows_per_item, error_flag);
-    } else {
-      WgradGemmKernel<1><<<grid, kThreads, smem, stream>>>(map_a, map_b, map_d, dw, M, N, K, *fused, rows_per_item, error_flag);
-    }
-    e = cudaGetLastError();
+  if (fused->nranks > 8 || !fused->out_mc || !fused->work_counter) return -1;
+  // All CTAs take part in the closing cross-GPU barrier, so the grid must be the same on
+  // every rank and fully resident: one CTA per SM at most.
+  static std::atomic<unsigned long long> allowed1{0}, allowed2{0};
+  AllowSmem(reinterpret_cast<const void*>(WgradGemmKernel<1>), smem, &allowed1);
+  AllowSmem(reinterpret_cast<const void*>(WgradGemmKernel<2>), smem, &allowed2);
+  // One CTA on every SM even when there are fewer tiles: the others only reduce (or broadcast).
+  // Work items of that: a few per warp of the grid, between 2 and 32 rows of a tile each.
+  const int grid = sms;
+  const long long owned_rows = static_cast<long long>((tiles + fused->nranks - 1) / fused->nranks) * kTileM;
+  const long long warps = static_cast<long long>(grid) * (kThreads / 32);
+  int rows_per_item = 32;
+  while (rows_per_item > 2 && owned_rows / rows_per_item < 2 * warps) rows_per_item >>= 1;
+  if (gather) {
+    const size_t bytes_a = static_cast<size_t>(K) * M * 2, bytes_b = static_cast<size_t>(K) * N * 2;
+    size_t vecs = (bytes_a + bytes_b) / 16;
+    int gblocks = static_cast<int>((vecs + 511) / 512);
+    if (gblocks > sms) gblocks = sms;
+    if (gblocks < 1) gblocks = 1;
+    WgradGatherKernel<<<gblocks, 512, 0, stream>>>(static_cast<const char*>(dy), static_cast<const char*>(x), *fused,
+                                                  bytes_a, bytes_b, static_cast<size_t>(tiles) + 148);
+    if (cudaGetLastError() != cudaSuccess) return -4;
+    WgradGemmKernel<2><<<grid, kThreads, smem, stream>>>(map_a, map_b, map_d, dw, M, N, k_rows, *fused, rows_per_item, error_flag);
   } else {
-    static bool attr_p = false;
-    if (!attr_p) {
-      cudaFuncSetAttribute(WgradGemmKernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-      attr_p = true;
-    }
-    WgradGemmKernel<0><<<grid, kThreads, smem, stream>>>(map_a, map_b, map_d, dw, M, N, K, none, 32, error_flag);
-    e = cudaGetLastError();
+    WgradGemmKernel<1><<<grid, kThreads, smem, stream>>>(map_a, map_b, map_d, dw, M, N, K, *fused, rows_per_item, error_flag);
   }
-  return e == cudaSuccess ? 0 : -4;
+  return cudaGetLastError() == cudaSuccess ? 0 : -4;
 }
+
+namespace {
+
+// How a product is spread over the GPU: tiles of 256 x TN, `splits` pairs of CTAs per tile.
+struct PairPlan {
+  int tn, splits, clusters;
+};
+
+template <int TN, int kSplits>
+cudaError_t LaunchPairs(const CUtensorMap& map_a, const CUtensorMap& map_b, const CUtensorMap& map_d, int M, int N, int K,
+                        const PairPlan& plan, int* error_flag, cudaStream_t stream) {
+  const size_t smem = sizeof(PairShared<TN>) + 1024;
+  static std::atomic<unsigned long long> allowed{0};
+  AllowSmem(reinterpret_cast<const void*>(WgradPairKernel<TN, kSplits>), smem, &allowed);
+  cudaLaunchConfig_t cfg;
+  memset(&cfg, 0, sizeof(cfg));
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = 2 * kSplits;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cfg.gridDim = dim3(static_cast<unsigned>(plan.clusters) * 2 * kSplits);
+  cfg.blockDim = dim3(kPairThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, WgradPairKernel<TN, kSplits>, map_a, map_b, map_d, M, N, K, error_flag);
+}
+
+// The plan with the least estimated time. A k-block costs about the same with either tile width (both
+// are bound by getting A into and out of shared memory), so narrow tiles pay only where they make
+// more of too few tiles; `fixed` is what a tile costs besides, in k-blocks, adding up partial sums included
+// (fitted to 18 shapes). 33 clusters of four CTAs and 15 of eight find room at the same time.
+PairPlan PlanPairs(int M, int N, int K, int sms) {
+  static const struct { int tn, splits; double fixed; } kinds[] = {{256, 1, 22}, {256, 2, 24}, {128, 2, 18}, {256, 4, 30}, {128, 4, 24}};
+  const int k_blocks = (K + kTileK - 1) / kTileK;
+  PairPlan best = {256, 1, 1};
+  double least = 1e30;
+  for (const auto& k : kinds) {
+    if (k.splits > k_blocks) continue;
+    const long long tiles = static_cast<long long>((M + 255) / 256) * ((N + k.tn - 1) / k.tn);
+    const int resident = k.splits == 1 ? sms / 2 : k.splits == 2 ? sms * 33 / 148 : sms * 15 / 148;
+    if (resident < 1) continue;
+    const double waves = static_cast<double>((tiles + resident - 1) / resident);
+    const double blocks = (k_blocks + k.splits - 1) / k.splits;
+    // Without a split the pairs are persistent: the fixed part comes once.
+    const double cost = k.splits == 1 ? waves * blocks + k.fixed : waves * (blocks + k.fixed);
+    if (cost < least) {
+      least = cost;
+      best.tn = k.tn;
+      best.splits = k.splits;
+      best.clusters = static_cast<int>(k.splits == 1 && tiles > resident ? resident : tiles);
+    }
+  }
+  return best;
+}
+
+}  // namespace
 
 extern "C" int switchml_wgrad_gemm_2cta(const void* dy, const void* x, float* dw, int M, int N, int K,
                                         int* error_flag, void* stream_ptr) {
@@ -850,24 +768,20 @@ extern "C" int switchml_wgrad_gemm_2cta(const void* dy, const void* x, float* dw
   CUtensorMap map_a, map_b, map_d;
   if (!MakeMap(&map_a, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, dy, K, M, kTileK, kAtomMN) ||
       !MakeMap(&map_b, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, x, K, N, kTileK, kAtomMN) ||
-      !MakeMap(&map_d, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, dw, M, N, kTileM, kEpiCols))
+      !MakeMap(&map_d, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, dw, M, N, 32, kEpiCols))
     return -3;
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 0 && dev < 64 && g_sm_count[dev] == 0)
     cudaDeviceGetAttribute(&g_sm_count[dev], cudaDevAttrMultiProcessorCount, dev);
   int sms = (dev >= 0 && dev < 64 && g_sm_count[dev] > 0) ? g_sm_count[dev] : 148;
-  int tiles = ((M + 255) / 256) * ((N + 255) / 256);
-  int pairs = tiles < sms / 2 ? tiles : sms / 2;
-  size_t smem = sizeof(SharedStorage2) + 1024;
-  static bool attr = false;
-  if (!attr) {
-    cudaFuncSetAttribute(WgradGemm2CtaKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-    attr = true;
-  }
-  WgradGemm2CtaKernel<<<pairs * 2, k2Threads, smem, static_cast<cudaStream_t>(stream_ptr)>>>(
-      map_a, map_b, map_d, M, N, K, error_flag);
-  return cudaGetLastError() == cudaSuccess ? 0 : -4;
+  PairPlan plan = PlanPairs(M, N, K, sms);
+  const cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
+  const auto launch = plan.splits == 1 ? LaunchPairs<256, 1>
+                    : plan.splits == 2 ? (plan.tn == 256 ? LaunchPairs<256, 2> : LaunchPairs<128, 2>)
+                                       : (plan.tn == 256 ? LaunchPairs<256, 4> : LaunchPairs<128, 4>);
+  const cudaError_t e = launch(map_a, map_b, map_d, M, N, K, plan, error_flag, stream);
+  return e == cudaSuccess ? 0 : -4;
 }
 
 extern "C" int switchml_wgrad_flag_words(int M, int N) {

@@ -12,9 +12,9 @@ import os
 import torch
 
 from .._native import library_path, NativeError
+from ..parallel.context import _current_stream
 
 _LIB = None
-_TWO_CTA_DEFAULT = True   # measured: 53 vs 58 us on 8192x4096x1024, 815 vs 923 us on 8192^3
 
 
 class _FusedArgs(ctypes.Structure):
@@ -53,31 +53,40 @@ _ERRORS = {-1: "bad argument", -2: "M and N must be multiples of 8 and all tenso
 def wgrad_gemm(dy, x, out=None, error_flag=None, two_cta=None):
     """dW[out_features, in_features] (fp32) = dY^T @ X for bf16 dY [K, M] and X [K, N].
 
-    `two_cta`: use the kernel in which two CTAs share a 256x256 tile (tcgen05 cta_group::2);
-    default: whenever the reduction dimension is at least 256, where shared-memory bandwidth
-    bounds the one-CTA kernel."""
+    `two_cta`: use the kernel in which two CTAs share a tile (tcgen05 cta_group::2); default: by
+    size, see _prefers_two_ctas."""
     assert dy.is_cuda and x.is_cuda and dy.dtype == torch.bfloat16 and x.dtype == torch.bfloat16
-    assert dy.dim() == 2 and x.dim() == 2 and dy.shape[0] == x.shape[0]
-    dy = dy.contiguous()
-    x = x.contiguous()
     K, M = dy.shape
-    N = x.shape[1]
+    rows, N = x.shape
+    assert rows == K
+    if not dy.is_contiguous():
+        dy = dy.contiguous()
+    if not x.is_contiguous():
+        x = x.contiguous()
     if out is None:
         out = torch.empty(M, N, dtype=torch.float32, device=dy.device)
     assert out.is_contiguous() and out.dtype == torch.float32 and out.numel() == M * N
-    stream = torch.cuda.current_stream(dy.device).cuda_stream
+    stream = _current_stream(dy.get_device())
     err_ptr = error_flag.data_ptr() if error_flag is not None else None
     if two_cta is None:
-        two_cta = _TWO_CTA_DEFAULT and K >= 256   # tiny K is output-bound: the one-CTA kernel wins there
+        two_cta = _prefers_two_ctas(K, M, N)
+    l = _LIB or _lib()
     if two_cta:
-        rc = _lib().switchml_wgrad_gemm_2cta(dy.data_ptr(), x.data_ptr(), out.data_ptr(), M, N, K, err_ptr,
-                                             ctypes.c_void_p(stream))
+        rc = l.switchml_wgrad_gemm_2cta(dy.data_ptr(), x.data_ptr(), out.data_ptr(), M, N, K, err_ptr, stream)
     else:
-        rc = _lib().switchml_wgrad_gemm(dy.data_ptr(), x.data_ptr(), out.data_ptr(), M, N, K, None, err_ptr,
-                                        ctypes.c_void_p(stream))
+        rc = l.switchml_wgrad_gemm(dy.data_ptr(), x.data_ptr(), out.data_ptr(), M, N, K, None, err_ptr, stream)
     if rc != 0:
         raise NativeError("wgrad_gemm: " + _ERRORS.get(rc, str(rc)))
-    return out.view(M, N)
+    return out if out.shape == (M, N) else out.view(M, N)
+
+
+def _prefers_two_ctas(K, M, N):
+    """Up to K = 256 writing the gradient takes longer than multiplying. Up to 512 the one-CTA kernel's
+    smaller tiles still win while there are at most two of them per SM (512 x 4096 x 1024: 10.4 against
+    12.4 us; with many tiles the pairs win, 300 x 8000 x 8000: 65 against 70 us)."""
+    if K > 512:
+        return True
+    return K > 256 and (M + 127) // 128 * ((N + 255) // 256) > 296
 
 
 def flag_words(M, N):

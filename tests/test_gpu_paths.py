@@ -150,3 +150,38 @@ def test_host_pipeline_chunks(ctx, mode, numel, chunk):
             want = np.concatenate([quant_allreduce_oracle([hx[lo:hi].numpy()], 64) for lo, hi in pipe.bounds])
             assert np.array_equal(hy.numpy(), want)
     pipe.close()
+
+
+@pytest.mark.parametrize("K", [1, 15, 16, 63, 64, 65, 100, 128, 129])
+@pytest.mark.parametrize("M,N", [(8, 8), (128, 128), (136, 264), (1000, 520)])
+def test_wgrad_short_reductions(K, M, N):
+    """The kernel for short reductions at the edges of its range: K around a step and a stage, tiles
+    that stick out of the matrix on either side. Neighbouring memory stays as it is."""
+    from switchml_b200.ops.wgrad import wgrad_gemm
+    gen = torch.Generator(device="cuda").manual_seed(K + M)
+    dy = torch.randn(K, M, device="cuda", generator=gen).bfloat16()
+    x = torch.randn(K, N, device="cuda", generator=gen).bfloat16()
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    frame = torch.full((M * N + 128,), 3.0, device="cuda")
+    out = frame[64:64 + M * N].view(M, N)
+    wgrad_gemm(dy, x, out=out, error_flag=err)
+    assert int(err) == 0
+    assert torch.allclose(out, dy.float().t() @ x.float(), rtol=1e-4, atol=1e-4 * K ** 0.5)
+    assert bool((frame[:64] == 3).all()) and bool((frame[64 + M * N:] == 3).all())
+
+
+@pytest.mark.parametrize("K,M,N", [(8192, 512, 512), (8192, 1024, 1024), (4160, 264, 520), (2048, 1000, 1032), (300, 256, 128),
+                                   (1000, 3000, 2000), (640, 2048, 4104), (65, 8, 8), (8192, 2304, 1024)])
+def test_wgrad_pairs_of_ctas_with_every_split(K, M, N):
+    """Two CTAs per tile, both tile widths, alone and two or four pairs to a tile; the same bits twice."""
+    from switchml_b200.ops.wgrad import wgrad_gemm
+    gen = torch.Generator(device="cuda").manual_seed(K + N)
+    dy = torch.randn(K, M, device="cuda", generator=gen).bfloat16()
+    x = torch.randn(K, N, device="cuda", generator=gen).bfloat16()
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    out = wgrad_gemm(dy, x, error_flag=err, two_cta=True)
+    assert int(err) == 0
+    ref = dy.double().t() @ x.double()
+    assert float((out - ref).norm() / ref.norm()) < 1e-5
+    assert torch.allclose(out.double(), ref, rtol=1e-4, atol=2e-4 * K ** 0.5)
+    assert torch.equal(wgrad_gemm(dy, x, two_cta=True), out)

@@ -152,6 +152,76 @@ __device__ __forceinline__ uint4 ReduceVec(const RankCtx& ctx, char* const* peer
   return r;
 }
 
+// 16-byte vector accumulators of the plain-sum mode.
+template <int ELEM> struct VecAcc;
+template <> struct VecAcc<ELEM_F32> {
+  float4 a;
+  __device__ __forceinline__ void Zero() { a = make_float4(0.f, 0.f, 0.f, 0.f); }
+  __device__ __forceinline__ void Init(uint4 v) { a = make_float4(__uint_as_float(v.x), __uint_as_float(v.y), __uint_as_float(v.z), __uint_as_float(v.w)); }
+  __device__ __forceinline__ void Add(uint4 v) { a.x += __uint_as_float(v.x); a.y += __uint_as_float(v.y); a.z += __uint_as_float(v.z); a.w += __uint_as_float(v.w); }
+  __device__ __forceinline__ uint4 Finish(float s) {
+    if (s != 1.0f) { a.x *= s; a.y *= s; a.z *= s; a.w *= s; }
+    return make_uint4(__float_as_uint(a.x), __float_as_uint(a.y), __float_as_uint(a.z), __float_as_uint(a.w));
+  }
+};
+template <> struct VecAcc<ELEM_I32> {
+  uint4 a;
+  __device__ __forceinline__ void Zero() { a = make_uint4(0, 0, 0, 0); }
+  __device__ __forceinline__ void Init(uint4 v) { a = v; }
+  __device__ __forceinline__ void Add(uint4 v) { a.x += v.x; a.y += v.y; a.z += v.z; a.w += v.w; }  // wrapping
+  __device__ __forceinline__ uint4 Finish(float) { return a; }
+};
+template <> struct VecAcc<ELEM_BF16> {
+  float a[8];
+  __device__ __forceinline__ void Zero() {
+#pragma unroll
+    for (int j = 0; j < 8; j++) a[j] = 0.f;
+  }
+  __device__ __forceinline__ void Init(uint4 v) {
+    float2 q;
+    q = Bf16x2ToFloat2(v.x); a[0] = q.x; a[1] = q.y;
+    q = Bf16x2ToFloat2(v.y); a[2] = q.x; a[3] = q.y;
+    q = Bf16x2ToFloat2(v.z); a[4] = q.x; a[5] = q.y;
+    q = Bf16x2ToFloat2(v.w); a[6] = q.x; a[7] = q.y;
+  }
+  __device__ __forceinline__ void Add(uint4 v) {
+    float2 q;
+    q = Bf16x2ToFloat2(v.x); a[0] += q.x; a[1] += q.y;
+    q = Bf16x2ToFloat2(v.y); a[2] += q.x; a[3] += q.y;
+    q = Bf16x2ToFloat2(v.z); a[4] += q.x; a[5] += q.y;
+    q = Bf16x2ToFloat2(v.w); a[6] += q.x; a[7] += q.y;
+  }
+  __device__ __forceinline__ uint4 Finish(float s) {
+    if (s != 1.0f) {
+#pragma unroll
+      for (int j = 0; j < 8; j++) a[j] *= s;
+    }
+    return make_uint4(Float2ToBf16x2(a[0], a[1]), Float2ToBf16x2(a[2], a[3]), Float2ToBf16x2(a[4], a[5]),
+                      Float2ToBf16x2(a[6], a[7]));
+  }
+};
+
+// Peer memory: U 16-byte vectors (at `off`, off + step, ...; those from `left` on are left alone) summed over
+// all ranks, post-scaled. Rank by rank with all U loads in flight; vector by vector, as ReduceVec
+// goes, a thread had one load in flight and four emulated ranks reduced at 0.7 TB/s.
+template <int ELEM, int U>
+__device__ __forceinline__ void ReducePeers(const RankCtx& ctx, char* const* peers, size_t off, size_t step, int left,
+                                            float post_scale, uint4 (&r)[U]) {
+  VecAcc<ELEM> acc[U];
+#pragma unroll
+  for (int u = 0; u < U; u++) acc[u].Zero();
+  for (int p = 0; p < ctx.nranks; p++) {
+    const char* src = peers[p] + off;
+    uint4 v[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) v[u] = u < left ? LoadCg16(src + u * step) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+    for (int u = 0; u < U; u++) acc[u].Add(v[u]);
+  }
+#pragma unroll
+  for (int u = 0; u < U; u++) r[u] = acc[u].Finish(post_scale);
+}
+
 // Write one 16-byte vector to every rank's copy.
 __device__ __forceinline__ void BroadcastVec(const RankCtx& ctx, char* const* peers, char* mc,
                                              size_t off, uint4 v) {
@@ -556,9 +626,37 @@ __device__ void RunStaged(const RankCtx& ctx, const JobArgs& job, int channel,
       // whole vectors would make it overlap the last vector of the previous rank's shard.
       if (sb >= se) {
       } else if (narrow) {
+        size_t from = sb;
+        if (!ctx.use_multimem) {
+          // Groups of four elements: 16 bytes of every rank's payload, 8 bytes of results.
+          constexpr int U = 8;
+          const size_t g0 = sb / 4, g1 = se / 4;  // sb is a multiple of the block
+          for (size_t g = g0 + t; g < g1; g += U * n) {
+            const int left = g1 - g > static_cast<size_t>(U - 1) * n ? U : static_cast<int>((g1 - g + n - 1) / n);
+            uint4 q[U];
+            ReducePeers<ELEM_I32, U>(ctx, ctx.stage_peer, slot_off + g * 16, static_cast<size_t>(n) * 16, left, 1.0f, q);
+            uint2 h[U];
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+              if (u >= left) continue;
+              const float f = sf[((g + static_cast<size_t>(u) * n) * 4) >> shift];
+              float y[4] = {quant::Dequantize(static_cast<int>(q[u].x), f), quant::Dequantize(static_cast<int>(q[u].y), f),
+                            quant::Dequantize(static_cast<int>(q[u].z), f), quant::Dequantize(static_cast<int>(q[u].w), f)};
+              if (job.post_scale != 1.0f) { y[0] *= job.post_scale; y[1] *= job.post_scale; y[2] *= job.post_scale; y[3] *= job.post_scale; }
+              h[u] = make_uint2(Float2ToBf16x2(y[0], y[1]), Float2ToBf16x2(y[2], y[3]));
+            }
+            for (int p = 0; p < ctx.nranks; p++) {
+              char* dst = dst_peer[p] + dst_off + g * 8;
+#pragma unroll
+              for (int u = 0; u < U; u++)
+                if (u < left) *reinterpret_cast<uint2*>(dst + static_cast<size_t>(u) * n * 8) = h[u];
+            }
+          }
+          from = g1 * 4;  // fewer than four elements, at the job's end
+        }
         // Two neighbouring lanes pair their results into one 32-bit store.
         char* mc = ctx.stage_mc + slot_off;
-        for (size_t i0 = sb + (t & ~31); i0 < se; i0 += n) {
+        for (size_t i0 = from + (t & ~31); i0 < se; i0 += n) {
           const size_t i = i0 + lane;
           int v = 0;
           if (i < se) {
@@ -646,28 +744,33 @@ __device__ void RunStaged(const RankCtx& ctx, const JobArgs& job, int channel,
               BroadcastVec(ctx, dst_peer, dst_mc, dst_off + v * 16, sum);
             }
           };
-          size_t v = v0 + t;
-          for (; v + (kUnrollLink - 1) * n < v1; v += kUnrollLink * n) {
-            uint4 r[kUnrollLink];
+          constexpr int U = 8;
+          for (size_t v = v0 + t; v < v1; v += U * n) {
+            const int left = v1 - v > static_cast<size_t>(U - 1) * n ? U : static_cast<int>((v1 - v + n - 1) / n);
+            uint4 r[U];
+            ReducePeers<ELEM_I32, U>(ctx, ctx.stage_peer, slot_off + v * 16, static_cast<size_t>(n) * 16, left, 1.0f, r);
 #pragma unroll
-            for (int u = 0; u < kUnrollLink; u++)
-              r[u] = ReduceVec<ELEM_I32>(ctx, ctx.stage_peer, ctx.stage_mc, slot_off + (v + u * n) * 16, 1.0f);
-#pragma unroll
-            for (int u = 0; u < kUnrollLink; u++) finish(v + u * n, r[u]);
-          }
-          if (v < v1) {  // the remainder in one go, see above
-            uint4 r[kUnrollLink];
-#pragma unroll
-            for (int u = 0; u < kUnrollLink; u++)
-              if (v + u * n < v1) r[u] = ReduceVec<ELEM_I32>(ctx, ctx.stage_peer, ctx.stage_mc, slot_off + (v + u * n) * 16, 1.0f);
-#pragma unroll
-            for (int u = 0; u < kUnrollLink; u++)
-              if (v + u * n < v1) finish(v + u * n, r[u]);
+            for (int u = 0; u < U; u++)
+              if (u < left) finish(v + static_cast<size_t>(u) * n, r[u]);
           }
         }
       } else {
         size_t v0 = sb / vec_elems, v1 = (se + vec_elems - 1) / vec_elems;
         size_t v = v0 + t;
+        if (!ctx.use_multimem) {
+          constexpr int U = ELEM == ELEM_BF16 ? 4 : 8;
+          for (; v < v1; v += U * n) {
+            const int left = v1 - v > static_cast<size_t>(U - 1) * n ? U : static_cast<int>((v1 - v + n - 1) / n);
+            uint4 r[U];
+            ReducePeers<ELEM, U>(ctx, ctx.stage_peer, slot_off + v * 16, static_cast<size_t>(n) * 16, left, job.post_scale, r);
+            for (int p = 0; p < ctx.nranks; p++) {
+              char* dst = ctx.stage_peer[p] + slot_off + v * 16;
+#pragma unroll
+              for (int u = 0; u < U; u++)
+                if (u < left) *reinterpret_cast<uint4*>(dst + static_cast<size_t>(u) * n * 16) = r[u];
+            }
+          }
+        }
         for (; v + (kUnrollLink - 1) * n < v1; v += kUnrollLink * n) {
           uint4 r[kUnrollLink];
 #pragma unroll
@@ -825,39 +928,70 @@ __device__ void RunOneShot(const RankCtx& ctx, const JobArgs& job, int channel,
   char* mine = ctx.stage_peer[ctx.rank];
   char* out = static_cast<char*>(job.out) + c0 * esz;
   if (MODE == MODE_QUANT) {
-    // One warp per block: exponent over all ranks' copies, then quantise, add, dequantise.
+    // One warp per block: the largest magnitude over all ranks' copies gives the exponent, then
+    // quantise, add, dequantise. Four elements per lane and load (the buffers and the blocks are
+    // vector aligned), the loads of all ranks in flight together: the buffers come out of L2, and a
+    // small message is nothing but these latencies.
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
     const size_t B = ctx.block_numel;
     const size_t nblocks = (len + B - 1) / B;
+    const size_t src_step = ctx.oneshot_bytes;
+    const char* src0 = mine + buf_off(0);
+    const bool wide_out = (reinterpret_cast<uintptr_t>(out) & (ELEM == ELEM_BF16 ? 7 : 15)) == 0;
     for (size_t b = warp; b < nblocks; b += nwarps) {
-      size_t base = b * B;
-      size_t n = len - base < B ? len - base : B;
+      const size_t base = b * B;
+      const size_t n = len - base < B ? len - base : B;
+      // Elements from `i` on, of rank `s`; zero beyond the message.
+      auto load4 = [&](int s, size_t i) {
+        const char* src = src0 + s * src_step;
+        if (i + 4 <= n) return LoadGroupAsFloat<ELEM>(src, (base + i) / 4);
+        float4 x;
+        x.x = i < n ? LoadAsFloat<ELEM>(src, base + i) : 0.f;
+        x.y = i + 1 < n ? LoadAsFloat<ELEM>(src, base + i + 1) : 0.f;
+        x.z = i + 2 < n ? LoadAsFloat<ELEM>(src, base + i + 2) : 0.f;
+        x.w = 0.f;
+        return x;
+      };
       float m = 0.f;
-      int e = quant::kZeroExponent;
-      for (int s = 0; s < ctx.nranks; s++) {
-        const char* src = mine + buf_off(s);
-        m = 0.f;
-        for (size_t i = lane; i < n; i += 32) {
-          float v = fabsf(LoadAsFloat<ELEM>(src, base + i));
-          if (v > m) m = v;
-        }
+      for (size_t i = lane * 4; i < n; i += 128) {
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-          float t = __shfl_xor_sync(0xffffffffu, m, o);
-          if (t > m) m = t;
+        for (int s = 0; s < kMaxRanks; s++) {
+          if (s >= ctx.nranks) continue;  // uniform
+          const float4 x = load4(s, i);
+          m = fmaxf(m, fmaxf(fmaxf(fabsf(x.x), fabsf(x.y)), fmaxf(fabsf(x.z), fabsf(x.w))));  // a NaN never wins
         }
-        int le = quant::LocalExponent(m);
-        if (le > e) e = le;
       }
-      float sf = quant::ScaleFactorFromBase(e, ctx.quant_base);
-      for (size_t i = lane; i < n; i += 32) {
-        unsigned acc = 0;
-        for (int s = 0; s < ctx.nranks; s++)
-          acc += static_cast<unsigned>(quant::Quantize(LoadAsFloat<ELEM>(mine + buf_off(s), base + i), sf));
-        float y = quant::Dequantize(static_cast<int>(acc), sf);
-        if (job.post_scale != 1.0f) y *= job.post_scale;
-        if (ELEM == ELEM_BF16) reinterpret_cast<unsigned short*>(out)[base + i] = FloatToBf16(y);
-        else reinterpret_cast<float*>(out)[base + i] = y;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+      const float sf = quant::ScaleFactorFromBase(quant::LocalExponent(m), ctx.quant_base);
+      for (size_t i = lane * 4; i < n; i += 128) {
+        unsigned acc[4] = {0, 0, 0, 0};
+#pragma unroll
+        for (int s = 0; s < kMaxRanks; s++) {
+          if (s >= ctx.nranks) continue;
+          const float4 x = load4(s, i);
+          acc[0] += static_cast<unsigned>(quant::Quantize(x.x, sf));
+          acc[1] += static_cast<unsigned>(quant::Quantize(x.y, sf));
+          acc[2] += static_cast<unsigned>(quant::Quantize(x.z, sf));
+          acc[3] += static_cast<unsigned>(quant::Quantize(x.w, sf));
+        }
+        float y[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+          y[j] = quant::Dequantize(static_cast<int>(acc[j]), sf);
+          if (job.post_scale != 1.0f) y[j] *= job.post_scale;
+        }
+        if (wide_out && i + 4 <= n) {
+          if (ELEM == ELEM_BF16) *reinterpret_cast<uint2*>(out + (base + i) * 2) = make_uint2(Float2ToBf16x2(y[0], y[1]), Float2ToBf16x2(y[2], y[3]));
+          else *reinterpret_cast<float4*>(out + (base + i) * 4) = make_float4(y[0], y[1], y[2], y[3]);
+        } else {
+#pragma unroll
+          for (int j = 0; j < 4; j++) {
+            if (i + j >= n) continue;
+            if (ELEM == ELEM_BF16) reinterpret_cast<unsigned short*>(out)[base + i + j] = FloatToBf16(y[j]);
+            else reinterpret_cast<float*>(out)[base + i + j] = y[j];
+          }
+        }
       }
     }
   } else {

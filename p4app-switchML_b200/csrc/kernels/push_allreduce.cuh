@@ -42,60 +42,6 @@ static const int kPushUnroll = 8;  // 16-byte vectors in flight per thread
 // Index of source rank `s` among the n-1 areas that destination `d` keeps (s != d).
 __device__ __forceinline__ int PushAreaIndex(int s, int d) { return s < d ? s : s - 1; }
 
-// Four consecutive elements of the input as floats (f32: one 16-byte load, bf16: 8 bytes).
-template <int ELEM>
-__device__ __forceinline__ float4 LoadGroupAsFloat(const char* in, size_t group) {
-  if (ELEM == ELEM_BF16) {
-    uint2 u = *reinterpret_cast<const uint2*>(in + group * 8);
-    float2 a = Bf16x2ToFloat2(u.x), b = Bf16x2ToFloat2(u.y);
-    return make_float4(a.x, a.y, b.x, b.y);
-  }
-  return *reinterpret_cast<const float4*>(in + group * 16);
-}
-
-// 16-byte vector accumulators of the plain-sum mode.
-template <int ELEM> struct VecAcc;
-template <> struct VecAcc<ELEM_F32> {
-  float4 a;
-  __device__ __forceinline__ void Init(uint4 v) { a = make_float4(__uint_as_float(v.x), __uint_as_float(v.y), __uint_as_float(v.z), __uint_as_float(v.w)); }
-  __device__ __forceinline__ void Add(uint4 v) { a.x += __uint_as_float(v.x); a.y += __uint_as_float(v.y); a.z += __uint_as_float(v.z); a.w += __uint_as_float(v.w); }
-  __device__ __forceinline__ uint4 Finish(float s) {
-    if (s != 1.0f) { a.x *= s; a.y *= s; a.z *= s; a.w *= s; }
-    return make_uint4(__float_as_uint(a.x), __float_as_uint(a.y), __float_as_uint(a.z), __float_as_uint(a.w));
-  }
-};
-template <> struct VecAcc<ELEM_I32> {
-  uint4 a;
-  __device__ __forceinline__ void Init(uint4 v) { a = v; }
-  __device__ __forceinline__ void Add(uint4 v) { a.x += v.x; a.y += v.y; a.z += v.z; a.w += v.w; }  // wrapping
-  __device__ __forceinline__ uint4 Finish(float) { return a; }
-};
-template <> struct VecAcc<ELEM_BF16> {
-  float a[8];
-  __device__ __forceinline__ void Init(uint4 v) {
-    float2 q;
-    q = Bf16x2ToFloat2(v.x); a[0] = q.x; a[1] = q.y;
-    q = Bf16x2ToFloat2(v.y); a[2] = q.x; a[3] = q.y;
-    q = Bf16x2ToFloat2(v.z); a[4] = q.x; a[5] = q.y;
-    q = Bf16x2ToFloat2(v.w); a[6] = q.x; a[7] = q.y;
-  }
-  __device__ __forceinline__ void Add(uint4 v) {
-    float2 q;
-    q = Bf16x2ToFloat2(v.x); a[0] += q.x; a[1] += q.y;
-    q = Bf16x2ToFloat2(v.y); a[2] += q.x; a[3] += q.y;
-    q = Bf16x2ToFloat2(v.z); a[4] += q.x; a[5] += q.y;
-    q = Bf16x2ToFloat2(v.w); a[6] += q.x; a[7] += q.y;
-  }
-  __device__ __forceinline__ uint4 Finish(float s) {
-    if (s != 1.0f) {
-#pragma unroll
-      for (int j = 0; j < 8; j++) a[j] *= s;
-    }
-    return make_uint4(Float2ToBf16x2(a[0], a[1]), Float2ToBf16x2(a[2], a[3]), Float2ToBf16x2(a[4], a[5]),
-                      Float2ToBf16x2(a[6], a[7]));
-  }
-};
-
 // Where the owner `me` writes its results on the n ranks: the output itself when it lies in
 // symmetric memory, else the result area that each peer's slot keeps for `me`.
 struct PushTargets {

@@ -49,6 +49,17 @@ __device__ __forceinline__ float TileLoadAsFloat(const void* in, size_t i, int e
   return reinterpret_cast<const float*>(in)[i];
 }
 
+// Four consecutive elements of the input as floats (f32: one 16-byte load, bf16: 8 bytes).
+template <int ELEM>
+__device__ __forceinline__ float4 LoadGroupAsFloat(const char* in, size_t group) {
+  if (ELEM == ELEM_BF16) {
+    const uint2 u = *reinterpret_cast<const uint2*>(in + group * 8);
+    return make_float4(__uint_as_float(u.x << 16), __uint_as_float(u.x & 0xffff0000u), __uint_as_float(u.y << 16),
+                       __uint_as_float(u.y & 0xffff0000u));
+  }
+  return *reinterpret_cast<const float4*>(in + group * 16);
+}
+
 // Local exponents of the `len` elements at `in` (one tile), published under `tag` into the
 // exponent words starting at byte offset `exp_off`. Called by all threads of a role of
 // `nwarps` warps; `warp` is the caller's warp index inside the role.
@@ -128,17 +139,16 @@ __device__ __forceinline__ void PublishTileExponents(const RankCtx& ctx, int war
                                                      const char* in, size_t len, size_t exp_off, Epoch tag) {
   const size_t B = ctx.block_numel;
   size_t first_block = 0;
-  if (ELEM == ELEM_F32 && (reinterpret_cast<uintptr_t>(in) & 15) == 0) {
-    // The tile as rows of 128 elements, one float4 per lane. A warp takes 8 consecutive rows
+  if (ELEM != ELEM_I32 && (reinterpret_cast<uintptr_t>(in) & (ELEM == ELEM_BF16 ? 7 : 15)) == 0) {
+    // The tile as rows of 128 elements, four per lane. A warp takes 8 consecutive rows
     // per step and issues all their loads before it looks at any value.
     constexpr int kRows = 8;
     const size_t whole_blocks = len / B;                          // blocks without a ragged end
     const size_t nrows = whole_blocks * B / 128 / kRows * kRows;  // rows handled here, in whole steps
-    const float4* p4 = reinterpret_cast<const float4*>(in);
     for (size_t r0 = static_cast<size_t>(warp) * kRows; r0 < nrows; r0 += static_cast<size_t>(nwarps) * kRows) {
       float4 x[kRows];
 #pragma unroll
-      for (int u = 0; u < kRows; u++) x[u] = p4[(r0 + u) * 32 + lane];
+      for (int u = 0; u < kRows; u++) x[u] = LoadGroupAsFloat<ELEM>(in, (r0 + u) * 32 + lane);
       PublishRows8(ctx, lane, x, r0, exp_off, tag);
     }
     first_block = nrows * 128 / B;
@@ -171,18 +181,19 @@ __device__ __forceinline__ void QuantizeRange(int tid, int nthreads, const char*
                                               size_t end, const float* sf, int shift) {
   if (begin >= end) return;
   const size_t n = end - begin;
-  if (ELEM == ELEM_F32 && ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(q)) & 15) == 0) {
-    const float4* in4 = reinterpret_cast<const float4*>(in) + begin / 4;
+  if (ELEM != ELEM_I32 && (reinterpret_cast<uintptr_t>(in) & (ELEM == ELEM_BF16 ? 7 : 15)) == 0 &&
+      (reinterpret_cast<uintptr_t>(q) & 15) == 0) {
     int4* q4 = reinterpret_cast<int4*>(q);
-    const size_t nvec = n / 4;
+    const size_t nvec = n / 4, first = begin / 4;
     const size_t nt = nthreads;
-    size_t i = tid;
-    for (; i + (UNROLL - 1) * nt < nvec; i += UNROLL * nt) {
+    for (size_t i = tid; i < nvec; i += UNROLL * nt) {
       float4 x[UNROLL];
 #pragma unroll
-      for (int u = 0; u < UNROLL; u++) x[u] = in4[i + u * nt];
+      for (int u = 0; u < UNROLL; u++)
+        if (i + u * nt < nvec) x[u] = LoadGroupAsFloat<ELEM>(in, first + i + u * nt);
 #pragma unroll
       for (int u = 0; u < UNROLL; u++) {
+        if (i + u * nt >= nvec) continue;
         const float f = sf[(begin + (i + u * nt) * 4) >> shift];
         int4 r;
         r.x = quant::Quantize(x[u].x, f);
@@ -192,18 +203,8 @@ __device__ __forceinline__ void QuantizeRange(int tid, int nthreads, const char*
         q4[i + u * nt] = r;
       }
     }
-    for (; i < nvec; i += nt) {
-      float4 x = in4[i];
-      const float f = sf[(begin + i * 4) >> shift];
-      int4 r;
-      r.x = quant::Quantize(x.x, f);
-      r.y = quant::Quantize(x.y, f);
-      r.z = quant::Quantize(x.z, f);
-      r.w = quant::Quantize(x.w, f);
-      q4[i] = r;
-    }
     for (size_t j = nvec * 4 + tid; j < n; j += nthreads)
-      q[j] = quant::Quantize(reinterpret_cast<const float*>(in)[begin + j], sf[(begin + j) >> shift]);
+      q[j] = quant::Quantize(TileLoadAsFloat(in, begin + j, ELEM), sf[(begin + j) >> shift]);
   } else {
     for (size_t j = tid; j < n; j += nthreads)
       q[j] = quant::Quantize(TileLoadAsFloat(in, begin + j, ELEM), sf[(begin + j) >> shift]);

@@ -106,6 +106,10 @@ SML_HD int32_t Quantize(float x, float sf) {
 
 SML_HD float Dequantize(int32_t q, float sf) {
 #if defined(__CUDA_ARCH__)
+  // With 1, 2, 4 or 8 workers sf is a power of two, and multiplying by its exact reciprocal (the
+  // exponent field mirrored at 127) gives the bits of the division, which costs ten times as much.
+  const uint32_t bits = __float_as_uint(sf);
+  if ((bits & 0x007fffffu) == 0) return __int2float_rn(q) * __uint_as_float(0x7f000000u - bits);
   return __fdiv_rn(__int2float_rn(q), sf);
 #else
   return static_cast<float>(q) / sf;

@@ -12,6 +12,7 @@ from .._native import lib, last_error, NativeError
 
 ELEM = {"float32": 0, "int32": 1, "bfloat16": 2}
 MODE = {"sum": 0, "quant": 1}
+_ARRAYS = {}  # pointer array types by length
 ALGO = {"staged": 0, "oneshot": 1, "push": 3}
 
 
@@ -24,19 +25,21 @@ def emulated_allreduce(inputs, mode="quant", algo="staged", block_numel=256, slo
     import torch
     n = len(inputs)
     x0 = inputs[0]
-    elem = {torch.float32: 0, torch.int32: 1, torch.bfloat16: 2}[x0.dtype]
+    dtype, numel = x0.dtype, x0.numel()
+    elem = {torch.float32: 0, torch.int32: 1, torch.bfloat16: 2}[dtype]
     for x in inputs:
-        assert x.is_cuda and x.is_contiguous() and x.dtype == x0.dtype and x.numel() == x0.numel()
+        assert x.is_cuda and x.is_contiguous() and x.dtype == dtype and x.numel() == numel
     if outputs is None:
         outputs = [torch.empty_like(x) for x in inputs]
     esz_unit = n * max(block_numel, 128) * 4
     slot_bytes = max(esz_unit, slot_bytes // esz_unit * esz_unit)
     if algo == "push":  # a slot holds n-1 receive areas and n-1 result areas of one shard each
         slot_bytes = max(slot_bytes, 2 * esz_unit)
-    ins = (ctypes.c_void_p * n)(*[x.data_ptr() for x in inputs])
-    outs = (ctypes.c_void_p * n)(*[o.data_ptr() for o in outputs])
+    array = _ARRAYS.get(n) or _ARRAYS.setdefault(n, ctypes.c_void_p * n)
+    ins = array(*[x.data_ptr() for x in inputs])
+    outs = array(*[o.data_ptr() for o in outputs])
     torch.cuda.synchronize()
-    rc = lib().sml_emu_allreduce(n, ins, outs, x0.numel(), elem, MODE[mode], ALGO[algo], block_numel,
+    rc = lib().sml_emu_allreduce(n, ins, outs, numel, elem, MODE[mode], ALGO[algo], block_numel,
                                  slot_bytes, slots_per_channel, channels, float(post_scale), repeats,
                                  int(exponent_lookahead))
     if rc != 0:

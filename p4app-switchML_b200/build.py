@@ -9,6 +9,7 @@ Products (all inside this directory, never installed elsewhere):
     lib/libswitchml_b200.a         the same as a static archive
     lib/libswitchml_gemm.so        tcgen05 weight-gradient GEMM (loaded on demand)
     lib/torch_switchml.so          native c10d backend for PyTorch (python build.py --torch)
+    lib/torch_switchml_linear.so   autograd node of FusedWgradLinear (python build.py --torch)
     build-checked/libswitchml_b200.so   the library with the kernels' bounds checks (--checked)
     lib/libnccl-net-switchml.so    NCCL collective-network plugin (bin/collnet_harness drives it)
     bin/switchml_switchd           stand-alone controller / software switch
@@ -56,7 +57,7 @@ LIB_SOURCES = [
     "csrc/kernels/allreduce_kernels.cu",
     "csrc/capi/switchml_c.cc",
 ]
-GEMM_SOURCES = ["csrc/kernels/wgrad_gemm.cu"]
+GEMM_SOURCES = ["csrc/kernels/wgrad_gemm.cu", "csrc/kernels/linear_ops.cu"]
 NCCL_PLUGIN_SOURCES = ["csrc/nccl/collnet_plugin.cc"]
 PROGRAMS = {
     "switchml_switchd": ["controller/switchd.cc"],
@@ -237,35 +238,49 @@ def build_checked(verbose=False, jobs=None):
     return target
 
 
+# Extensions of PyTorch: product, source, libraries of this package that it links.
+TORCH_EXTENSIONS = [("torch_switchml", "csrc/torch/process_group_sml.cc", ["switchml_b200"]),
+                    ("torch_switchml_linear", "csrc/torch/fused_linear.cc", ["switchml_gemm"])]
+
+
 def build_torch_extension(verbose=False):
-    """lib/torch_switchml.so: the native c10d backend. Needs the headers and libraries of the
-    installed PyTorch; returns None (with a note) when they are not usable."""
+    """lib/torch_switchml.so, the native c10d backend, and lib/torch_switchml_linear.so, the autograd node of
+    FusedWgradLinear. Needs the headers and libraries of the installed PyTorch; returns None (with a note) when
+    they are not usable, else the path of the former."""
     try:
         import torch
         from torch.utils import cpp_extension as ce
     except Exception as e:  # pragma: no cover
         print("torch extension skipped: %s" % e)
         return None
-    src = os.path.join(ROOT, "csrc", "torch", "process_group_sml.cc")
-    out = os.path.join(LIB, "torch_switchml.so")
-    if os.path.exists(out) and os.path.getmtime(out) > max(os.path.getmtime(src), _headers_mtime()):
-        return out
     import sysconfig
     tlib = ce.library_paths()[0]
     have_cuda = os.path.exists(os.path.join(tlib, "libc10_cuda.so"))
-    cmd = ["g++", "-std=c++17", "-O2", "-fPIC", "-shared", "-pthread", "-Wno-deprecated-declarations",
-           "-D_GLIBCXX_USE_CXX11_ABI=%d" % int(torch._C._GLIBCXX_USE_CXX11_ABI),
-           "-DTORCH_EXTENSION_NAME=torch_switchml", "-DTORCH_API_INCLUDE_EXTENSION_H"] + \
-          (["-DSWITCHML_TORCH_CUDA"] if have_cuda else []) + \
-          ["-I" + p for p in ce.include_paths()] + ["-I" + sysconfig.get_paths()["include"]] + INCLUDES + \
-          [src, "-o", out, "-L" + LIB, "-lswitchml_b200", "-Wl,-rpath,$ORIGIN", "-L" + tlib, "-Wl,-rpath," + tlib,
-           "-ltorch", "-ltorch_cpu", "-lc10", "-ltorch_python"] + (["-lc10_cuda"] if have_cuda else [])
-    if verbose:
-        print(" ".join(cmd), flush=True)
-    r = subprocess.run(cmd, capture_output=True, text=True)
-    if r.returncode != 0:
-        raise RuntimeError("torch extension failed to build:\n" + r.stdout + r.stderr[-4000:])
-    return out
+    hdr = _headers_mtime()
+
+    def one(name, source, libraries):
+        src, out = os.path.join(ROOT, source), os.path.join(LIB, name + ".so")
+        if os.path.exists(out) and os.path.getmtime(out) > max(os.path.getmtime(src), hdr):
+            return out
+        part = "%s.%d" % (out, os.getpid())  # several processes may build at once
+        cmd = ["g++", "-std=c++17", "-O2", "-fPIC", "-shared", "-pthread", "-Wno-deprecated-declarations",
+               "-D_GLIBCXX_USE_CXX11_ABI=%d" % int(torch._C._GLIBCXX_USE_CXX11_ABI),
+               "-DTORCH_EXTENSION_NAME=" + name, "-DTORCH_API_INCLUDE_EXTENSION_H"] + \
+              (["-DSWITCHML_TORCH_CUDA"] if have_cuda else []) + \
+              ["-I" + p for p in ce.include_paths()] + ["-I" + sysconfig.get_paths()["include"]] + INCLUDES + \
+              [src, "-o", part, "-L" + LIB] + ["-l" + l for l in libraries] + \
+              ["-Wl,-rpath,$ORIGIN", "-L" + tlib, "-Wl,-rpath," + tlib, "-ltorch", "-ltorch_cpu", "-lc10", "-ltorch_python"] + \
+              (["-lc10_cuda", "-ltorch_cuda"] if have_cuda else [])
+        if verbose:
+            print(" ".join(cmd), flush=True)
+        r = subprocess.run(cmd, capture_output=True, text=True)
+        if r.returncode != 0:
+            raise RuntimeError("torch extension failed to build:\n" + r.stdout + r.stderr[-4000:])
+        os.replace(part, out)
+        return out
+
+    with cf.ThreadPoolExecutor(max_workers=2) as ex:
+        return list(ex.map(lambda e: one(*e), TORCH_EXTENSIONS))[0]
 
 
 def clean():

@@ -784,6 +784,16 @@ extern "C" int switchml_wgrad_gemm_2cta(const void* dy, const void* x, float* dw
   return e == cudaSuccess ? 0 : -4;
 }
 
+// Up to K = 256 writing the gradient takes longer than multiplying. Up to 512 the one-CTA kernel's
+// smaller tiles still win while there are at most two of them per SM (512 x 4096 x 1024: 10.4 against
+// 12.4 us; with many tiles the pairs win, 300 x 8000 x 8000: 65 against 70 us).
+extern "C" int switchml_wgrad_gemm_auto(const void* dy, const void* x, float* dw, int M, int N, int K, int* error_flag,
+                                        void* stream) {
+  const long long tiles = static_cast<long long>((M + kTileM - 1) / kTileM) * ((N + kTileN - 1) / kTileN);
+  if (K > 512 || (K > 256 && tiles > 296)) return switchml_wgrad_gemm_2cta(dy, x, dw, M, N, K, error_flag, stream);
+  return switchml_wgrad_gemm(dy, x, dw, M, N, K, nullptr, error_flag, stream);
+}
+
 extern "C" int switchml_wgrad_flag_words(int M, int N) {
   int tiles = ((M + kTileM - 1) / kTileM) * ((N + kTileN - 1) / kTileN);
   return (tiles + 148 + 8) * 8;

@@ -64,7 +64,15 @@ int switchml_wgrad_gemm(const void* dy, const void* x, float* dw, int M, int N, 
 /* Same GEMM (no fused reduce) with pairs of CTAs sharing 256x256 tiles (tcgen05 cta_group::2). */
 int switchml_wgrad_gemm_2cta(const void* dy, const void* x, float* dw, int M, int N, int K,
                              int* error_flag, void* stream);
+/* The plain GEMM by whichever of the two suits the size. */
+int switchml_wgrad_gemm_auto(const void* dy, const void* x, float* dw, int M, int N, int K, int* error_flag, void* stream);
 int switchml_wgrad_flag_words(int M, int N);
+
+/* n fp32 values of a weight and nb of a bias (nb may be 0) to bf16, in one launch (linear_ops.cu). */
+int switchml_cast_weights(const float* w, void* w_low, unsigned long long n, const float* b, void* b_low,
+                          unsigned long long nb, void* stream);
+/* out[m] = sum over k of dy[k, m], bf16 [K, M] row-major, summed in fp32. M a multiple of 8, dy 16-byte aligned. */
+int switchml_column_sums(const void* dy, float* out, int K, int M, void* stream);
 
 #ifdef __cplusplus
 }

@@ -8,6 +8,7 @@ later tiles are still being computed.
 """
 import ctypes
 import os
+import weakref
 
 import torch
 
@@ -40,6 +41,10 @@ def _lib():
         l.switchml_wgrad_gemm_2cta.restype = ctypes.c_int
         l.switchml_wgrad_gemm_2cta.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int,
                                                ctypes.c_int, ctypes.c_int, ctypes.c_void_p, ctypes.c_void_p]
+        l.switchml_wgrad_gemm_auto.restype = ctypes.c_int
+        l.switchml_wgrad_gemm_auto.argtypes = l.switchml_wgrad_gemm_2cta.argtypes
+        l.switchml_column_sums.restype = ctypes.c_int
+        l.switchml_column_sums.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int, ctypes.c_int, ctypes.c_void_p]
         l.switchml_wgrad_flag_words.restype = ctypes.c_int
         l.switchml_wgrad_flag_words.argtypes = [ctypes.c_int, ctypes.c_int]
         _LIB = l
@@ -54,7 +59,7 @@ def wgrad_gemm(dy, x, out=None, error_flag=None, two_cta=None):
     """dW[out_features, in_features] (fp32) = dY^T @ X for bf16 dY [K, M] and X [K, N].
 
     `two_cta`: use the kernel in which two CTAs share a tile (tcgen05 cta_group::2); default: by
-    size, see _prefers_two_ctas."""
+    size (switchml_wgrad_gemm_auto)."""
     assert dy.is_cuda and x.is_cuda and dy.dtype == torch.bfloat16 and x.dtype == torch.bfloat16
     K, M = dy.shape
     rows, N = x.shape
@@ -68,25 +73,16 @@ def wgrad_gemm(dy, x, out=None, error_flag=None, two_cta=None):
     assert out.is_contiguous() and out.dtype == torch.float32 and out.numel() == M * N
     stream = _current_stream(dy.get_device())
     err_ptr = error_flag.data_ptr() if error_flag is not None else None
-    if two_cta is None:
-        two_cta = _prefers_two_ctas(K, M, N)
     l = _LIB or _lib()
-    if two_cta:
+    if two_cta is None:
+        rc = l.switchml_wgrad_gemm_auto(dy.data_ptr(), x.data_ptr(), out.data_ptr(), M, N, K, err_ptr, stream)
+    elif two_cta:
         rc = l.switchml_wgrad_gemm_2cta(dy.data_ptr(), x.data_ptr(), out.data_ptr(), M, N, K, err_ptr, stream)
     else:
         rc = l.switchml_wgrad_gemm(dy.data_ptr(), x.data_ptr(), out.data_ptr(), M, N, K, None, err_ptr, stream)
     if rc != 0:
         raise NativeError("wgrad_gemm: " + _ERRORS.get(rc, str(rc)))
     return out if out.shape == (M, N) else out.view(M, N)
-
-
-def _prefers_two_ctas(K, M, N):
-    """Up to K = 256 writing the gradient takes longer than multiplying. Up to 512 the one-CTA kernel's
-    smaller tiles still win while there are at most two of them per SM (512 x 4096 x 1024: 10.4 against
-    12.4 us; with many tiles the pairs win, 300 x 8000 x 8000: 65 against 70 us)."""
-    if K > 512:
-        return True
-    return K > 256 and (M + 127) // 128 * ((N + 255) // 256) > 296
 
 
 def flag_words(M, N):
@@ -155,6 +151,8 @@ class FusedWgrad:
                 ev.record(side_stream)
             _PENDING.append(ev)
             return out
+        if self.nranks == 1:
+            return wgrad_gemm(dy, x, out=self.grad, error_flag=self.error)
         K = dy.shape[0]
         operand_bytes = self.nranks * K * (self.M + self.N) * 2
         gather = self.fused and (self.policy == "gather" or
@@ -215,26 +213,38 @@ def _side_stream(device):
     return _SIDE_STREAMS[device]
 
 
-class _FusedLinearFn(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, x, weight, bias, layer):
-        ctx.layer = layer
-        ctx.save_for_backward(x, weight)
-        return torch.nn.functional.linear(x, weight, bias)
+def column_sums(dy):
+    """Sum over the rows of a bf16 matrix [K, M], in fp32 (M a multiple of 8, contiguous)."""
+    K, M = dy.shape
+    out = torch.empty(M, dtype=torch.float32, device=dy.device)
+    rc = (_LIB or _lib()).switchml_column_sums(dy.data_ptr(), out.data_ptr(), K, M, _current_stream(dy.get_device()))
+    if rc != 0:
+        raise NativeError("column_sums: " + _ERRORS.get(rc, str(rc)))
+    return out
 
-    @staticmethod
-    def backward(ctx, dy):
-        x, weight = ctx.saved_tensors
-        layer = ctx.layer
-        x2 = x.reshape(-1, x.shape[-1])
-        dy2 = dy.reshape(-1, dy.shape[-1])
-        dx = (dy2 @ weight.to(dy2.dtype)).reshape(x.shape) if ctx.needs_input_grad[0] else None
-        # dW on the tcgen05 tensor cores, summed over the workers in the same kernel,
-        # written straight into the parameter's gradient.
-        layer.wgrad.run(dy2.to(torch.bfloat16), x2.to(torch.bfloat16),
-                        side_stream=_side_stream(dy2.device) if layer.overlap else None)
-        dbias = dy2.sum(0).to(layer.bias.dtype) if layer.bias is not None else None
-        return dx, None, dbias, None
+
+_NODE = None
+
+
+def _node():
+    """lib/torch_switchml_linear.so, the layer's autograd node (csrc/torch/fused_linear.cc); built when it is
+    missing, like the main library."""
+    global _NODE
+    if _NODE is None:
+        import importlib.util
+        _lib()
+        path = library_path("torch_switchml_linear.so")
+        if not os.path.exists(path):
+            here = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+            spec = importlib.util.spec_from_file_location("_switchml_build", os.path.join(here, "build.py"))
+            build = importlib.util.module_from_spec(spec)
+            spec.loader.exec_module(build)
+            build.build_torch_extension()
+        spec = importlib.util.spec_from_file_location("torch_switchml_linear", path)
+        module = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(module)
+        _NODE = module
+    return _NODE
 
 
 class FusedWgradLinear(torch.nn.Linear):
@@ -243,19 +253,25 @@ class FusedWgradLinear(torch.nn.Linear):
     ``.grad`` then aliases the symmetric gradient buffer and arrives already reduced."""
 
     wgrad = None
-    overlap = True  # run the weight-gradient kernel on a side stream
+    overlap = True  # with several workers: run the weight-gradient kernel on a side stream
+    _plan = None
 
     def attach(self, ctx, scale=1.0):
         self.wgrad = FusedWgrad(ctx, self.out_features, self.in_features, scale)
         self.weight.grad = self.wgrad.grad
         self.weight._sml_reduced_in_backward = True
+        # The node keeps no reference to the layer: it would be one in a circle.
+        wgrad, layer = self.wgrad, weakref.ref(self)
+
+        def reduce_over_workers(dy, x):
+            alive = layer()
+            wgrad.run(dy, x, side_stream=_side_stream(dy.device) if alive is None or alive.overlap else None)
+
+        # The side stream hides the sum over the workers; one worker has none, and nothing to do in Python.
+        self._plan = _node().Plan(wgrad.grad, wgrad.error, reduce_over_workers if wgrad.nranks > 1 else None)
         return self
 
     def forward(self, x):
-        if self.wgrad is None or not torch.is_grad_enabled():
+        if self._plan is None or not torch.is_grad_enabled():
             return super().forward(x)
-        w = self.weight
-        if torch.is_autocast_enabled():
-            dt = torch.get_autocast_dtype("cuda")
-            return _FusedLinearFn.apply(x.to(dt), w.to(dt), self.bias.to(dt) if self.bias is not None else None, self)
-        return _FusedLinearFn.apply(x, w, self.bias, self)
+        return _node().fused_linear(x, self.weight, self.bias, self._plan)

@@ -185,3 +185,40 @@ def test_wgrad_pairs_of_ctas_with_every_split(K, M, N):
     assert float((out - ref).norm() / ref.norm()) < 1e-5
     assert torch.allclose(out.double(), ref, rtol=1e-4, atol=2e-4 * K ** 0.5)
     assert torch.equal(wgrad_gemm(dy, x, two_cta=True), out)
+
+
+@pytest.mark.parametrize("K,M", [(1, 8), (3, 72), (255, 64), (256, 128), (257, 520), (4097, 1000), (8192, 4096)])
+def test_column_sums(K, M):
+    """Clusters of one to eight CTAs, ragged rows and columns; the same bits twice."""
+    from switchml_b200.ops.wgrad import column_sums
+    dy = torch.randn(K, M, device="cuda", generator=torch.Generator(device="cuda").manual_seed(K + M)).bfloat16()
+    out = column_sums(dy)
+    assert torch.allclose(out.double(), dy.double().sum(0), rtol=1e-5, atol=1e-5 * K ** 0.5)
+    assert torch.equal(column_sums(dy), out)
+
+
+@pytest.mark.parametrize("shape,features", [((256, 64), 128), ((3, 17, 72), 40), ((1, 8), 8)])
+@pytest.mark.parametrize("bias", [True, False])
+@pytest.mark.parametrize("x_dtype", [torch.float32, torch.bfloat16])
+def test_fused_wgrad_linear_against_plain_linear(ctx, shape, features, bias, x_dtype):
+    """Forward and all gradients of the layer under autocast, against nn.Linear."""
+    from switchml_b200.ops.wgrad import FusedWgradLinear, wait_pending
+    assert ctx.start(sml.make_config("cuda", mode="float_sum", launch="inline", symm_heap_mb=16))
+    torch.manual_seed(3)
+    plain = torch.nn.Linear(shape[-1], features, bias=bias, device="cuda")
+    layer = FusedWgradLinear(shape[-1], features, bias=bias, device="cuda")
+    layer.load_state_dict(plain.state_dict())
+    layer.attach(ctx)
+    x = torch.randn(shape, device="cuda").to(x_dtype)
+    results = []
+    for module in (plain, layer):
+        xi = x.clone().requires_grad_()
+        with torch.autocast("cuda", dtype=torch.bfloat16):
+            y = module(xi)
+        y.backward(torch.linspace(-1, 1, y.numel(), device="cuda").view(y.shape).to(y.dtype))
+        wait_pending()
+        assert xi.grad.dtype == x_dtype and module.weight.grad.dtype == torch.float32
+        results.append([y.detach(), xi.grad, module.weight.grad] + ([module.bias.grad] if bias else []))
+    for got, want in zip(results[1], results[0]):
+        assert got.dtype == want.dtype and got.shape == want.shape
+        assert float((got.float() - want.float()).norm()) <= 1e-2 * float(want.float().norm()) + 1e-6

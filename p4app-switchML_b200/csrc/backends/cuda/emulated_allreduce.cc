@@ -164,7 +164,7 @@ int EmulatedAllReduce(int nranks, void* const* in_ptrs, void* const* out_ptrs,
   proto.nranks = nranks;
   proto.slot_bytes = slot_bytes;
   proto.slots_per_channel = slots_per_channel;
-  proto.sc_fence = 0;
+  proto.one_gpu = 1;
   proto.exp_ring = ExpRingDepth(slots_per_channel);
   proto.exp_lookahead = ExpLookahead(slots_per_channel, exponent_lookahead < 0 ? kDefaultExpLookahead : exponent_lookahead);
   proto.block_numel = block_numel;

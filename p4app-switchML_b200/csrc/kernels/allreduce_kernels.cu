@@ -282,7 +282,7 @@ __device__ __forceinline__ void RoleSignal(const RankCtx& ctx, const Role& role,
   role.Sync();
   if (role.tid < ctx.nranks) {
     if (ctx.sc_fence) __threadfence_system();
-    StoreReleaseSys(FlagPtr(ctx.stage_peer[role.tid], channel, phase, ctx.rank), epoch);
+    StoreRelease(ctx, FlagPtr(ctx.stage_peer[role.tid], channel, phase, ctx.rank), epoch);
   }
 }
 
@@ -294,7 +294,7 @@ __device__ __forceinline__ bool RoleWait(const RankCtx& ctx, const Role& role, i
     const Epoch* mine = FlagPtr(ctx.stage_peer[ctx.rank], channel, phase, role.tid);
     unsigned long long start = GlobalTimerNs();
     unsigned long long spins = 0;
-    while (LoadAcquireSys(mine) < epoch) {
+    while (LoadAcquire(ctx, mine) < epoch) {
       ++spins;
       if ((spins & 63) == 0) {
         if (*reinterpret_cast<volatile int*>(&sh->failed)) break;
@@ -351,7 +351,7 @@ __device__ __forceinline__ void RunSignaler(const RankCtx& ctx, StagedShared* sh
     for (int r = 0; r < 3; r++) {
       if (r >= nroles) continue;
       if (d[r] > told[r]) {
-        if (lane < ctx.nranks) StoreReleaseSys(FlagPtr(ctx.stage_peer[lane], channel, r + 1, ctx.rank), base + d[r]);
+        if (lane < ctx.nranks) StoreRelease(ctx, FlagPtr(ctx.stage_peer[lane], channel, r + 1, ctx.rank), base + d[r]);
         told[r] = d[r];
       }
       if (told[r] < ntiles) all = false;
@@ -1608,7 +1608,7 @@ extern "C" int switchml_local_allreduce_noalloc(const void* in, void* out,
   ctx.stage_peer[0] = scratch;
   ctx.slot_bytes = kNoAllocSlotBytes;
   ctx.slots_per_channel = kNoAllocSlots;
-  ctx.sc_fence = 1;
+  ctx.one_gpu = 1;
   ctx.exp_ring = ExpRingDepth(kNoAllocSlots);
   ctx.exp_lookahead = ExpLookahead(kNoAllocSlots, kDefaultExpLookahead);
   ctx.block_numel = block_numel;

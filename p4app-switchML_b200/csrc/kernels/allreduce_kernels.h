@@ -61,6 +61,7 @@ struct RankCtx {
   int slots_per_channel;
   int sc_fence;                  // 1: a sequentially consistent system fence before every flag store (signal_fence = sc);
                                  // 0: the flag's release store alone orders the data before it
+  int one_gpu;                   // 1: all ranks live on this GPU (flags need GPU scope only)
   int exp_ring;                  // exponent slots per channel: a ring of its own, ExpRingDepth(slots_per_channel)
   int exp_lookahead;             // how many tiles the exponents travel ahead of their data (2 * lookahead <= ring)
   int block_numel;               // quantisation block (= packet_numel)

@@ -62,11 +62,13 @@ __device__ __forceinline__ void PushSumStep(size_t v, size_t stride, const char*
                                             size_t recv_bytes, int n, int me, char* out,
                                             const PushTargets& tg, float post_scale) {
   VecAcc<ELEM> acc[U];
+  uint4 tmp[U];
 #pragma unroll
-  for (int u = 0; u < U; u++) acc[u].Init(*reinterpret_cast<const uint4*>(own + (v + u * stride) * 16));
+  for (int u = 0; u < U; u++) tmp[u] = *reinterpret_cast<const uint4*>(own + (v + u * stride) * 16);
+#pragma unroll
+  for (int u = 0; u < U; u++) acc[u].Init(tmp[u]);
   for (int j = 0; j < n - 1; j++) {
     const char* src = recv + static_cast<size_t>(j) * recv_bytes;
-    uint4 tmp[U];
 #pragma unroll
     for (int u = 0; u < U; u++) tmp[u] = *reinterpret_cast<const uint4*>(src + (v + u * stride) * 16);
 #pragma unroll
@@ -79,7 +81,7 @@ __device__ __forceinline__ void PushSumStep(size_t v, size_t stride, const char*
     *reinterpret_cast<uint4*>(out + (v + u * stride) * 16) = r[u];
   }
   for (int d = 1; d < n; d++) {
-    char* dst = tg.Of((me + d) % n);
+    char* dst = tg.Of(me + d < n ? me + d : me + d - n);
 #pragma unroll
     for (int u = 0; u < U; u++) *reinterpret_cast<uint4*>(dst + (v + u * stride) * 16) = r[u];
   }
@@ -92,22 +94,28 @@ template <int ELEM, int U, bool NARROW>
 __device__ __forceinline__ void PushQuantStep(size_t g, size_t stride, size_t first_elem, const char* own,
                                               const char* recv, size_t recv_bytes, int n, int me, char* out,
                                               const PushTargets& tg, float post_scale, const float* sf, int shift) {
-  uint4 acc[U];
+  float4 x[U];
+  uint4 acc[U], tmp[U];
   float f[U];
 #pragma unroll
+  for (int u = 0; u < U; u++) x[u] = LoadGroupAsFloat<ELEM>(own, g + u * stride);
+#pragma unroll
+  for (int u = 0; u < U; u++)  // the first peer's copy is on its way while the own values are quantised
+    tmp[u] = *reinterpret_cast<const uint4*>(recv + (g + u * stride) * 16);
+#pragma unroll
   for (int u = 0; u < U; u++) {
-    const float4 x = LoadGroupAsFloat<ELEM>(own, g + u * stride);
     f[u] = sf[(first_elem + (g + u * stride) * 4) >> shift];
-    acc[u] = make_uint4(static_cast<unsigned>(quant::Quantize(x.x, f[u])), static_cast<unsigned>(quant::Quantize(x.y, f[u])),
-                        static_cast<unsigned>(quant::Quantize(x.z, f[u])), static_cast<unsigned>(quant::Quantize(x.w, f[u])));
+    acc[u] = make_uint4(static_cast<unsigned>(quant::Quantize(x[u].x, f[u])), static_cast<unsigned>(quant::Quantize(x[u].y, f[u])),
+                        static_cast<unsigned>(quant::Quantize(x[u].z, f[u])), static_cast<unsigned>(quant::Quantize(x[u].w, f[u])));
   }
   for (int j = 0; j < n - 1; j++) {
-    const char* src = recv + static_cast<size_t>(j) * recv_bytes;
-    uint4 tmp[U];
-#pragma unroll
-    for (int u = 0; u < U; u++) tmp[u] = *reinterpret_cast<const uint4*>(src + (g + u * stride) * 16);
 #pragma unroll
     for (int u = 0; u < U; u++) { acc[u].x += tmp[u].x; acc[u].y += tmp[u].y; acc[u].z += tmp[u].z; acc[u].w += tmp[u].w; }
+    if (j + 1 < n - 1) {
+      const char* src = recv + static_cast<size_t>(j + 1) * recv_bytes;
+#pragma unroll
+      for (int u = 0; u < U; u++) tmp[u] = *reinterpret_cast<const uint4*>(src + (g + u * stride) * 16);
+    }
   }
   uint4 w[U];
   uint2 h[U];
@@ -125,10 +133,10 @@ __device__ __forceinline__ void PushQuantStep(size_t g, size_t stride, size_t fi
     else *reinterpret_cast<uint4*>(out + (g + u * stride) * 16) = w[u];
   }
   for (int d = 1; d < n; d++) {
-    char* dst = tg.Of((me + d) % n);
+    char* dst = tg.Of(me + d < n ? me + d : me + d - n);
 #pragma unroll
     for (int u = 0; u < U; u++) {
-      if (NARROW) *reinterpret_cast<uint2*>(dst + (g + u * stride) * 8) = h[u];
+        if (NARROW) *reinterpret_cast<uint2*>(dst + (g + u * stride) * 8) = h[u];
       else *reinterpret_cast<uint4*>(dst + (g + u * stride) * 16) = w[u];
     }
   }
@@ -272,17 +280,25 @@ __device__ void RunPush(const RankCtx& ctx, const JobArgs& job, int channel,
       const size_t per = len / n;  // a full tile: n shards of whole chunks
       if (MODE == MODE_QUANT && stream && len == tile_elems && per % (kWsChunk / 4) == 0) {
         // All n-1 foreign shards as one run of chunks, the right-hand neighbour's first.
-        const size_t cps = per / (kWsChunk / 4);  // chunks per shard
+        const unsigned cps = static_cast<unsigned>(per / (kWsChunk / 4));  // chunks per shard
         char* const* peers = ctx.stage_peer;
+        // Chunk c of the run: the rank it goes to and its place in that rank's shard, in elements.
+        auto place = [&](size_t c, size_t* off) {
+          const unsigned shard = static_cast<unsigned>(c) / cps;
+          *off = static_cast<size_t>(static_cast<unsigned>(c) - shard * cps) * (kWsChunk / 4);
+          const int p = me + 1 + static_cast<int>(shard);
+          return p < n ? p : p - n;
+        };
         streamed = WarpStreamRun(
-            ws, warp, kLoadWarps, lane, cps * (n - 1),
+            ws, warp, kLoadWarps, lane, static_cast<size_t>(cps) * (n - 1),
             [&](size_t c) {
-              const int p = (me + 1 + static_cast<int>(c / cps)) % n;
-              return in + (static_cast<size_t>(p) * per + (c % cps) * (kWsChunk / 4)) * 4;
+              size_t off;
+              const int p = place(c, &off);
+              return in + (static_cast<size_t>(p) * per + off) * 4;
             },
             [&](size_t c, const char* smem) {
-              const int p = (me + 1 + static_cast<int>(c / cps)) % n;
-              const size_t off = (c % cps) * (kWsChunk / 4);  // first element of the chunk inside its shard
+              size_t off;
+              const int p = place(c, &off);
               int4* dst = reinterpret_cast<int4*>(peers[p] + slot_off + static_cast<size_t>(PushAreaIndex(me, p)) * recv_bytes) + off / 4;
               const float* sfp = sf;
               float4 x[8];
@@ -349,21 +365,12 @@ __device__ void RunPush(const RankCtx& ctx, const JobArgs& job, int channel,
         const size_t t = role.tid, nt = role.nthreads;
         const uintptr_t both = reinterpret_cast<uintptr_t>(own) | reinterpret_cast<uintptr_t>(out);
         if (MODE == MODE_QUANT) {
-          const bool narrow = ELEM == ELEM_BF16;  // bf16 jobs receive bf16: in their output, or in the result areas
+          constexpr bool narrow = ELEM == ELEM_BF16;  // bf16 jobs receive bf16: in their output, or in the result areas
           const size_t ngroups = (both & (ELEM == ELEM_BF16 ? 7 : 15)) == 0 ? cnt / 4 : 0;
-          constexpr int U = 4;
-          size_t g = t;
-          if (narrow) {
-            for (; g + (U - 1) * nt < ngroups; g += U * nt)
-              PushQuantStep<ELEM, U, true>(g, nt, sb, own, recv, recv_bytes, n, me, out, tg, job.post_scale, sf, shift);
-            for (; g < ngroups; g += nt)
-              PushQuantStep<ELEM, 1, true>(g, nt, sb, own, recv, recv_bytes, n, me, out, tg, job.post_scale, sf, shift);
-          } else {
-            for (; g + (U - 1) * nt < ngroups; g += U * nt)
-              PushQuantStep<ELEM, U, false>(g, nt, sb, own, recv, recv_bytes, n, me, out, tg, job.post_scale, sf, shift);
-            for (; g < ngroups; g += nt)
-              PushQuantStep<ELEM, 1, false>(g, nt, sb, own, recv, recv_bytes, n, me, out, tg, job.post_scale, sf, shift);
-          }
+          Turns<4>(t, ngroups, nt, [&](auto width, size_t g) {
+            PushQuantStep<ELEM, decltype(width)::value, ELEM == ELEM_BF16>(g, nt, sb, own, recv, recv_bytes, n, me, out, tg,
+                                                                          job.post_scale, sf, shift);
+          });
           // Ragged end, or pointers that are not vector aligned: element by element.
           for (size_t i = ngroups * 4 + t; i < cnt; i += nt) {
             const float f = sf[(sb + i) >> shift];
@@ -383,11 +390,9 @@ __device__ void RunPush(const RankCtx& ctx, const JobArgs& job, int channel,
         } else {
           const size_t vec_elems = 16 / in_esz;
           const size_t nvec = (both & 15) == 0 ? cnt / vec_elems : 0;
-          size_t v = t;
-          for (; v + (kPushUnroll - 1) * nt < nvec; v += kPushUnroll * nt)
-            PushSumStep<ELEM, kPushUnroll>(v, nt, own, recv, recv_bytes, n, me, out, tg, job.post_scale);
-          for (; v < nvec; v += nt)
-            PushSumStep<ELEM, 1>(v, nt, own, recv, recv_bytes, n, me, out, tg, job.post_scale);
+          Turns<kPushUnroll>(t, nvec, nt, [&](auto width, size_t v) {
+            PushSumStep<ELEM, decltype(width)::value>(v, nt, own, recv, recv_bytes, n, me, out, tg, job.post_scale);
+          });
           for (size_t i = nvec * vec_elems + t; i < cnt; i += nt) {
             if (ELEM == ELEM_I32) {
               unsigned a = reinterpret_cast<const unsigned*>(own)[i];

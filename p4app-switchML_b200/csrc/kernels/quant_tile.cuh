@@ -60,6 +60,30 @@ __device__ __forceinline__ float4 LoadGroupAsFloat(const char* in, size_t group)
   return *reinterpret_cast<const float4*>(in + group * 16);
 }
 
+// Largest of each of NV values over groups of W neighbouring lanes: lane l returns the maximum of value
+// ((l % W) * NV) / W. The values are handed out while they are reduced (NV - 1 + log2(W / NV) shuffles
+// instead of NV * log2(W)).
+template <int NV, int W>
+__device__ __forceinline__ float GroupMaxima(const float (&v)[NV], int lane) {
+  static_assert(NV <= W, "a lane returns one value");
+  float t[NV];
+#pragma unroll
+  for (int i = 0; i < NV; i++) t[i] = v[i];
+  int o = W / 2;
+#pragma unroll
+  for (int half = NV / 2; half >= 1; half >>= 1, o >>= 1) {
+    const bool up = (lane & o) != 0;
+#pragma unroll
+    for (int i = 0; i < half; i++) {
+      const float other = __shfl_xor_sync(0xffffffffu, up ? t[i] : t[i + half], o);
+      t[i] = fmaxf(up ? t[i + half] : t[i], other);
+    }
+  }
+#pragma unroll
+  for (; o >= 1; o >>= 1) t[0] = fmaxf(t[0], __shfl_xor_sync(0xffffffffu, t[0], o));
+  return t[0];
+}
+
 // Local exponents of the `len` elements at `in` (one tile), published under `tag` into the
 // exponent words starting at byte offset `exp_off`. Called by all threads of a role of
 // `nwarps` warps; `warp` is the caller's warp index inside the role.
@@ -68,45 +92,41 @@ __device__ __forceinline__ float4 LoadGroupAsFloat(const char* in, size_t group)
 // Blocks of 32 or 64 elements are groups of 8 or 16 neighbouring lanes of one row; larger
 // blocks are 1, 2, 4 or 8 whole rows, which a step always holds completely because steps
 // start at multiples of 8 rows.
+// kLog2Block: log2 of the block size, so that all indexes are shifts (with the size known at run time
+// only, publishing a 16 Ki element tile took 9 us, most of it 64-bit divisions).
+template <int kLog2Block>
+__device__ __forceinline__ void PublishRows8As(const RankCtx& ctx, int lane, const float4* x, size_t row0, size_t exp_off, Epoch tag) {
+  constexpr int kLanes = kLog2Block >= 7 ? 32 : 1 << (kLog2Block - 2);  // lanes per block and row
+  constexpr int kRowsPerBlock = kLog2Block >= 7 ? 1 << (kLog2Block - 7) : 1;
+  constexpr int NV = 8 / kRowsPerBlock;
+  float m[NV];
+#pragma unroll
+  for (int u = 0; u < NV; u++) {
+    m[u] = 0.f;
+#pragma unroll
+    for (int r = 0; r < kRowsPerBlock; r++) {
+      const float4 v = x[u * kRowsPerBlock + r];
+      m[u] = fmaxf(m[u], fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
+    }
+  }
+  const float mine = GroupMaxima<NV, kLanes>(m, lane);
+  constexpr int kShare = kLanes / NV;  // lanes that hold the same value: the first publishes it
+  if ((lane & (kShare - 1)) == 0) {
+    const int value = (lane & (kLanes - 1)) / kShare;  // which of the NV
+    const size_t block = ((row0 * 128) >> kLog2Block) + (kLanes < 32 ? value * (32 / kLanes) + lane / kLanes : value);
+    ExpPublish(ctx, exp_off + block * kExpWordBytes, ExpWord(tag, quant::LocalExponent(mine)));
+  }
+}
+
 __device__ __forceinline__ void PublishRows8(const RankCtx& ctx, int lane, const float4* x, size_t row0,
                                              size_t exp_off, Epoch tag) {
-  constexpr int kRows = 8;
-  const size_t B = ctx.block_numel;
-  float m[kRows];
-#pragma unroll
-  for (int u = 0; u < kRows; u++)
-    m[u] = fmaxf(fmaxf(fabsf(x[u].x), fabsf(x[u].y)), fmaxf(fabsf(x[u].z), fabsf(x[u].w)));
-  if (B < 128) {
-    const int g = static_cast<int>(B / 4);  // lanes per block: 8 or 16
-    const size_t per_row = 128 / B;         // blocks per row: 4 or 2
-#pragma unroll
-    for (int u = 0; u < kRows; u++) {
-      float mm = m[u];
-      for (int o = g >> 1; o > 0; o >>= 1) mm = fmaxf(mm, __shfl_xor_sync(0xffffffffu, mm, o));
-      if ((lane % g) == 0)
-        ExpPublish(ctx, exp_off + ((row0 + u) * per_row + lane / g) * kExpWordBytes,
-                   ExpWord(tag, quant::LocalExponent(mm)));
-    }
-  } else {
-    const int rows_per_block = static_cast<int>(B / 128);  // 1, 2, 4 or 8
-    // fold the rows of one block into the first of them, then one butterfly per block
-#pragma unroll
-    for (int span = 1; span < kRows; span <<= 1) {
-      if (span < rows_per_block) {
-#pragma unroll
-        for (int u = 0; u + span < kRows; u += 2 * span) m[u] = fmaxf(m[u], m[u + span]);
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < kRows; u++) {
-      if ((u % rows_per_block) != 0) continue;  // warp-uniform
-      float mm = m[u];
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) mm = fmaxf(mm, __shfl_xor_sync(0xffffffffu, mm, o));
-      if (lane == 0)
-        ExpPublish(ctx, exp_off + ((row0 + u) / rows_per_block) * kExpWordBytes,
-                   ExpWord(tag, quant::LocalExponent(mm)));
-    }
+  switch (ctx.block_numel) {  // the same for all threads
+    case 32: return PublishRows8As<5>(ctx, lane, x, row0, exp_off, tag);
+    case 64: return PublishRows8As<6>(ctx, lane, x, row0, exp_off, tag);
+    case 128: return PublishRows8As<7>(ctx, lane, x, row0, exp_off, tag);
+    case 256: return PublishRows8As<8>(ctx, lane, x, row0, exp_off, tag);
+    case 512: return PublishRows8As<9>(ctx, lane, x, row0, exp_off, tag);
+    default: return PublishRows8As<10>(ctx, lane, x, row0, exp_off, tag);
   }
 }
 

@@ -38,7 +38,6 @@ def emulated_allreduce(inputs, mode="quant", algo="staged", block_numel=256, slo
     array = _ARRAYS.get(n) or _ARRAYS.setdefault(n, ctypes.c_void_p * n)
     ins = array(*[x.data_ptr() for x in inputs])
     outs = array(*[o.data_ptr() for o in outputs])
-    torch.cuda.synchronize()
     rc = lib().sml_emu_allreduce(n, ins, outs, numel, elem, MODE[mode], ALGO[algo], block_numel,
                                  slot_bytes, slots_per_channel, channels, float(post_scale), repeats,
                                  int(exponent_lookahead))

@@ -978,29 +978,43 @@ __device__ void RunOneShot(const RankCtx& ctx, const JobArgs& job, int channel,
         x.w = 0.f;
         return x;
       };
+      // A block of up to 256 elements stays in registers between the two passes (kHeld float4 per rank).
+      constexpr int kHeld = 2;
+      const bool held = n <= kHeld * 128 && (n & 3) == 0;
+      float4 x[kHeld][kMaxRanks];
       float m = 0.f;
-      for (size_t i = lane * 4; i < n; i += 128) {
+      auto largest = [&](float4 v) { m = fmaxf(m, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w)))); };  // a NaN never wins
+      if (held) {
 #pragma unroll
-        for (int s = 0; s < kMaxRanks; s++) {
-          if (s >= ctx.nranks) continue;  // uniform
-          const float4 x = load4(s, i);
-          m = fmaxf(m, fmaxf(fmaxf(fabsf(x.x), fabsf(x.y)), fmaxf(fabsf(x.z), fabsf(x.w))));  // a NaN never wins
+        for (int h = 0; h < kHeld; h++) {
+#pragma unroll
+          for (int s = 0; s < kMaxRanks; s++) {
+            x[h][s] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (s < ctx.nranks && h * 128 + lane * 4 < n) x[h][s] = LoadGroupAsFloat<ELEM>(src0 + s * src_step, base / 4 + h * 32 + lane);
+          }
+        }
+#pragma unroll
+        for (int h = 0; h < kHeld; h++) {
+#pragma unroll
+          for (int s = 0; s < kMaxRanks; s++) largest(x[h][s]);
+        }
+      } else {
+        for (size_t i = lane * 4; i < n; i += 128) {
+#pragma unroll
+          for (int s = 0; s < kMaxRanks; s++)
+            if (s < ctx.nranks) largest(load4(s, i));  // uniform
         }
       }
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
       const float sf = quant::ScaleFactorFromBase(quant::LocalExponent(m), ctx.quant_base);
-      for (size_t i = lane * 4; i < n; i += 128) {
-        unsigned acc[4] = {0, 0, 0, 0};
-#pragma unroll
-        for (int s = 0; s < kMaxRanks; s++) {
-          if (s >= ctx.nranks) continue;
-          const float4 x = load4(s, i);
-          acc[0] += static_cast<unsigned>(quant::Quantize(x.x, sf));
-          acc[1] += static_cast<unsigned>(quant::Quantize(x.y, sf));
-          acc[2] += static_cast<unsigned>(quant::Quantize(x.z, sf));
-          acc[3] += static_cast<unsigned>(quant::Quantize(x.w, sf));
-        }
+      auto add4 = [&](unsigned (&acc)[4], float4 v) {
+        acc[0] += static_cast<unsigned>(quant::Quantize(v.x, sf));
+        acc[1] += static_cast<unsigned>(quant::Quantize(v.y, sf));
+        acc[2] += static_cast<unsigned>(quant::Quantize(v.z, sf));
+        acc[3] += static_cast<unsigned>(quant::Quantize(v.w, sf));
+      };
+      auto finish = [&](size_t i, const unsigned (&acc)[4]) {
         float y[4];
 #pragma unroll
         for (int j = 0; j < 4; j++) {
@@ -1017,6 +1031,25 @@ __device__ void RunOneShot(const RankCtx& ctx, const JobArgs& job, int channel,
             if (ELEM == ELEM_BF16) reinterpret_cast<unsigned short*>(out)[base + i + j] = FloatToBf16(y[j]);
             else reinterpret_cast<float*>(out)[base + i + j] = y[j];
           }
+        }
+      };
+      if (held) {
+#pragma unroll
+        for (int h = 0; h < kHeld; h++) {
+          const size_t i = h * 128 + lane * 4;
+          unsigned acc[4] = {0, 0, 0, 0};
+#pragma unroll
+          for (int s = 0; s < kMaxRanks; s++)
+            if (s < ctx.nranks) add4(acc, x[h][s]);
+          if (i < n) finish(i, acc);
+        }
+      } else {
+        for (size_t i = lane * 4; i < n; i += 128) {
+          unsigned acc[4] = {0, 0, 0, 0};
+#pragma unroll
+          for (int s = 0; s < kMaxRanks; s++)
+            if (s < ctx.nranks) add4(acc, load4(s, i));
+          finish(i, acc);
         }
       }
     }

@@ -100,12 +100,27 @@ __device__ __forceinline__ void SetRawWord(RawVec<8>& r, int i, unsigned w) { if
 __device__ __forceinline__ void SetRawWord(RawVec<4>& r, int, unsigned w) { r.v = w; }
 __device__ __forceinline__ void SetRawWord(RawVec<2>& r, int, unsigned w) { r.v = static_cast<unsigned short>(w); }
 
+// The larger of two magnitudes. kNan: NaN if either is; else a NaN never wins.
+template <bool kNan>
+__device__ __forceinline__ float Larger(float a, float b) {
+  if (!kNan) return fmaxf(a, b);
+  float r;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+  return r;
+}
+
 // One chunk of kQuantChunk elements by one warp, in vectors of VB bytes (of VE elements): vector
 // u * 32 + lane is lane's u-th, so a row is the 32 * VE elements that a load instruction brings.
 // A quantisation block is a power of two of lanes of one row, or of whole rows. kGuard: the chunk
 // has only `valid` elements, VB is one element; what is missing counts as zero.
-template <int ELEM, int VB, bool kGuard>
-__device__ __forceinline__ void LocalQuantChunk(const char* in, char* out, int lane, int log2_block, float base,
+//
+// kFast: with one worker the trip x -> int32 -> float rounds x to a multiple of 2^(E-31), E the block's
+// exponent. That is (x + C) - C with C = +-2^(E-8): below C the sum's last bit is the grid's, from C on
+// x lies on the grid already. Conversions between float and int run at an eighth of the rate of additions,
+// two of them per element took 5.9 us of a 25 MB bf16 bucket (kernel 11.6 us -> 9.1 us). Nothing is done and
+// false comes back when a value is not finite or so large that the integer saturates; kFast = false takes those.
+template <int ELEM, int VB, bool kGuard, bool kFast>
+__device__ __forceinline__ bool LocalQuantChunk(const char* in, char* out, int lane, int log2_block, float base,
                                                 int valid) {
   constexpr int kEsz = ELEM == ELEM_BF16 ? 2 : 4;
   constexpr int VE = VB / kEsz;
@@ -129,10 +144,10 @@ __device__ __forceinline__ void LocalQuantChunk(const char* in, char* out, int l
     for (int w = 0; w < kWords; w++) {
       const unsigned raw = RawWord(x[u], w);
       if (ELEM == ELEM_F32) {
-        m[u] = fmaxf(m[u], fabsf(__uint_as_float(raw)));  // a NaN never wins
+        m[u] = Larger<kFast>(m[u], fabsf(__uint_as_float(raw)));
       } else {
-        m[u] = fmaxf(m[u], fabsf(__uint_as_float(raw << 16)));
-        if (VB >= 4) m[u] = fmaxf(m[u], fabsf(__uint_as_float(raw & 0xffff0000u)));
+        m[u] = Larger<kFast>(m[u], fabsf(__uint_as_float(raw << 16)));
+        if (VB >= 4) m[u] = Larger<kFast>(m[u], fabsf(__uint_as_float(raw & 0xffff0000u)));
       }
     }
   }
@@ -142,7 +157,7 @@ __device__ __forceinline__ void LocalQuantChunk(const char* in, char* out, int l
     for (int o = 16; o > 0; o >>= 1) {
       if (o < lanes) {  // warp-uniform
 #pragma unroll
-        for (int u = 0; u < kRows; u++) m[u] = fmaxf(m[u], __shfl_xor_sync(0xffffffffu, m[u], o));
+        for (int u = 0; u < kRows; u++) m[u] = Larger<kFast>(m[u], __shfl_xor_sync(0xffffffffu, m[u], o));
       }
     }
   } else {
@@ -152,14 +167,14 @@ __device__ __forceinline__ void LocalQuantChunk(const char* in, char* out, int l
     for (int span = 1; span < kRows; span <<= 1) {
       if (span < rows) {
 #pragma unroll
-        for (int u = 0; u + span < kRows; u += 2 * span) m[u] = fmaxf(m[u], m[u + span]);
+        for (int u = 0; u + span < kRows; u += 2 * span) m[u] = Larger<kFast>(m[u], m[u + span]);
       }
     }
 #pragma unroll
     for (int u = 0; u < kRows; u++) {
       if ((u & (rows - 1)) != 0) continue;
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) m[u] = fmaxf(m[u], __shfl_xor_sync(0xffffffffu, m[u], o));
+      for (int o = 16; o > 0; o >>= 1) m[u] = Larger<kFast>(m[u], __shfl_xor_sync(0xffffffffu, m[u], o));
     }
 #pragma unroll
     for (int span = kRows / 2; span >= 1; span >>= 1) {
@@ -169,13 +184,26 @@ __device__ __forceinline__ void LocalQuantChunk(const char* in, char* out, int l
       }
     }
   }
+  if (kFast) {
+    bool odd = false;
+#pragma unroll
+    for (int u = 0; u < kRows; u++) odd |= !(m[u] < 0x1p127f);
+    if (__any_sync(0xffffffffu, odd)) return false;
+  }
 #pragma unroll
   for (int u = 0; u < kRows; u++) {
-    // With one worker the scale factor is a power of two (2^31 over the block's power), so that
-    // multiplying by its exact reciprocal gives the bits of the division.
-    const float f = quant::ScaleFactorFromBase(quant::LocalExponent(m[u]), base);
+    const int exponent = quant::ClampExponent(quant::LocalExponent(m[u]));
+    const float c = __int_as_float((exponent - 8 + 127) << 23);
+    // (The scale factor is a power of two here, so that multiplying by its exact reciprocal gives the bits of
+    // the division.)
+    const float f = quant::ScaleFactorFromBase(exponent, base);
     const float inv = __frcp_rn(f);
-    auto trip = [&](float v) { return __int2float_rn(quant::Quantize(v, f)) * inv; };
+    auto trip = [&](float v) {
+      if (!kFast) return __int2float_rn(quant::Quantize(v, f)) * inv;
+      const float cv = __uint_as_float((__float_as_uint(v) & 0x80000000u) | __float_as_uint(c));
+      const float r = __fsub_rn(__fadd_rn(v, cv), cv);
+      return fabsf(v) < c ? r : v;
+    };
     RawVec<VB> y;
 #pragma unroll
     for (int w = 0; w < kWords; w++) {
@@ -192,6 +220,7 @@ __device__ __forceinline__ void LocalQuantChunk(const char* in, char* out, int l
     }
     if (!kGuard || u * 32 + lane < valid) reinterpret_cast<RawVec<VB>*>(out)[u * 32 + lane] = y;
   }
+  return true;
 }
 
 // One chunk per warp; the last warp takes what is left over (fewer than kQuantChunk elements).
@@ -203,9 +232,12 @@ LocalQuantKernel(const char* in, char* out, size_t numel, int log2_block, float 
   const size_t c = (static_cast<size_t>(blockIdx.x) * kQuantThreads + threadIdx.x) >> 5;
   const size_t off = c * kQuantChunk;
   if (off + kQuantChunk <= numel) {
-    LocalQuantChunk<ELEM, VB, false>(in + off * kEsz, out + off * kEsz, lane, log2_block, base, kQuantChunk);
+    const char* from = in + off * kEsz;
+    char* to = out + off * kEsz;
+    if (!LocalQuantChunk<ELEM, VB, false, true>(from, to, lane, log2_block, base, kQuantChunk))
+      LocalQuantChunk<ELEM, kEsz, true, false>(from, to, lane, log2_block, base, kQuantChunk);
   } else if (off < numel) {
-    LocalQuantChunk<ELEM, kEsz, true>(in + off * kEsz, out + off * kEsz, lane, log2_block, base, static_cast<int>(numel - off));
+    LocalQuantChunk<ELEM, kEsz, true, false>(in + off * kEsz, out + off * kEsz, lane, log2_block, base, static_cast<int>(numel - off));
   }
 }
 

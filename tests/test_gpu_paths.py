@@ -222,3 +222,34 @@ def test_fused_wgrad_linear_against_plain_linear(ctx, shape, features, bias, x_d
     for got, want in zip(results[1], results[0]):
         assert got.dtype == want.dtype and got.shape == want.shape
         assert float((got.float() - want.float()).norm()) <= 1e-2 * float(want.float().norm()) + 1e-6
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_one_worker_exact_pass_of_odd_values(ctx, dtype):
+    """Infinities, NaN, values whose integer saturates, denormals, negative zeros and halves of the grid:
+    whatever the arithmetic, the bits are the oracle's."""
+    block = 64
+    assert ctx.start(sml.make_config("cuda", packet_numel=block, mode="int32_quant", launch="inline"))
+    gen = torch.Generator().manual_seed(1)
+    x = torch.randn(40 * 1024 + 13, generator=gen)
+    x[0:3] = torch.tensor([float("inf"), -float("inf"), float("nan")])
+    x[1024] = 3.0e38
+    x[2048] = -2.0 ** 127
+    x[3072:3072 + block] = torch.randn(block, generator=gen) * 1e-42   # denormals
+    x[4096:4096 + block] = -0.0
+    x[5120] = float("nan")
+    # Halves of the grid of a block whose exponent is 1: multiples of 2^-31, ties to even.
+    ties = torch.randint(-2 ** 20, 2 ** 20, (1024,), generator=gen).float() * 2.0 ** -31
+    x[6144:7168] = ties
+    x[6144:7168:block] = 1.5
+    x[7168:8192] = torch.randn(1024, generator=gen) * 2.0 ** -119          # below the smallest exponent
+    x[8192:9216] = torch.randn(1024, generator=gen).clamp(-1.9, 1.9) * 2.0 ** 126
+    x = x.to(dtype)
+    want = torch.from_numpy(quant_allreduce_oracle([x.float().numpy()], block)).to(dtype)
+    for offset in (0, 1):
+        frame = torch.empty(x.numel() + offset, dtype=dtype, device="cuda")
+        d = frame[offset:]
+        d.copy_(x)
+        ctx.all_reduce(d)
+        bits = torch.int32 if dtype == torch.float32 else torch.int16
+        assert torch.equal(d.cpu().view(bits), want.view(bits)), offset

@@ -101,6 +101,7 @@ struct EventState : public DeviceJobState {
     const auto start = std::chrono::steady_clock::now();
     RelaxedCapture relaxed;
     for (;;) {
+      if (milliseconds < 0) cudaEventSynchronize(done);  // without a limit the driver waits, which answers fastest
       {
         std::lock_guard<std::mutex> lk(completions->mu);
         if (!completions->reap) return;
@@ -108,13 +109,10 @@ struct EventState : public DeviceJobState {
       }
       const JobStatus s = job.GetJobStatus();
       if (s == FINISHED || s == FAILED) return;
-      // Not fired yet. Without a limit the driver waits, which answers fastest.
-      if (milliseconds < 0) {
-        cudaEventSynchronize(done);
-      } else if (std::chrono::steady_clock::now() - start > std::chrono::duration<double, std::milli>(milliseconds)) {
-        return;
-      } else if (std::chrono::steady_clock::now() - start > std::chrono::microseconds(100)) {
-        std::this_thread::sleep_for(std::chrono::microseconds(10));
+      if (milliseconds >= 0) {
+        const auto passed = std::chrono::steady_clock::now() - start;
+        if (passed > std::chrono::duration<double, std::milli>(milliseconds)) return;
+        if (passed > std::chrono::microseconds(100)) std::this_thread::sleep_for(std::chrono::microseconds(10));
       }
       std::this_thread::yield();
     }
@@ -136,6 +134,7 @@ static const int kStatusSlots = 4096;
 // launch = worker: with this many jobs in flight the launcher thread takes over, which may wait for
 // room in the stream's queue (about a thousand launches) while the callers go on.
 static const size_t kDirectLaunches = 256;
+static const uint64_t kBriefBytes = 1 << 20;  // read + write at 6 TB/s: 0.4 us
 
 // One NVTX range per job for timeline tools; without one the name is not even put together.
 struct NvtxRange {
@@ -662,7 +661,10 @@ bool CudaBackend::OnSubmit(const std::shared_ptr<Job>& job) {
     cudaGetLastError();
   }
   const bool capturing = capture == cudaStreamCaptureStatusActive;
-  if (!inline_launch_) {
+  // launch = worker: a single worker's short pass takes less than handing over from the producer's stream to
+  // the backend's and back (two events and the GPU's wait for them), so it runs where its input was made.
+  const bool brief = n_ == 1 && job->tensor_.numel * DataTypeSize(job->tensor_.data_type) <= kBriefBytes;
+  if (!inline_launch_ && (capturing || !brief)) {
     // Where the producer stream is now: the job comes after it.
     f.ready = GetEvent();
     cudaEventRecord(f.ready, user_stream);
@@ -677,6 +679,7 @@ bool CudaBackend::OnSubmit(const std::shared_ptr<Job>& job) {
     job->SetJobStatus(QUEUED);
     job->SetJobStatus(RUNNING);
     cudaStreamWaitEvent(comm_stream_, f.ready, 0);
+    if (last_job_) last_job_->StreamWait(comm_stream_);
     LaunchJob(job, comm_stream_, &f);
     PushInFlight(std::move(f));
     return true;
@@ -687,6 +690,13 @@ bool CudaBackend::OnSubmit(const std::shared_ptr<Job>& job) {
   }
   {
     std::lock_guard<std::mutex> lk(launch_mu_);
+    if (!inline_launch_ && (queued_jobs_ > 0 || InFlightCount() >= kDirectLaunches)) {
+      f.ready = GetEvent();
+      cudaEventRecord(f.ready, user_stream);
+      job->ready_event_ = f.ready;
+      queued_jobs_++;
+      return false;  // in line behind the jobs that the launcher thread has not enqueued yet
+    }
     job->SetJobStatus(QUEUED);
     job->SetJobStatus(RUNNING);
     // Not while capturing: an event recorded outside the capture cannot be waited on inside
@@ -735,6 +745,7 @@ void CudaBackend::LauncherLoop() {
     {
       std::lock_guard<std::mutex> lk(launch_mu_);
       if (f.ready) cudaStreamWaitEvent(comm_stream_, f.ready, 0);
+      if (last_job_) last_job_->StreamWait(comm_stream_);
       LaunchJob(js.job, comm_stream_, &f);
       PushInFlight(std::move(f));
       queued_jobs_--;

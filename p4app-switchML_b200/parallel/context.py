@@ -5,6 +5,7 @@ import ctypes
 import enum
 import json
 
+from .. import _native
 from .._native import lib, last_error, read_string, NativeError
 
 
@@ -24,6 +25,7 @@ class JobStatus(enum.IntEnum):
 
 
 _STATUS = tuple(JobStatus)
+_FINISHED = JobStatus.FINISHED
 
 
 class ContextState(enum.IntEnum):
@@ -40,6 +42,10 @@ try:
     _raw_stream = getattr(_torch._C, "_cuda_getCurrentRawStream", None)
 except ImportError:  # numpy-only environments
     _torch, _TORCH_CODES, _raw_stream = None, {}, None
+
+
+def _current_device():
+    return _torch._C._cuda_getDevice() if _torch.cuda.is_initialized() else _torch.cuda.current_device()
 
 
 def _current_stream(device_index):
@@ -90,8 +96,8 @@ class Job:
 
     def stream_wait(self, stream=None):
         """Order a CUDA stream after the job without waiting on the host (cuda backend)."""
-        ptr = _current_stream(_torch.cuda.current_device()) if stream is None else getattr(stream, "cuda_stream", stream)
-        if lib().sml_job_stream_wait(self._h, ptr) != 0:
+        ptr = _current_stream(_current_device()) if stream is None else getattr(stream, "cuda_stream", stream)
+        if (_native._LIB or lib()).sml_job_stream_wait(self._h, ptr) != 0:
             raise NativeError(last_error())
 
     def error(self):
@@ -104,7 +110,7 @@ class Job:
 
     def release(self):
         if self._h:
-            lib().sml_job_release(self._h)
+            (_native._LIB or lib()).sml_job_release(self._h)
             self._h = 0
             self._keep = None
 
@@ -168,23 +174,29 @@ class Context:
     # -- jobs ------------------------------------------------------------------------
     def all_reduce_async(self, tensor, out=None, stream=None):
         """Submit a SUM allreduce of `tensor` (result in `out`, default in place)."""
-        ptr, numel, code, cur_stream, is_cuda = _describe(tensor)
-        optr = ptr
-        if out is not None:
+        ptr, numel, code, cur_stream, _ = _describe(tensor)
+        if out is None:
+            optr = ptr
+        elif _torch is not None and type(out) is _torch.Tensor and type(tensor) is _torch.Tensor:
+            if out.dtype != tensor.dtype or out.numel() != numel:
+                raise ValueError("out must match the input's size and dtype")
+            if not out.is_contiguous():
+                raise ValueError("tensor must be contiguous")
+            optr = out.data_ptr()
+        else:
             optr, onumel, ocode, _, _ = _describe(out)
             if onumel != numel or ocode != code:
                 raise ValueError("out must match the input's size and dtype")
         if stream is not None:
             cur_stream = getattr(stream, "cuda_stream", stream)
-        h = lib().sml_allreduce_async(ptr, optr, numel, code, cur_stream)
+        h = (_native._LIB or lib()).sml_allreduce_async(ptr, optr, numel, code, cur_stream)
         if h < 0:
             raise NativeError(last_error())
         return Job(h, (tensor, out))
 
     def all_reduce(self, tensor, out=None):
         job = self.all_reduce_async(tensor, out)
-        st = job.wait()
-        if st != JobStatus.FINISHED:
+        if job.wait() is not _FINISHED:
             raise NativeError("allreduce failed: " + job.error())
         return job
 

@@ -1479,7 +1479,17 @@ LaunchPlan PlanLaunch(const RankCtx& ctx, const JobArgs& job, int requested_chan
     unsigned long long unit = static_cast<unsigned long long>(ctx.nranks) *
                               (ctx.block_numel > 128 ? ctx.block_numel : 128);
     unsigned long long tile = (numel + 4ull * ch - 1) / (4ull * ch);
-    if (tile < 16384) tile = 16384;
+    if (ctx.one_gpu) {
+      // Meeting costs little on one GPU, an idle SM as much as anywhere: one to four tiles of 4 Ki to 14 Ki
+      // elements for every channel before they grow (2^18 elements were 16 tiles for 74 channels).
+      const unsigned long long per_channel = (numel + ch - 1) / ch;
+      unsigned long long count = (per_channel + 7168) / 14336;
+      count = count < 1 ? 1 : count > 4 ? 4 : count;
+      tile = (per_channel + count - 1) / count;
+      if (tile < 4096) tile = 4096;
+    } else if (tile < 16384) {
+      tile = 16384;
+    }
     tile = (tile + unit - 1) / unit * unit;
     if (tile > slot_elems) tile = slot_elems;
     p.tile_elems = tile;

@@ -10,6 +10,7 @@ Products (all inside this directory, never installed elsewhere):
     lib/libswitchml_gemm.so        tcgen05 weight-gradient GEMM (loaded on demand)
     lib/torch_switchml.so          native c10d backend for PyTorch (python build.py --torch)
     lib/torch_switchml_linear.so   autograd node of FusedWgradLinear (python build.py --torch)
+    lib/torch_switchml_jobs.so     submission of torch tensors without Python (python build.py --torch)
     build-checked/libswitchml_b200.so   the library with the kernels' bounds checks (--checked)
     lib/libnccl-net-switchml.so    NCCL collective-network plugin (bin/collnet_harness drives it)
     bin/switchml_switchd           stand-alone controller / software switch
@@ -240,12 +241,13 @@ def build_checked(verbose=False, jobs=None):
 
 # Extensions of PyTorch: product, source, libraries of this package that it links.
 TORCH_EXTENSIONS = [("torch_switchml", "csrc/torch/process_group_sml.cc", ["switchml_b200"]),
-                    ("torch_switchml_linear", "csrc/torch/fused_linear.cc", ["switchml_gemm"])]
+                    ("torch_switchml_linear", "csrc/torch/fused_linear.cc", ["switchml_gemm"]),
+                    ("torch_switchml_jobs", "csrc/torch/jobs.cc", [])]
 
 
 def build_torch_extension(verbose=False):
-    """lib/torch_switchml.so, the native c10d backend, and lib/torch_switchml_linear.so, the autograd node of
-    FusedWgradLinear. Needs the headers and libraries of the installed PyTorch; returns None (with a note) when
+    """lib/torch_switchml.so, the native c10d backend, lib/torch_switchml_linear.so, the autograd node of
+    FusedWgradLinear, and lib/torch_switchml_jobs.so, submission without Python. Needs the headers and libraries of the installed PyTorch; returns None (with a note) when
     they are not usable, else the path of the former."""
     try:
         import torch
@@ -279,7 +281,7 @@ def build_torch_extension(verbose=False):
         os.replace(part, out)
         return out
 
-    with cf.ThreadPoolExecutor(max_workers=2) as ex:
+    with cf.ThreadPoolExecutor(max_workers=3) as ex:
         return list(ex.map(lambda e: one(*e), TORCH_EXTENSIONS))[0]
 
 

@@ -6,7 +6,7 @@ import enum
 import json
 
 from .. import _native
-from .._native import lib, last_error, read_string, NativeError
+from .._native import lib, library_path, last_error, read_string, NativeError
 
 
 class DataType(enum.IntEnum):
@@ -122,6 +122,30 @@ class Job:
             pass
 
 
+def _load_native_jobs():
+    """(Job, submit) of lib/torch_switchml_jobs.so (csrc/torch/jobs.cc), which does what the class above and
+    ``all_reduce_async`` do for torch tensors; (Job, None) where it is not built."""
+    import os
+    path = library_path("torch_switchml_jobs.so")
+    if _torch is None or not os.path.exists(path):
+        return Job, None
+    import importlib.util
+    spec = importlib.util.spec_from_file_location("torch_switchml_jobs", path)
+    try:
+        native = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(native)
+    except ImportError:  # built for another PyTorch
+        return Job, None
+    l = lib()
+    native.init([ctypes.cast(f, ctypes.c_void_p).value for f in
+                 (l.sml_allreduce_async, l.sml_job_wait, l.sml_job_status, l.sml_job_stream_wait, l.sml_job_error,
+                  l.sml_job_release, l.sml_last_error)], _STATUS, NativeError)
+    return native.Job, native.submit
+
+
+Job, _submit = _load_native_jobs()
+
+
 class Context:
     """The library's singleton (``Context.get_instance()``)."""
 
@@ -174,6 +198,10 @@ class Context:
     # -- jobs ------------------------------------------------------------------------
     def all_reduce_async(self, tensor, out=None, stream=None):
         """Submit a SUM allreduce of `tensor` (result in `out`, default in place)."""
+        if _submit is not None:
+            job = _submit(tensor, out, stream)
+            if job is not None:
+                return job
         ptr, numel, code, cur_stream, _ = _describe(tensor)
         if out is None:
             optr = ptr

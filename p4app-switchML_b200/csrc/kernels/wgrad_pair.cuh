@@ -18,27 +18,30 @@
 // cycle is what an SM gets out of L2), whatever the number of stages and of issuing threads; the clock
 // under this load is 1.6 to 1.9 GHz.
 //
-// The epilogue's eight warps store 32 rows each on their own (StoreBox32) and never wait for one another.
+// The epilogue's warps store 32 rows each on their own (StoreBox32) and never wait for one another. While later
+// tiles are multiplied four of them do it, through one 4 KiB buffer each: eight warps' bursts of stores hold up the
+// main loop's loads (4096 x 8192 x 2048: 118 -> 124 us), and buffers beyond that would cost a stage of operands
+// (8192 x 4096 x 1024: 61.9 -> 63.1 us). A pair's last tile, which nothing hides, goes out by all eight through the
+// stages, every box of a warp in flight.
 constexpr int kPairThreads = 384;
 constexpr int kPairEpiWarps = 8;
-constexpr int kPairBufs = 2;
 constexpr uint32_t kPeerBitMask = 0xFEFFFFFFu;  // clears the lowest CTA-rank bit of a shared::cluster address
 constexpr int kPairABytes = kTileK * 128 * 2;   // 128 rows of A: 16 KiB
 
 template <int TN>
 struct __align__(1024) PairShared {
-  static constexpr int kStages = TN == 256 ? 5 : 6;
+  static constexpr int kStages = 6;
   static constexpr int kBBytes = kTileK * (TN / 2) * 2;
   static constexpr int kStageBytes = kPairABytes + kBBytes;
-  uint8_t stage[kStages][kStageBytes];  // split: later the partial sums for the other pairs, 128 rows x TN fp32
-  uint8_t epi[kPairEpiWarps][kPairBufs][32 * 128];
+  uint8_t stage[kStages][kStageBytes];  // later this CTA's part of the last tile, or its partial sums: 128 rows x TN fp32
+  uint8_t epi[4][32 * 128];
   uint64_t full[kStages];
   uint64_t empty[kStages];
   uint64_t acc_full[2];
   uint64_t acc_empty[2];
   uint32_t tmem_base;
   volatile int abort;
-  static_assert(kStages * kStageBytes >= 128 * TN * 4, "the partial sums must fit");
+  static_assert(kStages * kStageBytes >= 128 * TN * 4, "the result must fit");
 };
 
 __device__ __forceinline__ void ClusterSync() {
@@ -82,6 +85,18 @@ __device__ __forceinline__ void MbarArriveOn(uint64_t* bar, uint32_t rank) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(PeerAddr(SmemAddr(bar), rank)) : "memory");
 }
 
+// A barrier of the epilogue's warps that tells all of them whether any of them says yes.
+__device__ __forceinline__ bool EpilogueAny(bool yes) {
+  uint32_t any;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.u32 p, %1, 0;\n\t"
+      "barrier.cta.red.or.pred q, 1, %2, p;\n\t"
+      "selp.u32 %0, 1, 0, q;\n\t}"
+      : "=r"(any) : "r"(static_cast<uint32_t>(yes)), "n"(kPairEpiWarps * 32) : "memory");
+  return any != 0;
+}
+
 template <int TN, int kSplits>
 __global__ void __launch_bounds__(kPairThreads, 1)
 WgradPairKernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
@@ -112,7 +127,7 @@ WgradPairKernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
     }
     for (int b = 0; b < 2; b++) {
       MbarInit(&sh.acc_full[b], 1);
-      MbarInit(&sh.acc_empty[b], 2 * kPairEpiWarps);  // of both CTAs
+      MbarInit(&sh.acc_empty[b], 2 * 4);  // four warps of both CTAs
     }
     sh.abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -189,24 +204,34 @@ WgradPairKernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
         }
       }
     } else {
-      uint32_t local_tile = 0, stores = 0;
-      for (int tile = first_tile; tile < num_tiles; tile += stride, local_tile++) {
-        const int m0 = (tile / tiles_n) * 256 + static_cast<int>(side) * 128 + quarter * 32;
-        const int n0 = (tile % tiles_n) * TN;
+      const int last = first_tile + (num_tiles - 1 - first_tile) / stride * stride;
+      const int m = static_cast<int>(side) * 128 + quarter * 32;
+      uint32_t local_tile = 0;
+      bool ok = half == 0;
+      for (int tile = first_tile; tile < last && ok; tile += stride, local_tile++) {
         const int acc = local_tile & 1;
-        if (!MbarWait(&sh.acc_full[acc], (local_tile >> 1) & 1, &sh.abort)) break;
+        ok = MbarWait(&sh.acc_full[acc], (local_tile >> 1) & 1, &sh.abort);
+        if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        for (int g = half * (kGroups / 2); g < (half + 1) * (kGroups / 2); g++, stores++) {
+        for (int g = 0; g < kGroups; g++) {
           // The buffer is free once the store that used it last has read it.
-          if (stores >= kPairBufs) {
-            if (lane == 0) asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(kPairBufs - 1) : "memory");
-            __syncwarp();
-          }
-          StoreBox32(lanes + acc * TN + g * kEpiCols, sh.epi[e][stores % kPairBufs], lane, &map_d, n0 + g * kEpiCols, m0);
+          if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+          __syncwarp();
+          StoreBox32(lanes + acc * TN + g * kEpiCols, sh.epi[e], lane, &map_d, (tile % tiles_n) * TN + g * kEpiCols, (tile / tiles_n) * 256 + m);
         }
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncwarp();
         if (lane == 0) MbarArriveOn(&sh.acc_empty[acc], leader_rank);
+      }
+      // Once the last accumulator is full every load has landed and every MMA has read the stages.
+      local_tile = static_cast<uint32_t>((last - first_tile) / stride);
+      const int acc = local_tile & 1;
+      if (ok) ok = MbarWait(&sh.acc_full[acc], (local_tile >> 1) & 1, &sh.abort);
+      if (EpilogueAny(ok)) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        for (int g = half * (kGroups / 2); g < (half + 1) * (kGroups / 2); g++)
+          StoreBox32(lanes + acc * TN + g * kEpiCols, &sh.stage[0][0] + (g * 4 + quarter) * (32 * 128), lane, &map_d,
+                     (last % tiles_n) * TN + g * kEpiCols, (last / tiles_n) * 256 + m);
       }
     }
   }
@@ -214,21 +239,16 @@ WgradPairKernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
   if (kSplit) {
     ClusterSync();  // every pair's partial sums are in place
     if (warp >= 4 && !sh.abort) {
-      const int e = warp - 4, quarter = warp & 3, half = e >> 2;
+      const int quarter = warp & 3, half = (warp - 4) >> 2;
       const int m0 = (first_tile / tiles_n) * 256 + static_cast<int>(side) * 128 + quarter * 32;
       const int n0 = (first_tile % tiles_n) * TN;
       constexpr int mine = kGroups / kSplits;
-      uint32_t stores = 0;
-      for (int i = half; i < mine; i += 2, stores++) {
+      for (int i = half; i < mine; i += 2) {
         const int g = share * mine + i;
-        if (stores >= kPairBufs) {
-          if (lane == 0) asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(kPairBufs - 1) : "memory");
-          __syncwarp();
-        }
         // Box by box at the same offset in every CTA, so that a warp reads 512 bytes in a row; row by
         // row, as the accumulator is held, other CTAs' memory gave 6 bytes per ns.
-        const uint32_t box = SmemAddr(&sh.stage[0][0]) + (g * 4 + quarter) * (32 * 128) + lane * 16;
-        uint8_t* buf = sh.epi[e][stores % kPairBufs];
+        uint8_t* buf = &sh.stage[0][0] + (g * 4 + quarter) * (32 * 128);  // only this warp reads this pair's own
+        const uint32_t box = SmemAddr(buf) + lane * 16;
         float4 x[kSplits][8];  // all loads before the first sum: each takes about a microsecond
 #pragma unroll
         for (int p = 0; p < kSplits; p++) {

@@ -61,6 +61,7 @@ def wgrad_gemm(dy, x, out=None, error_flag=None, two_cta=None):
     `two_cta`: use the kernel in which two CTAs share a tile (tcgen05 cta_group::2); default: by
     size (switchml_wgrad_gemm_auto)."""
     assert dy.is_cuda and x.is_cuda and dy.dtype == torch.bfloat16 and x.dtype == torch.bfloat16
+    assert dy.dim() == 2 and x.dim() == 2
     K, M = dy.shape
     rows, N = x.shape
     assert rows == K

@@ -187,6 +187,20 @@ def test_wgrad_pairs_of_ctas_with_every_split(K, M, N):
     assert torch.equal(wgrad_gemm(dy, x, two_cta=True), out)
 
 
+@pytest.mark.parametrize("K,M,N", [(200, 5000, 9000), (64, 304, 20000), (1000, 8000, 4104)])
+def test_wgrad_pairs_with_many_tiles(K, M, N):
+    """More tiles than pairs of CTAs, whose epilogues run beside the next tile's multiplications but for the last."""
+    from switchml_b200.ops.wgrad import wgrad_gemm
+    gen = torch.Generator(device="cuda").manual_seed(K + N)
+    dy = torch.randn(K, M, device="cuda", generator=gen).bfloat16()
+    x = torch.randn(K, N, device="cuda", generator=gen).bfloat16()
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    out = wgrad_gemm(dy, x, error_flag=err, two_cta=True)
+    assert int(err) == 0
+    assert torch.allclose(out, dy.float().t() @ x.float(), rtol=1e-4, atol=2e-4 * K ** 0.5)
+    assert torch.equal(wgrad_gemm(dy, x, two_cta=True), out)
+
+
 @pytest.mark.parametrize("K,M", [(1, 8), (3, 72), (255, 64), (256, 128), (257, 520), (4097, 1000), (8192, 4096)])
 def test_column_sums(K, M):
     """Clusters of one to eight CTAs, ragged rows and columns; the same bits twice."""

@@ -13,9 +13,11 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
-#include <cstring>
-
+#include "kernels/dependent_launch.cuh"
 #include "kernels/wgrad_gemm.h"
+
+using switchml::kernels::LaunchOverlapped;
+using switchml::kernels::WaitForEarlierKernels;
 
 namespace {
 
@@ -46,6 +48,7 @@ __device__ __forceinline__ void CastTile(const float* in, __nv_bfloat16* out, si
 
 __global__ void __launch_bounds__(kCastThreads)
 CastWeightsKernel(const float* w, __nv_bfloat16* w_low, size_t n, unsigned w_tiles, const float* b, __nv_bfloat16* b_low, size_t nb) {
+  WaitForEarlierKernels();
   if (blockIdx.x < w_tiles) CastTile(w, w_low, n, blockIdx.x);
   else CastTile(b, b_low, nb, blockIdx.x - w_tiles);
 }
@@ -67,6 +70,7 @@ __global__ void __launch_bounds__(kSumThreads) ColumnSumKernel(const __nv_bfloat
   const int col = col0 + lane * 8;  // M is a multiple of 8: a thread's columns exist all or none
   const int k0 = static_cast<int>(static_cast<long long>(K) * rank / ranks), k1 = static_cast<int>(static_cast<long long>(K) * (rank + 1) / ranks);
   float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  WaitForEarlierKernels();
   if (col < M) {
     const __nv_bfloat16* p = in + col;
     for (int k = k0 + row; k < k1; k += kSumRows * kSumUnroll) {
@@ -74,7 +78,7 @@ __global__ void __launch_bounds__(kSumThreads) ColumnSumKernel(const __nv_bfloat
 #pragma unroll
       for (int u = 0; u < kSumUnroll; u++) {
         const int r = k + u * kSumRows;
-        v[u] = r < k1 ? __ldg(reinterpret_cast<const uint4*>(p + static_cast<size_t>(r) * M)) : make_uint4(0, 0, 0, 0);
+        v[u] = r < k1 ? *reinterpret_cast<const uint4*>(p + static_cast<size_t>(r) * M) : make_uint4(0, 0, 0, 0);
       }
 #pragma unroll
       for (int u = 0; u < kSumUnroll; u++) {
@@ -124,9 +128,10 @@ extern "C" int switchml_cast_weights(const float* w, void* w_low, unsigned long 
   if (!w || !w_low || n == 0 || (nb && (!b || !b_low))) return -1;
   const unsigned long long w_tiles = (n + kCastTile - 1) / kCastTile, b_tiles = (nb + kCastTile - 1) / kCastTile;
   if (w_tiles + b_tiles > 0x7fffffffull) return -1;
-  CastWeightsKernel<<<static_cast<unsigned>(w_tiles + b_tiles), kCastThreads, 0, static_cast<cudaStream_t>(stream)>>>(
-      w, static_cast<__nv_bfloat16*>(w_low), n, static_cast<unsigned>(w_tiles), b, static_cast<__nv_bfloat16*>(b_low), nb);
-  return cudaGetLastError() == cudaSuccess ? 0 : -4;
+  const cudaError_t e = LaunchOverlapped(CastWeightsKernel, static_cast<unsigned>(w_tiles + b_tiles), kCastThreads, 0, 1,
+                                         static_cast<cudaStream_t>(stream), w, static_cast<__nv_bfloat16*>(w_low), n,
+                                         static_cast<unsigned>(w_tiles), b, static_cast<__nv_bfloat16*>(b_low), nb);
+  return e == cudaSuccess ? 0 : -4;
 }
 
 extern "C" int switchml_column_sums(const void* dy, float* out, int K, int M, void* stream) {
@@ -135,16 +140,8 @@ extern "C" int switchml_column_sums(const void* dy, float* out, int K, int M, vo
   // A CTA gets at least one turn of its unrolled loop (256 rows).
   int ctas = 1;
   while (ctas < 8 && K >= 2 * ctas * kSumRows * kSumUnroll) ctas <<= 1;
-  cudaLaunchConfig_t cfg;
-  memset(&cfg, 0, sizeof(cfg));
-  cudaLaunchAttribute attr;
-  attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = ctas;
-  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-  cfg.gridDim = dim3(static_cast<unsigned>((M + kSumCols - 1) / kSumCols * ctas));
-  cfg.blockDim = dim3(kSumThreads);
-  cfg.stream = static_cast<cudaStream_t>(stream);
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, ColumnSumKernel, static_cast<const __nv_bfloat16*>(dy), out, K, M) == cudaSuccess ? 0 : -4;
+  const unsigned blocks = static_cast<unsigned>((M + kSumCols - 1) / kSumCols * ctas);
+  const cudaError_t e = LaunchOverlapped(ColumnSumKernel, blocks, kSumThreads, 0, ctas, static_cast<cudaStream_t>(stream),
+                                         static_cast<const __nv_bfloat16*>(dy), out, K, M);
+  return e == cudaSuccess ? 0 : -4;
 }

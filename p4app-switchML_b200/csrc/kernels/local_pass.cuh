@@ -14,6 +14,7 @@
 #include <stdint.h>
 
 #include "kernels/allreduce_kernels.h"
+#include "kernels/dependent_launch.cuh"
 #include "switchml/quant_math.h"
 
 namespace switchml {
@@ -37,6 +38,8 @@ __host__ __device__ __forceinline__ size_t CopyHead(const char* out, size_t byte
 // before, 25 MB took 0.5 ms. `in` and `out` do not overlap unless they are equal.
 template <bool kShifted>
 __global__ void __launch_bounds__(kCopyThreads) LocalCopyKernel(const char* in, char* out, size_t bytes) {
+  WaitForEarlierKernels();
+  LetNextKernelStart();
   const size_t head = CopyHead(out, bytes);
   const size_t nvec = (bytes - head) / 16;
   const size_t first = static_cast<size_t>(blockIdx.x) * (kCopyThreads * kCopyUnroll) + threadIdx.x;
@@ -78,10 +81,8 @@ cudaError_t LaunchLocalCopyImpl(const void* in, void* out, size_t bytes, cudaStr
   const char* i = static_cast<const char*>(in);
   char* o = static_cast<char*>(out);
   if (((reinterpret_cast<uintptr_t>(in) ^ reinterpret_cast<uintptr_t>(out)) & 15) == 0)
-    LocalCopyKernel<false><<<static_cast<unsigned>(blocks), kCopyThreads, 0, stream>>>(i, o, bytes);
-  else
-    LocalCopyKernel<true><<<static_cast<unsigned>(blocks), kCopyThreads, 0, stream>>>(i, o, bytes);
-  return cudaGetLastError();
+    return LaunchOverlapped(LocalCopyKernel<false>, static_cast<unsigned>(blocks), kCopyThreads, 0, 1, stream, i, o, bytes);
+  return LaunchOverlapped(LocalCopyKernel<true>, static_cast<unsigned>(blocks), kCopyThreads, 0, 1, stream, i, o, bytes);
 }
 
 // ---- exact mode ------------------------------------------------------------------------
@@ -227,6 +228,8 @@ __device__ __forceinline__ bool LocalQuantChunk(const char* in, char* out, int l
 template <int ELEM, int VB>
 __global__ void __launch_bounds__(kQuantThreads)
 LocalQuantKernel(const char* in, char* out, size_t numel, int log2_block, float base) {
+  WaitForEarlierKernels();
+  LetNextKernelStart();
   constexpr int kEsz = ELEM == ELEM_BF16 ? 2 : 4;
   const int lane = threadIdx.x & 31;
   const size_t c = (static_cast<size_t>(blockIdx.x) * kQuantThreads + threadIdx.x) >> 5;
@@ -250,13 +253,13 @@ cudaError_t LaunchLocalQuantElem(const void* in, void* out, size_t numel, int lo
   const unsigned blocks = static_cast<unsigned>((numel + per_block - 1) / per_block);
   const char* i = static_cast<const char*>(in);
   char* o = static_cast<char*>(out);
-  if ((both & 15) == 0) LocalQuantKernel<ELEM, 16><<<blocks, kQuantThreads, 0, stream>>>(i, o, numel, log2_block, base);
-  else if ((both & 7) == 0) LocalQuantKernel<ELEM, 8><<<blocks, kQuantThreads, 0, stream>>>(i, o, numel, log2_block, base);
-  else if ((both & 3) == 0) LocalQuantKernel<ELEM, 4><<<blocks, kQuantThreads, 0, stream>>>(i, o, numel, log2_block, base);
-  else if (ELEM == ELEM_BF16 && (both & 1) == 0)
-    LocalQuantKernel<ELEM_BF16, 2><<<blocks, kQuantThreads, 0, stream>>>(i, o, numel, log2_block, base);
+  void (*kernel)(const char*, char*, size_t, int, float) = nullptr;
+  if ((both & 15) == 0) kernel = LocalQuantKernel<ELEM, 16>;
+  else if ((both & 7) == 0) kernel = LocalQuantKernel<ELEM, 8>;
+  else if ((both & 3) == 0) kernel = LocalQuantKernel<ELEM, 4>;
+  else if (ELEM == ELEM_BF16 && (both & 1) == 0) kernel = LocalQuantKernel<ELEM_BF16, 2>;
   else return cudaErrorInvalidValue;
-  return cudaGetLastError();
+  return LaunchOverlapped(kernel, blocks, kQuantThreads, 0, 1, stream, i, o, numel, log2_block, base);
 }
 
 }  // namespace

@@ -39,7 +39,12 @@
 #include <cstring>
 #include <mutex>
 
+#include "kernels/dependent_launch.cuh"
 #include "kernels/wgrad_gemm.h"
+
+using switchml::kernels::LaunchOverlapped;
+using switchml::kernels::LetNextKernelStart;
+using switchml::kernels::WaitForEarlierKernels;
 
 namespace {
 
@@ -631,14 +636,13 @@ static int LaunchWide(const void* dy, const void* x, float* dw, int M, int N, in
   static std::atomic<unsigned long long> allowed_store{0}, allowed_load{0};
   if (K <= 4 * kTileK) {
     AllowSmem(reinterpret_cast<const void*>(WgradWideKernel<3, 2>), sizeof(WideShared<3, 2>) + 1024, &allowed_store);
-    WgradWideKernel<3, 2><<<static_cast<unsigned>(tiles), kWideThreads, sizeof(WideShared<3, 2>) + 1024, stream>>>(
-        map_a, map_b, map_d, tiles_n, K, error_flag);
+    return LaunchOverlapped(WgradWideKernel<3, 2>, static_cast<unsigned>(tiles), kWideThreads, sizeof(WideShared<3, 2>) + 1024, 1,
+                            stream, map_a, map_b, map_d, tiles_n, K, error_flag) == cudaSuccess ? 0 : -4;
   } else {
     AllowSmem(reinterpret_cast<const void*>(WgradWideKernel<4, 1>), sizeof(WideShared<4, 1>) + 1024, &allowed_load);
-    WgradWideKernel<4, 1><<<static_cast<unsigned>(tiles), kWideThreads, sizeof(WideShared<4, 1>) + 1024, stream>>>(
-        map_a, map_b, map_d, tiles_n, K, error_flag);
+    return LaunchOverlapped(WgradWideKernel<4, 1>, static_cast<unsigned>(tiles), kWideThreads, sizeof(WideShared<4, 1>) + 1024, 1,
+                            stream, map_a, map_b, map_d, tiles_n, K, error_flag) == cudaSuccess ? 0 : -4;
   }
-  return cudaGetLastError() == cudaSuccess ? 0 : -4;
 }
 
 extern "C" int switchml_wgrad_gemm(const void* dy, const void* x, float* dw, int M, int N, int K,
@@ -714,19 +718,8 @@ cudaError_t LaunchPairs(const CUtensorMap& map_a, const CUtensorMap& map_b, cons
   const size_t smem = sizeof(PairShared<TN>) + 1024;
   static std::atomic<unsigned long long> allowed{0};
   AllowSmem(reinterpret_cast<const void*>(WgradPairKernel<TN, kSplits>), smem, &allowed);
-  cudaLaunchConfig_t cfg;
-  memset(&cfg, 0, sizeof(cfg));
-  cudaLaunchAttribute attr;
-  attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = 2 * kSplits;
-  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-  cfg.gridDim = dim3(static_cast<unsigned>(plan.clusters) * 2 * kSplits);
-  cfg.blockDim = dim3(kPairThreads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = stream;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, WgradPairKernel<TN, kSplits>, map_a, map_b, map_d, M, N, K, error_flag);
+  return LaunchOverlapped(WgradPairKernel<TN, kSplits>, static_cast<unsigned>(plan.clusters) * 2 * kSplits, kPairThreads, smem,
+                          2 * kSplits, stream, map_a, map_b, map_d, M, N, K, error_flag);
 }
 
 // The plan with the least estimated time. A k-block costs about the same with either tile width (both

@@ -142,6 +142,7 @@ WgradPairKernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
   ClusterSync();  // both CTAs' barriers exist before anybody signals across the pair
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_base = sh.tmem_base;
+  WaitForEarlierKernels();
 
   if (warp == 0) {
     if (lane == 0) {
@@ -195,6 +196,7 @@ WgradPairKernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
     if (kSplit) {
       // This pair's partial sums into shared memory, box by box as a TMA store would want them.
       if (MbarWait(&sh.acc_full[0], 0, &sh.abort)) {
+        LetNextKernelStart();
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         for (int g = half * (kGroups / 2); g < (half + 1) * (kGroups / 2); g++) {
           uint32_t v[32];
@@ -228,6 +230,7 @@ WgradPairKernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
       const int acc = local_tile & 1;
       if (ok) ok = MbarWait(&sh.acc_full[acc], (local_tile >> 1) & 1, &sh.abort);
       if (EpilogueAny(ok)) {
+        LetNextKernelStart();
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         for (int g = half * (kGroups / 2); g < (half + 1) * (kGroups / 2); g++)
           StoreBox32(lanes + acc * TN + g * kEpiCols, &sh.stage[0][0] + (g * 4 + quarter) * (32 * 128), lane, &map_d,

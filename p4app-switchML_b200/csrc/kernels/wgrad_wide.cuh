@@ -56,6 +56,7 @@ WgradWideKernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_base = sh.tmem_base;
+  WaitForEarlierKernels();
 
   if (warp == 0) {
     uint32_t it = 0;

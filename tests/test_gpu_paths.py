@@ -267,3 +267,51 @@ def test_one_worker_exact_pass_of_odd_values(ctx, dtype):
         ctx.all_reduce(d)
         bits = torch.int32 if dtype == torch.float32 else torch.int16
         assert torch.equal(d.cpu().view(bits), want.view(bits)), offset
+
+
+@pytest.mark.parametrize("K,M,N", [(16, 64, 64), (64, 1000, 2056), (2048, 512, 512), (1024, 2048, 4096)])
+def test_kernels_launched_early_keep_the_order_of_the_stream(ctx, K, M, N):
+    """Each kernel reads what the one before it wrote, and writes what the one before that read; also with an
+    ordinary kernel between, on a stream of its own and out of a graph."""
+    from switchml_b200.ops.wgrad import column_sums, wgrad_gemm
+    assert ctx.start(sml.make_config("cuda", mode="float_sum", launch="inline"))
+    gen = torch.Generator(device="cuda").manual_seed(K)
+    source = torch.randint(-2, 3, (6, K, M), device="cuda", generator=gen).bfloat16()
+    x = torch.randint(-2, 3, (K, N), device="cuda", generator=gen).bfloat16()
+    a, b = torch.empty_like(source[0]), torch.empty_like(source[0])
+    dw, kept = torch.empty(M, N, device="cuda"), torch.empty(6, M, N, device="cuda")
+    sums = []
+
+    def walk(i):
+        j = [ctx.all_reduce_async(source[i].view(-1), a.view(-1)), ctx.all_reduce_async(a.view(-1), b.view(-1))]
+        wgrad_gemm(b, x, out=dw)
+        j.append(ctx.all_reduce_async(dw.view(-1), kept[i].view(-1)))
+        sums.append(column_sums(b))
+        if i % 2:
+            b.zero_()
+        return j
+
+    stream = torch.cuda.Stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(stream):
+        jobs = [j for i in range(6) for j in walk(i)]
+    stream.synchronize()
+    for j in jobs:
+        assert j.wait() == sml.JobStatus.FINISHED
+        j.release()
+    for i in range(6):  # whole numbers: exact in any order
+        assert torch.equal(kept[i], source[i].float().t() @ x.float()), i
+        assert torch.equal(sums[i], source[i].float().sum(0)), i
+
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        wgrad_gemm(a, x, out=dw)
+        kept[0].copy_(dw)
+        wgrad_gemm(b, x, out=dw)
+        wgrad_gemm(a, x, out=kept[1])
+    for i in (2, 4):
+        a.copy_(source[i])
+        b.copy_(source[i + 1])
+        graph.replay()
+        for out, d in ((kept[0], a), (kept[1], a), (dw, b)):
+            assert torch.equal(out, d.float().t() @ x.float())

@@ -97,6 +97,14 @@ struct EventState : public DeviceJobState {
   void StreamWait(void* other) override {
     if (!SameStream(stream, static_cast<cudaStream_t>(other))) cudaStreamWaitEvent(static_cast<cudaStream_t>(other), done, 0);
   }
+  // Whether work on `other` that is enqueued from now on comes after the job without waiting for it.
+  bool BehindWithoutWaiting(cudaStream_t other) {
+    if (SameStream(stream, other)) return true;
+    RelaxedCapture relaxed;
+    const cudaError_t e = cudaEventQuery(done);
+    if (e != cudaSuccess) cudaGetLastError();
+    return e == cudaSuccess;
+  }
   void HelpComplete(Job& job, double milliseconds) override {
     const auto start = std::chrono::steady_clock::now();
     RelaxedCapture relaxed;
@@ -128,13 +136,15 @@ struct InFlight {
   int status_slot = -1;  // -1: the job's kernel reports no status
   unsigned long long tiles = 0;
   std::string launch_error;
+  // Whether input and output are ordinary device memory, once CheckOperands has looked.
+  bool checked = false, in_device = true, out_device = true;
 };
 
 static const int kStatusSlots = 4096;
 // launch = worker: with this many jobs in flight the launcher thread takes over, which may wait for
 // room in the stream's queue (about a thousand launches) while the callers go on.
 static const size_t kDirectLaunches = 256;
-static const uint64_t kBriefBytes = 1 << 20;  // read + write at 6 TB/s: 0.4 us
+static const uint64_t kBriefBytes = 1 << 20;  // read + write at 6 TB/s: 0.4 us (device memory only: over PCIe it is 40 us)
 
 // One NVTX range per job for timeline tools; without one the name is not even put together.
 struct NvtxRange {
@@ -201,6 +211,8 @@ class CudaBackend : public CudaBackendInterface {
   void LaunchJob(const std::shared_ptr<Job>& job, cudaStream_t stream, InFlight* f, bool capturing = false);
   // The same for a single worker, whose job is one pass over the tensor (or none).
   cudaError_t LaunchLocalJob(const Tensor& t, cudaStream_t stream, InFlight* f);
+  // Looks at the job's addresses, once: fills `f`, with the error if the GPU cannot reach them.
+  void CheckOperands(const Tensor& t, InFlight* f);
   // What follows the kernels (`e`: how their launch went): the job's event and its ordering hooks.
   void FinishLaunch(const std::shared_ptr<Job>& job, cudaStream_t stream, InFlight* f, cudaError_t e, bool capturing);
   cudaEvent_t GetEvent() { return events_->Get(); }
@@ -456,23 +468,26 @@ static const char* GpuCannotAccess(const void* p, bool* device) {
   return nullptr;
 }
 
+// The kernels dereference both pointers on the GPU: refuse anything the GPU cannot be
+// trusted to reach (ordinary malloc'ed host memory) instead of launching into a fault.
+// Device, managed and pinned (cudaHostAlloc / cudaHostRegister) memory pass.
+void CudaBackend::CheckOperands(const Tensor& t, InFlight* f) {
+  if (f->checked) return;
+  f->checked = true;
+  if (t.numel == 0) return;
+  const char* why = GpuCannotAccess(t.in_ptr, &f->in_device);
+  f->out_device = f->in_device;
+  if (!why && t.out_ptr != t.in_ptr) why = GpuCannotAccess(t.out_ptr, &f->out_device);
+  if (why) f->launch_error = std::string("backend = cuda needs device, managed or pinned memory: ") + why;
+}
+
 void CudaBackend::LaunchJob(const std::shared_ptr<Job>& job, cudaStream_t stream, InFlight* f, bool capturing) {
   const CudaBackendConfig& c = config_.backend_.cuda;
   Tensor t = job->tensor_;
   const Tensor& user = job->tensor_;
-  // The kernels dereference both pointers on the GPU: refuse anything the GPU cannot be
-  // trusted to reach (ordinary malloc'ed host memory) instead of launching into a fault.
-  // Device, managed and pinned (cudaHostAlloc / cudaHostRegister) memory pass.
-  bool in_device = true, out_device = true;
-  if (t.numel > 0) {
-    const char* why = GpuCannotAccess(t.in_ptr, &in_device);
-    out_device = in_device;
-    if (!why && t.out_ptr != t.in_ptr) why = GpuCannotAccess(t.out_ptr, &out_device);
-    if (why) {
-      f->launch_error = std::string("backend = cuda needs device, managed or pinned memory: ") + why;
-      return;
-    }
-  }
+  CheckOperands(t, f);
+  if (!f->launch_error.empty()) return;
+  bool in_device = f->in_device, out_device = f->out_device;
   NvtxRange range(*job, user);
   if (n_ == 1) {
     FinishLaunch(job, stream, f, LaunchLocalJob(t, stream, f), capturing);
@@ -661,49 +676,45 @@ bool CudaBackend::OnSubmit(const std::shared_ptr<Job>& job) {
     cudaGetLastError();
   }
   const bool capturing = capture == cudaStreamCaptureStatusActive;
-  // launch = worker: a single worker's short pass takes less than handing over from the producer's stream to
-  // the backend's and back (two events and the GPU's wait for them), so it runs where its input was made.
-  const bool brief = n_ == 1 && job->tensor_.numel * DataTypeSize(job->tensor_.data_type) <= kBriefBytes;
-  if (!inline_launch_ && (capturing || !brief)) {
-    // Where the producer stream is now: the job comes after it.
-    f.ready = GetEvent();
-    cudaEventRecord(f.ready, user_stream);
-    std::lock_guard<std::mutex> lk(launch_mu_);
-    if (capturing || queued_jobs_ > 0 || InFlightCount() >= kDirectLaunches) {
-      queued_jobs_++;
-      job->ready_event_ = f.ready;
-      return false;  // goes through the scheduler, so that the caller does not wait for the stream's queue
-    }
-    // Nobody is ahead of this job: enqueueing it here costs less than waking the launcher thread
-    // (a blocking allreduce of 64 Ki elements took 38 us with the hand-over).
-    job->SetJobStatus(QUEUED);
-    job->SetJobStatus(RUNNING);
-    cudaStreamWaitEvent(comm_stream_, f.ready, 0);
-    if (last_job_) last_job_->StreamWait(comm_stream_);
-    LaunchJob(job, comm_stream_, &f);
-    PushInFlight(std::move(f));
-    return true;
-  }
-  if (InFlightCount() > kStatusSlots / 4) {  // a status word must have been read before its slot comes round again
+  if (inline_launch_ && InFlightCount() > kStatusSlots / 4) {  // a status word must have been read before its slot comes round again
     std::lock_guard<std::mutex> lk(completions_->mu);
     Reap();
   }
+  // launch = worker: a single worker's short pass takes less than handing over from the producer's stream to
+  // the backend's and back (two events and the GPU's wait for them), so it may run where its input was made.
+  bool brief = false;
+  if (!inline_launch_ && !capturing && n_ == 1 && job->tensor_.numel * DataTypeSize(job->tensor_.data_type) <= kBriefBytes) {
+    CheckOperands(job->tensor_, &f);
+    brief = f.in_device && f.out_device;
+  }
   {
     std::lock_guard<std::mutex> lk(launch_mu_);
-    if (!inline_launch_ && (queued_jobs_ > 0 || InFlightCount() >= kDirectLaunches)) {
-      f.ready = GetEvent();
-      cudaEventRecord(f.ready, user_stream);
-      job->ready_event_ = f.ready;
-      queued_jobs_++;
-      return false;  // in line behind the jobs that the launcher thread has not enqueued yet
+    cudaStream_t stream = user_stream;
+    if (!inline_launch_) {
+      const bool queue = capturing || queued_jobs_ > 0 || InFlightCount() >= kDirectLaunches;
+      // The producer's stream must not wait for a job before this one: whoever computes there has not asked for that.
+      if (queue || !brief || (last_job_ && !last_job_->BehindWithoutWaiting(user_stream))) {
+        // Where the producer stream is now: the job comes after it.
+        f.ready = GetEvent();
+        cudaEventRecord(f.ready, user_stream);
+        if (queue) {
+          queued_jobs_++;
+          job->ready_event_ = f.ready;
+          return false;  // goes through the scheduler, so that the caller does not wait for the stream's queue
+        }
+        // Nobody is ahead of this job: enqueueing it here costs less than waking the launcher thread
+        // (a blocking allreduce of 64 Ki elements took 38 us with the hand-over).
+        stream = comm_stream_;
+        cudaStreamWaitEvent(stream, f.ready, 0);
+      }
     }
     job->SetJobStatus(QUEUED);
     job->SetJobStatus(RUNNING);
     // Not while capturing: an event recorded outside the capture cannot be waited on inside
     // it. A captured job is ordered by the graph it becomes part of; whoever replays that
     // graph next to other jobs of this context orders the two.
-    if (!capturing && last_job_) last_job_->StreamWait(user_stream);
-    LaunchJob(job, user_stream, &f, capturing);
+    if (!capturing && last_job_) last_job_->StreamWait(stream);
+    LaunchJob(job, stream, &f, capturing);
     if (!capturing) PushInFlight(std::move(f));
   }
   if (capturing) {

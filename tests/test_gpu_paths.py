@@ -132,6 +132,24 @@ def test_many_jobs_from_several_threads_and_streams(ctx, launch):
     assert st["jobs_finished"] == 1600 and st["jobs_failed"] == 0
 
 
+def test_a_brief_job_does_not_hold_up_its_producer(ctx):
+    """launch = worker: jobs run beside what the producer's stream does. A short job behind long ones comes after
+    them, but the stream that it was submitted on does not."""
+    assert ctx.start(sml.make_config("cuda", mode="float_sum", launch="worker"))
+    x = torch.ones(1 << 28, device="cuda")
+    y, z = torch.zeros_like(x), torch.zeros(1000, device="cuda")
+    ctx.all_reduce(z, torch.empty_like(z))  # the first launch of a kernel loads it
+    torch.cuda.synchronize()
+    long_jobs = [ctx.all_reduce_async(x, y) for _ in range(20)]  # some 300 us each
+    brief = ctx.all_reduce_async(y[:1000], z)
+    here = torch.cuda.Event()
+    here.record()
+    here.synchronize()
+    assert long_jobs[-1].status() != sml.JobStatus.FINISHED
+    assert brief.wait() == sml.JobStatus.FINISHED and bool((z == 1).all())
+    assert [j.wait() for j in long_jobs] == [sml.JobStatus.FINISHED] * 20
+
+
 @pytest.mark.parametrize("mode", ["float_sum", "int32_quant"])
 @pytest.mark.parametrize("numel,chunk", [(1, 1 << 24), (3, 2), ((1 << 18) + 1, 1 << 24), ((1 << 20) + 77, 1 << 18),
                                          (5_000_003, 1 << 24)])

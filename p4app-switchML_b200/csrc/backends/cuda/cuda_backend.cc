@@ -82,24 +82,40 @@ struct RelaxedCapture {
   ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
 };
 
-// Two work items on the same stream are in order by themselves. The handle of the per-thread
-// default stream names another stream in every thread.
-inline bool SameStream(cudaStream_t a, cudaStream_t b) { return a == b && a != cudaStreamPerThread; }
+// What tells a stream from every other one of the process's life. Handles do not: that of a destroyed stream may
+// come back as another one's, and those of the default streams stand for another stream on every device (or in
+// every thread).
+struct StreamIdentity {
+  unsigned long long id = 0;
+  int device = -1;  // current when the stream was looked at; -1: there is no telling
+  StreamIdentity() {}
+  explicit StreamIdentity(cudaStream_t s) {
+    if (cudaStreamGetId(s, &id) != cudaSuccess || cudaGetDevice(&device) != cudaSuccess) {
+      cudaGetLastError();
+      device = -1;
+    }
+  }
+  bool Is(const StreamIdentity& o) const { return device >= 0 && device == o.device && id == o.id; }
+};
 
 struct EventState : public DeviceJobState {
   cudaEvent_t done = nullptr;
-  cudaStream_t stream = nullptr;  // where the job runs
+  StreamIdentity stream;  // where the job runs
   std::shared_ptr<EventPool> pool;
   std::shared_ptr<Completions> completions;
   ~EventState() override {
     if (pool) pool->Put(done);
   }
   void StreamWait(void* other) override {
-    if (!SameStream(stream, static_cast<cudaStream_t>(other))) cudaStreamWaitEvent(static_cast<cudaStream_t>(other), done, 0);
+    OrderAfter(static_cast<cudaStream_t>(other), StreamIdentity(static_cast<cudaStream_t>(other)));
   }
-  // Whether work on `other` that is enqueued from now on comes after the job without waiting for it.
-  bool BehindWithoutWaiting(cudaStream_t other) {
-    if (SameStream(stream, other)) return true;
+  // Two work items on the same stream are in order by themselves.
+  void OrderAfter(cudaStream_t other, const StreamIdentity& id) {
+    if (!stream.Is(id)) cudaStreamWaitEvent(other, done, 0);
+  }
+  // Whether work on the stream `other` that is enqueued from now on comes after the job without waiting for it.
+  bool BehindWithoutWaiting(const StreamIdentity& other) {
+    if (stream.Is(other)) return true;
     RelaxedCapture relaxed;
     const cudaError_t e = cudaEventQuery(done);
     if (e != cudaSuccess) cudaGetLastError();
@@ -128,6 +144,7 @@ struct EventState : public DeviceJobState {
 };
 
 struct InFlight {
+  StreamIdentity stream;  // where the job runs
   std::shared_ptr<Job> job;
   bool via_scheduler = false;
   JobSlice slice;
@@ -232,6 +249,7 @@ class CudaBackend : public CudaBackendInterface {
   kernels::RankCtx ctx_;
   int max_channels_ = 1;
   cudaStream_t comm_stream_ = nullptr;
+  StreamIdentity comm_identity_;
   int* dev_status_ = nullptr;
   unsigned long long* dev_counters_ = nullptr;
   unsigned long long* dev_trace_ = nullptr;  // kTraceWords, only with [backend.cuda] trace
@@ -358,6 +376,7 @@ void CudaBackend::SetupWorker() {
   int lo = 0, hi = 0;
   cudaDeviceGetStreamPriorityRange(&lo, &hi);
   SML_CUDA_CHECK(cudaStreamCreateWithPriority(&comm_stream_, cudaStreamNonBlocking, hi));
+  comm_identity_ = StreamIdentity(comm_stream_);
   last_job_.reset();
   queued_jobs_ = 0;
   SML_CUDA_CHECK(cudaMalloc(&dev_counters_, 16 * sizeof(unsigned long long)));
@@ -646,7 +665,7 @@ void CudaBackend::FinishLaunch(const std::shared_ptr<Job>& job, cudaStream_t str
   if (f->done) {
     auto st = std::make_shared<EventState>();
     st->done = f->done;
-    st->stream = stream;
+    st->stream = f->stream;
     st->pool = events_;
     st->completions = completions_;
     last_job_ = st;
@@ -687,13 +706,14 @@ bool CudaBackend::OnSubmit(const std::shared_ptr<Job>& job) {
     CheckOperands(job->tensor_, &f);
     brief = f.in_device && f.out_device;
   }
+  if (!capturing) f.stream = StreamIdentity(user_stream);
   {
     std::lock_guard<std::mutex> lk(launch_mu_);
     cudaStream_t stream = user_stream;
     if (!inline_launch_) {
       const bool queue = capturing || queued_jobs_ > 0 || InFlightCount() >= kDirectLaunches;
       // The producer's stream must not wait for a job before this one: whoever computes there has not asked for that.
-      if (queue || !brief || (last_job_ && !last_job_->BehindWithoutWaiting(user_stream))) {
+      if (queue || !brief || (last_job_ && !last_job_->BehindWithoutWaiting(f.stream))) {
         // Where the producer stream is now: the job comes after it.
         f.ready = GetEvent();
         cudaEventRecord(f.ready, user_stream);
@@ -705,6 +725,7 @@ bool CudaBackend::OnSubmit(const std::shared_ptr<Job>& job) {
         // Nobody is ahead of this job: enqueueing it here costs less than waking the launcher thread
         // (a blocking allreduce of 64 Ki elements took 38 us with the hand-over).
         stream = comm_stream_;
+        f.stream = comm_identity_;
         cudaStreamWaitEvent(stream, f.ready, 0);
       }
     }
@@ -713,7 +734,7 @@ bool CudaBackend::OnSubmit(const std::shared_ptr<Job>& job) {
     // Not while capturing: an event recorded outside the capture cannot be waited on inside
     // it. A captured job is ordered by the graph it becomes part of; whoever replays that
     // graph next to other jobs of this context orders the two.
-    if (!capturing && last_job_) last_job_->StreamWait(stream);
+    if (!capturing && last_job_) last_job_->OrderAfter(stream, f.stream);
     LaunchJob(job, stream, &f, capturing);
     if (!capturing) PushInFlight(std::move(f));
   }
@@ -756,7 +777,8 @@ void CudaBackend::LauncherLoop() {
     {
       std::lock_guard<std::mutex> lk(launch_mu_);
       if (f.ready) cudaStreamWaitEvent(comm_stream_, f.ready, 0);
-      if (last_job_) last_job_->StreamWait(comm_stream_);
+      f.stream = comm_identity_;
+      if (last_job_) last_job_->OrderAfter(comm_stream_, f.stream);
       LaunchJob(js.job, comm_stream_, &f);
       PushInFlight(std::move(f));
       queued_jobs_--;

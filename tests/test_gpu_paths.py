@@ -1,5 +1,6 @@
 """Edges of the kernels' dispatch and of the host path around them, each against the CPU oracle
 or a plain PyTorch reference of the same operation."""
+import ctypes
 import threading
 
 import numpy as np
@@ -148,6 +149,36 @@ def test_a_brief_job_does_not_hold_up_its_producer(ctx):
     assert long_jobs[-1].status() != sml.JobStatus.FINISHED
     assert brief.wait() == sml.JobStatus.FINISHED and bool((z == 1).all())
     assert [j.wait() for j in long_jobs] == [sml.JobStatus.FINISHED] * 20
+
+
+def test_a_stream_whose_handle_was_another_ones_waits(ctx):
+    """A stream that is made after the job's own one was destroyed, and may have got its handle, comes after the
+    job when it is told to."""
+    assert ctx.start(sml.make_config("cuda", mode="float_sum", launch="inline"))
+    cudart = torch.cuda.cudart()
+
+    def new_stream():
+        handle = ctypes.c_void_p()
+        assert int(cudart.cudaStreamCreate(ctypes.addressof(handle))) == 0
+        return handle.value
+
+    x = torch.ones(1 << 27, device="cuda")
+    y, z = torch.zeros_like(x), torch.zeros(1000, device="cuda")
+    torch.cuda.synchronize()
+    first, others = new_stream(), []
+    jobs = [ctx.all_reduce_async(x, y, stream=first) for _ in range(10)]
+    cudart.cudaStreamDestroy(first)
+    while len(others) < 64 and (not others or others[-1] != first):
+        others.append(new_stream())
+    jobs[-1].stream_wait(others[-1])
+    with torch.cuda.stream(torch.cuda.ExternalStream(others[-1])):
+        z.copy_(y[-1000:])
+    torch.cuda.synchronize()
+    assert bool((z == 1).all())
+    for j in jobs:
+        assert j.wait() == sml.JobStatus.FINISHED
+    for handle in others:
+        cudart.cudaStreamDestroy(handle)
 
 
 @pytest.mark.parametrize("mode", ["float_sum", "int32_quant"])

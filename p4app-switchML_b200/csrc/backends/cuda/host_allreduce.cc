@@ -26,6 +26,26 @@ struct ChunkEvent {
     if (e) cudaEventDestroy(e);
   }
 };
+
+// Nothing may be in flight on the caller's buffers when the call returns, whatever happened: also not when
+// AllReduceAsync throws because the context has been stopped.
+struct Submitted {
+  cudaStream_t in, comm, out;
+  std::vector<std::shared_ptr<Job>> jobs;
+  bool over = false;
+  cudaError_t Finish() {
+    if (over) return cudaSuccess;
+    over = true;
+    cudaError_t e = cudaSuccess;
+    for (const cudaStream_t s : {in, comm, out}) {
+      const cudaError_t this_one = cudaStreamSynchronize(s);
+      if (e == cudaSuccess) e = this_one;
+    }
+    for (auto& job : jobs) job->WaitToComplete();
+    return e;
+  }
+  ~Submitted() { Finish(); }
+};
 }  // namespace
 
 int HostPipelinedAllReduce(const void* host_in, void* host_out, void* device, uint64_t numel, DataType type,
@@ -36,7 +56,8 @@ int HostPipelinedAllReduce(const void* host_in, void* host_out, void* device, ui
   const cudaStream_t s_comm = ctx.GetConfig().general_.num_workers == 1 ? s_out : static_cast<cudaStream_t>(stream_comm);
   const size_t esz = DataTypeSize(type);
   ChunkEvent arrived;
-  std::vector<std::shared_ptr<Job>> jobs;
+  Submitted submitted{s_in, s_comm, s_out, {}};
+  std::vector<std::shared_ptr<Job>>& jobs = submitted.jobs;
   jobs.reserve(numel / chunk_numel + 1);
   cudaError_t e = arrived.e ? cudaSuccess : cudaErrorMemoryAllocation;
   for (uint64_t lo = 0; lo < numel && e == cudaSuccess; lo += chunk_numel) {
@@ -50,11 +71,9 @@ int HostPipelinedAllReduce(const void* host_in, void* host_out, void* device, ui
     if (!jobs.back()->StreamWait(s_out)) break;  // failed: reported below
     e = cudaMemcpyAsync(static_cast<char*>(host_out) + lo * esz, d, len * esz, cudaMemcpyDeviceToHost, s_out);
   }
-  // Nothing may be in flight on the caller's buffers when this returns, whatever happened.
-  const cudaError_t in = cudaStreamSynchronize(s_in), out = cudaStreamSynchronize(s_out);
-  if (e == cudaSuccess) e = in != cudaSuccess ? in : out;
+  const cudaError_t finished = submitted.Finish();
+  if (e == cudaSuccess) e = finished;
   for (auto& job : jobs) {
-    job->WaitToComplete();
     if (job->GetJobStatus() != FINISHED) {
       *error = job->failure_reason_;
       return -1;

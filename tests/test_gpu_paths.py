@@ -201,6 +201,19 @@ def test_host_pipeline_chunks(ctx, mode, numel, chunk):
     pipe.close()
 
 
+def test_host_pipeline_leaves_nothing_in_flight_when_it_fails(ctx):
+    """A call that ends with an error, here because the context was stopped, has ended on the GPU too."""
+    from switchml_b200.parallel.host_pipeline import HostAllReduce
+    assert ctx.start(sml.make_config("cuda", mode="float_sum", launch="inline"))
+    numel = 1 << 26
+    hx, hy = torch.ones(numel, pin_memory=True), torch.zeros(numel, pin_memory=True)
+    pipe = HostAllReduce(ctx, numel, torch.float32)
+    ctx.stop()
+    with pytest.raises(RuntimeError):
+        pipe.run(hx, hy)
+    assert pipe.s_in.query() and pipe.s_comm.query() and pipe.s_out.query()
+
+
 @pytest.mark.parametrize("K", [1, 15, 16, 63, 64, 65, 100, 128, 129])
 @pytest.mark.parametrize("M,N", [(8, 8), (128, 128), (136, 264), (1000, 520)])
 def test_wgrad_short_reductions(K, M, N):

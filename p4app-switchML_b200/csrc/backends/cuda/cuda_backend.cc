@@ -615,7 +615,7 @@ void CudaBackend::LaunchJob(const std::shared_ptr<Job>& job, cudaStream_t stream
   f->tiles = plan.tiles;
   // Replays of a captured launch share one status word that nobody waits on; a timeout in
   // a replay still shows up in the device counters.
-  f->status_slot = capturing ? kStatusSlots - 2 : static_cast<int>(launched_jobs_++ % (kStatusSlots - 2));
+  f->status_slot = capturing ? kStatusSlots - 2 : static_cast<int>(launched_jobs_ % (kStatusSlots - 2));
 
   cudaError_t e = cudaSuccess;
   host_status_[f->status_slot] = kernels::STATUS_OK;  // the ring is far longer than the queue
@@ -656,6 +656,7 @@ cudaError_t CudaBackend::LaunchLocalJob(const Tensor& t, cudaStream_t stream, In
 }
 
 void CudaBackend::FinishLaunch(const std::shared_ptr<Job>& job, cudaStream_t stream, InFlight* f, cudaError_t e, bool capturing) {
+  if (!capturing) launched_jobs_++;  // (its old value was the job's place in the ring of status words)
   f->done = capturing ? nullptr : GetEvent();
   if (e == cudaSuccess && f->done) e = cudaEventRecord(f->done, stream);
   if (e != cudaSuccess) {

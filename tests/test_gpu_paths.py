@@ -133,6 +133,17 @@ def test_many_jobs_from_several_threads_and_streams(ctx, launch):
     assert st["jobs_finished"] == 1600 and st["jobs_failed"] == 0
 
 
+@pytest.mark.parametrize("launch", ["worker", "inline"])
+def test_one_worker_counts_its_jobs(ctx, launch):
+    """Jobs with a kernel and without one (a sum of one term, in place)."""
+    assert ctx.start(sml.make_config("cuda", mode="float_sum", launch=launch))
+    x = torch.zeros(1000, device="cuda")
+    for out in (None, torch.empty_like(x), None):
+        ctx.all_reduce(x, out)
+    counted = ctx.get_stats()["backend"]
+    assert counted["jobs_launched"] == 3 and counted["kernel_launches"] == 1
+
+
 def test_a_brief_job_does_not_hold_up_its_producer(ctx):
     """launch = worker: jobs run beside what the producer's stream does. A short job behind long ones comes after
     them, but the stream that it was submitted on does not."""

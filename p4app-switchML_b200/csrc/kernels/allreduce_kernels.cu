@@ -39,6 +39,7 @@
 #include "kernels/device_sync.cuh"
 #include "kernels/local_pass.cuh"
 #include "kernels/multimem.cuh"
+#include "kernels/once_per_device.h"
 #include "kernels/quant_tile.cuh"
 #include "switchml/quant_math.h"
 
@@ -1315,17 +1316,15 @@ __global__ void WaitProbeKernel(const RankCtx ctx) {
   ChannelBarrier(ctx, kMaxChannels - 1, kNumPhases - 1, ~0ull, &s_failed, false);
 }
 
-// Lets `kernel` use `bytes` of dynamic shared memory on the current device: once per device (`done`: a bit
-// for each), not 0.6 us on every launch.
+// Lets `kernel` use `bytes` of dynamic shared memory on the current device: once per device, not 0.6 us on
+// every launch.
 cudaError_t AllowDynamicSmem(const void* kernel, size_t bytes, std::atomic<unsigned long long>* done) {
   if (bytes == 0) return cudaSuccess;
   int dev = 0;
   cudaGetDevice(&dev);
-  const unsigned long long bit = 1ull << (dev & 63);
-  if (done->load(std::memory_order_acquire) & bit) return cudaSuccess;
-  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
-  if (e == cudaSuccess) done->fetch_or(bit, std::memory_order_release);
-  return e;
+  return OncePerDevice(dev, done, [&] {
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
+  });
 }
 
 template <int ELEM, int MODE, int ALGO>

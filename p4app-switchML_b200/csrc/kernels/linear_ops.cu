@@ -21,6 +21,13 @@ using switchml::kernels::WaitForEarlierKernels;
 
 namespace {
 
+// As in wgrad_gemm.cu: a failed launch does not leave its error for the next caller of cudaGetLastError().
+int Launched(cudaError_t e) {
+  if (e == cudaSuccess) return 0;
+  cudaGetLastError();
+  return -4;
+}
+
 constexpr int kCastThreads = 256;
 constexpr int kCastVecs = 4;  // vectors of 4 elements per thread
 constexpr int kCastTile = kCastThreads * kCastVecs * 4;
@@ -131,7 +138,7 @@ extern "C" int switchml_cast_weights(const float* w, void* w_low, unsigned long 
   const cudaError_t e = LaunchOverlapped(CastWeightsKernel, static_cast<unsigned>(w_tiles + b_tiles), kCastThreads, 0, 1,
                                          static_cast<cudaStream_t>(stream), w, static_cast<__nv_bfloat16*>(w_low), n,
                                          static_cast<unsigned>(w_tiles), b, static_cast<__nv_bfloat16*>(b_low), nb);
-  return e == cudaSuccess ? 0 : -4;
+  return Launched(e);
 }
 
 extern "C" int switchml_column_sums(const void* dy, float* out, int K, int M, void* stream) {
@@ -143,5 +150,5 @@ extern "C" int switchml_column_sums(const void* dy, float* out, int K, int M, vo
   const unsigned blocks = static_cast<unsigned>((M + kSumCols - 1) / kSumCols * ctas);
   const cudaError_t e = LaunchOverlapped(ColumnSumKernel, blocks, kSumThreads, 0, ctas, static_cast<cudaStream_t>(stream),
                                          static_cast<const __nv_bfloat16*>(dy), out, K, M);
-  return e == cudaSuccess ? 0 : -4;
+  return Launched(e);
 }

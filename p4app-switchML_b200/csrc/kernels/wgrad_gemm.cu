@@ -40,6 +40,7 @@
 #include <mutex>
 
 #include "kernels/dependent_launch.cuh"
+#include "kernels/once_per_device.h"
 #include "kernels/wgrad_gemm.h"
 
 using switchml::kernels::LaunchOverlapped;
@@ -608,15 +609,32 @@ bool MakeMap(CUtensorMap* map, CUtensorMapDataType type, int esz, const void* ba
 
 int g_sm_count[64] = {0};
 
-// Lets `kernel` use `bytes` of dynamic shared memory on the current device; once per device (`done`: a
-// bit for each).
-void AllowSmem(const void* kernel, size_t bytes, std::atomic<unsigned long long>* done) {
+// Lets `kernel` use `bytes` of dynamic shared memory on the current device.
+cudaError_t AllowSmem(const void* kernel, size_t bytes, std::atomic<unsigned long long>* done) {
   int dev = 0;
   cudaGetDevice(&dev);
-  const unsigned long long bit = 1ull << (dev & 63);
-  if (done->load(std::memory_order_acquire) & bit) return;
-  cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
-  done->fetch_or(bit, std::memory_order_release);
+  return switchml::kernels::OncePerDevice(dev, done, [&] {
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
+  });
+}
+
+// What the entry points return: 0, or -4 with the runtime's last error taken, which whoever asks for it next
+// would otherwise find.
+int Launched(cudaError_t e) {
+  if (e == cudaSuccess) return 0;
+  cudaGetLastError();
+  return -4;
+}
+
+template <int kWideStages, int kWideBufs>
+cudaError_t LaunchWideKernel(const CUtensorMap& map_a, const CUtensorMap& map_b, const CUtensorMap& map_d, unsigned tiles,
+                             int tiles_n, int K, int* error_flag, cudaStream_t stream) {
+  const auto kernel = WgradWideKernel<kWideStages, kWideBufs>;
+  const size_t smem = sizeof(WideShared<kWideStages, kWideBufs>) + 1024;
+  static std::atomic<unsigned long long> allowed{0};
+  const cudaError_t e = AllowSmem(reinterpret_cast<const void*>(kernel), smem, &allowed);
+  if (e != cudaSuccess) return e;
+  return LaunchOverlapped(kernel, tiles, kWideThreads, smem, 1, stream, map_a, map_b, map_d, tiles_n, K, error_flag);
 }
 
 }  // namespace
@@ -633,16 +651,8 @@ static int LaunchWide(const void* dy, const void* x, float* dw, int M, int N, in
   const long long tiles = static_cast<long long>((M + kTileM - 1) / kTileM) * tiles_n;
   if (tiles > 0x7fffffffll) return -1;
   // Short reductions want room to store, long ones to load.
-  static std::atomic<unsigned long long> allowed_store{0}, allowed_load{0};
-  if (K <= 4 * kTileK) {
-    AllowSmem(reinterpret_cast<const void*>(WgradWideKernel<3, 2>), sizeof(WideShared<3, 2>) + 1024, &allowed_store);
-    return LaunchOverlapped(WgradWideKernel<3, 2>, static_cast<unsigned>(tiles), kWideThreads, sizeof(WideShared<3, 2>) + 1024, 1,
-                            stream, map_a, map_b, map_d, tiles_n, K, error_flag) == cudaSuccess ? 0 : -4;
-  } else {
-    AllowSmem(reinterpret_cast<const void*>(WgradWideKernel<4, 1>), sizeof(WideShared<4, 1>) + 1024, &allowed_load);
-    return LaunchOverlapped(WgradWideKernel<4, 1>, static_cast<unsigned>(tiles), kWideThreads, sizeof(WideShared<4, 1>) + 1024, 1,
-                            stream, map_a, map_b, map_d, tiles_n, K, error_flag) == cudaSuccess ? 0 : -4;
-  }
+  const auto launch = K <= 4 * kTileK ? LaunchWideKernel<3, 2> : LaunchWideKernel<4, 1>;
+  return Launched(launch(map_a, map_b, map_d, static_cast<unsigned>(tiles), tiles_n, K, error_flag, stream));
 }
 
 extern "C" int switchml_wgrad_gemm(const void* dy, const void* x, float* dw, int M, int N, int K,
@@ -680,8 +690,9 @@ extern "C" int switchml_wgrad_gemm(const void* dy, const void* x, float* dw, int
   // All CTAs take part in the closing cross-GPU barrier, so the grid must be the same on
   // every rank and fully resident: one CTA per SM at most.
   static std::atomic<unsigned long long> allowed1{0}, allowed2{0};
-  AllowSmem(reinterpret_cast<const void*>(WgradGemmKernel<1>), smem, &allowed1);
-  AllowSmem(reinterpret_cast<const void*>(WgradGemmKernel<2>), smem, &allowed2);
+  const cudaError_t e = gather ? AllowSmem(reinterpret_cast<const void*>(WgradGemmKernel<2>), smem, &allowed2)
+                               : AllowSmem(reinterpret_cast<const void*>(WgradGemmKernel<1>), smem, &allowed1);
+  if (e != cudaSuccess) return Launched(e);
   // One CTA on every SM even when there are fewer tiles: the others only reduce (or broadcast).
   // Work items of that: a few per warp of the grid, between 2 and 32 rows of a tile each.
   const int grid = sms;
@@ -697,12 +708,13 @@ extern "C" int switchml_wgrad_gemm(const void* dy, const void* x, float* dw, int
     if (gblocks < 1) gblocks = 1;
     WgradGatherKernel<<<gblocks, 512, 0, stream>>>(static_cast<const char*>(dy), static_cast<const char*>(x), *fused,
                                                   bytes_a, bytes_b, static_cast<size_t>(tiles) + 148);
-    if (cudaGetLastError() != cudaSuccess) return -4;
+    const cudaError_t gathered = cudaGetLastError();
+    if (gathered != cudaSuccess) return Launched(gathered);
     WgradGemmKernel<2><<<grid, kThreads, smem, stream>>>(map_a, map_b, map_d, dw, M, N, k_rows, *fused, rows_per_item, error_flag);
   } else {
     WgradGemmKernel<1><<<grid, kThreads, smem, stream>>>(map_a, map_b, map_d, dw, M, N, K, *fused, rows_per_item, error_flag);
   }
-  return cudaGetLastError() == cudaSuccess ? 0 : -4;
+  return Launched(cudaGetLastError());
 }
 
 namespace {
@@ -717,7 +729,8 @@ cudaError_t LaunchPairs(const CUtensorMap& map_a, const CUtensorMap& map_b, cons
                         const PairPlan& plan, int* error_flag, cudaStream_t stream) {
   const size_t smem = sizeof(PairShared<TN>) + 1024;
   static std::atomic<unsigned long long> allowed{0};
-  AllowSmem(reinterpret_cast<const void*>(WgradPairKernel<TN, kSplits>), smem, &allowed);
+  const cudaError_t e = AllowSmem(reinterpret_cast<const void*>(WgradPairKernel<TN, kSplits>), smem, &allowed);
+  if (e != cudaSuccess) return e;
   return LaunchOverlapped(WgradPairKernel<TN, kSplits>, static_cast<unsigned>(plan.clusters) * 2 * kSplits, kPairThreads, smem,
                           2 * kSplits, stream, map_a, map_b, map_d, M, N, K, error_flag);
 }
@@ -773,8 +786,7 @@ extern "C" int switchml_wgrad_gemm_2cta(const void* dy, const void* x, float* dw
   const auto launch = plan.splits == 1 ? LaunchPairs<256, 1>
                     : plan.splits == 2 ? (plan.tn == 256 ? LaunchPairs<256, 2> : LaunchPairs<128, 2>)
                                        : (plan.tn == 256 ? LaunchPairs<256, 4> : LaunchPairs<128, 4>);
-  const cudaError_t e = launch(map_a, map_b, map_d, M, N, K, plan, error_flag, stream);
-  return e == cudaSuccess ? 0 : -4;
+  return Launched(launch(map_a, map_b, map_d, M, N, K, plan, error_flag, stream));
 }
 
 // Up to K = 256 writing the gradient takes longer than multiplying. Up to 512 the one-CTA kernel's

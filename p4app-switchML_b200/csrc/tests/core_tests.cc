@@ -12,6 +12,7 @@
 
 #include "backends/softswitch/soft_switch.h"
 #include "backends/timeout_queue.h"
+#include "kernels/once_per_device.h"
 #include "ppp/cpu_exponent_quantizer_ppp.h"
 #include "rendezvous/control.h"
 #include "simd/simd_kernels.h"
@@ -124,6 +125,19 @@ static void TestSimdMatchesScalar() {
   simd::Enable(true);
 }
 
+// What fails is tried again; what has worked is not, on that device.
+static void TestOncePerDevice() {
+  std::atomic<unsigned long long> done{0};
+  int calls = 0;
+  auto act = [&] { return ++calls == 1 ? 2 : 0; };
+  EXPECT(kernels::OncePerDevice(3, &done, act) == 2);
+  EXPECT(kernels::OncePerDevice(3, &done, act) == 0);
+  EXPECT(kernels::OncePerDevice(3, &done, act) == 0);
+  EXPECT(calls == 2);
+  EXPECT(kernels::OncePerDevice(4, &done, act) == 0);
+  EXPECT(calls == 3);
+}
+
 static void TestNumaHelpers() {
   int ids[1024], count = 0;
   // Node 0 exists on every Linux machine with NUMA information; without it the helpers say no.
@@ -136,6 +150,7 @@ static void TestNumaHelpers() {
   }
   EXPECT(!GetCoresNuma(-1, ids, 1024, &count) && !GetCoresNuma(4095, ids, 1024, &count));
   EXPECT(GetDeviceNuma("ffff:ff:1f.7") == -1);
+  TestOncePerDevice();
 }
 
 static void TestStaticSlice() {

@@ -27,9 +27,12 @@ Job::Job(Tensor tensor, JobType job_type, ExtraJobInfo extra_job_info)
       extra_job_info_(extra_job_info),
       job_status_(INIT) {}
 
-void Job::WaitToComplete() { WaitToCompleteFor(-1); }
+void Job::WaitToComplete() { Wait(-1); }
 
-bool Job::WaitToCompleteFor(double milliseconds) {
+bool Job::WaitToCompleteFor(double milliseconds) { return Wait(milliseconds > 0 ? milliseconds : 0); }
+
+// < 0: without a limit.
+bool Job::Wait(double milliseconds) {
   const auto deadline = std::chrono::steady_clock::now() + std::chrono::duration<double, std::milli>(milliseconds < 0 ? 0 : milliseconds);
   auto wait = [&](std::unique_lock<std::mutex>& lk, auto condition) {
     if (milliseconds >= 0) return job_event_.wait_until(lk, deadline, condition);

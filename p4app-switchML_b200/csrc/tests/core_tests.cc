@@ -213,6 +213,7 @@ static void TestJobFsm() {
   try { j.SetJobStatus(QUEUED); } catch (const FatalError&) { threw = true; }
   EXPECT(threw);
   EXPECT(!j.WaitToCompleteFor(5));
+  EXPECT(!j.WaitToCompleteFor(0) && !j.WaitToCompleteFor(-1));
   std::thread fin([&] { j.SetJobStatus(FINISHED); });
   j.WaitToComplete();
   fin.join();

@@ -73,7 +73,7 @@ class Job {
 
   // Block until the job is FINISHED or FAILED.
   void WaitToComplete();
-  // Same with a limit; returns false on timeout.
+  // Same with a limit; returns false on timeout (at once with a limit of 0 or less).
   bool WaitToCompleteFor(double milliseconds);
   JobStatus GetJobStatus();
   void SetJobStatus(JobStatus job_status);
@@ -100,6 +100,8 @@ class Job {
   std::function<void()> on_success_;
 
  private:
+  bool Wait(double milliseconds);
+
   static std::atomic<JobId> next_id_;
   JobStatus job_status_;
   std::mutex access_mutex_;

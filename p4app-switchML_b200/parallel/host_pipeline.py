@@ -31,7 +31,7 @@ def _chunk_bytes(nbytes):
     not overlap is one chunk, and a chunk costs some 10 us to start: at 55 GB/s the sum is least at
     sqrt(nbytes * 550 kB). A power of two, because copies of odd sizes ran a fifth slower (128 MiB:
     2.97 ms in 8 MiB chunks, 3.56 ms in 10.7 MiB chunks, 3.77 ms unchunked)."""
-    return 1 << max(0, round(math.log2(math.sqrt(nbytes * 550e3))))
+    return 1 << max(0, round(math.log2(math.sqrt(max(nbytes, 1) * 550e3))))
 
 
 class HostAllReduce:

@@ -212,6 +212,14 @@ def test_host_pipeline_chunks(ctx, mode, numel, chunk):
     pipe.close()
 
 
+def test_host_pipeline_of_nothing(ctx):
+    from switchml_b200.parallel.host_pipeline import HostAllReduce
+    assert ctx.start(sml.make_config("cuda", mode="float_sum", launch="inline"))
+    hx, hy = torch.empty(0, pin_memory=True), torch.empty(0, pin_memory=True)
+    pipe = HostAllReduce(ctx, 0, torch.float32)
+    assert pipe.bounds == [] and pipe.run(hx, hy) is hy
+
+
 def test_host_pipeline_leaves_nothing_in_flight_when_it_fails(ctx):
     """A call that ends with an error, here because the context was stopped, has ended on the GPU too."""
     from switchml_b200.parallel.host_pipeline import HostAllReduce

@@ -80,7 +80,8 @@ class HostAllReduce:
             return host_out
         src, dst = host_in, host_out
         if not self._plain(src):
-            src = host_in[:self.numel].to(self.dx.dtype).cpu().contiguous()
+            # (an input of another shape is refused here)
+            src = torch.empty(self.numel, dtype=self.dx.dtype, pin_memory=True).copy_(host_in[:self.numel])
         if not self._plain(dst):
             dst = torch.empty(self.numel, dtype=self.dx.dtype, pin_memory=True)
         with torch.cuda.device(self.dx.device):
@@ -94,7 +95,8 @@ class HostAllReduce:
         return host_out
 
     def _plain(self, t):
-        return t.device.type == "cpu" and t.dtype == self.dx.dtype and t.is_contiguous() and t.numel() >= self.numel
+        return (t.device.type == "cpu" and t.dtype == self.dx.dtype and t.dim() == 1 and t.is_contiguous()
+                and t.numel() >= self.numel)
 
     def close(self):
         self.dx = None

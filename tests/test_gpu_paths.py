@@ -212,6 +212,25 @@ def test_host_pipeline_chunks(ctx, mode, numel, chunk):
     pipe.close()
 
 
+def test_host_pipeline_looks_at_its_tensors(ctx):
+    """Tensors that are too short or of another shape are refused, longer, strided and converted ones are not."""
+    from switchml_b200.parallel.host_pipeline import HostAllReduce
+    assert ctx.start(sml.make_config("cuda", mode="float_sum", launch="inline"))
+    numel = 1000
+    pipe = HostAllReduce(ctx, numel, torch.float32)
+    x, y = torch.arange(2.0 * numel).pin_memory(), torch.zeros(numel).pin_memory()
+    for bad in (x[:numel - 1], x[:numel].view(10, 100), x.view(2, numel)):
+        with pytest.raises(RuntimeError):
+            pipe.run(bad, y)
+    for bad in (y[:numel - 1], y.view(10, 100)):
+        with pytest.raises(RuntimeError):
+            pipe.run(x, bad)
+    for good in (x, x[::2], x.to(torch.int32), x.cuda()):
+        out = torch.zeros(2 * numel)
+        assert pipe.run(good, out[::2]) is not None
+        assert torch.equal(out[::2], good[:numel].float().cpu()) and bool((out[1::2] == 0).all())
+
+
 def test_host_pipeline_of_nothing(ctx):
     from switchml_b200.parallel.host_pipeline import HostAllReduce
     assert ctx.start(sml.make_config("cuda", mode="float_sum", launch="inline"))

@@ -22,8 +22,7 @@ import math
 import torch
 
 from .._native import last_error, lib
-from .context import _TORCH_CODES
-
+from .context import _describe
 
 
 def _chunk_bytes(nbytes):
@@ -78,6 +77,7 @@ class HostAllReduce:
                     raise RuntimeError("allreduce into pinned memory failed: " + j.error())
                 j.release()
             return host_out
+        _, _, code, _, _ = _describe(self.dx)  # a type that the context does not take is refused here
         src, dst = host_in, host_out
         if not self._plain(src):
             # (an input of another shape is refused here)
@@ -86,7 +86,7 @@ class HostAllReduce:
             dst = torch.empty(self.numel, dtype=self.dx.dtype, pin_memory=True)
         with torch.cuda.device(self.dx.device):
             rc = lib().sml_host_allreduce(src.data_ptr(), dst.data_ptr(), self.dx.data_ptr(), self.numel,
-                                          _TORCH_CODES[self.dx.dtype], self.chunk, self.s_in.cuda_stream,
+                                          code, self.chunk, self.s_in.cuda_stream,
                                           self.s_comm.cuda_stream, self.s_out.cuda_stream)
         if rc != 0:
             raise RuntimeError("allreduce of host memory failed: " + last_error())

@@ -231,6 +231,14 @@ def test_host_pipeline_looks_at_its_tensors(ctx):
         assert torch.equal(out[::2], good[:numel].float().cpu()) and bool((out[1::2] == 0).all())
 
 
+def test_host_pipeline_refuses_types_as_the_context_does(ctx):
+    from switchml_b200.parallel.host_pipeline import HostAllReduce
+    assert ctx.start(sml.make_config("cuda", mode="float_sum", launch="inline"))
+    x = torch.zeros(10, dtype=torch.float64).pin_memory()
+    with pytest.raises(TypeError):
+        HostAllReduce(ctx, 10, torch.float64).run(x, torch.empty_like(x))
+
+
 def test_host_pipeline_of_nothing(ctx):
     from switchml_b200.parallel.host_pipeline import HostAllReduce
     assert ctx.start(sml.make_config("cuda", mode="float_sum", launch="inline"))

@@ -216,6 +216,7 @@ def _side_stream(device):
 
 def column_sums(dy):
     """Sum over the rows of a bf16 matrix [K, M], in fp32 (M a multiple of 8, contiguous)."""
+    assert dy.is_cuda and dy.dtype == torch.bfloat16 and dy.dim() == 2 and dy.is_contiguous()
     K, M = dy.shape
     out = torch.empty(M, dtype=torch.float32, device=dy.device)
     rc = (_LIB or _lib()).switchml_column_sums(dy.data_ptr(), out.data_ptr(), K, M, _current_stream(dy.get_device()))

@@ -93,6 +93,9 @@ class FusedLinear : public torch::autograd::Function<FusedLinear> {
       at::NoGradGuard no_grad;
       const Tensor dyl = dy2.to(at::kBFloat16).contiguous(), xl = x2.to(at::kBFloat16).contiguous();
       if (!plan->run) {
+        // (The weight may be another one than the layer had when it was attached.)
+        TORCH_CHECK(dyl.is_cuda() && xl.is_cuda() && dyl.size(1) * xl.size(1) == plan->grad.numel(), "the weight gradient is [",
+                    dyl.size(1), ", ", xl.size(1), "], the buffer from attach() has ", plan->grad.numel(), " elements");
         Check(switchml_wgrad_gemm_auto(dyl.const_data_ptr(), xl.const_data_ptr(), plan->grad.data_ptr<float>(),
                                        static_cast<int>(dyl.size(1)), static_cast<int>(xl.size(1)), static_cast<int>(dyl.size(0)),
                                        plan->error.data_ptr<int>(), CurrentStream()),

@@ -346,6 +346,21 @@ def test_fused_wgrad_linear_against_plain_linear(ctx, shape, features, bias, x_d
         assert float((got.float() - want.float()).norm()) <= 1e-2 * float(want.float().norm()) + 1e-6
 
 
+@pytest.mark.parametrize("features", [64, 192])
+def test_fused_wgrad_linear_with_another_weight(ctx, features):
+    """A weight that the gradient's buffer does not fit is refused, and the buffer's neighbours stay as they are."""
+    from switchml_b200.ops.wgrad import FusedWgradLinear
+    assert ctx.start(sml.make_config("cuda", mode="float_sum", launch="inline", symm_heap_mb=16))
+    layer = FusedWgradLinear(64, 128, bias=False, device="cuda").attach(ctx)
+    after = ctx.symmetric_empty(1 << 16, torch.float32).fill_(5.0)
+    layer.weight = torch.nn.Parameter(torch.randn(features, 64, device="cuda"))
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        y = layer(torch.randn(32, 64, device="cuda"))
+    with pytest.raises(RuntimeError):
+        y.sum().backward()
+    assert bool((after == 5).all())
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_one_worker_exact_pass_of_odd_values(ctx, dtype):
     """Infinities, NaN, values whose integer saturates, denormals, negative zeros and halves of the grid:

@@ -8,6 +8,7 @@ later tiles are still being computed.
 """
 import ctypes
 import os
+import warnings
 import weakref
 
 import torch
@@ -225,27 +226,67 @@ def column_sums(dy):
     return out
 
 
+class _FusedLinearFn(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, x, weight, bias, plan):
+        ctx.plan = plan
+        ctx.save_for_backward(x, weight)
+        ctx.bias_dtype = None if bias is None else bias.dtype
+        return torch.nn.functional.linear(x, weight, bias)
+
+    @staticmethod
+    def backward(ctx, dy):
+        x, weight = ctx.saved_tensors
+        x2 = x.reshape(-1, x.shape[-1])
+        dy2 = dy.reshape(-1, dy.shape[-1])
+        dx = (dy2 @ weight.to(dy2.dtype)).reshape(x.shape) if ctx.needs_input_grad[0] else None
+        with torch.no_grad():
+            ctx.plan.run(dy2.to(torch.bfloat16), x2.to(torch.bfloat16))
+        return dx, None, dy2.sum(0).to(ctx.bias_dtype) if ctx.bias_dtype is not None else None, None
+
+
+class _PythonNode:
+    """What lib/torch_switchml_linear.so offers, in Python: 150 instead of 20 us on the host for forward and backward
+    of a small layer."""
+
+    class Plan:
+        def __init__(self, grad, error, run):
+            self.run = run or (lambda dy, x: wgrad_gemm(dy, x, out=grad, error_flag=error))
+
+    @staticmethod
+    def fused_linear(x, weight, bias, plan):
+        if torch.is_autocast_enabled():
+            dt = torch.get_autocast_dtype("cuda")
+            x, weight, bias = x.to(dt), weight.to(dt), bias.to(dt) if bias is not None else None
+        return _FusedLinearFn.apply(x, weight, bias, plan)
+
+
 _NODE = None
 
 
 def _node():
     """lib/torch_switchml_linear.so, the layer's autograd node (csrc/torch/fused_linear.cc); built when it is
-    missing, like the main library."""
+    missing, like the main library. Where it cannot be built or loaded (no headers of this PyTorch, no compiler) the
+    node in Python does its work."""
     global _NODE
     if _NODE is None:
         import importlib.util
         _lib()
         path = library_path("torch_switchml_linear.so")
-        if not os.path.exists(path):
-            here = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
-            spec = importlib.util.spec_from_file_location("_switchml_build", os.path.join(here, "build.py"))
-            build = importlib.util.module_from_spec(spec)
-            spec.loader.exec_module(build)
-            build.build_torch_extension()
-        spec = importlib.util.spec_from_file_location("torch_switchml_linear", path)
-        module = importlib.util.module_from_spec(spec)
-        spec.loader.exec_module(module)
-        _NODE = module
+        try:
+            if not os.path.exists(path):
+                here = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+                spec = importlib.util.spec_from_file_location("_switchml_build", os.path.join(here, "build.py"))
+                build = importlib.util.module_from_spec(spec)
+                spec.loader.exec_module(build)
+                build.build_torch_extension()
+            spec = importlib.util.spec_from_file_location("torch_switchml_linear", path)
+            module = importlib.util.module_from_spec(spec)
+            spec.loader.exec_module(module)
+            _NODE = module
+        except (ImportError, OSError, RuntimeError) as e:
+            warnings.warn("FusedWgradLinear runs without lib/torch_switchml_linear.so: %s" % e)
+            _NODE = _PythonNode
     return _NODE
 
 

@@ -626,33 +626,25 @@ int Launched(cudaError_t e) {
   return -4;
 }
 
-template <int kWideStages, int kWideBufs>
-cudaError_t LaunchWideKernel(const CUtensorMap& map_a, const CUtensorMap& map_b, const CUtensorMap& map_d, unsigned tiles,
-                             int tiles_n, int K, int* error_flag, cudaStream_t stream) {
-  const auto kernel = WgradWideKernel<kWideStages, kWideBufs>;
-  const size_t smem = sizeof(WideShared<kWideStages, kWideBufs>) + 1024;
-  static std::atomic<unsigned long long> allowed{0};
-  const cudaError_t e = AllowSmem(reinterpret_cast<const void*>(kernel), smem, &allowed);
-  if (e != cudaSuccess) return e;
-  return LaunchOverlapped(kernel, tiles, kWideThreads, smem, 1, stream, map_a, map_b, map_d, tiles_n, K, error_flag);
-}
-
 }  // namespace
 
-// The plain GEMM, one CTA per tile. fc6 (32 x 4096 x 25088): 76.1 us -> 67.2 us (6.1 TB/s of
-// output; the stores alone take 63.5), 100 x 8000 x 8000: 56 -> 47 us.
+// The plain GEMM, one CTA per tile.
+template <bool kWholeBoxes>
 static int LaunchWide(const void* dy, const void* x, float* dw, int M, int N, int K, int* error_flag, cudaStream_t stream) {
   CUtensorMap map_a, map_b, map_d;
   if (!MakeMap(&map_a, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, dy, K, M, kTileK, kAtomMN) ||
       !MakeMap(&map_b, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, x, K, N, kTileK, kAtomMN) ||
-      !MakeMap(&map_d, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, dw, M, N, 32, kEpiCols))
+      !MakeMap(&map_d, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, dw, M, N, kWholeBoxes ? kTileM : 32, kEpiCols))
     return -3;
   const int tiles_n = (N + kTileN - 1) / kTileN;
   const long long tiles = static_cast<long long>((M + kTileM - 1) / kTileM) * tiles_n;
   if (tiles > 0x7fffffffll) return -1;
-  // Short reductions want room to store, long ones to load.
-  const auto launch = K <= 4 * kTileK ? LaunchWideKernel<3, 2> : LaunchWideKernel<4, 1>;
-  return Launched(launch(map_a, map_b, map_d, static_cast<unsigned>(tiles), tiles_n, K, error_flag, stream));
+  const size_t smem = sizeof(WideShared) + 1024;
+  static std::atomic<unsigned long long> allowed{0};
+  const cudaError_t e = AllowSmem(reinterpret_cast<const void*>(WgradWideKernel<kWholeBoxes>), smem, &allowed);
+  if (e != cudaSuccess) return Launched(e);
+  return Launched(LaunchOverlapped(WgradWideKernel<kWholeBoxes>, static_cast<unsigned>(tiles), kWideThreads, smem, 1, stream,
+                                   map_a, map_b, map_d, tiles_n, K, error_flag));
 }
 
 extern "C" int switchml_wgrad_gemm(const void* dy, const void* x, float* dw, int M, int N, int K,
@@ -663,7 +655,7 @@ extern "C" int switchml_wgrad_gemm(const void* dy, const void* x, float* dw, int
   if ((reinterpret_cast<uintptr_t>(dy) | reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(dw)) & 15)
     return -2;
   if (!fused || fused->nranks <= 1)
-    return LaunchWide(dy, x, dw, M, N, K, error_flag, static_cast<cudaStream_t>(stream_ptr));
+    return (K > 4 * kTileK ? LaunchWide<true> : LaunchWide<false>)(dy, x, dw, M, N, K, error_flag, static_cast<cudaStream_t>(stream_ptr));
   const bool gather = fused->mode == 1;
   if (gather && (!fused->gather_local || !fused->gather_mc || !fused->gather_counter || !fused->out_mc || !fused->work_counter ||
                  fused->nranks > 8))

@@ -278,6 +278,24 @@ def test_wgrad_short_reductions(K, M, N):
     assert bool((frame[:64] == 3).all()) and bool((frame[64 + M * N:] == 3).all())
 
 
+@pytest.mark.parametrize("K", [256, 257, 300, 320, 448, 1000, 4096])
+@pytest.mark.parametrize("M,N", [(8, 8), (136, 264), (1000, 520), (4000, 5000)])
+def test_wgrad_one_cta_per_tile_and_long_reductions(K, M, N):
+    """The kernel for short reductions beyond their range: whole boxes of 128 rows, last stages that K fills and that
+    it does not, one tile and several per CTA."""
+    from switchml_b200.ops.wgrad import wgrad_gemm
+    gen = torch.Generator(device="cuda").manual_seed(K + M)
+    dy = torch.randn(K, M, device="cuda", generator=gen).bfloat16()
+    x = torch.randn(K, N, device="cuda", generator=gen).bfloat16()
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    frame = torch.full((M * N + 128,), 3.0, device="cuda")
+    out = wgrad_gemm(dy, x, out=frame[64:64 + M * N].view(M, N), error_flag=err, two_cta=False)
+    assert int(err) == 0
+    ref = dy.double().t() @ x.double()
+    assert float((out - ref).norm() / ref.norm()) < 1e-5
+    assert bool((frame[:64] == 3).all()) and bool((frame[64 + M * N:] == 3).all())
+
+
 @pytest.mark.parametrize("K,M,N", [(8192, 512, 512), (8192, 1024, 1024), (4160, 264, 520), (2048, 1000, 1032), (300, 256, 128),
                                    (1000, 3000, 2000), (640, 2048, 4104), (65, 8, 8), (8192, 2304, 1024)])
 def test_wgrad_pairs_of_ctas_with_every_split(K, M, N):

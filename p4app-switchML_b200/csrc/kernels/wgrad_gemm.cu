@@ -148,15 +148,12 @@ constexpr uint32_t kInstrDesc = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) 
                                 (static_cast<uint32_t>(kTileN >> 3) << 17) |
                                 (static_cast<uint32_t>(kTileM >> 4) << 24);
 
-__device__ __forceinline__ void MmaWith(uint32_t tmem_d, uint64_t a_desc, uint64_t b_desc, uint32_t instr, uint32_t accumulate) {
+__device__ __forceinline__ void Mma(uint32_t tmem_d, uint64_t a_desc, uint64_t b_desc, uint32_t accumulate) {
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
       "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "l"(a_desc), "l"(b_desc), "r"(instr), "r"(accumulate) : "memory");
-}
-__device__ __forceinline__ void Mma(uint32_t tmem_d, uint64_t a_desc, uint64_t b_desc, uint32_t accumulate) {
-  MmaWith(tmem_d, a_desc, b_desc, kInstrDesc, accumulate);
+      ::"r"(tmem_d), "l"(a_desc), "l"(b_desc), "r"(kInstrDesc), "r"(accumulate) : "memory");
 }
 
 // Arrive on an mbarrier once every tcgen05 operation issued so far by this thread is done.
@@ -781,13 +778,13 @@ extern "C" int switchml_wgrad_gemm_2cta(const void* dy, const void* x, float* dw
   return Launched(launch(map_a, map_b, map_d, M, N, K, plan, error_flag, stream));
 }
 
-// Up to K = 256 writing the gradient takes longer than multiplying. Up to 512 the one-CTA kernel's
-// smaller tiles still win while there are at most two of them per SM (512 x 4096 x 1024: 10.4 against
-// 12.4 us; with many tiles the pairs win, 300 x 8000 x 8000: 65 against 70 us).
+// Up to K = 512 the one-CTA kernel's smaller tiles and open epilogue win, whatever the number of tiles (one CTA against two,
+// back to back: 512 x 4096 x 1024 8.6 and 9.2 us, 300 x 8192 x 8192 57 and 70, 512 x 8192 x 8192 80 and 87, 512 x 4096 x
+// 25088 136 and 150); beyond it the pairs' halved traffic for X does (640 x 8192 x 8192: 102 and 97, 768 x 4096 x 4096: 36
+// and 32.5). Around the line they differ by a few percent.
 extern "C" int switchml_wgrad_gemm_auto(const void* dy, const void* x, float* dw, int M, int N, int K, int* error_flag,
                                         void* stream) {
-  const long long tiles = static_cast<long long>((M + kTileM - 1) / kTileM) * ((N + kTileN - 1) / kTileN);
-  if (K > 512 || (K > 256 && tiles > 296)) return switchml_wgrad_gemm_2cta(dy, x, dw, M, N, K, error_flag, stream);
+  if (K > 512) return switchml_wgrad_gemm_2cta(dy, x, dw, M, N, K, error_flag, stream);
   return switchml_wgrad_gemm(dy, x, dw, M, N, K, nullptr, error_flag, stream);
 }
 

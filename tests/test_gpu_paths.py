@@ -296,6 +296,19 @@ def test_wgrad_one_cta_per_tile_and_long_reductions(K, M, N):
     assert bool((frame[:64] == 3).all()) and bool((frame[64 + M * N:] == 3).all())
 
 
+@pytest.mark.parametrize("K", [511, 512, 513, 576])
+def test_wgrad_at_the_line_between_its_kernels(K):
+    """Either kernel, and whichever is chosen, for more tiles than there are CTAs."""
+    from switchml_b200.ops.wgrad import wgrad_gemm
+    gen = torch.Generator(device="cuda").manual_seed(K)
+    dy = torch.randn(K, 4104, device="cuda", generator=gen).bfloat16()
+    x = torch.randn(K, 3000, device="cuda", generator=gen).bfloat16()
+    ref = dy.double().t() @ x.double()
+    for two_cta in (None, False, True):
+        out = wgrad_gemm(dy, x, two_cta=two_cta)
+        assert float((out - ref).norm() / ref.norm()) < 1e-5, two_cta
+
+
 @pytest.mark.parametrize("K,M,N", [(8192, 512, 512), (8192, 1024, 1024), (4160, 264, 520), (2048, 1000, 1032), (300, 256, 128),
                                    (1000, 3000, 2000), (640, 2048, 4104), (65, 8, 8), (8192, 2304, 1024)])
 def test_wgrad_pairs_of_ctas_with_every_split(K, M, N):

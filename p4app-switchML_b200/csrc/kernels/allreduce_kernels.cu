@@ -224,14 +224,15 @@ template <> struct VecAcc<ELEM_BF16> {
 };
 
 // Peer memory: U 16-byte vectors (at `off`, off + step, ...; those from `left` on are left alone) summed over
-// all ranks, post-scaled. Rank by rank with all U loads in flight; vector by vector, as ReduceVec
-// goes, a thread had one load in flight and four emulated ranks reduced at 0.7 TB/s.
-template <int ELEM, int U>
+// all ranks, post-scaled. Rank by rank with all U loads in flight (on one GPU those of several ranks where U is small);
+// vector by vector, as ReduceVec goes, a thread had one load in flight and four emulated ranks reduced at 0.7 TB/s.
+template <int ELEM, int U, bool kOneGpu>
 __device__ __forceinline__ void ReducePeers(const RankCtx& ctx, char* const* peers, size_t off, size_t step, int left,
                                             float post_scale, uint4 (&r)[U]) {
   VecAcc<ELEM> acc[U];
 #pragma unroll
   for (int u = 0; u < U; u++) acc[u].Zero();
+#pragma unroll (kOneGpu && U <= 4 ? 4 : 1)
   for (int p = 0; p < ctx.nranks; p++) {
     const char* src = peers[p] + off;
     uint4 v[U];
@@ -444,13 +445,16 @@ __device__ __forceinline__ void RoleLocalCopy(const RankCtx& ctx, const Role& ro
 #define SML_GEOMETRY_CHECK(CTX, CHANNEL, FAILED, COND)
 #endif
 
-template <int ELEM, int MODE, int kLoadWarps = kDefaultLoadWarps, int kReduceWarps = kDefaultReduceWarps,
+// kOneGpu: all ranks live on this GPU, and the reducer's loads from them come out of its own L2: it keeps twice as many
+// in flight as of loads that cross NVLink (kUnrollLink, where 8 measured slower).
+template <int ELEM, int MODE, bool kOneGpu, int kLoadWarps = kDefaultLoadWarps, int kReduceWarps = kDefaultReduceWarps,
           int kUnrollLink = kDefaultUnrollLink>
 __device__ void RunStaged(const RankCtx& ctx, const JobArgs& job, int channel,
                           unsigned long long elems_per_channel, Epoch base, StagedShared* sh, float* s_sf) {
   constexpr int kStoreWarps = kThreads / 32 - kLoadWarps - kReduceWarps - 1;  // the last warp tells the peers
   static_assert(kStoreWarps >= 1, "the storer needs a warp");
   constexpr int kUnrollInt = 4 * kUnrollLink;  // 4-byte integer lanes in flight per thread
+  constexpr int kPeerLoads = kOneGpu ? 8 : kUnrollLink;
   const int in_esz = ELEM == ELEM_BF16 ? 2 : 4;
   const int st_esz = MODE == MODE_QUANT ? 4 : in_esz;
   const size_t slot_elems = ctx.slot_bytes / st_esz;  // what the checked build verifies tiles against
@@ -649,12 +653,12 @@ __device__ void RunStaged(const RankCtx& ctx, const JobArgs& job, int channel,
         size_t from = sb;
         if (!ctx.use_multimem) {
           // Groups of four elements: 16 bytes of every rank's payload, 8 bytes of results.
-          constexpr int U = 8;
+          constexpr int U = kPeerLoads;
           const size_t g0 = sb / 4, g1 = se / 4;  // sb is a multiple of the block
           for (size_t g = g0 + t; g < g1; g += U * n) {
             const int left = StepsLeft<U>(g1 - g, n);
             uint4 q[U];
-            ReducePeers<ELEM_I32, U>(ctx, ctx.stage_peer, slot_off + g * 16, static_cast<size_t>(n) * 16, left, 1.0f, q);
+            ReducePeers<ELEM_I32, U, kOneGpu>(ctx, ctx.stage_peer, slot_off + g * 16, static_cast<size_t>(n) * 16, left, 1.0f, q);
             uint2 h[U];
 #pragma unroll
             for (int u = 0; u < U; u++) {
@@ -764,25 +768,24 @@ __device__ void RunStaged(const RankCtx& ctx, const JobArgs& job, int channel,
               BroadcastVec(ctx, dst_peer, dst_mc, dst_off + v * 16, sum);
             }
           };
-          constexpr int U = 8;
-          auto turn = [&](size_t v, int left) {
-            uint4 r[U];
-            ReducePeers<ELEM_I32, U>(ctx, ctx.stage_peer, slot_off + v * 16, static_cast<size_t>(n) * 16, left, 1.0f, r);
+          for (size_t v = v0 + t; v < v1; v += kPeerLoads * n) {
+            const int left = StepsLeft<kPeerLoads>(v1 - v, n);
+            uint4 r[kPeerLoads];
+            ReducePeers<ELEM_I32, kPeerLoads, kOneGpu>(ctx, ctx.stage_peer, slot_off + v * 16, static_cast<size_t>(n) * 16, left, 1.0f, r);
 #pragma unroll
-            for (int u = 0; u < U; u++)
+            for (int u = 0; u < kPeerLoads; u++)
               if (u < left) finish(v + static_cast<size_t>(u) * n, r[u]);
-          };
-          for (size_t v = v0 + t; v < v1; v += U * n) turn(v, StepsLeft<U>(v1 - v, n));
+          }
         }
       } else {
         size_t v0 = sb / vec_elems, v1 = (se + vec_elems - 1) / vec_elems;
         size_t v = v0 + t;
         if (!ctx.use_multimem) {
-          constexpr int U = ELEM == ELEM_BF16 ? 4 : 8;
+          constexpr int U = ELEM == ELEM_BF16 ? 4 : kPeerLoads;
           for (; v < v1; v += U * n) {
             const int left = StepsLeft<U>(v1 - v, n);
             uint4 r[U];
-            ReducePeers<ELEM, U>(ctx, ctx.stage_peer, slot_off + v * 16, static_cast<size_t>(n) * 16, left, job.post_scale, r);
+            ReducePeers<ELEM, U, kOneGpu>(ctx, ctx.stage_peer, slot_off + v * 16, static_cast<size_t>(n) * 16, left, job.post_scale, r);
             for (int p = 0; p < ctx.nranks; p++) {
               char* dst = ctx.stage_peer[p] + slot_off + v * 16;
 #pragma unroll
@@ -1183,16 +1186,16 @@ __device__ void RunZeroCopy(const RankCtx& ctx, const JobArgs& job, int channel,
 }
 
 // ------------------------------------------------------------------------------------
-template <int ELEM, int MODE, int ALGO>
+template <int ELEM, int MODE, int ALGO, bool kOneGpu>
 __device__ __forceinline__ void RunJob(const RankCtx& ctx, const JobArgs& job, int channel,
                                        unsigned long long epc, Epoch base, int* s_failed, float* s_sf) {
   // The quantising loader reads its input twice and meets its peers once more per tile,
   // so it gets more warps than the plain copy-in of the SUM modes (8-GPU measurements with
   // 1 GiB: 4/8/4 3.72 ms, 6/8/2 3.30 ms, 8/6/2 3.07 ms before the loader was vectorised).
   if (ALGO == ALGO_STAGED && MODE == MODE_QUANT)
-    RunStaged<ELEM, MODE, 6, 8>(ctx, job, channel, epc, base, reinterpret_cast<StagedShared*>(s_failed), s_sf);
+    RunStaged<ELEM, MODE, kOneGpu, 6, 8>(ctx, job, channel, epc, base, reinterpret_cast<StagedShared*>(s_failed), s_sf);
   else if (ALGO == ALGO_STAGED)
-    RunStaged<ELEM, MODE>(ctx, job, channel, epc, base, reinterpret_cast<StagedShared*>(s_failed), s_sf);
+    RunStaged<ELEM, MODE, kOneGpu>(ctx, job, channel, epc, base, reinterpret_cast<StagedShared*>(s_failed), s_sf);
   else if (ALGO == ALGO_PUSH)
     RunPush<ELEM, MODE>(ctx, job, channel, epc, base, reinterpret_cast<StagedShared*>(s_failed), s_sf);
   else if (ALGO == ALGO_ONESHOT) RunOneShot<ELEM, MODE>(ctx, job, channel, epc, base, s_failed);
@@ -1238,9 +1241,16 @@ AllReduceKernel(const __grid_constant__ RankCtx ctx, const __grid_constant__ Job
   __shared__ StagedShared s_state;
   __shared__ float s_sf[(MODE == MODE_QUANT && (ALGO == ALGO_STAGED || ALGO == ALGO_PUSH)) ? kMaxBlocksPerSlot : 1];
   SML_EPOCH_PROLOGUE(ctx, job, blockIdx.x, ALGO)
-  RunJob<ELEM, MODE, ALGO>(ctx, job, blockIdx.x, epc, s_base, &s_state.failed, s_sf);
+  RunJob<ELEM, MODE, ALGO, false>(ctx, job, blockIdx.x, epc, s_base, &s_state.failed, s_sf);
   SML_EPOCH_EPILOGUE(ctx, job, blockIdx.x)
 }
+
+// The checked build emulates with the code for ranks on GPUs of their own: on one GPU it runs nowhere else.
+#ifdef SWITCHML_CHECKED
+static constexpr bool kEmuOneGpu = false;
+#else
+static constexpr bool kEmuOneGpu = true;
+#endif
 
 // All ranks in one grid: blockIdx.y selects the rank whose role this CTA plays.
 template <int ELEM, int MODE, int ALGO>
@@ -1259,7 +1269,7 @@ AllReduceEmuKernel(const __grid_constant__ EmuArgs args, unsigned long long epc)
   for (unsigned i = threadIdx.x; i < sizeof(JobArgs) / 4; i += blockDim.x) reinterpret_cast<unsigned*>(&s_job)[i] = from_job[i];
   __syncthreads();
   SML_EPOCH_PROLOGUE(s_ctx, s_job, blockIdx.x, ALGO)
-  RunJob<ELEM, MODE, ALGO>(s_ctx, s_job, blockIdx.x, epc, s_base, &s_state.failed, s_sf);
+  RunJob<ELEM, MODE, ALGO, kEmuOneGpu>(s_ctx, s_job, blockIdx.x, epc, s_base, &s_state.failed, s_sf);
   SML_EPOCH_EPILOGUE(s_ctx, s_job, blockIdx.x)
 }
 

@@ -82,3 +82,35 @@ def test_a_region_that_is_too_small_is_reported_not_touched(algo):
     assert "refused:" in out and "kernel status" in out
     status = int(out.split("kernel status")[1].split()[0])
     assert status & 0xf == 3
+
+
+@pytest.mark.parametrize("algo", ["staged", "push"])
+def test_code_for_ranks_on_gpus_of_their_own(algo):
+    """The checked build emulates with the code that ranks on several GPUs run over peer memory, which is not the one that
+    the library emulates with: every element type and mode, ragged ends, tensors that are not vector aligned."""
+    out = _child("""
+        for n, numel, off in ((2, 70, 0), (2, 300001, 0), (3, 50001, 1), (4, 123457, 0), (8, (1 << 18) + 5, 2)):
+            g = torch.Generator().manual_seed(numel)
+            def place(t):
+                frame = torch.zeros(numel + off, dtype=t.dtype, device="cuda")
+                frame[off:].copy_(t)
+                return frame[off:]
+            opts = dict(algo=%r, block_numel=64, slot_bytes=32768)
+            xs = [torch.randn(numel, generator=g) * 10.0 ** (r %% 3) for r in range(n)]
+            for dtype in (torch.float32, torch.bfloat16):
+                ys = [x.to(dtype) for x in xs]
+                want = torch.from_numpy(quant_allreduce_oracle([y.float().numpy() for y in ys], 64)).to(dtype)
+                for o in emulated_allreduce([place(y) for y in ys], mode="quant", **opts):
+                    assert torch.equal(o.cpu(), want), (n, numel, dtype, "quant")
+                # Sums in fp32 in some order of the ranks, and at most one rounding to bf16: one unit of 2^-8.
+                want = sum(y.double() for y in ys)
+                bound = 2.0 ** -20 * sum(y.double().abs() for y in ys) + (2.0 ** -8 * want.abs() if dtype == torch.bfloat16 else 0)
+                for o in emulated_allreduce([place(y) for y in ys], mode="sum", **opts):
+                    assert bool(((o.cpu().double() - want).abs() <= bound).all()), (n, numel, dtype, "sum")
+            xi = [torch.randint(-2 ** 30, 2 ** 30, (numel,), generator=g, dtype=torch.int32) for r in range(n)]
+            want = int_allreduce_oracle([x.numpy() for x in xi])
+            for o in emulated_allreduce([place(x) for x in xi], mode="sum", **opts):
+                assert np.array_equal(o.cpu().numpy(), want), (n, numel, "int")
+        print("as on several GPUs")
+    """ % algo)
+    assert "as on several GPUs" in out

@@ -32,7 +32,6 @@
 #include <stdlib.h>
 
 #include <atomic>
-#include <type_traits>
 
 #include "kernels/allreduce_kernels.h"
 #include "kernels/bulk_copy.cuh"
@@ -41,6 +40,7 @@
 #include "kernels/multimem.cuh"
 #include "kernels/once_per_device.h"
 #include "kernels/quant_tile.cuh"
+#include "kernels/turns.cuh"
 #include "switchml/quant_math.h"
 
 namespace switchml {
@@ -84,17 +84,6 @@ template <int U>
 __device__ __forceinline__ int StepsLeft(size_t remaining, int n) {
   if (remaining > static_cast<size_t>((U - 1) * n)) return U;
   return static_cast<int>((static_cast<unsigned>(remaining) + n - 1) / static_cast<unsigned>(n));
-}
-
-// Walks the elements i, i + n, i + 2n, ... below `count`: whole turns of U of them, then what is left in turns
-// of U/2, U/4, ... 1 (log2(U) trips to memory instead of U - 1; predicating one whole turn instead cost
-// registers, and a third of the speed of the loop before it). f(width, i) takes `width` of them.
-template <int U, typename F>
-__device__ __forceinline__ void Turns(size_t i, size_t count, size_t n, F f) {
-  for (; i + (U - 1) * n < count; i += U * n) f(std::integral_constant<int, U>(), i);
-  if constexpr (U > 1) {
-    if (i < count) Turns<U / 2>(i, count, n, f);
-  }
 }
 
 // Element `i` of the input as float (QUANT mode reads f32 or bf16).
@@ -1197,7 +1186,7 @@ __device__ __forceinline__ void RunJob(const RankCtx& ctx, const JobArgs& job, i
   else if (ALGO == ALGO_STAGED)
     RunStaged<ELEM, MODE, kOneGpu>(ctx, job, channel, epc, base, reinterpret_cast<StagedShared*>(s_failed), s_sf);
   else if (ALGO == ALGO_PUSH)
-    RunPush<ELEM, MODE>(ctx, job, channel, epc, base, reinterpret_cast<StagedShared*>(s_failed), s_sf);
+    RunPush<ELEM, MODE, kOneGpu>(ctx, job, channel, epc, base, reinterpret_cast<StagedShared*>(s_failed), s_sf);
   else if (ALGO == ALGO_ONESHOT) RunOneShot<ELEM, MODE>(ctx, job, channel, epc, base, s_failed);
   else if (ctx.use_multimem) RunZeroCopy<ELEM, kZeroCopyUnrollLink>(ctx, job, channel, epc, base, s_failed);
   else RunZeroCopy<ELEM, kZeroCopyUnrollPeer>(ctx, job, channel, epc, base, s_failed);

@@ -136,13 +136,13 @@ __device__ __forceinline__ void PushQuantStep(size_t g, size_t stride, size_t fi
     char* dst = tg.Of(me + d < n ? me + d : me + d - n);
 #pragma unroll
     for (int u = 0; u < U; u++) {
-        if (NARROW) *reinterpret_cast<uint2*>(dst + (g + u * stride) * 8) = h[u];
+      if (NARROW) *reinterpret_cast<uint2*>(dst + (g + u * stride) * 8) = h[u];
       else *reinterpret_cast<uint4*>(dst + (g + u * stride) * 16) = w[u];
     }
   }
 }
 
-template <int ELEM, int MODE>
+template <int ELEM, int MODE, bool kOneGpu>
 __device__ void RunPush(const RankCtx& ctx, const JobArgs& job, int channel,
                         unsigned long long elems_per_channel, Epoch base, StagedShared* sh, float* s_sf) {
   constexpr int kLoadWarps = MODE == MODE_QUANT ? 6 : 5;
@@ -367,7 +367,7 @@ __device__ void RunPush(const RankCtx& ctx, const JobArgs& job, int channel,
         if (MODE == MODE_QUANT) {
           constexpr bool narrow = ELEM == ELEM_BF16;  // bf16 jobs receive bf16: in their output, or in the result areas
           const size_t ngroups = (both & (ELEM == ELEM_BF16 ? 7 : 15)) == 0 ? cnt / 4 : 0;
-          Turns<4>(t, ngroups, nt, [&](auto width, size_t g) {
+          Turns<4, kOneGpu>(t, ngroups, nt, [&](auto width, size_t g) {
             PushQuantStep<ELEM, decltype(width)::value, ELEM == ELEM_BF16>(g, nt, sb, own, recv, recv_bytes, n, me, out, tg,
                                                                           job.post_scale, sf, shift);
           });
@@ -390,7 +390,7 @@ __device__ void RunPush(const RankCtx& ctx, const JobArgs& job, int channel,
         } else {
           const size_t vec_elems = 16 / in_esz;
           const size_t nvec = (both & 15) == 0 ? cnt / vec_elems : 0;
-          Turns<kPushUnroll>(t, nvec, nt, [&](auto width, size_t v) {
+          Turns<kPushUnroll, kOneGpu>(t, nvec, nt, [&](auto width, size_t v) {
             PushSumStep<ELEM, decltype(width)::value>(v, nt, own, recv, recv_bytes, n, me, out, tg, job.post_scale);
           });
           for (size_t i = nvec * vec_elems + t; i < cnt; i += nt) {

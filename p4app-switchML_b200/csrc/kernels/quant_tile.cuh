@@ -22,6 +22,7 @@
 
 #include "kernels/allreduce_kernels.h"
 #include "kernels/device_sync.cuh"
+#include "kernels/turns.cuh"
 #include "kernels/warp_stream.cuh"
 #include "switchml/quant_math.h"
 
@@ -206,14 +207,15 @@ __device__ __forceinline__ void QuantizeRange(int tid, int nthreads, const char*
     int4* q4 = reinterpret_cast<int4*>(q);
     const size_t nvec = n / 4, first = begin / 4;
     const size_t nt = nthreads;
-    for (size_t i = tid; i < nvec; i += UNROLL * nt) {
-      float4 x[UNROLL];
+    // (Predicating the last turn in every turn instead cost registers: up to 35 words per thread of the kernels that
+    // call this were spilled for it.)
+    Turns<UNROLL>(tid, nvec, nt, [&](auto width, size_t i) {
+      constexpr int U = decltype(width)::value;
+      float4 x[U];
 #pragma unroll
-      for (int u = 0; u < UNROLL; u++)
-        if (i + u * nt < nvec) x[u] = LoadGroupAsFloat<ELEM>(in, first + i + u * nt);
+      for (int u = 0; u < U; u++) x[u] = LoadGroupAsFloat<ELEM>(in, first + i + u * nt);
 #pragma unroll
-      for (int u = 0; u < UNROLL; u++) {
-        if (i + u * nt >= nvec) continue;
+      for (int u = 0; u < U; u++) {
         const float f = sf[(begin + (i + u * nt) * 4) >> shift];
         int4 r;
         r.x = quant::Quantize(x[u].x, f);
@@ -222,7 +224,7 @@ __device__ __forceinline__ void QuantizeRange(int tid, int nthreads, const char*
         r.w = quant::Quantize(x[u].w, f);
         q4[i + u * nt] = r;
       }
-    }
+    });
     for (size_t j = nvec * 4 + tid; j < n; j += nthreads)
       q[j] = quant::Quantize(TileLoadAsFloat(in, begin + j, ELEM), sf[(begin + j) >> shift]);
   } else {

@@ -164,7 +164,8 @@ int EmulatedAllReduce(int nranks, void* const* in_ptrs, void* const* out_ptrs,
   // Plain sums through the slots are bound by memory, and here every rank's slots share one L2: a ring that
   // stays in it spares each tile two trips to HBM (4 ranks x 2^24 float32: 272 us with 155 MB of slots, 200 us
   // with 43 MB; three slots of 64 to 96 KiB, two of 128 KiB and four of 64 KiB come to the same). The
-  // exact mode pays too much per tile for smaller ones (256 KiB: 400 us, 128 KiB: 453 us).
+  // exact mode pays too much per tile for smaller ones (256 KiB: 400 us, 128 KiB: 453 us). The caller's geometry is an
+  // upper bound there; the results do not depend on it.
   const size_t unit_bytes = static_cast<size_t>(nranks) * (block_numel > 128 ? block_numel : 128) * 4;
   const size_t ring = kL2Slots / (static_cast<size_t>(max_channels) * nranks);  // bytes of a channel's slots
   if (algo == ALGO_STAGED && mode == MODE_SUM && numel * esz * nranks > kL2Slots && slot_bytes * slots_per_channel > ring) {

@@ -21,7 +21,11 @@ def emulated_allreduce(inputs, mode="quant", algo="staged", block_numel=256, slo
                        exponent_lookahead=-1):
     """Allreduce `inputs` (a list of equally sized 1-D CUDA tensors, one per virtual rank,
     all on the current device). Returns the list of per-rank outputs. `exponent_lookahead`:
-    tiles by which the exact mode's exponents run ahead of their data (-1: the library's default)."""
+    tiles by which the exact mode's exponents run ahead of their data (-1: the library's default).
+
+    `slot_bytes` and `slots_per_channel` are taken as they are (rounded to whole units of a tile), but for plain sums
+    through the slots (mode "sum", algo "staged") of more than 44 MB over all ranks: there they are upper bounds, and the ring is cut
+    to what stays in L2 (csrc/backends/cuda/emulated_allreduce.cc). The results do not depend on either."""
     import torch
     n = len(inputs)
     x0 = inputs[0]

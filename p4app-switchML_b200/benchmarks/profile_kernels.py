@@ -9,9 +9,12 @@ emulated in one cooperative launch over peer memory, 2^24 elements per rank: inp
 outputs of 512 MiB together exceed the 126 MB L2 while staying far below a few GB);
 wgrad / wgrad_2cta (tcgen05 weight-gradient GEMM, one CTA per 128x256 tile / two CTAs per
 256x256 tile, BERT FFN shape 8192 x 4096 x 1024);
+wgrad_split (the same with K split over two pairs of CTAs per tile, 8192 x 1024 x 1024);
 wgrad_fc6 (VGG fc6 shape, K = 32: output-bandwidth bound);
 local_copy (what `bench.py --gpus 1` times: a one-worker, out-of-place float_sum allreduce of
-2^26 elements through the Context, i.e. LocalCopyKernel over 256 MiB in and 256 MiB out).
+2^26 elements through the Context, i.e. LocalCopyKernel over 256 MiB in and 256 MiB out);
+local_quant (the same in the exact mode: LocalQuantKernel).
+The plain GEMMs are the kernels WgradWideKernel (one CTA) and WgradPairKernel (two).
 Prints CUDA-event timings.
 """
 import argparse
@@ -46,10 +49,12 @@ def main():
     ap.add_argument("--algo", default="staged", choices=["staged", "push"],
                     help="streamed aggregation: whole tiles through the slots, or shards pushed to their owners")
     a = ap.parse_args()
-    if a.kernel == "local_copy":
+    if a.kernel in ("local_copy", "local_quant"):
+        exact = a.kernel == "local_quant"
         import switchml_b200 as sml
         ctx = sml.Context.get_instance()
-        assert ctx.start(sml.make_config("cuda", packet_numel=256, mode="float_sum", launch="inline"))
+        assert ctx.start(sml.make_config("cuda", packet_numel=256, mode="int32_quant" if exact else "float_sum",
+                                         launch="inline"))
         numel = 1 << 26
         x = torch.rand(numel, device="cuda")
         y = torch.empty_like(x)
@@ -59,9 +64,9 @@ def main():
             job.stream_wait()
             job.release()
         ms = timed(one, a.iters)
-        assert torch.equal(x, y)
+        assert torch.allclose(x, y, rtol=0, atol=2.0 ** -30 if exact else 0.0)  # (blocks below 1: a grid of 2^-31)
         ctx.stop()
-        print("local_copy: %d elements, %.4f ms, %.0f GB/s read+write" % (numel, ms, 2 * numel * 4 / ms / 1e6))
+        print("%s: %d elements, %.4f ms, %.0f GB/s read+write" % (a.kernel, numel, ms, 2 * numel * 4 / ms / 1e6))
     elif a.kernel.startswith("allreduce"):
         from switchml_b200.ops.emulation import emulated_allreduce
         numel = 1 << a.log2_numel
@@ -74,15 +79,15 @@ def main():
         mode = "quant" if a.kernel == "allreduce_quant" else "sum"
         ms = timed(lambda: emulated_allreduce(xs, mode=mode, algo=a.algo, block_numel=256, slot_bytes=262144,
                                               slots_per_channel=4, outputs=outs), a.iters)
-        # includes allocation of the staging regions; the kernel itself is what ncu captures
-        print("%s (%s): %d ranks x %d elements, %.3f ms per call (with staging setup)" % (a.kernel, a.algo, a.ranks, numel, ms))
+        # with launch and two synchronisations; the kernel itself is what ncu captures
+        print("%s (%s): %d ranks x %d elements, %.3f ms per call" % (a.kernel, a.algo, a.ranks, numel, ms))
     else:
         from switchml_b200.ops.wgrad import wgrad_gemm
-        K, M, N = (32, 4096, 25088) if a.kernel == "wgrad_fc6" else (8192, 4096, 1024)
+        K, M, N = {"wgrad_fc6": (32, 4096, 25088), "wgrad_split": (8192, 1024, 1024)}.get(a.kernel, (8192, 4096, 1024))
         dy = torch.randn(K, M, device="cuda", dtype=torch.bfloat16)
         x = torch.randn(K, N, device="cuda", dtype=torch.bfloat16)
         out = torch.empty(M, N, device="cuda")
-        two = a.kernel == "wgrad_2cta"
+        two = a.kernel in ("wgrad_2cta", "wgrad_split")
         ms = timed(lambda: wgrad_gemm(dy, x, out=out, two_cta=two), a.iters)
         print("%s: K=%d M=%d N=%d, %.3f ms, %.0f TFLOP/s, output %.0f GB/s" %
               (a.kernel, K, M, N, ms, 2.0 * K * M * N / ms / 1e9, M * N * 4 / ms / 1e6))

@@ -1,12 +1,14 @@
 """Small, self-terminating workloads for profiling one kernel at a time on ONE GPU.
 
     python p4app-switchML_b200/benchmarks/profile_kernels.py --kernel allreduce_quant
-    ncu --set full --clock-control none -k regex:AllReduceEmuKernel -c 1 -o prof \
+    ncu --set full --clock-control none -k regex:AllReduceOneGpuKernel -c 1 -o prof \
         python p4app-switchML_b200/benchmarks/profile_kernels.py --kernel allreduce_quant
 
 Kernels: allreduce_quant / allreduce_sum / allreduce_int (streamed aggregation, 4 ranks
 emulated in one cooperative launch over peer memory, 2^24 elements per rank: inputs and
-outputs of 512 MiB together exceed the 126 MB L2 while staying far below a few GB);
+outputs of 512 MiB together exceed the 126 MB L2 while staying far below a few GB; messages of
+2^18 elements and more run AllReduceOneGpuKernel, shorter ones and the checked build, which
+SWITCHML_B200_LIBRARY selects, AllReduceEmuKernel);
 wgrad / wgrad_2cta (tcgen05 weight-gradient GEMM, one CTA per 128x256 tile / two CTAs per
 256x256 tile, BERT FFN shape 8192 x 4096 x 1024);
 wgrad_split (the same with K split over two pairs of CTAs per tile, 8192 x 1024 x 1024);

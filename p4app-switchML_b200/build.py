@@ -55,7 +55,7 @@ LIB_SOURCES = [
     "csrc/backends/cuda/driver_api.cc", "csrc/backends/cuda/fd_channel.cc",
     "csrc/backends/cuda/symmetric_memory.cc", "csrc/backends/cuda/cuda_backend.cc",
     "csrc/backends/cuda/emulated_allreduce.cc", "csrc/backends/cuda/host_allreduce.cc",
-    "csrc/kernels/allreduce_kernels.cu",
+    "csrc/kernels/allreduce_kernels.cu", "csrc/kernels/one_gpu_allreduce.cu",
     "csrc/capi/switchml_c.cc",
 ]
 GEMM_SOURCES = ["csrc/kernels/wgrad_gemm.cu", "csrc/kernels/linear_ops.cu"]

@@ -34,6 +34,7 @@ struct EmuWorkspace {
   int* status = nullptr;            // kMaxRanks words of pinned host memory that the kernel writes
   int* status_dev = nullptr;
   std::string layout;               // geometry that the flags and exponent words in `memory` belong to
+  unsigned long long epochs = 0;    // that any channel may have used since they were cleared
 
   ~EmuWorkspace() {
     int current = -1;
@@ -45,6 +46,7 @@ struct EmuWorkspace {
   }
 };
 
+constexpr unsigned long long kDirectNumel = 1ull << 18;
 constexpr size_t kL2Slots = size_t(44) << 20;  // of 126 MB: inputs and outputs stream through it as well
 
 constexpr size_t kEpochBytes = size_t(kMaxRanks) * kMaxChannels * sizeof(unsigned long long);
@@ -161,6 +163,16 @@ int EmulatedAllReduce(int nranks, void* const* in_ptrs, void* const* out_ptrs,
   if (max_channels < 1) max_channels = 1;
   if (channels > 0 && channels < max_channels) max_channels = channels;
 
+  // Every rank can address all tensors here, so that results may go straight into the outputs (one_gpu_allreduce.cu), for
+  // whole vectors of device memory. Below 2^18 elements per rank, where a message between GPUs takes neither of these
+  // algorithms but ALGO_ONESHOT, and in the checked build, the kernels run as they do between GPUs: that is what one
+  // looks at there (2 ranks push exact, whole calls: 2^18 elements 36 us with them and 28 straight, 2^22 72 and 46).
+  bool direct = (algo == ALGO_STAGED || algo == ALGO_PUSH) && numel >= kDirectNumel && !CheckedBuild();
+  uintptr_t bits = 0;
+  for (int r = 0; r < nranks; r++) bits |= reinterpret_cast<uintptr_t>(in_ptrs[r]) | reinterpret_cast<uintptr_t>(out_ptrs[r]);
+  if (bits & 15) direct = false;
+  for (int r = 0; direct && r < nranks; r++) direct = DeviceMemory(in_ptrs[r]) && DeviceMemory(out_ptrs[r]);  // 0.3 us each
+
   // Plain sums through the slots are bound by memory, and here every rank's slots share one L2: a ring that
   // stays in it spares each tile two trips to HBM (4 ranks x 2^24 float32: 272 us with 155 MB of slots, 200 us
   // with 43 MB; three slots of 64 to 96 KiB, two of 128 KiB and four of 64 KiB come to the same). The
@@ -168,7 +180,7 @@ int EmulatedAllReduce(int nranks, void* const* in_ptrs, void* const* out_ptrs,
   // upper bound there; the results do not depend on it.
   const size_t unit_bytes = static_cast<size_t>(nranks) * (block_numel > 128 ? block_numel : 128) * 4;
   const size_t ring = kL2Slots / (static_cast<size_t>(max_channels) * nranks);  // bytes of a channel's slots
-  if (algo == ALGO_STAGED && mode == MODE_SUM && numel * esz * nranks > kL2Slots && slot_bytes * slots_per_channel > ring) {
+  if (!direct && algo == ALGO_STAGED && mode == MODE_SUM && numel * esz * nranks > kL2Slots && slot_bytes * slots_per_channel > ring) {
     if (slots_per_channel > 3) slots_per_channel = 3;
     const size_t fits = ring / slots_per_channel / unit_bytes * unit_bytes;
     if (fits < slot_bytes) slot_bytes = fits > unit_bytes ? fits : unit_bytes;
@@ -186,27 +198,41 @@ int EmulatedAllReduce(int nranks, void* const* in_ptrs, void* const* out_ptrs,
   proto.quant_base = quant::QuantBase(nranks);
   proto.oneshot_bytes = oneshot_bytes;
   proto.timeout_ns = 2000000000ull;  // 2 s: generous for one GPU, still bounded
-  const size_t bytes = StagingBytes(slot_bytes, slots_per_channel, block_numel, max_channels,
+  JobArgs proto_job;
+  memset(&proto_job, 0, sizeof(proto_job));
+  proto_job.elem_type = elem_type;
+  proto_job.mode = mode;
+  proto_job.algo = algo;
+  if (direct && !OneGpuFits(proto, proto_job)) direct = false;
+  size_t bytes = StagingBytes(slot_bytes, slots_per_channel, block_numel, max_channels,
                                     oneshot_bytes, nranks, &proto.data_offset, &proto.exp_offset,
                                     &proto.oneshot_offset);
+  const size_t own_words = direct && mode == MODE_QUANT ? OneGpuExponentBytes(nranks, block_numel, max_channels) : 0;
+  if (own_words > 0) {
+    proto.exp_offset = bytes;
+    bytes += (own_words + 4095) / 4096 * 4096;
+  }
   proto.stage_bytes = ReportedStageBytes(bytes);
   if (algo == ALGO_PUSH && PushTileCapacity(proto, elem_type, mode) == 0)
     return fail("ALGO_PUSH needs at least two ranks and slots of about twice nranks * max(block, 128) * 4 bytes", -1);
 
   // Flags and exponent words of another layout are noise in this one, so they are cleared (with
-  // the epochs, which start over) when the layout changes, and only then.
+  // the epochs, which start over) when the layout changes, and only then; or when the epochs outgrow the tags of
+  // one_gpu_allreduce.cu, after hours.
   char layout[128];
-  snprintf(layout, sizeof(layout), "%d/%zu/%d/%d/%d/%zu", nranks, slot_bytes, slots_per_channel, block_numel, max_channels, bytes);
+  snprintf(layout, sizeof(layout), "%d/%d/%zu/%d/%d/%d/%zu", direct, nranks, slot_bytes, slots_per_channel, block_numel, max_channels, bytes);
   const size_t need = kHeadBytes + bytes * nranks;
   cudaError_t e = cudaSuccess;
   std::unique_ptr<EmuWorkspace> ws = WorkspacePool::Get().Take(dev, need, layout);
   if (!ws) ws = NewWorkspace(dev, need, &e);
   if (!ws) return fail(std::string("allocation failed: ") + cudaGetErrorString(e), -3);
   char* const stage0 = ws->memory + kHeadBytes;
-  if (ws->layout != layout) {
+  if (ws->layout != layout || ws->epochs > (1u << 23)) {
     ws->layout.clear();
+    ws->epochs = 0;
     e = cudaMemsetAsync(ws->memory, 0, kHeadBytes, 0);
     if (e == cudaSuccess) e = cudaMemset2DAsync(stage0, bytes, 0, proto.oneshot_offset, nranks, 0);
+    if (e == cudaSuccess && own_words > 0) e = cudaMemset2DAsync(stage0 + proto.exp_offset, bytes, 0, own_words, nranks, 0);
     if (e != cudaSuccess) return fail(std::string("allocation failed: ") + cudaGetErrorString(e), -3);
   }
 
@@ -234,7 +260,12 @@ int EmulatedAllReduce(int nranks, void* const* in_ptrs, void* const* out_ptrs,
       j.mode = mode;
       j.algo = algo;
       j.post_scale = post_scale;
-      if (it == 0 && algo != ALGO_ONESHOT) j.bulk_copy = DeviceMemory(j.in) && DeviceMemory(j.out);  // 0.3 us each
+      if (it == 0 && algo != ALGO_ONESHOT) j.bulk_copy = direct || (DeviceMemory(j.in) && DeviceMemory(j.out));
+      if (direct) {
+        j.out_zero_copy = 1;
+        for (int p = 0; p < nranks; p++) j.user_peer[p] = static_cast<char*>(out_ptrs[p]);
+        j.user_bytes = numel * esz;
+      }
       j.oneshot_parity = it & 1;
     }
     if (it == 0) {
@@ -245,6 +276,7 @@ int EmulatedAllReduce(int nranks, void* const* in_ptrs, void* const* out_ptrs,
       args.job[r].tile_elems = plan.tile_elems;
       args.job[r].epochs = plan.epochs;
     }
+    ws->epochs += plan.epochs;
     e = LaunchAllReduceEmulated(args, nranks, plan, 0);
     if (e != cudaSuccess) break;
   }

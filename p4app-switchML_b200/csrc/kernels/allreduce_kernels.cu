@@ -41,6 +41,7 @@
 #include "kernels/once_per_device.h"
 #include "kernels/quant_tile.cuh"
 #include "kernels/turns.cuh"
+#include "kernels/vector_sum.cuh"
 #include "switchml/quant_math.h"
 
 namespace switchml {
@@ -61,22 +62,6 @@ __device__ __forceinline__ bool Aligned16(const void* p) {
 
 __device__ __forceinline__ uint4 LoadCg16(const void* p) {
   return __ldcg(reinterpret_cast<const uint4*>(p));
-}
-
-// bf16 pair helpers -----------------------------------------------------------------
-__device__ __forceinline__ float2 Bf16x2ToFloat2(unsigned u) {
-  return make_float2(__uint_as_float(u << 16), __uint_as_float(u & 0xffff0000u));
-}
-__device__ __forceinline__ unsigned Float2ToBf16x2(float a, float b) {
-  __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
-  return *reinterpret_cast<unsigned*>(&h);
-}
-__device__ __forceinline__ float Bf16ToFloat(unsigned short u) {
-  return __uint_as_float(static_cast<unsigned>(u) << 16);
-}
-__device__ __forceinline__ unsigned short FloatToBf16(float f) {
-  __nv_bfloat16 h = __float2bfloat16_rn(f);
-  return *reinterpret_cast<unsigned short*>(&h);
 }
 
 // Of U steps of `n` threads each, those that a thread with `remaining` elements from its own on still has.
@@ -162,55 +147,6 @@ __device__ __forceinline__ uint4 ReduceVec(const RankCtx& ctx, char* const* peer
   }
   return r;
 }
-
-// 16-byte vector accumulators of the plain-sum mode.
-template <int ELEM> struct VecAcc;
-template <> struct VecAcc<ELEM_F32> {
-  float4 a;
-  __device__ __forceinline__ void Zero() { a = make_float4(0.f, 0.f, 0.f, 0.f); }
-  __device__ __forceinline__ void Init(uint4 v) { a = make_float4(__uint_as_float(v.x), __uint_as_float(v.y), __uint_as_float(v.z), __uint_as_float(v.w)); }
-  __device__ __forceinline__ void Add(uint4 v) { a.x += __uint_as_float(v.x); a.y += __uint_as_float(v.y); a.z += __uint_as_float(v.z); a.w += __uint_as_float(v.w); }
-  __device__ __forceinline__ uint4 Finish(float s) {
-    if (s != 1.0f) { a.x *= s; a.y *= s; a.z *= s; a.w *= s; }
-    return make_uint4(__float_as_uint(a.x), __float_as_uint(a.y), __float_as_uint(a.z), __float_as_uint(a.w));
-  }
-};
-template <> struct VecAcc<ELEM_I32> {
-  uint4 a;
-  __device__ __forceinline__ void Zero() { a = make_uint4(0, 0, 0, 0); }
-  __device__ __forceinline__ void Init(uint4 v) { a = v; }
-  __device__ __forceinline__ void Add(uint4 v) { a.x += v.x; a.y += v.y; a.z += v.z; a.w += v.w; }  // wrapping
-  __device__ __forceinline__ uint4 Finish(float) { return a; }
-};
-template <> struct VecAcc<ELEM_BF16> {
-  float a[8];
-  __device__ __forceinline__ void Zero() {
-#pragma unroll
-    for (int j = 0; j < 8; j++) a[j] = 0.f;
-  }
-  __device__ __forceinline__ void Init(uint4 v) {
-    float2 q;
-    q = Bf16x2ToFloat2(v.x); a[0] = q.x; a[1] = q.y;
-    q = Bf16x2ToFloat2(v.y); a[2] = q.x; a[3] = q.y;
-    q = Bf16x2ToFloat2(v.z); a[4] = q.x; a[5] = q.y;
-    q = Bf16x2ToFloat2(v.w); a[6] = q.x; a[7] = q.y;
-  }
-  __device__ __forceinline__ void Add(uint4 v) {
-    float2 q;
-    q = Bf16x2ToFloat2(v.x); a[0] += q.x; a[1] += q.y;
-    q = Bf16x2ToFloat2(v.y); a[2] += q.x; a[3] += q.y;
-    q = Bf16x2ToFloat2(v.z); a[4] += q.x; a[5] += q.y;
-    q = Bf16x2ToFloat2(v.w); a[6] += q.x; a[7] += q.y;
-  }
-  __device__ __forceinline__ uint4 Finish(float s) {
-    if (s != 1.0f) {
-#pragma unroll
-      for (int j = 0; j < 8; j++) a[j] *= s;
-    }
-    return make_uint4(Float2ToBf16x2(a[0], a[1]), Float2ToBf16x2(a[2], a[3]), Float2ToBf16x2(a[4], a[5]),
-                      Float2ToBf16x2(a[6], a[7]));
-  }
-};
 
 // Peer memory: U 16-byte vectors (at `off`, off + step, ...; those from `left` on are left alone) summed over
 // all ranks, post-scaled. Rank by rank with all U loads in flight (on one GPU those of several ranks where U is small);
@@ -1465,7 +1401,9 @@ LaunchPlan PlanLaunch(const RankCtx& ctx, const JobArgs& job, int requested_chan
   const unsigned long long numel = job.numel ? job.numel : 1;
   if (max_channels > kMaxChannels) max_channels = kMaxChannels;
   p.tile_elems = 0;
-  if (job.algo == ALGO_STAGED || job.algo == ALGO_PUSH) {
+  if (ctx.one_gpu && job.out_zero_copy) {
+    PlanOneGpu(ctx, job, requested_channels, max_channels, &p);
+  } else if (job.algo == ALGO_STAGED || job.algo == ALGO_PUSH) {
     size_t slot_elems = job.algo == ALGO_PUSH ? PushTileCapacity(ctx, job.elem_type, job.mode)
                                               : SlotElems(ctx, job.elem_type, job.mode);
     int ch = requested_channels > 0 ? requested_channels : max_channels;
@@ -1478,6 +1416,7 @@ LaunchPlan PlanLaunch(const RankCtx& ctx, const JobArgs& job, int requested_chan
                               (ctx.block_numel > 128 ? ctx.block_numel : 128);
     unsigned long long tile = (numel + 4ull * ch - 1) / (4ull * ch);
     if (ctx.one_gpu) {
+      // (Short messages and tensors off their boundaries; the others: one_gpu_allreduce.cu.)
       // Meeting costs little on one GPU, an idle SM as much as anywhere: one to four tiles of 4 Ki to 14 Ki
       // elements for every channel before they grow (2^18 elements were 16 tiles for 74 channels). Whole calls, this rule,
       // always four tiles, and tiles of at least 16 Ki as between GPUs: 2 ranks x 2^18 push exact 39 / 39 / 44 us, 2 x 2^20
@@ -1545,6 +1484,7 @@ cudaError_t LaunchAllReduce(const RankCtx& ctx, const JobArgs& job, const Launch
 cudaError_t LaunchAllReduceEmulated(const EmuArgs& args, int nranks, const LaunchPlan& plan,
                                     cudaStream_t stream) {
   if (nranks < 1 || nranks > kMaxRanks || plan.channels > kMaxChannels) return cudaErrorInvalidValue;
+  if (args.job[0].out_zero_copy) return LaunchOneGpuAllReduce(args, nranks, plan, stream);
   SML_DISPATCH(LaunchOneEmu, args.job[0].elem_type, args.job[0].mode, args.job[0].algo, args, nranks, plan, stream);
 }
 

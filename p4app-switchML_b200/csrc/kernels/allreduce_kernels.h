@@ -91,7 +91,8 @@ struct JobArgs {
   int bulk_copy;     // `in` and `out` are ordinary device memory of this GPU: whole-tile copies may go through the
                      // TMA unit (never set for pinned host or managed memory)
   int out_zero_copy; // ALGO_STAGED / ALGO_PUSH: `out` lies in the symmetric user region (user_* and out_offset are
-                     // set): finished shards are broadcast straight into every rank's output, no copy-out
+                     // set): finished shards are broadcast straight into every rank's output, no copy-out. With all
+                     // ranks on one GPU (one_gpu) user_peer are the outputs themselves
   unsigned long long tile_elems;  // ALGO_STAGED: elements per tile (<= elements of a slot)
   // ALGO_ZEROCOPY (and out_zero_copy): offsets of in/out inside the symmetric user region and its mappings
   char* user_peer[kMaxRanks];
@@ -158,6 +159,13 @@ struct EmuArgs {
 };
 cudaError_t LaunchAllReduceEmulated(const EmuArgs& args, int nranks, const LaunchPlan& plan,
                                     cudaStream_t stream);
+// ALGO_STAGED and ALGO_PUSH with out_zero_copy and all ranks on this GPU (one_gpu_allreduce.cu): whether the slots have
+// room for it, the bytes of its exponent words (RankCtx::exp_offset; cleared before the first use, and after 2^23 epochs at
+// the latest), its geometry, its launch (LaunchAllReduceEmulated comes here).
+size_t OneGpuExponentBytes(int nranks, int block_numel, int max_channels);
+bool OneGpuFits(const RankCtx& ctx, const JobArgs& job);
+void PlanOneGpu(const RankCtx& ctx, const JobArgs& job, int requested_channels, int max_channels, LaunchPlan* plan);
+cudaError_t LaunchOneGpuAllReduce(const EmuArgs& args, int nranks, const LaunchPlan& plan, cudaStream_t stream);
 // Single worker, plain sum, out of place: copy `bytes` bytes with one kernel.
 cudaError_t LaunchLocalCopy(const void* in, void* out, size_t bytes, cudaStream_t stream);
 // Single worker, exact mode (float32 or bfloat16, element-aligned): the quantise / dequantise round

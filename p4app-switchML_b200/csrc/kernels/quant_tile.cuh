@@ -95,8 +95,9 @@ __device__ __forceinline__ float GroupMaxima(const float (&v)[NV], int lane) {
 // start at multiples of 8 rows.
 // kLog2Block: log2 of the block size, so that all indexes are shifts (with the size known at run time
 // only, publishing a 16 Ki element tile took 9 us, most of it 64-bit divisions).
-template <int kLog2Block>
-__device__ __forceinline__ void PublishRows8As(const RankCtx& ctx, int lane, const float4* x, size_t row0, size_t exp_off, Epoch tag) {
+// `publish(block, exponent)` is called by one lane for each block.
+template <int kLog2Block, typename Publish>
+__device__ __forceinline__ void PublishRows8As(int lane, const float4* x, size_t row0, Publish publish) {
   constexpr int kLanes = kLog2Block >= 7 ? 32 : 1 << (kLog2Block - 2);  // lanes per block and row
   constexpr int kRowsPerBlock = kLog2Block >= 7 ? 1 << (kLog2Block - 7) : 1;
   constexpr int NV = 8 / kRowsPerBlock;
@@ -115,20 +116,26 @@ __device__ __forceinline__ void PublishRows8As(const RankCtx& ctx, int lane, con
   if ((lane & (kShare - 1)) == 0) {
     const int value = (lane & (kLanes - 1)) / kShare;  // which of the NV
     const size_t block = ((row0 * 128) >> kLog2Block) + (kLanes < 32 ? value * (32 / kLanes) + lane / kLanes : value);
-    ExpPublish(ctx, exp_off + block * kExpWordBytes, ExpWord(tag, quant::LocalExponent(mine)));
+    publish(block, quant::LocalExponent(mine));
   }
 }
 
+template <typename Publish>
+__device__ __forceinline__ void PublishRows8(int block_numel, int lane, const float4* x, size_t row0, Publish publish) {
+  switch (block_numel) {  // the same for all threads
+    case 32: return PublishRows8As<5>(lane, x, row0, publish);
+    case 64: return PublishRows8As<6>(lane, x, row0, publish);
+    case 128: return PublishRows8As<7>(lane, x, row0, publish);
+    case 256: return PublishRows8As<8>(lane, x, row0, publish);
+    case 512: return PublishRows8As<9>(lane, x, row0, publish);
+    default: return PublishRows8As<10>(lane, x, row0, publish);
+  }
+}
 __device__ __forceinline__ void PublishRows8(const RankCtx& ctx, int lane, const float4* x, size_t row0,
                                              size_t exp_off, Epoch tag) {
-  switch (ctx.block_numel) {  // the same for all threads
-    case 32: return PublishRows8As<5>(ctx, lane, x, row0, exp_off, tag);
-    case 64: return PublishRows8As<6>(ctx, lane, x, row0, exp_off, tag);
-    case 128: return PublishRows8As<7>(ctx, lane, x, row0, exp_off, tag);
-    case 256: return PublishRows8As<8>(ctx, lane, x, row0, exp_off, tag);
-    case 512: return PublishRows8As<9>(ctx, lane, x, row0, exp_off, tag);
-    default: return PublishRows8As<10>(ctx, lane, x, row0, exp_off, tag);
-  }
+  PublishRows8(ctx.block_numel, lane, x, row0, [&](size_t block, int exponent) {
+    ExpPublish(ctx, exp_off + block * kExpWordBytes, ExpWord(tag, exponent));
+  });
 }
 
 // The blocks [first_block, nblocks) of a tile, one block per warp and step, any element type

@@ -4,7 +4,10 @@ Kernels of different ranks wait for each other, so they cannot be tested as sepa
 launches on a single device. Instead one cooperative launch plays all ranks: its
 ``blockIdx.y`` is the rank, every rank's staging memory lives on the same device and the
 peer-memory code path runs unchanged (csrc/kernels/allreduce_kernels.cu,
-``AllReduceEmuKernel``). Used by the GPU tests and for kernel profiling on one device.
+``AllReduceEmuKernel``). Messages of 2^18 elements per rank and more ("staged" and "push") take
+pipelines made for ranks that share a GPU instead, whose results go straight into all outputs
+(csrc/kernels/one_gpu_allreduce.cu); the checked build of the library keeps to the kernels between
+GPUs at every size. Used by the GPU tests and for kernel profiling on one device.
 """
 import ctypes
 
@@ -23,9 +26,9 @@ def emulated_allreduce(inputs, mode="quant", algo="staged", block_numel=256, slo
     all on the current device). Returns the list of per-rank outputs. `exponent_lookahead`:
     tiles by which the exact mode's exponents run ahead of their data (-1: the library's default).
 
-    `slot_bytes` and `slots_per_channel` are taken as they are (rounded to whole units of a tile), but for plain sums
-    through the slots (mode "sum", algo "staged") of more than 44 MB over all ranks: there they are upper bounds, and the ring is cut
-    to what stays in L2 (csrc/backends/cuda/emulated_allreduce.cc). The results do not depend on either."""
+    `slot_bytes` and `slots_per_channel` are taken as they are (rounded to whole units of a tile) below 2^18 elements per rank. Above
+    they are upper bounds: tiles and rings are cut to what stays in L2 and in shared memory. The results do not depend on either, but
+    for the order in which plain sums add ("push": the owner of a shard first)."""
     import torch
     n = len(inputs)
     x0 = inputs[0]

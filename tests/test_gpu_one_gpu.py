@@ -1,0 +1,91 @@
+"""The aggregation pipelines for ranks that share a GPU (csrc/kernels/one_gpu_allreduce.cu), which messages of 2^18
+elements per rank and more take: against the CPU oracle, and with plain sums against float64."""
+import numpy as np
+import pytest
+import torch
+
+from switchml_b200.ops.emulation import emulated_allreduce
+from switchml_b200.ops.oracle import int_allreduce_oracle, quant_allreduce_oracle
+
+pytestmark = pytest.mark.gpu
+
+SMALLEST = 1 << 18
+
+
+def _inputs(n, numel, dtype, seed):
+    g = torch.Generator().manual_seed(seed)
+    if dtype == torch.int32:
+        return [torch.randint(-2 ** 30, 2 ** 30, (numel,), generator=g, dtype=dtype) for _ in range(n)]
+    xs = [((torch.rand(numel, generator=g) * 2 - 1) * 10.0 ** (r % 4 - 2)) for r in range(n)]
+    for x in xs:
+        x[1000:5000] = 0.0  # blocks of zeros
+        x[-3:] = 2.0 ** -100
+    return [x.to(dtype) for x in xs]
+
+
+# The last tile: full, one element, one short of a chunk, whole chunks and a ragged one; one channel: many more tiles than
+# slots, stages and exponent slots.
+@pytest.mark.parametrize("numel, channels", [(SMALLEST, 0), (SMALLEST + 1, 0), (8192 * 40 - 1, 1), (SMALLEST + 9 * 1024 + 5, 3)])
+@pytest.mark.parametrize("n, block, slot_bytes, slots", [(1, 256, 32768, 2), (2, 32, 131072, 1), (3, 1024, 12288, 3), (4, 64, 16384, 4),
+                                                        (5, 256, 65536, 5), (7, 64, 1, 2), (8, 1024, 32768, 1), (8, 256, 262144, 4)])
+@pytest.mark.parametrize("algo", ["staged", "push"])
+def test_exact(algo, n, block, slot_bytes, slots, numel, channels):
+    if algo == "push" and n == 1:
+        pytest.skip("pushing needs a peer")
+    for dtype in (torch.float32, torch.bfloat16):
+        xs = _inputs(n, numel, dtype, numel + n)
+        want = torch.from_numpy(quant_allreduce_oracle([x.float().numpy() for x in xs], block)).to(dtype)
+        for inplace in (False, True):
+            ys = [x.cuda() for x in xs]
+            outs = emulated_allreduce(ys, mode="quant", algo=algo, block_numel=block, slot_bytes=slot_bytes, slots_per_channel=slots,
+                                      channels=channels, repeats=1 if inplace else 2, outputs=ys if inplace else None)
+            for r, o in enumerate(outs):
+                assert torch.equal(o.cpu(), want), (dtype, inplace, r)
+
+
+@pytest.mark.parametrize("numel, channels", [(SMALLEST, 0), (SMALLEST + 1, 1), (SMALLEST + 16387, 3)])
+@pytest.mark.parametrize("n, slot_bytes, slots", [(1, 65536, 2), (2, 65536, 1), (3, 1536, 2), (4, 16384, 4), (6, 131072, 3), (8, 262144, 4)])
+@pytest.mark.parametrize("algo", ["staged", "push"])
+def test_plain_sums(algo, n, slot_bytes, slots, numel, channels):
+    if algo == "push" and n == 1:
+        pytest.skip("pushing needs a peer")
+    options = {"mode": "sum", "algo": algo, "slot_bytes": slot_bytes, "slots_per_channel": slots, "channels": channels}
+    xs = _inputs(n, numel, torch.int32, n)
+    for o in emulated_allreduce([x.cuda() for x in xs], **options):
+        assert np.array_equal(o.cpu().numpy(), int_allreduce_oracle([x.numpy() for x in xs]))
+    for dtype, eps in ((torch.float32, 2.0 ** -24), (torch.bfloat16, 2.0 ** -8)):  # half an ulp of 24 and of 8 bits
+        xs = _inputs(n, numel, dtype, n)
+        ys = [x.cuda() for x in xs]
+        outs = emulated_allreduce(ys, post_scale=0.5, outputs=ys, **options)
+        exact = sum(x.double() for x in xs) / 2
+        # n - 1 float32 additions (n for what they add to the last rounding), each off by half an ulp, and the result's rounding
+        bound = sum(x.double().abs() for x in xs) / 2 * (n * 2.0 ** -24) + exact.abs() * eps + 1e-38
+        assert bool(((outs[0].cpu().double() - exact).abs() <= bound).all()), dtype
+        for o in outs[1:]:
+            assert torch.equal(o, outs[0]), "all ranks hold the same bits"
+
+
+def test_values_that_are_not_finite():
+    """Infinities and NaN come out as between GPUs: as the same job in pieces below 2^18 elements gives them."""
+    n, numel, block = 2, SMALLEST, 64
+    xs = _inputs(n, numel, torch.float32, 5)
+    xs[0][64] = float("inf")
+    xs[1][128 * 64 + 3] = float("nan")
+    xs[1][300 * 64] = -float("inf")
+    xs[0][400 * 64] = 3.4e38
+    for algo in ("staged", "push"):
+        outs = emulated_allreduce([x.cuda() for x in xs], mode="quant", algo=algo, block_numel=block)
+        for at in range(0, numel, numel // 4):
+            part = emulated_allreduce([x[at:at + numel // 4].cuda() for x in xs], mode="quant", algo=algo, block_numel=block)
+            for o, p in zip(outs, part):
+                assert torch.equal(o[at:at + numel // 4].view(torch.int32), p.view(torch.int32)), (algo, at)
+
+
+def test_a_rank_without_alignment_takes_the_streaming_kernels():
+    numel = SMALLEST + 7
+    xs = _inputs(2, numel + 1, torch.float32, 3)
+    ys = [xs[0].cuda()[1:], xs[1].cuda()[:-1]]
+    want = quant_allreduce_oracle([y.cpu().numpy() for y in ys], 64)
+    for algo in ("staged", "push"):
+        for o in emulated_allreduce(ys, mode="quant", algo=algo, block_numel=64):
+            assert np.array_equal(o.cpu().numpy(), want)

@@ -97,6 +97,18 @@ __device__ __forceinline__ bool EpilogueAny(bool yes) {
   return any != 0;
 }
 
+// Tile number `t`, in tiles from the top left corner. The shorter side comes first, so that the tiles that are multiplied
+// at the same time share strips of both operands: row by row, 3 x 79 tiles read X from memory once for every row
+// (2000 x 520 x 20000: 74.2 -> 65.3 us, 6000 x 800 x 16000: 197 -> 183; as many columns as rows: no difference).
+struct TilePlace {
+  int m, n;
+};
+__device__ __forceinline__ TilePlace PlaceOf(int t, int tiles_m, int tiles_n) {
+  const bool down = tiles_m < tiles_n;
+  const int side = down ? tiles_m : tiles_n, q = t / side, r = t - q * side;
+  return {down ? r : q, down ? q : r};
+}
+
 template <int TN, int kSplits>
 __global__ void __launch_bounds__(kPairThreads, 1)
 WgradPairKernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
@@ -148,8 +160,9 @@ WgradPairKernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
     if (lane == 0) {
       uint32_t it = 0;
       for (int tile = first_tile; tile < num_tiles && !sh.abort; tile += stride) {
-        const int m0 = (tile / tiles_n) * 256 + static_cast<int>(side) * 128;
-        const int n0 = (tile % tiles_n) * TN + static_cast<int>(side) * (TN / 2);
+        const TilePlace at = PlaceOf(tile, tiles_m, tiles_n);
+        const int m0 = at.m * 256 + static_cast<int>(side) * 128;
+        const int n0 = at.n * TN + static_cast<int>(side) * (TN / 2);
         for (int kb = kb0; kb < kb1; kb++, it++) {
           const int s = it % kStages;
           if (!MbarWait(&sh.empty[s], ((it / kStages) & 1) ^ 1, &sh.abort)) break;
@@ -215,11 +228,12 @@ WgradPairKernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
         ok = MbarWait(&sh.acc_full[acc], (local_tile >> 1) & 1, &sh.abort);
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const TilePlace at = PlaceOf(tile, tiles_m, tiles_n);
         for (int g = 0; g < kGroups; g++) {
           // The buffer is free once the store that used it last has read it.
           if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
           __syncwarp();
-          StoreBox32(lanes + acc * TN + g * kEpiCols, sh.epi[e], lane, &map_d, (tile % tiles_n) * TN + g * kEpiCols, (tile / tiles_n) * 256 + m);
+          StoreBox32(lanes + acc * TN + g * kEpiCols, sh.epi[e], lane, &map_d, at.n * TN + g * kEpiCols, at.m * 256 + m);
         }
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncwarp();
@@ -232,9 +246,10 @@ WgradPairKernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
       if (EpilogueAny(ok)) {
         LetNextKernelStart();
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const TilePlace at = PlaceOf(last, tiles_m, tiles_n);
         for (int g = half * (kGroups / 2); g < (half + 1) * (kGroups / 2); g++)
           StoreBox32(lanes + acc * TN + g * kEpiCols, &sh.stage[0][0] + (g * 4 + quarter) * (32 * 128), lane, &map_d,
-                     (last % tiles_n) * TN + g * kEpiCols, (last / tiles_n) * 256 + m);
+                     at.n * TN + g * kEpiCols, at.m * 256 + m);
       }
     }
   }
@@ -243,8 +258,9 @@ WgradPairKernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
     ClusterSync();  // every pair's partial sums are in place
     if (warp >= 4 && !sh.abort) {
       const int quarter = warp & 3, half = (warp - 4) >> 2;
-      const int m0 = (first_tile / tiles_n) * 256 + static_cast<int>(side) * 128 + quarter * 32;
-      const int n0 = (first_tile % tiles_n) * TN;
+      const TilePlace at = PlaceOf(first_tile, tiles_m, tiles_n);
+      const int m0 = at.m * 256 + static_cast<int>(side) * 128 + quarter * 32;
+      const int n0 = at.n * TN;
       constexpr int mine = kGroups / kSplits;
       for (int i = half; i < mine; i += 2) {
         const int g = share * mine + i;

@@ -19,12 +19,14 @@
 // under this load is 1.6 to 1.9 GHz.
 //
 // The epilogue's warps store 32 rows each on their own (StoreBox32) and never wait for one another. While later
-// tiles are multiplied four of them do it, through one 4 KiB buffer each: eight warps' bursts of stores hold up the
-// main loop's loads (4096 x 8192 x 2048: 118 -> 124 us), and buffers beyond that would cost a stage of operands
-// (8192 x 4096 x 1024: 61.9 -> 63.1 us). A pair's last tile, which nothing hides, goes out by all eight through the
-// stages, every box of a warp in flight.
+// tiles are multiplied four of them do it: eight warps' bursts of stores hold up the main loop's loads (4096 x 8192 x 2048:
+// 118 -> 124 us). So do two boxes of a warp in flight, where the main loop is long enough to hide them one by one
+// (1024 x 4096 x 4096: 38.1 -> 39.9 us, 2000 x 10000 x 4000: 147 -> 157); up to kShortKBlocks it is not, and a warp has two buffers of
+// 4 KiB (559 x 680 x 13744: 24.2 -> 22.7 us, 640 x 8192 x 8192: 105 -> 99). A pair's last tile, which nothing hides, goes
+// out by all eight through the stages, every box of a warp in flight.
 constexpr int kPairThreads = 384;
 constexpr int kPairEpiWarps = 8;
+constexpr int kShortKBlocks = 14;  // 900 rows: 900 x 3000 x 3000 24.4 and 24.0 us with one and with two buffers
 constexpr uint32_t kPeerBitMask = 0xFEFFFFFFu;  // clears the lowest CTA-rank bit of a shared::cluster address
 constexpr int kPairABytes = kTileK * 128 * 2;   // 128 rows of A: 16 KiB
 
@@ -34,7 +36,7 @@ struct __align__(1024) PairShared {
   static constexpr int kBBytes = kTileK * (TN / 2) * 2;
   static constexpr int kStageBytes = kPairABytes + kBBytes;
   uint8_t stage[kStages][kStageBytes];  // later this CTA's part of the last tile, or its partial sums: 128 rows x TN fp32
-  uint8_t epi[4][32 * 128];
+  uint8_t epi[4][2][32 * 128];
   uint64_t full[kStages];
   uint64_t empty[kStages];
   uint64_t acc_full[2];
@@ -221,6 +223,7 @@ WgradPairKernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
     } else {
       const int last = first_tile + (num_tiles - 1 - first_tile) / stride * stride;
       const int m = static_cast<int>(side) * 128 + quarter * 32;
+      const bool two_bufs = all_k_blocks <= kShortKBlocks;
       uint32_t local_tile = 0;
       bool ok = half == 0;
       for (int tile = first_tile; tile < last && ok; tile += stride, local_tile++) {
@@ -231,9 +234,12 @@ WgradPairKernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
         const TilePlace at = PlaceOf(tile, tiles_m, tiles_n);
         for (int g = 0; g < kGroups; g++) {
           // The buffer is free once the store that used it last has read it.
-          if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+          if (lane == 0) {
+            if (two_bufs) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+            else asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+          }
           __syncwarp();
-          StoreBox32(lanes + acc * TN + g * kEpiCols, sh.epi[e], lane, &map_d, at.n * TN + g * kEpiCols, at.m * 256 + m);
+          StoreBox32(lanes + acc * TN + g * kEpiCols, sh.epi[e][two_bufs ? g & 1 : 0], lane, &map_d, at.n * TN + g * kEpiCols, at.m * 256 + m);
         }
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncwarp();

@@ -727,9 +727,10 @@ cudaError_t LaunchPairs(const CUtensorMap& map_a, const CUtensorMap& map_b, cons
 // The plan with the least estimated time. A k-block costs about the same with either tile width (both
 // are bound by getting A into and out of shared memory), so narrow tiles pay only where they make
 // more of too few tiles; `fixed` is what a tile costs besides, in k-blocks, adding up partial sums included
-// (fitted to 18 shapes). 33 clusters of four CTAs and 15 of eight find room at the same time.
+// (fitted to 18 shapes; 17 to 33 tiles wide split from 13 k-blocks on only: 2048 x 1024 at K = 384 8.4 us split and 7.4 not, at K = 1024
+// 10.1 and 10.5). 33 clusters of four CTAs and 15 of eight find room at the same time.
 PairPlan PlanPairs(int M, int N, int K, int sms) {
-  static const struct { int tn, splits; double fixed; } kinds[] = {{256, 1, 22}, {256, 2, 24}, {128, 2, 18}, {256, 4, 30}, {128, 4, 24}};
+  static const struct { int tn, splits; double fixed; } kinds[] = {{256, 1, 22}, {256, 2, 28}, {128, 2, 18}, {256, 4, 30}, {128, 4, 22}};
   const int k_blocks = (K + kTileK - 1) / kTileK;
   PairPlan best = {256, 1, 1};
   double least = 1e30;
@@ -778,13 +779,22 @@ extern "C" int switchml_wgrad_gemm_2cta(const void* dy, const void* x, float* dw
   return Launched(launch(map_a, map_b, map_d, M, N, K, plan, error_flag, stream));
 }
 
-// Up to K = 512 the one-CTA kernel's smaller tiles and open epilogue win, whatever the number of tiles (one CTA against two,
-// back to back: 512 x 4096 x 1024 8.6 and 9.2 us, 300 x 8192 x 8192 57 and 70, 512 x 8192 x 8192 80 and 87, 512 x 4096 x
-// 25088 136 and 150); beyond it the pairs' halved traffic for X does (640 x 8192 x 8192: 102 and 97, 768 x 4096 x 4096: 36
-// and 32.5). Around the line they differ by a few percent.
+// One CTA or two per tile, by what both took (back to back, us, one and two):
+//   K > 512: two, for the pairs' halved traffic for X (640 x 8192 x 8192: 111 and 102, 640 x 4096 x 4096: 32 and 29).
+//   Fewer: one, for its smaller tiles and open epilogue (512 x 8192 x 8192: 92 and 95, 256 x 4096 x 4096: 18.0 and 20.8,
+//   512 x 4096 x 1024: 8.2 and 8.6), but
+//   - few tiles are split over pairs that add up in shared memory (512 x 512 x 512 7.6 and 6.2, 256 x 1024 x 1024: 6.4 and 6.2,
+//     192 x 1024 x 1024: 5.9 and 6.1);
+//   - rows that are not whole lines of 128 bytes make loads cost half as much again, and the pairs load less: with more tiles than
+//     pairs from K = 384 on (448 x 3000 x 3000: 16.8 and 15.3, 512 x 6000 x 2000: 22.5 and 20.9, 384 x 6000 x 2000: 18.7 and 19.0), with
+//     at most half as many, where a tile's epilogue is hidden by nothing in either kernel, as with few tiles (384 x 1200 x
+//     1000: 8.3 and 7.6). Between them the one-CTA kernel keeps ahead (512 x 2000 x 2000: 8.6 and 9.0).
 extern "C" int switchml_wgrad_gemm_auto(const void* dy, const void* x, float* dw, int M, int N, int K, int* error_flag,
                                         void* stream) {
-  if (K > 512) return switchml_wgrad_gemm_2cta(dy, x, dw, M, N, K, error_flag, stream);
+  const long long tiles = static_cast<long long>((M + 255) / 256) * ((N + 255) / 256);
+  const bool ragged = (M | N) % 64 != 0;
+  const bool two = K > 512 || (K > 384 && ragged && tiles > 74) || (K > 192 && tiles <= (ragged ? 33 : 16));
+  if (two) return switchml_wgrad_gemm_2cta(dy, x, dw, M, N, K, error_flag, stream);
   return switchml_wgrad_gemm(dy, x, dw, M, N, K, nullptr, error_flag, stream);
 }
 

@@ -87,16 +87,13 @@ cudaError_t LaunchLocalCopyImpl(const void* in, void* out, size_t bytes, cudaStr
 
 // ---- exact mode ------------------------------------------------------------------------
 template <int BYTES> struct RawVec;
-template <> struct RawVec<16> { uint4 v; };
 template <> struct RawVec<8> { uint2 v; };
 template <> struct RawVec<4> { unsigned v; };
 template <> struct RawVec<2> { unsigned short v; };
 
-__device__ __forceinline__ unsigned RawWord(const RawVec<16>& r, int i) { return i == 0 ? r.v.x : i == 1 ? r.v.y : i == 2 ? r.v.z : r.v.w; }
 __device__ __forceinline__ unsigned RawWord(const RawVec<8>& r, int i) { return i == 0 ? r.v.x : r.v.y; }
 __device__ __forceinline__ unsigned RawWord(const RawVec<4>& r, int) { return r.v; }
 __device__ __forceinline__ unsigned RawWord(const RawVec<2>& r, int) { return r.v; }
-__device__ __forceinline__ void SetRawWord(RawVec<16>& r, int i, unsigned w) { if (i == 0) r.v.x = w; else if (i == 1) r.v.y = w; else if (i == 2) r.v.z = w; else r.v.w = w; }
 __device__ __forceinline__ void SetRawWord(RawVec<8>& r, int i, unsigned w) { if (i == 0) r.v.x = w; else r.v.y = w; }
 __device__ __forceinline__ void SetRawWord(RawVec<4>& r, int, unsigned w) { r.v = w; }
 __device__ __forceinline__ void SetRawWord(RawVec<2>& r, int, unsigned w) { r.v = static_cast<unsigned short>(w); }
@@ -108,6 +105,56 @@ __device__ __forceinline__ float Larger(float a, float b) {
   float r;
   asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
   return r;
+}
+
+// The largest of each quantisation block, in every lane and row that holds some of it: m[u] is what a lane has of row u. A
+// block is a power of two of lanes of one row of 2^kLog2Row elements, or of whole rows.
+template <int kRows, int kLog2Row, bool kNan>
+__device__ __forceinline__ void BlockMaxima(float (&m)[kRows], int log2_block) {
+  if (log2_block < kLog2Row) {
+    const int lanes = 1 << (log2_block - (kLog2Row - 5));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      if (o < lanes) {  // warp-uniform
+#pragma unroll
+        for (int u = 0; u < kRows; u++) m[u] = Larger<kNan>(m[u], __shfl_xor_sync(0xffffffffu, m[u], o));
+      }
+    }
+  } else {
+    // Fold a block's rows into its first, one butterfly per block, and hand the maximum back.
+    const int rows = 1 << (log2_block - kLog2Row);
+#pragma unroll
+    for (int span = 1; span < kRows; span <<= 1) {
+      if (span < rows) {
+#pragma unroll
+        for (int u = 0; u + span < kRows; u += 2 * span) m[u] = Larger<kNan>(m[u], m[u + span]);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < kRows; u++) {
+      if ((u & (rows - 1)) != 0) continue;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) m[u] = Larger<kNan>(m[u], __shfl_xor_sync(0xffffffffu, m[u], o));
+    }
+#pragma unroll
+    for (int span = kRows / 2; span >= 1; span >>= 1) {
+      if (span < rows) {
+#pragma unroll
+        for (int u = 0; u + span < kRows; u += 2 * span) m[u + span] = m[u];
+      }
+    }
+  }
+}
+
+template <int ELEM>
+__device__ __forceinline__ float LoadElement(const char* p, int i) {
+  if (ELEM == ELEM_BF16) return __uint_as_float(static_cast<unsigned>(reinterpret_cast<const unsigned short*>(p)[i]) << 16);
+  return reinterpret_cast<const float*>(p)[i];
+}
+template <int ELEM>
+__device__ __forceinline__ void StoreElement(char* p, int i, float x) {
+  if (ELEM == ELEM_BF16) reinterpret_cast<__nv_bfloat16*>(p)[i] = __float2bfloat16_rn(x);
+  else reinterpret_cast<float*>(p)[i] = x;
 }
 
 // One chunk of kQuantChunk elements by one warp, in vectors of VB bytes (of VE elements): vector
@@ -126,7 +173,7 @@ __device__ __forceinline__ bool LocalQuantChunk(const char* in, char* out, int l
   constexpr int kEsz = ELEM == ELEM_BF16 ? 2 : 4;
   constexpr int VE = VB / kEsz;
   constexpr int kRows = kQuantChunk / (32 * VE);
-  constexpr int kLog2Row = (VE == 8 ? 8 : VE == 4 ? 7 : VE == 2 ? 6 : 5);
+  constexpr int kLog2Row = (VE == 4 ? 7 : VE == 2 ? 6 : 5);
   constexpr int kWords = VB >= 4 ? VB / 4 : 1;
   RawVec<VB> x[kRows];
 #pragma unroll
@@ -152,39 +199,7 @@ __device__ __forceinline__ bool LocalQuantChunk(const char* in, char* out, int l
       }
     }
   }
-  if (log2_block < kLog2Row) {
-    const int lanes = 1 << (log2_block - (kLog2Row - 5));
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      if (o < lanes) {  // warp-uniform
-#pragma unroll
-        for (int u = 0; u < kRows; u++) m[u] = Larger<kFast>(m[u], __shfl_xor_sync(0xffffffffu, m[u], o));
-      }
-    }
-  } else {
-    // Fold a block's rows into its first, one butterfly per block, and hand the maximum back.
-    const int rows = 1 << (log2_block - kLog2Row);
-#pragma unroll
-    for (int span = 1; span < kRows; span <<= 1) {
-      if (span < rows) {
-#pragma unroll
-        for (int u = 0; u + span < kRows; u += 2 * span) m[u] = Larger<kFast>(m[u], m[u + span]);
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < kRows; u++) {
-      if ((u & (rows - 1)) != 0) continue;
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) m[u] = Larger<kFast>(m[u], __shfl_xor_sync(0xffffffffu, m[u], o));
-    }
-#pragma unroll
-    for (int span = kRows / 2; span >= 1; span >>= 1) {
-      if (span < rows) {
-#pragma unroll
-        for (int u = 0; u + span < kRows; u += 2 * span) m[u + span] = m[u];
-      }
-    }
-  }
+  BlockMaxima<kRows, kLog2Row, kFast>(m, log2_block);
   if (kFast) {
     bool odd = false;
 #pragma unroll
@@ -224,7 +239,137 @@ __device__ __forceinline__ bool LocalQuantChunk(const char* in, char* out, int l
   return true;
 }
 
+// The same chunk in whole 16-byte vectors where the first element lies S elements behind a 16-byte boundary, in the input
+// and in the output alike (a slice of a flat buffer). Vector v holds the elements v * VE - S to v * VE - S + VE - 1. The first S
+// of them belong to the block of the vector before it, of whatever block they are: they count for its
+// maximum, and its exponent is theirs, which takes a shuffle each way per row. The neighbours' elements in
+// the first vector are left alone, and the chunk's last S elements lie in a vector of the next chunk: both ends go
+// element by element. Vectors of one element, which such tensors used to go in, cost their instructions (2^25
+// elements in place, blocks of 64: bfloat16 one element off 64.5 us, float32 63.5; of 256: 51 and 50).
+//
+// kGuard: the chunk has only `valid` elements. False, and nothing done, as in LocalQuantChunk<kFast>.
+template <int ELEM, int S, bool kGuard>
+__device__ __forceinline__ bool LocalQuantRows(const char* in, char* out, int lane, int log2_block, int valid) {
+  constexpr int kEsz = ELEM == ELEM_BF16 ? 2 : 4, VE = 16 / kEsz;
+  constexpr int kRows = kQuantChunk / (32 * VE), kLog2Row = VE == 8 ? 8 : 7;
+  const uint4* const from = reinterpret_cast<const uint4*>(in - S * kEsz);
+  uint4* const to = reinterpret_cast<uint4*>(out - S * kEsz);
+  auto element = [&](int e) { return LoadElement<ELEM>(in, e); };
+  // Element i of a vector.
+  auto get = [](const uint4& v, int i) {
+    const unsigned w = ELEM == ELEM_BF16 ? (i < 2 ? v.x : i < 4 ? v.y : i < 6 ? v.z : v.w) : (i == 0 ? v.x : i == 1 ? v.y : i == 2 ? v.z : v.w);
+    return __uint_as_float(ELEM == ELEM_F32 ? w : i & 1 ? w & 0xffff0000u : w << 16);
+  };
+  auto put = [](float x[VE]) {
+    if constexpr (ELEM == ELEM_F32) {
+      return make_uint4(__float_as_uint(x[0]), __float_as_uint(x[1]), __float_as_uint(x[2]), __float_as_uint(x[3]));
+    } else {
+      unsigned w[4];
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        const __nv_bfloat162 h = __floats2bfloat162_rn(x[2 * i], x[2 * i + 1]);
+        w[i] = *reinterpret_cast<const unsigned*>(&h);
+      }
+      return make_uint4(w[0], w[1], w[2], w[3]);
+    }
+  };
+  uint4 x[kRows];
+#pragma unroll
+  for (int u = 0; u < kRows; u++) {
+    const int first = (u * 32 + lane) * VE - S;
+    if (!kGuard || first + VE <= valid) {
+      x[u] = from[u * 32 + lane];
+      if (S > 0 && u == 0 && lane == 0) {  // the chunk before this one's
+        float y[VE];
+#pragma unroll
+        for (int i = 0; i < VE; i++) y[i] = i < S ? 0.f : get(x[u], i);
+        x[u] = put(y);
+      }
+    } else {
+      float y[VE];
+#pragma unroll
+      for (int i = 0; i < VE; i++) y[i] = first + i >= 0 && first + i < valid ? element(first + i) : 0.f;
+      x[u] = put(y);
+    }
+  }
+  float end = 0.f;  // lane i: element i of the last S
+  const int at_end = kQuantChunk - S + lane;
+  if (S > 0 && lane < S && (!kGuard || at_end < valid)) end = element(at_end);
+  float m[kRows], low[kRows];
+#pragma unroll
+  for (int u = 0; u < kRows; u++) {
+    m[u] = low[u] = 0.f;
+#pragma unroll
+    for (int i = 0; i < VE; i++) {
+      if (i < S) low[u] = Larger<true>(low[u], fabsf(get(x[u], i)));
+      else m[u] = Larger<true>(m[u], fabsf(get(x[u], i)));
+    }
+  }
+  if (S > 0) {
+    float end_max = fabsf(end);
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) end_max = Larger<true>(end_max, __shfl_xor_sync(0xffffffffu, end_max, o));
+#pragma unroll
+    for (int u = 0; u < kRows; u++) {
+      const float next = u + 1 < kRows ? low[u + 1 < kRows ? u + 1 : u] : end_max;
+      m[u] = Larger<true>(m[u], __shfl_sync(0xffffffffu, lane == 0 ? next : low[u], (lane + 1) & 31));
+    }
+  }
+  BlockMaxima<kRows, kLog2Row, true>(m, log2_block);
+  bool odd = false;
+#pragma unroll
+  for (int u = 0; u < kRows; u++) odd |= !(m[u] < 0x1p127f);
+  if (__any_sync(0xffffffffu, odd)) return false;
+  auto trip = [](float v, float c) {
+    const float cv = __uint_as_float((__float_as_uint(v) & 0x80000000u) | __float_as_uint(c));
+    const float r = __fsub_rn(__fadd_rn(v, cv), cv);
+    return fabsf(v) < c ? r : v;
+  };
+  float c[kRows];
+#pragma unroll
+  for (int u = 0; u < kRows; u++) c[u] = __int_as_float((quant::ClampExponent(quant::LocalExponent(m[u])) - 8 + 127) << 23);
+#pragma unroll
+  for (int u = 0; u < kRows; u++) {
+    float before = c[u];
+    if (S > 0) before = __shfl_sync(0xffffffffu, lane == 31 && u > 0 ? c[u > 0 ? u - 1 : 0] : c[u], (lane + 31) & 31);
+    float y[VE];
+#pragma unroll
+    for (int i = 0; i < VE; i++) y[i] = trip(get(x[u], i), i < S ? before : c[u]);
+    const int first = (u * 32 + lane) * VE - S;
+    if ((!kGuard || first + VE <= valid) && !(S > 0 && u == 0 && lane == 0)) {
+      to[u * 32 + lane] = put(y);
+    } else {
+#pragma unroll
+      for (int i = 0; i < VE; i++)
+        if (first + i >= 0 && (!kGuard || first + i < valid)) StoreElement<ELEM>(out, first + i, y[i]);
+    }
+  }
+  if (S > 0) {
+    const float last = __shfl_sync(0xffffffffu, c[kRows - 1], 31);
+    if (lane < S && (!kGuard || at_end < valid)) StoreElement<ELEM>(out, at_end, trip(end, last));
+  }
+  return true;
+}
+
 // One chunk per warp; the last warp takes what is left over (fewer than kQuantChunk elements).
+template <int ELEM, int S>
+__global__ void __launch_bounds__(kQuantThreads)
+LocalQuantRowsKernel(const char* in, char* out, size_t numel, int log2_block, float base) {
+  WaitForEarlierKernels();
+  LetNextKernelStart();
+  constexpr int kEsz = ELEM == ELEM_BF16 ? 2 : 4;
+  const int lane = threadIdx.x & 31;
+  const size_t off = ((static_cast<size_t>(blockIdx.x) * kQuantThreads + threadIdx.x) >> 5) * kQuantChunk;
+  if (off >= numel) return;
+  const char* from = in + off * kEsz;
+  char* to = out + off * kEsz;
+  const int valid = static_cast<int>(numel - off < kQuantChunk ? numel - off : kQuantChunk);
+  const bool done = valid == kQuantChunk ? LocalQuantRows<ELEM, S, false>(from, to, lane, log2_block, valid)
+                                         : LocalQuantRows<ELEM, S, true>(from, to, lane, log2_block, valid);
+  if (!done) LocalQuantChunk<ELEM, kEsz, true, false>(from, to, lane, log2_block, base, valid);
+}
+
+// The same where input and output lie differently to a 16-byte boundary, in the widest vectors that both addresses allow.
 template <int ELEM, int VB>
 __global__ void __launch_bounds__(kQuantThreads)
 LocalQuantKernel(const char* in, char* out, size_t numel, int log2_block, float base) {
@@ -244,22 +389,34 @@ LocalQuantKernel(const char* in, char* out, size_t numel, int log2_block, float 
   }
 }
 
-// The widest vectors that both addresses allow. Narrow ones cost instructions, not bandwidth: a
-// warp's load still covers a contiguous stretch.
 template <int ELEM>
 cudaError_t LaunchLocalQuantElem(const void* in, void* out, size_t numel, int log2_block, float base, cudaStream_t stream) {
-  const uintptr_t both = reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out);
+  constexpr int kEsz = ELEM == ELEM_BF16 ? 2 : 4;
+  const uintptr_t a = reinterpret_cast<uintptr_t>(in), b = reinterpret_cast<uintptr_t>(out);
+  if ((a | b) % kEsz != 0) return cudaErrorInvalidValue;
   const size_t per_block = static_cast<size_t>(kQuantChunk) * (kQuantThreads / 32);
   const unsigned blocks = static_cast<unsigned>((numel + per_block - 1) / per_block);
-  const char* i = static_cast<const char*>(in);
-  char* o = static_cast<char*>(out);
   void (*kernel)(const char*, char*, size_t, int, float) = nullptr;
-  if ((both & 15) == 0) kernel = LocalQuantKernel<ELEM, 16>;
-  else if ((both & 7) == 0) kernel = LocalQuantKernel<ELEM, 8>;
-  else if ((both & 3) == 0) kernel = LocalQuantKernel<ELEM, 4>;
-  else if (ELEM == ELEM_BF16 && (both & 1) == 0) kernel = LocalQuantKernel<ELEM_BF16, 2>;
-  else return cudaErrorInvalidValue;
-  return LaunchOverlapped(kernel, blocks, kQuantThreads, 0, 1, stream, i, o, numel, log2_block, base);
+  if (((a ^ b) & 15) == 0) {
+    const int shift = static_cast<int>(a & 15) / kEsz;
+    if constexpr (ELEM == ELEM_BF16) {
+      static constexpr decltype(kernel) kShifted[8] = {LocalQuantRowsKernel<ELEM, 0>, LocalQuantRowsKernel<ELEM, 1>, LocalQuantRowsKernel<ELEM, 2>,
+                                                       LocalQuantRowsKernel<ELEM, 3>, LocalQuantRowsKernel<ELEM, 4>, LocalQuantRowsKernel<ELEM, 5>,
+                                                       LocalQuantRowsKernel<ELEM, 6>, LocalQuantRowsKernel<ELEM, 7>};
+      kernel = kShifted[shift];
+    } else {
+      static constexpr decltype(kernel) kShifted[4] = {LocalQuantRowsKernel<ELEM, 0>, LocalQuantRowsKernel<ELEM, 1>, LocalQuantRowsKernel<ELEM, 2>,
+                                                       LocalQuantRowsKernel<ELEM, 3>};
+      kernel = kShifted[shift];
+    }
+  } else if (((a | b) & 7) == 0) {
+    kernel = LocalQuantKernel<ELEM, 8>;
+  } else if (((a | b) & 3) == 0) {
+    kernel = LocalQuantKernel<ELEM, 4>;
+  } else {
+    kernel = LocalQuantKernel<ELEM, kEsz>;
+  }
+  return LaunchOverlapped(kernel, blocks, kQuantThreads, 0, 1, stream, static_cast<const char*>(in), static_cast<char*>(out), numel, log2_block, base);
 }
 
 }  // namespace

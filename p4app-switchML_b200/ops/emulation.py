@@ -12,6 +12,7 @@ GPUs at every size. Used by the GPU tests and for kernel profiling on one device
 import ctypes
 
 from .._native import lib, last_error, NativeError
+from ..parallel.context import _emulate
 
 ELEM = {"float32": 0, "int32": 1, "bfloat16": 2}
 MODE = {"sum": 0, "quant": 1}
@@ -29,6 +30,11 @@ def emulated_allreduce(inputs, mode="quant", algo="staged", block_numel=256, slo
     `slot_bytes` and `slots_per_channel` are taken as they are (rounded to whole units of a tile) below 2^18 elements per rank. Above
     they are upper bounds: tiles and rings are cut to what stays in L2 and in shared memory. The results do not depend on either, but
     for the order in which plain sums add ("push": the owner of a shard first)."""
+    if _emulate is not None and mode in MODE and algo in ALGO:
+        done = _emulate(inputs, outputs, MODE[mode], ALGO[algo], block_numel, slot_bytes, slots_per_channel, channels, post_scale,
+                        repeats, exponent_lookahead)
+        if done is not None:
+            return done
     import torch
     n = len(inputs)
     x0 = inputs[0]

@@ -123,27 +123,27 @@ class Job:
 
 
 def _load_native_jobs():
-    """(Job, submit) of lib/torch_switchml_jobs.so (csrc/torch/jobs.cc), which does what the class above and
-    ``all_reduce_async`` do for torch tensors; (Job, None) where it is not built."""
+    """(Job, submit, emulate) of lib/torch_switchml_jobs.so (csrc/torch/jobs.cc), which do what the class above,
+    ``all_reduce_async`` and ``emulated_allreduce`` do, for torch tensors; (Job, None, None) where it is not built."""
     import os
     path = library_path("torch_switchml_jobs.so")
     if _torch is None or not os.path.exists(path):
-        return Job, None
+        return Job, None, None
     import importlib.util
     spec = importlib.util.spec_from_file_location("torch_switchml_jobs", path)
     try:
         native = importlib.util.module_from_spec(spec)
         spec.loader.exec_module(native)
     except ImportError:  # built for another PyTorch
-        return Job, None
+        return Job, None, None
     l = lib()
     native.init([ctypes.cast(f, ctypes.c_void_p).value for f in
                  (l.sml_allreduce_async, l.sml_job_wait, l.sml_job_status, l.sml_job_stream_wait, l.sml_job_error,
-                  l.sml_job_release, l.sml_last_error)], _STATUS, NativeError)
-    return native.Job, native.submit
+                  l.sml_job_release, l.sml_last_error, l.sml_emu_allreduce)], _STATUS, NativeError)
+    return native.Job, native.submit, native.emulate
 
 
-Job, _submit = _load_native_jobs()
+Job, _submit, _emulate = _load_native_jobs()
 
 
 class Context:

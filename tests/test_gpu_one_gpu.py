@@ -89,3 +89,16 @@ def test_a_rank_without_alignment_takes_the_streaming_kernels():
     for algo in ("staged", "push"):
         for o in emulated_allreduce(ys, mode="quant", algo=algo, block_numel=64):
             assert np.array_equal(o.cpu().numpy(), want)
+
+
+def test_arguments_that_python_looks_at():
+    xs = [torch.ones(5000, device="cuda") * r for r in range(3)]
+    for seq in (xs, tuple(xs)):  # with and without the native call
+        for o in emulated_allreduce(seq, mode="sum"):
+            assert torch.equal(o, torch.full_like(o, 3.0))
+    with pytest.raises(AssertionError):
+        emulated_allreduce([xs[0], xs[1][:100]], mode="sum")
+    with pytest.raises(KeyError):
+        emulated_allreduce([x.double() for x in xs], mode="sum")
+    with pytest.raises(KeyError):
+        emulated_allreduce(xs, mode="maximum")

@@ -777,7 +777,10 @@ namespace kernels {
 namespace {
 
 // ------------------------------------------------------------------------------------
-template <int ELEM, int MODE>
+// kOneGpu: all ranks live on this GPU. A rank then parks its input in its own buffer only, and the others read it there:
+// posted stores to everybody spare a trip back over a link that is not there, and cost the stores (8 ranks x 262143, whole
+// calls: plain sums 38 -> 28 us, exact 47 -> 38; 4 x 65536 24.4 -> 22.7).
+template <int ELEM, int MODE, bool kOneGpu>
 __device__ void RunOneShot(const RankCtx& ctx, const JobArgs& job, int channel,
                            unsigned long long elems_per_channel, Epoch base, int* s_failed) {
   const int esz = ELEM == ELEM_BF16 ? 2 : 4;
@@ -849,6 +852,7 @@ __device__ void RunOneShot(const RankCtx& ctx, const JobArgs& job, int channel,
   }
 
   const size_t my_off = buf_off(ctx.rank);
+  const int first_peer = kOneGpu ? ctx.rank : 0, end_peer = kOneGpu ? ctx.rank + 1 : ctx.nranks;
   // ---- push my range to everybody ----
   if (Aligned16(in)) {
     size_t nvec = bytes / 16;
@@ -861,17 +865,20 @@ __device__ void RunOneShot(const RankCtx& ctx, const JobArgs& job, int channel,
         if (i + u * stride < nvec) v[u] = reinterpret_cast<const uint4*>(in)[i + u * stride];
 #pragma unroll
       for (int u = 0; u < U; u++)
-        if (i + u * stride < nvec) BroadcastVec(ctx, ctx.stage_peer, ctx.stage_mc, my_off + (i + u * stride) * 16, v[u]);
+        if (i + u * stride < nvec) {
+          if (kOneGpu) *reinterpret_cast<uint4*>(ctx.stage_peer[ctx.rank] + my_off + (i + u * stride) * 16) = v[u];
+          else BroadcastVec(ctx, ctx.stage_peer, ctx.stage_mc, my_off + (i + u * stride) * 16, v[u]);
+        }
     }
     for (size_t b = nvec * 16 + threadIdx.x * esz; b < bytes; b += blockDim.x * esz) {
-      for (int p = 0; p < ctx.nranks; p++) {
+      for (int p = first_peer; p < end_peer; p++) {
         if (esz == 4) *reinterpret_cast<unsigned*>(ctx.stage_peer[p] + my_off + b) = *reinterpret_cast<const unsigned*>(in + b);
         else *reinterpret_cast<unsigned short*>(ctx.stage_peer[p] + my_off + b) = *reinterpret_cast<const unsigned short*>(in + b);
       }
     }
   } else {
     for (size_t b = threadIdx.x * esz; b < bytes; b += blockDim.x * esz) {
-      for (int p = 0; p < ctx.nranks; p++) {
+      for (int p = first_peer; p < end_peer; p++) {
         if (esz == 4) *reinterpret_cast<unsigned*>(ctx.stage_peer[p] + my_off + b) = *reinterpret_cast<const unsigned*>(in + b);
         else *reinterpret_cast<unsigned short*>(ctx.stage_peer[p] + my_off + b) = *reinterpret_cast<const unsigned short*>(in + b);
       }
@@ -879,8 +886,10 @@ __device__ void RunOneShot(const RankCtx& ctx, const JobArgs& job, int channel,
   }
   if (!ChannelBarrier(ctx, channel, 3, epoch, s_failed)) return;
 
-  // ---- reduce the n local copies ----
-  char* mine = ctx.stage_peer[ctx.rank];
+  // ---- reduce the n copies ----
+  // Those of the ranks' are `apart` bytes from one another (on one GPU the staging regions lie side by side).
+  const char* const first_copy = ctx.stage_peer[kOneGpu ? 0 : ctx.rank] + buf_off(0);
+  const size_t apart = ctx.oneshot_bytes + (kOneGpu ? ctx.stage_bytes : 0);
   char* out = static_cast<char*>(job.out) + c0 * esz;
   if (MODE == MODE_QUANT) {
     // One warp per block: the largest magnitude over all ranks' copies gives the exponent, then
@@ -890,8 +899,8 @@ __device__ void RunOneShot(const RankCtx& ctx, const JobArgs& job, int channel,
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
     const size_t B = ctx.block_numel;
     const size_t nblocks = (len + B - 1) / B;
-    const size_t src_step = ctx.oneshot_bytes;
-    const char* src0 = mine + buf_off(0);
+    const size_t src_step = apart;
+    const char* src0 = first_copy;
     const bool wide_out = (reinterpret_cast<uintptr_t>(out) & (ELEM == ELEM_BF16 ? 7 : 15)) == 0;
     for (size_t b = warp; b < nblocks; b += nwarps) {
       const size_t base = b * B;
@@ -995,9 +1004,9 @@ __device__ void RunOneShot(const RankCtx& ctx, const JobArgs& job, int channel,
         VecAcc<ELEM> acc[U];
 #pragma unroll
         for (int u = 0; u < U; u++)
-          if (u < left) acc[u].Init(*reinterpret_cast<const uint4*>(mine + buf_off(0) + (v + u * stride) * 16));
+          if (u < left) acc[u].Init(*reinterpret_cast<const uint4*>(first_copy + (v + u * stride) * 16));
         for (int s = 1; s < ctx.nranks; s++) {
-          const char* src = mine + buf_off(s);
+          const char* src = first_copy + s * apart;
           uint4 t[U];
 #pragma unroll
           for (int u = 0; u < U; u++)
@@ -1015,11 +1024,11 @@ __device__ void RunOneShot(const RankCtx& ctx, const JobArgs& job, int channel,
     for (size_t i = first + threadIdx.x; i < len; i += blockDim.x) {
       if (ELEM == ELEM_I32) {
         unsigned acc = 0;
-        for (int s = 0; s < ctx.nranks; s++) acc += reinterpret_cast<const unsigned*>(mine + buf_off(s))[i];
+        for (int s = 0; s < ctx.nranks; s++) acc += reinterpret_cast<const unsigned*>(first_copy + s * apart)[i];
         reinterpret_cast<unsigned*>(out)[i] = acc;
       } else {
         float acc = 0.f;
-        for (int s = 0; s < ctx.nranks; s++) acc += LoadAsFloat<ELEM>(mine + buf_off(s), i);
+        for (int s = 0; s < ctx.nranks; s++) acc += LoadAsFloat<ELEM>(first_copy + s * apart, i);
         if (job.post_scale != 1.0f) acc *= job.post_scale;
         if (ELEM == ELEM_BF16) reinterpret_cast<unsigned short*>(out)[i] = FloatToBf16(acc);
         else reinterpret_cast<float*>(out)[i] = acc;
@@ -1123,7 +1132,7 @@ __device__ __forceinline__ void RunJob(const RankCtx& ctx, const JobArgs& job, i
     RunStaged<ELEM, MODE, kOneGpu>(ctx, job, channel, epc, base, reinterpret_cast<StagedShared*>(s_failed), s_sf);
   else if (ALGO == ALGO_PUSH)
     RunPush<ELEM, MODE, kOneGpu>(ctx, job, channel, epc, base, reinterpret_cast<StagedShared*>(s_failed), s_sf);
-  else if (ALGO == ALGO_ONESHOT) RunOneShot<ELEM, MODE>(ctx, job, channel, epc, base, s_failed);
+  else if (ALGO == ALGO_ONESHOT) RunOneShot<ELEM, MODE, kOneGpu>(ctx, job, channel, epc, base, s_failed);
   else if (ctx.use_multimem) RunZeroCopy<ELEM, kZeroCopyUnrollLink>(ctx, job, channel, epc, base, s_failed);
   else RunZeroCopy<ELEM, kZeroCopyUnrollPeer>(ctx, job, channel, epc, base, s_failed);
 }
@@ -1445,11 +1454,13 @@ LaunchPlan PlanLaunch(const RankCtx& ctx, const JobArgs& job, int requested_chan
     // Whole quantisation blocks per channel; a few CTAs are enough for small messages.
     unsigned long long unit = ctx.block_numel > 128 ? ctx.block_numel : 128;
     unsigned long long units = (numel + unit - 1) / unit;
-    // A few CTAs are enough for small messages; from 256 Ki elements on every SM takes part.
-    int ch = requested_channels > 0 ? requested_channels : (numel >= (256u << 10) ? max_channels : 64);
+    // A few CTAs are enough for small messages; from 256 Ki elements, and on one GPU, every SM takes part.
+    int ch = requested_channels > 0 ? requested_channels : (numel >= (256u << 10) || ctx.one_gpu ? max_channels : 64);
     if (ch > max_channels) ch = max_channels;
     unsigned long long per = (units + ch - 1) / ch;
-    unsigned long long min_per = (4096 + unit - 1) / unit;  // at least 4 Ki elements per CTA
+    // At least 4 Ki elements per CTA. Without links the meeting costs the same however many meet: 2 Ki (2 x 262143
+    // exact 24.2 -> 21.1 us, 4 x 16384 22.9 -> 20.3; 1 Ki is no faster).
+    unsigned long long min_per = ((ctx.one_gpu ? 2048 : 4096) + unit - 1) / unit;
     if (per < min_per) per = min_per;
     p.elems_per_channel = per * unit;
     p.channels = static_cast<int>((numel + p.elems_per_channel - 1) / p.elems_per_channel);

@@ -15,7 +15,7 @@ wgrad_split (the same with K split over two pairs of CTAs per tile, 8192 x 1024 
 wgrad_fc6 (VGG fc6 shape, K = 32: output-bandwidth bound);
 local_copy (what `bench.py --gpus 1` times: a one-worker, out-of-place float_sum allreduce of
 2^26 elements through the Context, i.e. LocalCopyKernel over 256 MiB in and 256 MiB out);
-local_quant (the same in the exact mode: LocalQuantKernel).
+local_quant (the same in the exact mode: LocalQuantRowsKernel).
 The plain GEMMs are the kernels WgradWideKernel (one CTA) and WgradPairKernel (two).
 Prints CUDA-event timings.
 """

@@ -15,6 +15,7 @@
 
 #include "kernels/allreduce_kernels.h"
 #include "kernels/dependent_launch.cuh"
+#include "kernels/warp_max.cuh"
 #include "switchml/quant_math.h"
 
 namespace switchml {
@@ -98,15 +99,6 @@ __device__ __forceinline__ void SetRawWord(RawVec<8>& r, int i, unsigned w) { if
 __device__ __forceinline__ void SetRawWord(RawVec<4>& r, int, unsigned w) { r.v = w; }
 __device__ __forceinline__ void SetRawWord(RawVec<2>& r, int, unsigned w) { r.v = static_cast<unsigned short>(w); }
 
-// The larger of two magnitudes. kNan: NaN if either is; else a NaN never wins.
-template <bool kNan>
-__device__ __forceinline__ float Larger(float a, float b) {
-  if (!kNan) return fmaxf(a, b);
-  float r;
-  asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
-  return r;
-}
-
 // The largest of each quantisation block, in every lane and row that holds some of it: m[u] is what a lane has of row u. A
 // block is a power of two of lanes of one row of 2^kLog2Row elements, or of whole rows.
 template <int kRows, int kLog2Row, bool kNan>
@@ -121,7 +113,7 @@ __device__ __forceinline__ void BlockMaxima(float (&m)[kRows], int log2_block) {
       }
     }
   } else {
-    // Fold a block's rows into its first, one butterfly per block, and hand the maximum back.
+    // Fold a block's rows into its first, one reduction per block, and hand the maximum back.
     const int rows = 1 << (log2_block - kLog2Row);
 #pragma unroll
     for (int span = 1; span < kRows; span <<= 1) {
@@ -132,9 +124,7 @@ __device__ __forceinline__ void BlockMaxima(float (&m)[kRows], int log2_block) {
     }
 #pragma unroll
     for (int u = 0; u < kRows; u++) {
-      if ((u & (rows - 1)) != 0) continue;
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) m[u] = Larger<kNan>(m[u], __shfl_xor_sync(0xffffffffu, m[u], o));
+      if ((u & (rows - 1)) == 0) m[u] = WarpLargest<kNan>(m[u]);
     }
 #pragma unroll
     for (int span = kRows / 2; span >= 1; span >>= 1) {
@@ -358,10 +348,11 @@ __device__ __noinline__ void LocalQuantSlow(const char* in, char* out, int lane,
 }
 
 // One chunk per warp; the last warp takes what is left over (fewer than kQuantChunk elements).
-// Three blocks per SM (float32, 80 registers) and four (bfloat16, 64) keep 96 and 64 KB in flight. With two and three, and
-// the slow way inlined: 25 MB float32 7.5 us instead of 6.7, bfloat16 8.5 instead of 8.1, 2^27 elements 168 instead of 155
+// Three blocks per SM (float32, 80 registers) and four (bfloat16, 64) keep 96 and 64 KB in flight. With two and three, the
+// slow way inlined, and maxima by shuffles in all of these: 25 MB float32 7.5 us instead of 6.7, bfloat16 8.5 instead of 8.1, 2^27 elements 168 instead of 155
 // and 96 instead of 84 (blocks of 256, in place), bfloat16 one element off 133 instead of 98. One block more
-// costs registers that the fast way needs (bfloat16 25 MB 10.6).
+// costs registers that the fast way needs (bfloat16 25 MB 10.6). With WarpLargest() instead of shuffles 25 MB take 6.2 and
+// 7.0 us, 2^27 elements of bfloat16 78.7 instead of 81.7, one element off 87.5 instead of 91.7.
 template <int ELEM, int S>
 __global__ void __launch_bounds__(kQuantThreads, ELEM == ELEM_BF16 ? 4 : 3)
 LocalQuantRowsKernel(const char* in, char* out, size_t numel, int log2_block, float base) {

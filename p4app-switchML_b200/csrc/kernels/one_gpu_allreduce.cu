@@ -21,8 +21,8 @@
 //   - MODE_SUM: two warps drive the TMA unit, each through a ring of its own and for every second tile, so that the end of
 //     one tile's stores is not waited for by the next tile.
 //   - The host passes all geometry; with divisions in it a warp's way through a tile was half again as long.
-// Kernel times against the streaming kernels, us: 2 ranks x 2^22 push exact 49 -> 23, 8 x 2^20 push exact 67 -> 27, 2 x 2^25
-// push exact 252 -> 130, 4 x 2^24 staged exact 276 -> 136, staged sum 174 -> 113, push sum 225 -> 114 (82 us at the
+// Kernel times against the streaming kernels, us: 2 ranks x 2^22 push exact 49 -> 22, 8 x 2^20 push exact 67 -> 26, 2 x 2^25
+// push exact 252 -> 128, 4 x 2^24 staged exact 276 -> 135, staged sum 174 -> 113, push sum 225 -> 114 (82 us at the
 // speed of memory). Tiles of half the size 20 to 60 % slower, twice as many slots up to 15 %, half as many 15 to 20 %.
 //
 // Flow control (S slots per channel, E = kExpRing exponent slots, A = kOneAhead; "through k": tiles up to k from everybody):

@@ -23,6 +23,7 @@
 #include "kernels/allreduce_kernels.h"
 #include "kernels/device_sync.cuh"
 #include "kernels/turns.cuh"
+#include "kernels/warp_max.cuh"
 #include "kernels/warp_stream.cuh"
 #include "switchml/quant_math.h"
 
@@ -62,11 +63,20 @@ __device__ __forceinline__ float4 LoadGroupAsFloat(const char* in, size_t group)
 }
 
 // Largest of each of NV values over groups of W neighbouring lanes: lane l returns the maximum of value
-// ((l % W) * NV) / W. The values are handed out while they are reduced (NV - 1 + log2(W / NV) shuffles
-// instead of NV * log2(W)).
+// ((l % W) * NV) / W. Whole warps have an instruction for it; otherwise the values are handed out while they are
+// reduced (NV - 1 + log2(W / NV) shuffles instead of NV * log2(W)).
 template <int NV, int W>
 __device__ __forceinline__ float GroupMaxima(const float (&v)[NV], int lane) {
   static_assert(NV <= W, "a lane returns one value");
+  if (W == 32) {
+    float mine = 0.f;
+#pragma unroll
+    for (int i = 0; i < NV; i++) {
+      const float all = WarpLargest<false>(v[i]);
+      if (lane / (W / NV) == i) mine = all;
+    }
+    return mine;
+  }
   float t[NV];
 #pragma unroll
   for (int i = 0; i < NV; i++) t[i] = v[i];

@@ -81,6 +81,24 @@ def test_values_that_are_not_finite():
                 assert torch.equal(o[at:at + numel // 4].view(torch.int32), p.view(torch.int32)), (algo, at)
 
 
+@pytest.mark.parametrize("block", [64, 128, 256, 512, 1024])
+def test_the_largest_of_a_block_wherever_it_lies(block):
+    """... with both signs, beside NaN, which never wins, and in blocks of nothing else than zeros of both signs."""
+    for numel in (1 << 17, SMALLEST):  # the streaming kernels, and those for ranks that share a GPU
+        xs = [x * 1e-3 for x in _inputs(2, numel, torch.float32, block)]
+        blocks = numel // block
+        at = torch.arange(blocks) * block + torch.arange(blocks) * 37 % block
+        xs[0][at] = torch.where(torch.arange(blocks) % 2 == 0, 1.0, -1.0) * 2.0 ** (torch.arange(blocks) % 40 - 20)
+        xs[1][at[::3] // block * block + (at[::3] + 5) % block] = float("nan")
+        for x in xs:
+            x.view(blocks, block)[::7] = 0.0
+            x.view(blocks, block)[::7, ::3] = -0.0
+        want = quant_allreduce_oracle([x.numpy() for x in xs], block)
+        for algo in ("staged", "push"):
+            for o in emulated_allreduce([x.cuda() for x in xs], mode="quant", algo=algo, block_numel=block):
+                assert np.array_equal(o.cpu().numpy().view(np.int32), want.view(np.int32)), (algo, numel)
+
+
 def test_a_rank_without_alignment_takes_the_streaming_kernels():
     numel = SMALLEST + 7
     xs = _inputs(2, numel + 1, torch.float32, 3)

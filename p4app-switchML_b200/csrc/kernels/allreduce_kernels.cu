@@ -892,102 +892,132 @@ __device__ void RunOneShot(const RankCtx& ctx, const JobArgs& job, int channel,
   const size_t apart = ctx.oneshot_bytes + (kOneGpu ? ctx.stage_bytes : 0);
   char* out = static_cast<char*>(job.out) + c0 * esz;
   if (MODE == MODE_QUANT) {
-    // One warp per block: the largest magnitude over all ranks' copies gives the exponent, then
-    // quantise, add, dequantise. Four elements per lane and load (the buffers and the blocks are
-    // vector aligned), the loads of all ranks in flight together: the buffers come out of L2, and a
-    // small message is nothing but these latencies.
+    // The largest magnitude over all ranks' copies of a block gives its exponent, then quantise, add, dequantise. Four elements
+    // per lane and load (the buffers and the blocks are vector aligned), the loads of all ranks in flight together: the
+    // buffers come out of L2, and a small message is nothing but these latencies.
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
     const size_t B = ctx.block_numel;
-    const size_t nblocks = (len + B - 1) / B;
     const size_t src_step = apart;
     const char* src0 = first_copy;
     const bool wide_out = (reinterpret_cast<uintptr_t>(out) & (ELEM == ELEM_BF16 ? 7 : 15)) == 0;
-    for (size_t b = warp; b < nblocks; b += nwarps) {
-      const size_t base = b * B;
-      const size_t n = len - base < B ? len - base : B;
-      // Elements from `i` on, of rank `s`; zero beyond the message.
-      auto load4 = [&](int s, size_t i) {
-        const char* src = src0 + s * src_step;
-        if (i + 4 <= n) return LoadGroupAsFloat<ELEM>(src, (base + i) / 4);
-        float4 x;
-        x.x = i < n ? LoadAsFloat<ELEM>(src, base + i) : 0.f;
-        x.y = i + 1 < n ? LoadAsFloat<ELEM>(src, base + i + 1) : 0.f;
-        x.z = i + 2 < n ? LoadAsFloat<ELEM>(src, base + i + 2) : 0.f;
-        x.w = 0.f;
-        return x;
-      };
-      // A block of up to 256 elements stays in registers between the two passes (kHeld float4 per rank).
-      constexpr int kHeld = 2;
-      const bool held = n <= kHeld * 128 && (n & 3) == 0;
-      float4 x[kHeld][kMaxRanks];
-      float m = 0.f;
-      auto largest = [&](float4 v) { m = fmaxf(m, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w)))); };  // a NaN never wins
-      if (held) {
+    // With 2, 4 or 8 ranks the scale factors are powers of two: dividing by them is multiplying by their reciprocals.
+    const bool pow2 = ctx.nranks > 1 && (ctx.nranks & (ctx.nranks - 1)) == 0;
+    constexpr int kRows = 2;  // of 128 elements, which stay in registers between the two passes
+    // Four elements per row and rank of a lane; zero beyond the message. Whole rows without a look at the lanes (with one, 8 ranks'
+    // 262143 bfloat16 took 42 us instead of 32).
+    auto load = [&](size_t base, float4 (&x)[kRows][kMaxRanks]) {
+      if (base + kRows * 128 <= len) {
 #pragma unroll
-        for (int h = 0; h < kHeld; h++) {
+        for (int h = 0; h < kRows; h++)
 #pragma unroll
           for (int s = 0; s < kMaxRanks; s++) {
             x[h][s] = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (s < ctx.nranks && h * 128 + lane * 4 < n) x[h][s] = LoadGroupAsFloat<ELEM>(src0 + s * src_step, base / 4 + h * 32 + lane);
+            if (s < ctx.nranks) x[h][s] = LoadGroupAsFloat<ELEM>(src0 + s * src_step, base / 4 + h * 32 + lane);
           }
-        }
-#pragma unroll
-        for (int h = 0; h < kHeld; h++) {
-#pragma unroll
-          for (int s = 0; s < kMaxRanks; s++) largest(x[h][s]);
-        }
-      } else {
-        for (size_t i = lane * 4; i < n; i += 128) {
-#pragma unroll
-          for (int s = 0; s < kMaxRanks; s++)
-            if (s < ctx.nranks) largest(load4(s, i));  // uniform
-        }
+        return;
       }
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-      const float sf = quant::ScaleFactorFromBase(quant::LocalExponent(m), ctx.quant_base);
-      auto add4 = [&](unsigned (&acc)[4], float4 v) {
-        acc[0] += static_cast<unsigned>(quant::Quantize(v.x, sf));
-        acc[1] += static_cast<unsigned>(quant::Quantize(v.y, sf));
-        acc[2] += static_cast<unsigned>(quant::Quantize(v.z, sf));
-        acc[3] += static_cast<unsigned>(quant::Quantize(v.w, sf));
-      };
-      auto finish = [&](size_t i, const unsigned (&acc)[4]) {
-        float y[4];
+      for (int h = 0; h < kRows; h++) {
+        const size_t i = base + h * 128 + lane * 4;
+#pragma unroll
+        for (int s = 0; s < kMaxRanks; s++) {
+          const char* src = src0 + s * src_step;
+          x[h][s] = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (s >= ctx.nranks || i >= len) continue;
+          x[h][s].x = LoadAsFloat<ELEM>(src, i);
+          if (i + 1 < len) x[h][s].y = LoadAsFloat<ELEM>(src, i + 1);
+          if (i + 2 < len) x[h][s].z = LoadAsFloat<ELEM>(src, i + 2);
+          if (i + 3 < len) x[h][s].w = LoadAsFloat<ELEM>(src, i + 3);
+        }
+      }
+    };
+    auto largest = [](float m, float4 v) { return fmaxf(m, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w)))); };  // a NaN never wins
+    auto add4 = [](unsigned (&acc)[4], float4 v, float sf) {
+      acc[0] += static_cast<unsigned>(quant::Quantize(v.x, sf));
+      acc[1] += static_cast<unsigned>(quant::Quantize(v.y, sf));
+      acc[2] += static_cast<unsigned>(quant::Quantize(v.z, sf));
+      acc[3] += static_cast<unsigned>(quant::Quantize(v.w, sf));
+    };
+    auto finish = [&](size_t i, const unsigned (&acc)[4], float sf) {
+      float y[4];
+      const float inv = __uint_as_float(0x7f000000u - __float_as_uint(sf));
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        y[j] = pow2 ? __int2float_rn(static_cast<int>(acc[j])) * inv : quant::Dequantize(static_cast<int>(acc[j]), sf);
+        if (job.post_scale != 1.0f) y[j] *= job.post_scale;
+      }
+      if (wide_out && i + 4 <= len) {
+        if (ELEM == ELEM_BF16) *reinterpret_cast<uint2*>(out + i * 2) = make_uint2(Float2ToBf16x2(y[0], y[1]), Float2ToBf16x2(y[2], y[3]));
+        else *reinterpret_cast<float4*>(out + i * 4) = make_float4(y[0], y[1], y[2], y[3]);
+      } else {
 #pragma unroll
         for (int j = 0; j < 4; j++) {
-          y[j] = quant::Dequantize(static_cast<int>(acc[j]), sf);
-          if (job.post_scale != 1.0f) y[j] *= job.post_scale;
+          if (i + j >= len) continue;
+          if (ELEM == ELEM_BF16) reinterpret_cast<unsigned short*>(out)[i + j] = FloatToBf16(y[j]);
+          else reinterpret_cast<float*>(out)[i + j] = y[j];
         }
-        if (wide_out && i + 4 <= n) {
-          if (ELEM == ELEM_BF16) *reinterpret_cast<uint2*>(out + (base + i) * 2) = make_uint2(Float2ToBf16x2(y[0], y[1]), Float2ToBf16x2(y[2], y[3]));
-          else *reinterpret_cast<float4*>(out + (base + i) * 4) = make_float4(y[0], y[1], y[2], y[3]);
+      }
+    };
+    auto sum = [&](const float4 (&x)[kMaxRanks], float sf, size_t i) {
+      unsigned acc[4] = {0, 0, 0, 0};
+#pragma unroll
+      for (int s = 0; s < kMaxRanks; s++)
+        if (s < ctx.nranks) add4(acc, x[s], sf);
+      if (i < len) finish(i, acc, sf);
+    };
+    if (B <= kRows * 128) {
+      // A warp takes two rows, whatever blocks they consist of: with a warp per block, blocks of 64 left three quarters of
+      // the lanes and registers idle. Whole calls on one GPU, blocks of 64: 8 x 131072 float32 34 -> 24 us, 8 x 262143
+      // 49 -> 30, 2 x 4096 bfloat16 21 -> 19; of 256: 8 x 262143 36 -> 29, 2 x 4096 as before.
+      for (size_t base = warp * (kRows * 128); base < len; base += nwarps * (kRows * 128)) {
+        float4 x[kRows][kMaxRanks];
+        float m[kRows];
+        load(base, x);
+#pragma unroll
+        for (int h = 0; h < kRows; h++) {
+          m[h] = 0.f;
+#pragma unroll
+          for (int s = 0; s < kMaxRanks; s++) m[h] = largest(m[h], x[h][s]);
+        }
+        if (B >= 128) {
+          if (B > 128) m[0] = m[1] = fmaxf(m[0], m[1]);
+          m[0] = WarpLargest<false>(m[0]);
+          m[1] = B > 128 ? m[0] : WarpLargest<false>(m[1]);
         } else {
 #pragma unroll
-          for (int j = 0; j < 4; j++) {
-            if (i + j >= n) continue;
-            if (ELEM == ELEM_BF16) reinterpret_cast<unsigned short*>(out)[base + i + j] = FloatToBf16(y[j]);
-            else reinterpret_cast<float*>(out)[base + i + j] = y[j];
+          for (int o = 8; o > 0; o >>= 1) {
+            if (o * 4 >= static_cast<int>(B)) continue;  // the same for all threads
+#pragma unroll
+            for (int h = 0; h < kRows; h++) m[h] = fmaxf(m[h], __shfl_xor_sync(0xffffffffu, m[h], o));
           }
         }
-      };
-      if (held) {
 #pragma unroll
-        for (int h = 0; h < kHeld; h++) {
-          const size_t i = h * 128 + lane * 4;
-          unsigned acc[4] = {0, 0, 0, 0};
-#pragma unroll
-          for (int s = 0; s < kMaxRanks; s++)
-            if (s < ctx.nranks) add4(acc, x[h][s]);
-          if (i < n) finish(i, acc);
+        for (int h = 0; h < kRows; h++) {
+          const float sf = quant::ScaleFactorFromBase(quant::LocalExponent(m[h]), ctx.quant_base);
+          sum(x[h], sf, base + h * 128 + lane * 4);
         }
-      } else {
-        for (size_t i = lane * 4; i < n; i += 128) {
-          unsigned acc[4] = {0, 0, 0, 0};
+      }
+    } else {
+      // A warp per block, by two rows: 8 x 4096 float32 in blocks of 1024 47 -> 26 us, 2 x 4096 30 -> 27 (by single rows with a
+      // look at every load: one trip to L2 after the other).
+      for (size_t base = warp * B; base < len; base += nwarps * B) {
+        const size_t end = len - base < B ? len : base + B;
+        float4 x[kRows][kMaxRanks];
+        float m = 0.f;
+#pragma unroll 1
+        for (size_t i = base; i < end; i += kRows * 128) {
+          load(i, x);
 #pragma unroll
-          for (int s = 0; s < kMaxRanks; s++)
-            if (s < ctx.nranks) add4(acc, load4(s, i));
-          finish(i, acc);
+          for (int h = 0; h < kRows; h++)
+#pragma unroll
+            for (int s = 0; s < kMaxRanks; s++) m = largest(m, x[h][s]);
+        }
+        const float sf = quant::ScaleFactorFromBase(quant::LocalExponent(WarpLargest<false>(m)), ctx.quant_base);
+#pragma unroll 1
+        for (size_t i = base; i < end; i += kRows * 128) {
+          load(i, x);
+          sum(x[0], sf, i + lane * 4);
+          sum(x[1], sf, i + 128 + lane * 4);
         }
       }
     }

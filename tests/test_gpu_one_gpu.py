@@ -99,6 +99,21 @@ def test_the_largest_of_a_block_wherever_it_lies(block):
                 assert np.array_equal(o.cpu().numpy().view(np.int32), want.view(np.int32)), (algo, numel)
 
 
+@pytest.mark.parametrize("block", [32, 64, 128, 256, 512, 1024])
+def test_one_barrier_exact_at_the_ends_of_rows_and_blocks(block):
+    for n in (1, 2, 3, 8):
+        for numel in (1, 127, 129, 255, 256, 257, 1023, 1025, 2048 + 130, 20000 + 3):
+            for dtype in (torch.float32, torch.bfloat16):
+                xs = _inputs(n, numel, dtype, numel + n)
+                want = torch.from_numpy(quant_allreduce_oracle([x.float().numpy() for x in xs], block)).to(dtype)
+                outs = [torch.full((numel + 2,), 7.0, dtype=dtype, device="cuda") for _ in range(n)]
+                views = [o[r % 2:r % 2 + numel] for r, o in enumerate(outs)]  # every other one begins beside a vector
+                emulated_allreduce([x.cuda() for x in xs], mode="quant", algo="oneshot", block_numel=block, outputs=views)
+                for r, o in enumerate(outs):
+                    assert torch.equal(views[r].cpu(), want), (n, numel, dtype)
+                    assert bool((o[:r % 2] == 7).all()) and bool((o[r % 2 + numel:] == 7).all())
+
+
 def test_a_rank_without_alignment_takes_the_streaming_kernels():
     numel = SMALLEST + 7
     xs = _inputs(2, numel + 1, torch.float32, 3)

@@ -150,6 +150,7 @@ int EmulatedAllReduce(int nranks, void* const* in_ptrs, void* const* out_ptrs,
     return code;
   };
   if (nranks < 1 || nranks > kMaxRanks) return fail("nranks out of range", -1);
+  if (block_numel < 1) return fail("block_numel out of range", -1);
   if (algo == ALGO_ZEROCOPY) return fail("zero-copy needs real symmetric memory", -1);
   if (slot_bytes / 4 / block_numel * slots_per_channel > 8192)
     return fail("slots_per_channel * slot_bytes / (4 * block_numel) exceeds 8192", -1);

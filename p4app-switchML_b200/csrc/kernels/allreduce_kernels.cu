@@ -777,6 +777,31 @@ namespace kernels {
 namespace {
 
 // ------------------------------------------------------------------------------------
+// Exact mode of RunOneShot for blocks that its rows do not hold: a warp per block, element by element. `src` + r * apart is
+// rank r's copy. Only ops/emulation.py comes here: a context's blocks are powers of two from 32 to 1024.
+template <int ELEM>
+__device__ __noinline__ void ReduceBlocksOfAnySize(int nranks, size_t B, float quant_base, const char* src, size_t apart, char* out,
+                                                   size_t len, float post_scale) {
+  const int lane = threadIdx.x & 31;
+  for (size_t base = (threadIdx.x >> 5) * B; base < len; base += (blockDim.x >> 5) * B) {
+    const size_t end = len - base < B ? len : base + B;
+    float m = 0.f;
+    for (size_t i = base + lane; i < end; i += 32)
+      for (int s = 0; s < nranks; s++) m = fmaxf(m, fabsf(LoadAsFloat<ELEM>(src + s * apart, i)));  // a NaN never wins
+    __syncwarp();
+    const float sf = quant::ScaleFactorFromBase(quant::LocalExponent(WarpLargest<false>(m)), quant_base);
+    for (size_t i = base + lane; i < end; i += 32) {
+      unsigned acc = 0;
+      for (int s = 0; s < nranks; s++) acc += static_cast<unsigned>(quant::Quantize(LoadAsFloat<ELEM>(src + s * apart, i), sf));
+      float y = quant::Dequantize(static_cast<int>(acc), sf);
+      if (post_scale != 1.0f) y *= post_scale;
+      if (ELEM == ELEM_BF16) reinterpret_cast<unsigned short*>(out)[i] = FloatToBf16(y);
+      else reinterpret_cast<float*>(out)[i] = y;
+    }
+    __syncwarp();
+  }
+}
+
 // kOneGpu: all ranks live on this GPU. A rank then parks its input in its own buffer only, and the others read it there:
 // posted stores to everybody spare a trip back over a link that is not there, and cost the stores (8 ranks x 262143, whole
 // calls: plain sums 38 -> 28 us, exact 47 -> 38; 4 x 65536 24.4 -> 22.7).
@@ -965,7 +990,9 @@ __device__ void RunOneShot(const RankCtx& ctx, const JobArgs& job, int channel,
         if (s < ctx.nranks) add4(acc, x[s], sf);
       if (i < len) finish(i, acc, sf);
     };
-    if (B <= kRows * 128) {
+    if (B < 4 || (B <= kRows * 128 ? (B & (B - 1)) != 0 : B % (kRows * 128) != 0)) {
+      ReduceBlocksOfAnySize<ELEM>(ctx.nranks, B, ctx.quant_base, src0, src_step, out, len, job.post_scale);
+    } else if (B <= kRows * 128) {
       // A warp takes two rows, whatever blocks they consist of: with a warp per block, blocks of 64 left three quarters of
       // the lanes and registers idle. Whole calls on one GPU, blocks of 64: 8 x 131072 float32 34 -> 24 us, 8 x 262143
       // 49 -> 30, 2 x 4096 bfloat16 21 -> 19; of 256: 8 x 262143 36 -> 29, 2 x 4096 as before.
@@ -1481,8 +1508,9 @@ LaunchPlan PlanLaunch(const RankCtx& ctx, const JobArgs& job, int requested_chan
     p.epochs = static_cast<unsigned>(tiles_per_channel);
     p.tiles = tiles;
   } else if (job.algo == ALGO_ONESHOT) {
-    // Whole quantisation blocks per channel; a few CTAs are enough for small messages.
+    // Whole quantisation blocks and whole vectors per channel; a few CTAs are enough for small messages.
     unsigned long long unit = ctx.block_numel > 128 ? ctx.block_numel : 128;
+    while (unit % ctx.block_numel != 0 || unit % 8 != 0) unit += ctx.block_numel > 128 ? ctx.block_numel : 8;
     unsigned long long units = (numel + unit - 1) / unit;
     // A few CTAs are enough for small messages; from 256 Ki elements, and on one GPU, every SM takes part.
     int ch = requested_channels > 0 ? requested_channels : (numel >= (256u << 10) || ctx.one_gpu ? max_channels : 64);

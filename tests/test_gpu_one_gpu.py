@@ -114,6 +114,18 @@ def test_one_barrier_exact_at_the_ends_of_rows_and_blocks(block):
                     assert bool((o[:r % 2] == 7).all()) and bool((o[r % 2 + numel:] == 7).all())
 
 
+@pytest.mark.parametrize("block", [1, 6, 16, 96, 100, 129, 384, 2048])
+def test_one_barrier_exact_with_blocks_of_any_size(block):
+    """... which no context has: not a power of two, or not from 32 to 1024. Over several channels, too."""
+    for n in (2, 3, 8):
+        for numel in (1, 95, 383, 385, 4096, 20000 + 3):
+            for dtype in (torch.float32, torch.bfloat16):
+                xs = _inputs(n, numel, dtype, numel + n)
+                want = torch.from_numpy(quant_allreduce_oracle([x.float().numpy() for x in xs], block)).to(dtype)
+                for o in emulated_allreduce([x.cuda() for x in xs], mode="quant", algo="oneshot", block_numel=block, slot_bytes=16384):
+                    assert torch.equal(o.cpu(), want), (n, numel, dtype)
+
+
 def test_a_rank_without_alignment_takes_the_streaming_kernels():
     numel = SMALLEST + 7
     xs = _inputs(2, numel + 1, torch.float32, 3)

@@ -43,6 +43,7 @@
 #include "kernels/bulk_copy.cuh"
 #include "kernels/device_sync.cuh"
 #include "kernels/once_per_device.h"
+#include "kernels/one_gpu_waits.cuh"
 #include "kernels/quant_tile.cuh"
 #include "kernels/vector_sum.cuh"
 #include "switchml/quant_math.h"
@@ -73,53 +74,14 @@ struct OneGpuWarps {
   static constexpr int kThreads = (kLoad + kReduce + kFeeders + 2) * 32;  // two more talk to the peers
 };
 
-constexpr int kNoteLoaded = 8, kNoteReduced = 16;  // (eight and sixteen warps at most)
-struct OneGpuShared {
-  int failed;
-  unsigned next[32];  // per warp and role: the first tile that it has not finished
-  unsigned seen[3];   // per phase (1 and 2): tiles that all ranks have signalled
-  unsigned long long full[kOneCopyWarps * kOneCopyStages];  // mbarriers of the stages in shared memory
-};
-static_assert(kOneLoadStages + kOneReduceStages <= kOneCopyWarps * kOneCopyStages, "a barrier per stage");
-
-__device__ __forceinline__ bool Failed(OneGpuShared* sh) { return *reinterpret_cast<volatile int*>(&sh->failed) != 0; }
-__device__ __forceinline__ void SetFailed(OneGpuShared* sh) { *reinterpret_cast<volatile int*>(&sh->failed) = 1; }
-
-// All lanes of a warp: what it wrote so far belongs to the tiles before `next`.
-__device__ __forceinline__ void Note(OneGpuShared* sh, int which, int lane, unsigned next) {
-  __syncwarp();
-  if (lane == 0) asm volatile("st.release.cta.shared::cta.u32 [%0], %1;" ::"r"(BulkSmemAddr(&sh->next[which])), "r"(next) : "memory");
-}
-
-// All lanes of a warp: until eight neighbouring warps have finished the tiles before `tile`. False after a failure.
-__device__ __forceinline__ bool WaitForNotes(const RankCtx& ctx, OneGpuShared* sh, int which, unsigned tile) {
-  const int lane = threadIdx.x & 31;
-  unsigned long long start = 0;
-  for (unsigned spins = 0;;) {
-    unsigned v;
-    asm volatile("ld.acquire.cta.shared::cta.u32 %0, [%1];" : "=r"(v) : "r"(BulkSmemAddr(&sh->next[which + (lane & 7)])) : "memory");
-    if (__all_sync(0xffffffffu, v >= tile)) break;
-    if ((++spins & 63) == 0) {
-      const unsigned long long now = GlobalTimerNs();
-      if (start == 0) start = now;
-      if (__any_sync(0xffffffffu, Failed(sh) || now - start > 2 * ctx.timeout_ns)) {  // the other warps' waits end first
-        SetFailed(sh);
-        return false;
-      }
-    }
-    __nanosleep(20);
-  }
-  __syncwarp();
-  return true;
-}
+static_assert(kOneLoadStages + kOneReduceStages <= kOneBarriers && kOneCopyWarps * kOneCopyStages <= kOneBarriers, "a barrier per stage");
 
 __device__ __forceinline__ void RunOneGpuSignaler(const RankCtx& ctx, OneGpuShared* sh, int channel, Epoch base, unsigned ntiles) {
   const int lane = threadIdx.x & 31, phase = lane < 8 ? 0 : lane < 16 ? 1 : 2, peer = lane & 7;
   Epoch* const flag = phase > 0 && lane < 24 && peer < ctx.nranks ? FlagPtr(ctx.stage_peer[peer], channel, phase, ctx.rank) : nullptr;
   unsigned told = phase == 0 ? ntiles : 0;  // (nothing is told in phase 0)
   for (;;) {
-    unsigned v;
-    asm volatile("ld.acquire.cta.shared::cta.u32 %0, [%1];" : "=r"(v) : "r"(BulkSmemAddr(&sh->next[lane])) : "memory");
+    unsigned v = LoadSharedAcquire(&sh->next[lane]);
     __syncwarp();
 #pragma unroll
     for (int o = 1; o < 8; o <<= 1) v = min(v, __shfl_xor_sync(0xffffffffu, v, o));
@@ -156,7 +118,7 @@ __device__ __forceinline__ void RunOneGpuListener(const RankCtx& ctx, OneGpuShar
     for (int o = 1; o < 8; o <<= 1) v = min(v, __shfl_xor_sync(0xffffffffu, v, o));
     if (v > seen) {
       seen = v;
-      if (rank == 0 && lane < 24) asm volatile("st.release.cta.shared::cta.u32 [%0], %1;" ::"r"(BulkSmemAddr(&sh->seen[phase])), "r"(v) : "memory");
+      if (rank == 0 && lane < 24) StoreSharedRelease(&sh->seen[phase], v);
     }
     // What the CTA's warps will still ask for: all of phase 1, and room for the last tile.
     if (__all_sync(0xffffffffu, seen >= ntiles || (phase == 2 && seen + slots >= ntiles))) return;
@@ -164,72 +126,10 @@ __device__ __forceinline__ void RunOneGpuListener(const RankCtx& ctx, OneGpuShar
   }
 }
 
-// Tiles that all ranks are known to have signalled in a phase.
-struct Seen {
-  unsigned tiles = 0;
-  // All lanes of a warp: until that are at least `need`. False when the wait ran out or another warp failed.
-  __device__ __forceinline__ bool Reach(const RankCtx& ctx, int channel, int phase, unsigned need, OneGpuShared* sh) {
-    if (tiles >= need) return true;
-    unsigned long long start = 0;
-    for (unsigned spins = 0;;) {
-      asm volatile("ld.acquire.cta.shared::cta.u32 %0, [%1];" : "=r"(tiles) : "r"(BulkSmemAddr(&sh->seen[phase])) : "memory");
-      if (__all_sync(0xffffffffu, tiles >= need)) return true;
-      if ((++spins & 63) == 0) {
-        const unsigned long long now = GlobalTimerNs();
-        if (start == 0) start = now;
-        const bool late = now - start > ctx.timeout_ns;
-        if (__any_sync(0xffffffffu, late || Failed(sh))) {
-          if ((threadIdx.x & 31) == 0 && !Failed(sh)) {
-            ReportStatus(ctx, STATUS_TIMEOUT | (phase << 4) | (channel << 8));
-            atomicAdd(ctx.counters + 2, 1ull);
-          }
-          SetFailed(sh);
-          return false;
-        }
-      }
-      __nanosleep(20);
-    }
-  }
-};
-
-// All lanes of a warp: until the phase of `bar` with this parity is complete. The same answer in every lane.
-__device__ __forceinline__ bool WaitForBytes(const RankCtx& ctx, unsigned long long* bar, uint32_t parity, OneGpuShared* sh) {
-  const uint32_t addr = BulkSmemAddr(bar);
-  unsigned long long start = 0;
-  bool ok = true;
-  for (unsigned spins = 0;;) {
-    uint32_t done;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(done) : "r"(addr), "r"(parity) : "memory");
-    if (done) break;
-    if ((++spins & 255) == 0) {
-      const unsigned long long now = GlobalTimerNs();
-      if (start == 0) start = now;
-      if (Failed(sh) || now - start > ctx.timeout_ns) {
-        ok = false;
-        break;
-      }
-    }
-  }
-  ok = __all_sync(0xffffffffu, ok);
-  if (!ok) SetFailed(sh);
-  return ok;
-}
-
-// The same on the way out, with a limit of its own.
+// On the way out: until the phase of `bar` with this parity is complete, with a limit of its own.
 __device__ __forceinline__ void Drain(unsigned long long* bar, uint32_t parity) {
-  for (int spins = 0; spins < (1 << 16); spins++) {
-    uint32_t done;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(done) : "r"(BulkSmemAddr(bar)), "r"(parity) : "memory");
-    if (done) return;
-  }
+  for (int spins = 0; spins < (1 << 16); spins++)
+    if (TryWaitParity(bar, parity)) return;
 }
 
 // One lane: a bulk load of `bytes` (a multiple of 16) that completes on `bar`.
@@ -350,6 +250,7 @@ __device__ __forceinline__ void FeedReducer(const Tiles<ELEM, MODE_QUANT, kPush,
       asm volatile("fence.proxy.async.global;" ::: "memory");  // the slots were filled with ordinary stores
       BulkLoad(ring + (kOneLoadStages + s) * kOneStageBytes + to, from, count * (lane == 0 ? kIn : 4), bar);
     }
+    __syncwarp();
   }
   for (unsigned t = k > kOneReduceStages ? k - kOneReduceStages : 0; t < k; t++)  // as above
     Drain(&sh->full[kOneLoadStages + t % kOneReduceStages], (t / kOneReduceStages) & 1);
@@ -782,7 +683,7 @@ AllReduceOneGpuKernel(const __grid_constant__ EmuArgs args, const __grid_constan
     sh.next[i] = next;
     if (i < 3) sh.seen[i] = 0;
     if (i == 0) sh.failed = 0;
-    for (int b = i; b < kOneCopyWarps * kOneCopyStages; b += 32) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(BulkSmemAddr(&sh.full[b])));
+    for (int b = i; b < kOneBarriers; b += 32) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(BulkSmemAddr(&sh.full[b])));
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncthreads();

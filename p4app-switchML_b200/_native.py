@@ -62,6 +62,8 @@ def _declare(l):
         "sml_static_slice": (None, [u64, i32, i32, c.POINTER(u64), c.POINTER(u64)]),
         "sml_emu_allreduce": (i32, [i32, c.POINTER(vp), c.POINTER(vp), u64, i32, i32, i32, i32, u64,
                                     i32, i32, c.c_float, i32, i32]),
+        "sml_emu_allreduce_with": (i32, [vp, i32, c.POINTER(vp), c.POINTER(vp), u64, i32, i32, i32, i32, u64,
+                                         i32, i32, c.c_float, i32, i32]),
         "sml_host_allreduce": (i32, [vp, vp, vp, u64, i32, u64, vp, vp, vp]),
         "sml_emu_release": (None, []),
         "sml_convert_u8": (i32, [i32, vp, vp, u64, vp]),

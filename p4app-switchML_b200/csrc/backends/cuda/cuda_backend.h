@@ -49,6 +49,12 @@ class CudaBackendInterface : public Backend {
 // Factory used by Backend::CreateInstance. Throws FatalError when no usable GPU exists.
 Backend* CreateCudaBackend(Context& context, Config& config);
 
+// What only tests ask of EmulatedAllReduce. Zero: nothing of the kind.
+struct EmulationOptions {
+  int present = 0;                    // only the first `present` ranks come; what the others wait for runs out
+  unsigned long long timeout_ns = 0;  // of every wait
+};
+
 // Stand-alone multi-rank emulation on one GPU (no Context needed): `nranks` virtual
 // ranks, all memory on the current device, one cooperative kernel. in/out are arrays of
 // `nranks` device pointers. `exponent_lookahead` < 0 takes the default. Returns 0 or a negative error / positive kernels::Status.
@@ -56,7 +62,7 @@ Backend* CreateCudaBackend(Context& context, Config& config);
 int EmulatedAllReduce(int nranks, void* const* in_ptrs, void* const* out_ptrs,
                       unsigned long long numel, int elem_type, int mode, int algo, int block_numel,
                       size_t slot_bytes, int slots_per_channel, int channels, float post_scale,
-                      int repeats, int exponent_lookahead, std::string* error);
+                      int repeats, int exponent_lookahead, const EmulationOptions& options, std::string* error);
 
 // Free the staging memory that EmulatedAllReduce keeps.
 void ReleaseEmulationWorkspaces();

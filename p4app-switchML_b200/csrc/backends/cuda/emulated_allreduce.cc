@@ -144,12 +144,13 @@ void ReleaseEmulationWorkspaces() { WorkspacePool::Get().Clear(); }
 int EmulatedAllReduce(int nranks, void* const* in_ptrs, void* const* out_ptrs,
                       unsigned long long numel, int elem_type, int mode, int algo, int block_numel,
                       size_t slot_bytes, int slots_per_channel, int channels, float post_scale,
-                      int repeats, int exponent_lookahead, std::string* error) {
+                      int repeats, int exponent_lookahead, const EmulationOptions& options, std::string* error) {
   auto fail = [&](const std::string& m, int code) {
     if (error) *error = m;
     return code;
   };
   if (nranks < 1 || nranks > kMaxRanks) return fail("nranks out of range", -1);
+  if (options.present < 0 || options.present > nranks) return fail("more ranks come than there are", -1);
   if (block_numel < 1) return fail("block_numel out of range", -1);
   if (algo == ALGO_ZEROCOPY) return fail("zero-copy needs real symmetric memory", -1);
   if (slot_bytes / 4 / block_numel * slots_per_channel > 8192)
@@ -198,7 +199,7 @@ int EmulatedAllReduce(int nranks, void* const* in_ptrs, void* const* out_ptrs,
   proto.block_numel = block_numel;
   proto.quant_base = quant::QuantBase(nranks);
   proto.oneshot_bytes = oneshot_bytes;
-  proto.timeout_ns = 2000000000ull;  // 2 s: generous for one GPU, still bounded
+  proto.timeout_ns = options.timeout_ns ? options.timeout_ns : 2000000000ull;  // 2 s: generous for one GPU, still bounded
   JobArgs proto_job;
   memset(&proto_job, 0, sizeof(proto_job));
   proto_job.elem_type = elem_type;
@@ -278,7 +279,7 @@ int EmulatedAllReduce(int nranks, void* const* in_ptrs, void* const* out_ptrs,
       args.job[r].epochs = plan.epochs;
     }
     ws->epochs += plan.epochs;
-    e = LaunchAllReduceEmulated(args, nranks, plan, 0);
+    e = LaunchAllReduceEmulated(args, nranks, options.present ? options.present : nranks, plan, 0);
     if (e != cudaSuccess) break;
   }
   if (e == cudaSuccess) e = cudaDeviceSynchronize();

@@ -257,10 +257,21 @@ int sml_emu_allreduce(int nranks, void* const* in_ptrs, void* const* out_ptrs, u
                       int elem_type, int mode, int algo, int block_numel, uint64_t slot_bytes,
                       int slots_per_channel, int channels, float post_scale, int repeats,
                       int exponent_lookahead) {
+  const sml_emu_options none = {};
+  return sml_emu_allreduce_with(&none, nranks, in_ptrs, out_ptrs, numel, elem_type, mode, algo, block_numel, slot_bytes,
+                                slots_per_channel, channels, post_scale, repeats, exponent_lookahead);
+}
+
+int sml_emu_allreduce_with(const sml_emu_options* options, int nranks, void* const* in_ptrs, void* const* out_ptrs,
+                           uint64_t numel, int elem_type, int mode, int algo, int block_numel, uint64_t slot_bytes,
+                           int slots_per_channel, int channels, float post_scale, int repeats, int exponent_lookahead) {
   std::string err;
+  EmulationOptions o;
+  o.present = options->present;
+  o.timeout_ns = options->timeout_ns;
   int r = EmulatedAllReduce(nranks, in_ptrs, out_ptrs, numel, elem_type, mode, algo, block_numel,
                             slot_bytes, slots_per_channel, channels, post_scale, repeats,
-                            exponent_lookahead, &err);
+                            exponent_lookahead, o, &err);
   if (r != 0) g_error = err;
   return r;
 }

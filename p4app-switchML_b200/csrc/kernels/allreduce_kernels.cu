@@ -1340,10 +1340,10 @@ cudaError_t LaunchOne(const RankCtx& ctx, const JobArgs& job, const LaunchPlan& 
 }
 
 template <int ELEM, int MODE, int ALGO>
-cudaError_t LaunchOneEmu(const EmuArgs& emu, int nranks, const LaunchPlan& plan, cudaStream_t stream) {
+cudaError_t LaunchOneEmu(const EmuArgs& emu, int present, const LaunchPlan& plan, cudaStream_t stream) {
   unsigned long long epc = plan.elems_per_channel;
   void* args[] = {const_cast<EmuArgs*>(&emu), &epc};
-  dim3 grid(plan.channels, nranks);
+  dim3 grid(plan.channels, present);
   // Cooperative launch: the runtime refuses the launch unless all CTAs can be resident
   // together, which the cross-"rank" barriers need.
   constexpr size_t dyn = DynamicSmemBytes<ALGO>();
@@ -1550,11 +1550,11 @@ cudaError_t LaunchAllReduce(const RankCtx& ctx, const JobArgs& job, const Launch
   SML_DISPATCH(LaunchOne, job.elem_type, job.mode, job.algo, ctx, job, plan, stream);
 }
 
-cudaError_t LaunchAllReduceEmulated(const EmuArgs& args, int nranks, const LaunchPlan& plan,
+cudaError_t LaunchAllReduceEmulated(const EmuArgs& args, int nranks, int present, const LaunchPlan& plan,
                                     cudaStream_t stream) {
-  if (nranks < 1 || nranks > kMaxRanks || plan.channels > kMaxChannels) return cudaErrorInvalidValue;
-  if (args.job[0].out_zero_copy) return LaunchOneGpuAllReduce(args, nranks, plan, stream);
-  SML_DISPATCH(LaunchOneEmu, args.job[0].elem_type, args.job[0].mode, args.job[0].algo, args, nranks, plan, stream);
+  if (nranks < 1 || nranks > kMaxRanks || present < 1 || present > nranks || plan.channels > kMaxChannels) return cudaErrorInvalidValue;
+  if (args.job[0].out_zero_copy) return LaunchOneGpuAllReduce(args, nranks, present, plan, stream);
+  SML_DISPATCH(LaunchOneEmu, args.job[0].elem_type, args.job[0].mode, args.job[0].algo, args, present, plan, stream);
 }
 
 cudaError_t LaunchLocalCopy(const void* in, void* out, size_t bytes, cudaStream_t stream) {

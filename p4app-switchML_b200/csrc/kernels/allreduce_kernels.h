@@ -152,12 +152,13 @@ cudaError_t LaunchAllReduce(const RankCtx& ctx, const JobArgs& job, const Launch
                             cudaStream_t stream);
 // Single-GPU emulation of `nranks` ranks: one cooperative launch whose blockIdx.y is the
 // rank, every "peer" region living on the same device. Exercises the peer-memory code path
-// bit for bit. The ranks' arguments travel with the launch.
+// bit for bit. The ranks' arguments travel with the launch. Only the first `present` ranks have
+// CTAs: the others are ranks that never come.
 struct EmuArgs {
   RankCtx ctx[kMaxRanks];
   JobArgs job[kMaxRanks];
 };
-cudaError_t LaunchAllReduceEmulated(const EmuArgs& args, int nranks, const LaunchPlan& plan,
+cudaError_t LaunchAllReduceEmulated(const EmuArgs& args, int nranks, int present, const LaunchPlan& plan,
                                     cudaStream_t stream);
 // ALGO_STAGED and ALGO_PUSH with out_zero_copy and all ranks on this GPU (one_gpu_allreduce.cu): whether the slots have
 // room for it, the bytes of its exponent words (RankCtx::exp_offset; cleared before the first use, and after 2^23 epochs at
@@ -165,7 +166,7 @@ cudaError_t LaunchAllReduceEmulated(const EmuArgs& args, int nranks, const Launc
 size_t OneGpuExponentBytes(int nranks, int block_numel, int max_channels);
 bool OneGpuFits(const RankCtx& ctx, const JobArgs& job);
 void PlanOneGpu(const RankCtx& ctx, const JobArgs& job, int requested_channels, int max_channels, LaunchPlan* plan);
-cudaError_t LaunchOneGpuAllReduce(const EmuArgs& args, int nranks, const LaunchPlan& plan, cudaStream_t stream);
+cudaError_t LaunchOneGpuAllReduce(const EmuArgs& args, int nranks, int present, const LaunchPlan& plan, cudaStream_t stream);
 // Single worker, plain sum, out of place: copy `bytes` bytes with one kernel.
 cudaError_t LaunchLocalCopy(const void* in, void* out, size_t bytes, cudaStream_t stream);
 // Single worker, exact mode (float32 or bfloat16, element-aligned): the quantise / dequantise round

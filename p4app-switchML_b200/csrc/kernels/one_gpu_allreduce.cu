@@ -215,7 +215,7 @@ __device__ __forceinline__ void FeedLoader(const Tiles<ELEM, MODE_QUANT, kPush, 
   unsigned k = 0;
   if (lane == 0) asm volatile("fence.proxy.async.global;" ::: "memory");  // the input's producers used ordinary stores
   for (; k < tiles.ntiles; k++) {
-    if (k >= kOneLoadStages && !WaitForNotes(tiles.ctx, sh, kNoteLoaded, k + 1 - kOneLoadStages)) break;
+    if (k >= kOneLoadStages && !WaitForNotes(tiles.ctx, tiles.channel, sh, kNoteLoaded, k + 1 - kOneLoadStages)) break;
     const unsigned s = k % kOneLoadStages, bytes = tiles.Len(k) / kOneChunk * kOneChunk * kIn;
     if (lane == 0) {
       ExpectBytes(&sh->full[s], bytes);
@@ -239,7 +239,7 @@ __device__ __forceinline__ void FeedReducer(const Tiles<ELEM, MODE_QUANT, kPush,
   unsigned k = 0;
   for (; k < tiles.ntiles; k++) {
     if (!loaded.Reach(ctx, tiles.channel, 1, k + 1, sh)) break;
-    if (k >= kOneReduceStages && !WaitForNotes(ctx, sh, kNoteReduced, k + 1 - kOneReduceStages)) break;
+    if (k >= kOneReduceStages && !WaitForNotes(ctx, tiles.channel, sh, kNoteReduced, k + 1 - kOneReduceStages)) break;
     const unsigned s = k % kOneReduceStages, len = tiles.Len(k), per = tiles.Per(k);
     const unsigned sb = min(per * tiles.me, len), count = (min(sb + per, len) - sb) & ~7u;
     unsigned long long* bar = &sh->full[kOneLoadStages + s];
@@ -297,7 +297,7 @@ __device__ __forceinline__ void QuantLoader(const Tiles<ELEM, MODE_QUANT, kPush,
   };
   unsigned published = 0;
   auto publish = [&](unsigned k) {
-    if (!WaitForBytes(ctx, &sh->full[k % kOneLoadStages], (k / kOneLoadStages) & 1, sh)) return false;
+    if (!WaitForBytes(ctx, tiles.channel, &sh->full[k % kOneLoadStages], (k / kOneLoadStages) & 1, sh)) return false;
     if (c0 < tiles.Len(k)) {
       float4 x[8];
       rows(k, x);
@@ -343,11 +343,7 @@ __device__ __forceinline__ void QuantLoader(const Tiles<ELEM, MODE_QUANT, kPush,
         if (start == 0) start = now;
         const bool late = now - start > ctx.timeout_ns;
         if (__any_sync(0xffffffffu, late || Failed(sh))) {
-          if (lane == 0 && !Failed(sh)) {
-            ReportStatus(ctx, STATUS_TIMEOUT | (tiles.channel << 8));
-            atomicAdd(ctx.counters + 2, 1ull);
-          }
-          SetFailed(sh);
+          if (lane == 0) Fail(ctx, sh, tiles.channel, 0);
           return false;
         }
       }
@@ -461,7 +457,7 @@ __device__ __forceinline__ void CopyLoader(const Tiles<ELEM, MODE_SUM, kPush, kR
         const unsigned bytes = (e - b) * kEsz & ~15u;
         for (unsigned off = 0; off < bytes; off += kOneCopyBytes) {
           const unsigned s = stores % kOneCopyStages;
-          if (!WaitForBytes(ctx, full + s, (stores / kOneCopyStages) & 1, sh)) return;
+          if (!WaitForBytes(ctx, tiles.channel, full + s, (stores / kOneCopyStages) & 1, sh)) return;
           ++stores;
           if (lane == 0) {
             asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;"
@@ -639,7 +635,7 @@ __device__ __forceinline__ void Reducer(const Tiles<ELEM, MODE, kPush, R>& tiles
       const unsigned stage = k % kOneReduceStages, area = tiles.MostPer() * 4;
       const char* held = ring + (kOneLoadStages + stage) * kOneStageBytes;
       const char* others = held + tiles.MostPer() * T::kIn;
-      if (!WaitForBytes(ctx, &sh->full[kOneLoadStages + stage], (k / kOneReduceStages) & 1, sh)) return;
+      if (!WaitForBytes(ctx, tiles.channel, &sh->full[kOneLoadStages + stage], (k / kOneReduceStages) & 1, sh)) return;
 #pragma unroll 1
       for (; (r + (U - 1) * kWarps) * 32 + 31 < nvec; r += U * kWarps) QuantGroups<ELEM, R, U>(tiles, s, held, others, area, r * 32 + lane);
 #pragma unroll 1
@@ -735,7 +731,7 @@ size_t TileCapacity(const RankCtx& ctx, const JobArgs& job) {
 }
 
 template <int ELEM, int MODE, bool kPush, int R>
-cudaError_t LaunchRanks(const EmuArgs& emu, int nranks, const OneGpuPlan& plan, int channels, cudaStream_t stream) {
+cudaError_t LaunchRanks(const EmuArgs& emu, int present, const OneGpuPlan& plan, int channels, cudaStream_t stream) {
   void* args[] = {const_cast<EmuArgs*>(&emu), const_cast<OneGpuPlan*>(&plan)};
   const void* kernel = reinterpret_cast<const void*>(AllReduceOneGpuKernel<ELEM, MODE, kPush, R>);
   static std::atomic<unsigned long long> allowed{0};
@@ -746,11 +742,11 @@ cudaError_t LaunchRanks(const EmuArgs& emu, int nranks, const OneGpuPlan& plan, 
   });
   if (e != cudaSuccess) return e;
   // Cooperative: all CTAs are resident together, which their waiting for one another needs.
-  return cudaLaunchCooperativeKernel(kernel, dim3(channels, nranks), dim3(OneGpuWarps<MODE>::kThreads), args, kOneRingBytes, stream);
+  return cudaLaunchCooperativeKernel(kernel, dim3(channels, present), dim3(OneGpuWarps<MODE>::kThreads), args, kOneRingBytes, stream);
 }
 
 template <int ELEM, int MODE>
-cudaError_t LaunchMode(const EmuArgs& emu, int nranks, const LaunchPlan& launch, cudaStream_t stream) {
+cudaError_t LaunchMode(const EmuArgs& emu, int nranks, int present, const LaunchPlan& launch, cudaStream_t stream) {
   const RankCtx& ctx = emu.ctx[0];
   const JobArgs& job = emu.job[0];
   const unsigned unit = MODE == MODE_QUANT && ctx.block_numel > 128 ? ctx.block_numel : 128;
@@ -781,7 +777,7 @@ cudaError_t LaunchMode(const EmuArgs& emu, int nranks, const LaunchPlan& launch,
                    : nranks == 4 ? (push ? LaunchRanks<ELEM, MODE, true, 4> : LaunchRanks<ELEM, MODE, false, 4>)
                    : nranks == 8 ? (push ? LaunchRanks<ELEM, MODE, true, 8> : LaunchRanks<ELEM, MODE, false, 8>)
                                  : (push ? LaunchRanks<ELEM, MODE, true, 0> : LaunchRanks<ELEM, MODE, false, 0>);
-  return start(emu, nranks, plan, launch.channels, stream);
+  return start(emu, present, plan, launch.channels, stream);
 }
 
 }  // namespace
@@ -807,12 +803,12 @@ void PlanOneGpu(const RankCtx& ctx, const JobArgs& job, int requested_channels, 
   plan->epochs = static_cast<unsigned>(tiles_per_channel);
 }
 
-cudaError_t LaunchOneGpuAllReduce(const EmuArgs& args, int nranks, const LaunchPlan& plan, cudaStream_t stream) {
+cudaError_t LaunchOneGpuAllReduce(const EmuArgs& args, int nranks, int present, const LaunchPlan& plan, cudaStream_t stream) {
   const JobArgs& job = args.job[0];
-  if (job.elem_type == ELEM_I32) return LaunchMode<ELEM_I32, MODE_SUM>(args, nranks, plan, stream);
+  if (job.elem_type == ELEM_I32) return LaunchMode<ELEM_I32, MODE_SUM>(args, nranks, present, plan, stream);
   if (job.mode == MODE_QUANT)
-    return (job.elem_type == ELEM_F32 ? LaunchMode<ELEM_F32, MODE_QUANT> : LaunchMode<ELEM_BF16, MODE_QUANT>)(args, nranks, plan, stream);
-  return (job.elem_type == ELEM_F32 ? LaunchMode<ELEM_F32, MODE_SUM> : LaunchMode<ELEM_BF16, MODE_SUM>)(args, nranks, plan, stream);
+    return (job.elem_type == ELEM_F32 ? LaunchMode<ELEM_F32, MODE_QUANT> : LaunchMode<ELEM_BF16, MODE_QUANT>)(args, nranks, present, plan, stream);
+  return (job.elem_type == ELEM_F32 ? LaunchMode<ELEM_F32, MODE_SUM> : LaunchMode<ELEM_BF16, MODE_SUM>)(args, nranks, present, plan, stream);
 }
 
 }  // namespace kernels

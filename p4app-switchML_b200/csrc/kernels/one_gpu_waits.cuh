@@ -49,7 +49,14 @@ struct OneGpuShared {
 };
 
 __device__ __forceinline__ bool Failed(OneGpuShared* sh) { return *reinterpret_cast<volatile int*>(&sh->failed) != 0; }
-__device__ __forceinline__ void SetFailed(OneGpuShared* sh) { *reinterpret_cast<volatile int*>(&sh->failed) = 1; }
+// One lane: the CTA has failed. Its first failure is reported, whichever wait that ended: the waits that follow from it end
+// quietly, and none may end the CTA without a status.
+__device__ __forceinline__ void Fail(const RankCtx& ctx, OneGpuShared* sh, int channel, int phase) {
+  if (atomicExch(&sh->failed, 1) != 0) return;
+  ReportStatus(ctx, STATUS_TIMEOUT | (phase << 4) | (channel << 8));
+  atomicAdd(ctx.counters + 2, 1ull);
+}
+constexpr int kInsideCta = 3;  // the phase of a wait that is for the CTA's own warps or copies
 
 // All lanes of a warp: what it wrote so far belongs to the tiles before `next`.
 __device__ __forceinline__ void Note(OneGpuShared* sh, int which, int lane, unsigned next) {
@@ -58,7 +65,7 @@ __device__ __forceinline__ void Note(OneGpuShared* sh, int which, int lane, unsi
 }
 
 // All lanes of a warp: until eight neighbouring warps have finished the tiles before `tile`. False after a failure.
-__device__ __forceinline__ bool WaitForNotes(const RankCtx& ctx, OneGpuShared* sh, int which, unsigned tile) {
+__device__ __forceinline__ bool WaitForNotes(const RankCtx& ctx, int channel, OneGpuShared* sh, int which, unsigned tile) {
   const int lane = threadIdx.x & 31;
   unsigned long long start = 0;
   for (unsigned spins = 0;;) {
@@ -66,8 +73,9 @@ __device__ __forceinline__ bool WaitForNotes(const RankCtx& ctx, OneGpuShared* s
     if ((++spins & 63) == 0) {
       const unsigned long long now = GlobalTimerNs();
       if (start == 0) start = now;
-      if (__any_sync(0xffffffffu, Failed(sh) || now - start > 2 * ctx.timeout_ns)) {  // the other warps' waits end first
-        SetFailed(sh);
+      // (Twice the time: the wait that holds up the other warps says more than this one.)
+      if (__any_sync(0xffffffffu, Failed(sh) || now - start > 2 * ctx.timeout_ns)) {
+        if (lane == 0) Fail(ctx, sh, channel, kInsideCta);
         return false;
       }
     }
@@ -93,11 +101,7 @@ struct Seen {
         if (start == 0) start = now;
         const bool late = now - start > ctx.timeout_ns;
         if (__any_sync(0xffffffffu, late || Failed(sh))) {
-          if ((threadIdx.x & 31) == 0 && !Failed(sh)) {
-            ReportStatus(ctx, STATUS_TIMEOUT | (phase << 4) | (channel << 8));
-            atomicAdd(ctx.counters + 2, 1ull);
-          }
-          SetFailed(sh);
+          if ((threadIdx.x & 31) == 0) Fail(ctx, sh, channel, phase);
           return false;
         }
       }
@@ -107,7 +111,7 @@ struct Seen {
 };
 
 // All lanes of a warp: until the phase of `bar` with this parity is complete. The same answer in every lane.
-__device__ __forceinline__ bool WaitForBytes(const RankCtx& ctx, unsigned long long* bar, uint32_t parity, OneGpuShared* sh) {
+__device__ __forceinline__ bool WaitForBytes(const RankCtx& ctx, int channel, unsigned long long* bar, uint32_t parity, OneGpuShared* sh) {
   unsigned long long start = 0;
   bool ok = true;
   for (unsigned spins = 0;;) {
@@ -122,7 +126,7 @@ __device__ __forceinline__ bool WaitForBytes(const RankCtx& ctx, unsigned long l
     }
   }
   ok = __all_sync(0xffffffffu, ok);
-  if (!ok) SetFailed(sh);
+  if (!ok && (threadIdx.x & 31) == 0) Fail(ctx, sh, channel, kInsideCta);
   return ok;
 }
 

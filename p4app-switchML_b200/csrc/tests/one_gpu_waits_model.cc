@@ -180,6 +180,33 @@ int LanesThatReadDifferentCounts() {
   return fails;
 }
 
+// Each of the waits runs out: it ends in all lanes, and the CTA has a status, once.
+int AWaitThatRunsOutIsReported() {
+  int fails = 0;
+  for (int wait = 0; wait < 3; wait++) {
+    for (bool late : {true, false}) {  // its own time is up, or another warp has failed
+      Cta cta;
+      cta.sh.failed = !late;
+      bool answer[kLanes];
+      const std::string why = RunWarp([&] {
+        Seen seen;
+        answer[t_lane] = wait == 0   ? WaitForNotes(cta.ctx, 5, &cta.sh, kNoteLoaded, 1)
+                         : wait == 1 ? seen.Reach(cta.ctx, 5, 2, 1, &cta.sh)
+                                     : WaitForBytes(cta.ctx, 5, &cta.sh.full[0], 0, &cta.sh);
+        __syncwarp();
+      });
+      if (!why.empty()) printf("  %s\n", why.c_str());
+      EXPECT(why.empty());
+      for (int l = 0; l < kLanes; l++) EXPECT(why.empty() && !answer[l]);
+      EXPECT(cta.sh.failed == 1);
+      const int phase = wait == 1 ? 2 : kInsideCta;
+      EXPECT(cta.status == (late ? STATUS_TIMEOUT | (phase << 4) | (5 << 8) : STATUS_OK));
+      EXPECT(g_reports.size() == (late ? 1 : 0) && cta.counters[2] == (late ? 1 : 0));
+    }
+  }
+  return fails;
+}
+
 void Run(const char* name, int (*test)()) {
   const int fails = test();
   printf("%s %s\n", fails ? "FAIL" : "ok  ", name);
@@ -193,5 +220,6 @@ void Run(const char* name, int (*test)()) {
 int main() {
   using namespace switchml::kernels;
   Run("lanes_that_read_different_counts", LanesThatReadDifferentCounts);
+  Run("a_wait_that_runs_out_is_reported", AWaitThatRunsOutIsReported);
   return g_failures;
 }

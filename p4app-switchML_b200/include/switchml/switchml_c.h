@@ -85,6 +85,16 @@ int sml_emu_allreduce(int nranks, void* const* in_ptrs, void* const* out_ptrs, u
                       int elem_type, int mode, int algo, int block_numel, uint64_t slot_bytes,
                       int slots_per_channel, int channels, float post_scale, int repeats,
                       int exponent_lookahead);
+/* The same for tests, with what they ask of it (zero: nothing of the kind):
+ * present: only the first `present` ranks come, and the waits for the others run out;
+ * timeout_ns: of every wait. */
+typedef struct sml_emu_options {
+  int present;
+  uint64_t timeout_ns;
+} sml_emu_options;
+int sml_emu_allreduce_with(const sml_emu_options* options, int nranks, void* const* in_ptrs, void* const* out_ptrs,
+                           uint64_t numel, int elem_type, int mode, int algo, int block_numel, uint64_t slot_bytes,
+                           int slots_per_channel, int channels, float post_scale, int repeats, int exponent_lookahead);
 /* Allreduce of pinned host memory: chunks go to `device` (room for numel elements), are reduced there and
  * come back, on three streams of the current device. Returns when host_out is complete. */
 int sml_host_allreduce(const void* host_in, void* host_out, void* device, uint64_t numel, int dtype,

@@ -35,6 +35,25 @@ def emulated_allreduce(inputs, mode="quant", algo="staged", block_numel=256, slo
                         repeats, exponent_lookahead)
         if done is not None:
             return done
+    return _through_ctypes(None, inputs, mode, algo, block_numel, slot_bytes, slots_per_channel, channels, post_scale, repeats, outputs,
+                           exponent_lookahead)
+
+
+class _Options(ctypes.Structure):
+    _fields_ = [("present", ctypes.c_int), ("timeout_ns", ctypes.c_uint64)]
+
+
+def emulated_allreduce_with(inputs, present=0, timeout=0.0, mode="quant", algo="staged", block_numel=256, slot_bytes=131072,
+                            slots_per_channel=2, channels=0, post_scale=1.0, repeats=1, outputs=None, exponent_lookahead=-1):
+    """The same for tests. `present`: only the first `present` ranks come, so that the others' waits for the rest run out;
+    `timeout`: seconds until any wait does (0: the library's 2 s)."""
+    options = _Options(present, int(timeout * 1e9))
+    return _through_ctypes(options, inputs, mode, algo, block_numel, slot_bytes, slots_per_channel, channels, post_scale, repeats, outputs,
+                           exponent_lookahead)
+
+
+def _through_ctypes(options, inputs, mode, algo, block_numel, slot_bytes, slots_per_channel, channels, post_scale, repeats, outputs,
+                    exponent_lookahead):
     import torch
     n = len(inputs)
     x0 = inputs[0]
@@ -51,9 +70,9 @@ def emulated_allreduce(inputs, mode="quant", algo="staged", block_numel=256, slo
     array = _ARRAYS.get(n) or _ARRAYS.setdefault(n, ctypes.c_void_p * n)
     ins = array(*[x.data_ptr() for x in inputs])
     outs = array(*[o.data_ptr() for o in outputs])
-    rc = lib().sml_emu_allreduce(n, ins, outs, numel, elem, MODE[mode], ALGO[algo], block_numel,
-                                 slot_bytes, slots_per_channel, channels, float(post_scale), repeats,
-                                 int(exponent_lookahead))
+    rc = lib().sml_emu_allreduce_with(ctypes.byref(options or _Options()), n, ins, outs, numel, elem, MODE[mode], ALGO[algo], block_numel,
+                                      slot_bytes, slots_per_channel, channels, float(post_scale), repeats,
+                                      int(exponent_lookahead))
     if rc != 0:
         raise NativeError("emulated allreduce failed (%d): %s" % (rc, last_error()))
     return outputs

@@ -4,7 +4,8 @@ import numpy as np
 import pytest
 import torch
 
-from switchml_b200.ops.emulation import emulated_allreduce
+from switchml_b200._native import NativeError
+from switchml_b200.ops.emulation import emulated_allreduce, emulated_allreduce_with
 from switchml_b200.ops.oracle import int_allreduce_oracle, quant_allreduce_oracle
 
 pytestmark = pytest.mark.gpu
@@ -134,6 +135,42 @@ def test_a_rank_without_alignment_takes_the_streaming_kernels():
     for algo in ("staged", "push"):
         for o in emulated_allreduce(ys, mode="quant", algo=algo, block_numel=64):
             assert np.array_equal(o.cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("mode", ["quant", "sum"])
+@pytest.mark.parametrize("n, algo", [(2, "push"), (2, "staged"), (3, "staged"), (8, "push")])
+def test_a_rank_that_never_comes(n, algo, mode):
+    """The waits for it run out: the call says so, whichever of them is the first, and the next one is as good as ever."""
+    xs = _inputs(n, SMALLEST + 5, torch.float32, n)
+    for timeout in (0.02, 0.001):
+        with pytest.raises(NativeError, match="kernel status") as e:
+            emulated_allreduce_with([x.cuda() for x in xs], present=n - 1, timeout=timeout, mode=mode, algo=algo)
+        assert int(str(e.value).split("kernel status")[1].split()[0]) & 15 == 1  # timeout
+    outs = emulated_allreduce([x.cuda() for x in xs], mode=mode, algo=algo)
+    if mode == "quant":
+        want = quant_allreduce_oracle([x.numpy() for x in xs], 256)
+        assert all(np.array_equal(o.cpu().numpy(), want) for o in outs)
+    else:
+        assert torch.allclose(outs[0].cpu().double(), sum(x.double() for x in xs), rtol=1e-5, atol=1e-5)
+
+
+@pytest.mark.parametrize("mode", ["quant", "sum"])
+@pytest.mark.parametrize("n", [1, 2, 4])
+def test_waits_that_run_out_at_once(n, mode):
+    """Limits in the range of what the waits take, so that any of them may be the first to run out: a call either fails or
+    has the result."""
+    xs = _inputs(n, (1 << 21) + 5, torch.int32 if mode == "sum" else torch.float32, n)
+    want = int_allreduce_oracle([x.numpy() for x in xs]) if mode == "sum" else quant_allreduce_oracle([x.numpy() for x in xs], 256)
+    ys = [x.cuda() for x in xs]
+    for algo in ("staged",) if n == 1 else ("staged", "push"):
+        for timeout in (1e-9, 1e-6, 4e-6, 8e-6, 12e-6, 16e-6, 20e-6, 30e-6):
+            outs = [torch.zeros_like(y) for y in ys]
+            try:
+                emulated_allreduce_with(ys, timeout=timeout, mode=mode, algo=algo, outputs=outs)
+            except NativeError as e:
+                assert int(str(e).split("kernel status")[1].split()[0]) & 15 == 1
+                continue
+            assert all(np.array_equal(o.cpu().numpy(), want) for o in outs), (algo, timeout)
 
 
 def test_arguments_that_python_looks_at():

@@ -17,6 +17,6 @@ def output(tmp_path_factory):
     return subprocess.run([exe], capture_output=True, text=True, timeout=120).stdout
 
 
-@pytest.mark.parametrize("case", ["lanes_that_read_different_counts"])
+@pytest.mark.parametrize("case", ["lanes_that_read_different_counts", "a_wait_that_runs_out_is_reported"])
 def test_case(output, case):
     assert "ok   " + case in output, output

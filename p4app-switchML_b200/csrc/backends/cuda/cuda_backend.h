@@ -51,6 +51,8 @@ Backend* CreateCudaBackend(Context& context, Config& config);
 
 // What only tests ask of EmulatedAllReduce. Zero: nothing of the kind.
 struct EmulationOptions {
+  enum Kernels : int { kAny = 0, kStreaming = 1, kOneGpu = 2 };
+  int kernels = kAny;                 // for ALGO_STAGED and ALGO_PUSH: those between GPUs, or those of one_gpu_allreduce.cu
   int present = 0;                    // only the first `present` ranks come; what the others wait for runs out
   unsigned long long timeout_ns = 0;  // of every wait
 };

@@ -169,7 +169,9 @@ int EmulatedAllReduce(int nranks, void* const* in_ptrs, void* const* out_ptrs,
   // whole vectors of device memory. Below 2^18 elements per rank, where a message between GPUs takes neither of these
   // algorithms but ALGO_ONESHOT, and in the checked build, the kernels run as they do between GPUs: that is what one
   // looks at there (2 ranks push exact, whole calls: 2^18 elements 36 us with them and 28 straight, 2^22 72 and 46).
-  bool direct = (algo == ALGO_STAGED || algo == ALGO_PUSH) && numel >= kDirectNumel && !CheckedBuild();
+  const bool only_direct = options.kernels == EmulationOptions::kOneGpu;
+  bool direct = (algo == ALGO_STAGED || algo == ALGO_PUSH) && numel > 0 && options.kernels != EmulationOptions::kStreaming &&
+                (only_direct || (numel >= kDirectNumel && !CheckedBuild()));
   uintptr_t bits = 0;
   for (int r = 0; r < nranks; r++) bits |= reinterpret_cast<uintptr_t>(in_ptrs[r]) | reinterpret_cast<uintptr_t>(out_ptrs[r]);
   if (bits & 15) direct = false;
@@ -206,6 +208,7 @@ int EmulatedAllReduce(int nranks, void* const* in_ptrs, void* const* out_ptrs,
   proto_job.mode = mode;
   proto_job.algo = algo;
   if (direct && !OneGpuFits(proto, proto_job)) direct = false;
+  if (only_direct && !direct) return fail("not a call for the kernels of ranks that share a GPU", -1);
   size_t bytes = StagingBytes(slot_bytes, slots_per_channel, block_numel, max_channels,
                                     oneshot_bytes, nranks, &proto.data_offset, &proto.exp_offset,
                                     &proto.oneshot_offset);
@@ -266,7 +269,7 @@ int EmulatedAllReduce(int nranks, void* const* in_ptrs, void* const* out_ptrs,
       if (direct) {
         j.out_zero_copy = 1;
         for (int p = 0; p < nranks; p++) j.user_peer[p] = static_cast<char*>(out_ptrs[p]);
-        j.user_bytes = numel * esz;
+        j.user_bytes = ReportedOutputBytes(numel * esz);
       }
       j.oneshot_parity = it & 1;
     }

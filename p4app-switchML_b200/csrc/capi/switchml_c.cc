@@ -267,6 +267,7 @@ int sml_emu_allreduce_with(const sml_emu_options* options, int nranks, void* con
                            int slots_per_channel, int channels, float post_scale, int repeats, int exponent_lookahead) {
   std::string err;
   EmulationOptions o;
+  o.kernels = options->kernels;
   o.present = options->present;
   o.timeout_ns = options->timeout_ns;
   int r = EmulatedAllReduce(nranks, in_ptrs, out_ptrs, numel, elem_type, mode, algo, block_numel,

@@ -1453,13 +1453,16 @@ bool CheckedBuild() {
 #endif
 }
 
-size_t ReportedStageBytes(size_t actual) {
+static size_t Pretended(const char* name, size_t actual) {
 #ifdef SWITCHML_CHECKED
-  const char* e = getenv("SWITCHML_CHECKED_PRETEND_STAGE_BYTES");
+  const char* e = getenv(name);
   if (e && *e) return static_cast<size_t>(strtoull(e, nullptr, 0));
 #endif
+  (void)name;
   return actual;
 }
+size_t ReportedStageBytes(size_t actual) { return Pretended("SWITCHML_CHECKED_PRETEND_STAGE_BYTES", actual); }
+size_t ReportedOutputBytes(size_t actual) { return Pretended("SWITCHML_CHECKED_PRETEND_OUTPUT_BYTES", actual); }
 
 LaunchPlan PlanLaunch(const RankCtx& ctx, const JobArgs& job, int requested_channels,
                       int max_channels) {

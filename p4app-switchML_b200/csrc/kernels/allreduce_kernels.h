@@ -98,7 +98,7 @@ struct JobArgs {
   char* user_peer[kMaxRanks];
   char* user_mc;
   size_t in_offset, out_offset;
-  size_t user_bytes;  // size of the symmetric user region (checked build)
+  size_t user_bytes;  // size of the symmetric user region, or of each output with all ranks on one GPU (checked build)
 };
 
 // Geometry chosen on the host; identical on every rank for the same job.
@@ -142,6 +142,8 @@ size_t StagingBytes(size_t slot_bytes, int slots_per_channel, int block_numel, i
 // can watch the geometry checks refuse every tile (the memory itself stays as large as it
 // was, and a refused tile is not touched anyway).
 size_t ReportedStageBytes(size_t actual);
+// The same for the bytes of the outputs of ranks that share a GPU (SWITCHML_CHECKED_PRETEND_OUTPUT_BYTES).
+size_t ReportedOutputBytes(size_t actual);
 // True if the library was compiled with -DSWITCHML_CHECKED.
 bool CheckedBuild();
 

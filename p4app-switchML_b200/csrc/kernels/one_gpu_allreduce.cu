@@ -168,9 +168,18 @@ struct Tiles {
   const char* in;            // there, in this rank's tensor
   char* mine;                // the channel's slots in this rank's staging region
   size_t slot0;              // where they begin in any rank's region
+#ifdef SWITCHML_CHECKED
+  const OneGpuPlan& plan;
+  OneGpuShared* const sh;
+  const char* const ring;
+#endif
 
-  __device__ __forceinline__ Tiles(const RankCtx& c, const JobArgs& j, const OneGpuPlan& plan, int ch)
-      : ctx(c), job(j), channel(ch), n(kRanks ? kRanks : c.nranks), me(c.rank), size(plan.size), slots(plan.slots) {
+  __device__ __forceinline__ Tiles(const RankCtx& c, const JobArgs& j, const OneGpuPlan& plan, int ch, OneGpuShared* sh, const char* ring)
+      : ctx(c), job(j), channel(ch), n(kRanks ? kRanks : c.nranks), me(c.rank), size(plan.size), slots(plan.slots)
+#ifdef SWITCHML_CHECKED
+        , plan(plan), sh(sh), ring(ring)
+#endif
+  {
     const unsigned t0 = static_cast<unsigned>(ch) * plan.channel_tiles;
     ntiles = min(plan.channel_tiles, plan.tiles - t0);
     const bool last = t0 + ntiles == plan.tiles;
@@ -203,6 +212,51 @@ struct Tiles {
   __device__ __forceinline__ size_t Apart() const { return kPush ? AreaBytes() : ctx.stage_bytes; }
   __device__ __forceinline__ char* Out(int p, unsigned long long e) const { return job.user_peer[p] + (job.out_offset + e * kIn); }
 
+  // Whether an access lies in what it is meant for: this channel's part of the tensor, of rank r's slots, exponent words and
+  // output; the stages; the scale factors. The checked build (-DSWITCHML_CHECKED) asks for each: one that does not is left out,
+  // and the CTA fails with STATUS_BOUNDS. Otherwise always true.
+#ifdef SWITCHML_CHECKED
+  __device__ __forceinline__ bool Inside(const void* p, size_t bytes, const void* begin, size_t room, unsigned aligned) const {
+    const char *a = static_cast<const char*>(p), *b = static_cast<const char*>(begin);
+    if (a >= b && bytes <= room && static_cast<size_t>(a - b) <= room - bytes && reinterpret_cast<uintptr_t>(p) % aligned == 0) return true;
+    if (atomicExch(&sh->failed, 1) == 0) ReportStatus(ctx, STATUS_BOUNDS | (channel << 8));
+    return false;
+  }
+  __device__ __forceinline__ size_t Bytes() const { return (static_cast<size_t>(ntiles - 1) * size + end_len_) * kIn; }
+  __device__ __forceinline__ bool InTensor(const void* p, unsigned bytes, unsigned aligned = 1) const {
+    return Inside(p, bytes, in, first * kIn + Bytes() <= job.numel * kIn ? Bytes() : 0, aligned);
+  }
+  __device__ __forceinline__ bool InSlots(int r, const void* p, unsigned bytes, unsigned aligned = 1) const {
+    const size_t room = static_cast<size_t>(slots) * size * kSlot;
+    return Inside(p, bytes, ctx.stage_peer[r] + slot0, room <= plan.slot_pitch && slot0 + room <= ctx.stage_bytes ? room : 0, aligned);
+  }
+  __device__ __forceinline__ bool InWords(int r, const void* p, unsigned bytes) const {
+    const size_t begin = plan.exp0 + channel * plan.exp_pitch;
+    return Inside(p, bytes, ctx.stage_peer[r] + begin, begin + plan.exp_pitch <= ctx.stage_bytes ? plan.exp_pitch : 0, bytes);
+  }
+  __device__ __forceinline__ bool InOut(int r, const void* p, unsigned bytes) const {
+    const size_t begin = job.out_offset + first * kIn;
+    return Inside(p, bytes, job.user_peer[r] + begin, begin + Bytes() <= job.user_bytes ? Bytes() : 0, bytes);
+  }
+  __device__ __forceinline__ bool InStages(const void* p, unsigned bytes, unsigned aligned = 16) const {
+    return Inside(p, bytes, ring, kOneRingBytes, aligned);
+  }
+  __device__ __forceinline__ bool InStage(int s, const void* p, unsigned bytes) const {
+    return Inside(p, bytes, ring + s * kOneStageBytes, kOneStageBytes, bytes);
+  }
+  __device__ __forceinline__ bool InScales(const float* all, const float* p) const {
+    return Inside(p, 4, all, kOneQuantSlots * (kOneQuantTile / 32) * sizeof(float), 4);
+  }
+#else
+  __device__ __forceinline__ bool InTensor(const void*, unsigned, unsigned = 1) const { return true; }
+  __device__ __forceinline__ bool InSlots(int, const void*, unsigned, unsigned = 1) const { return true; }
+  __device__ __forceinline__ bool InWords(int, const void*, unsigned) const { return true; }
+  __device__ __forceinline__ bool InOut(int, const void*, unsigned) const { return true; }
+  __device__ __forceinline__ bool InStages(const void*, unsigned, unsigned = 16) const { return true; }
+  __device__ __forceinline__ bool InStage(int, const void*, unsigned) const { return true; }
+  __device__ __forceinline__ bool InScales(const float*, const float*) const { return true; }
+#endif
+
  private:
   unsigned end_len_, per_, end_per_;
 };
@@ -219,7 +273,8 @@ __device__ __forceinline__ void FeedLoader(const Tiles<ELEM, MODE_QUANT, kPush, 
     const unsigned s = k % kOneLoadStages, bytes = tiles.Len(k) / kOneChunk * kOneChunk * kIn;
     if (lane == 0) {
       ExpectBytes(&sh->full[s], bytes);
-      if (bytes > 0) BulkLoad(ring + s * kOneStageBytes, tiles.In(k), bytes, &sh->full[s]);
+      if (bytes > 0 && tiles.InTensor(tiles.In(k), bytes, 16) && bytes <= kOneStageBytes)
+        BulkLoad(ring + s * kOneStageBytes, tiles.In(k), bytes, &sh->full[s]);
     }
   }
   // Nothing may land in this shared memory once the CTA has gone; after a failure nobody else waits for it.
@@ -247,8 +302,12 @@ __device__ __forceinline__ void FeedReducer(const Tiles<ELEM, MODE_QUANT, kPush,
     __syncwarp();
     if (lane < tiles.n && count > 0) {
       const char* from = lane == 0 ? tiles.In(k) + static_cast<size_t>(sb) * kIn : tiles.Others(sb) + skip + tiles.SlotOff(k);
+      const unsigned bytes = count * (lane == 0 ? kIn : 4);
+      char* const stage = ring + (kOneLoadStages + s) * kOneStageBytes + to;
       asm volatile("fence.proxy.async.global;" ::: "memory");  // the slots were filled with ordinary stores
-      BulkLoad(ring + (kOneLoadStages + s) * kOneStageBytes + to, from, count * (lane == 0 ? kIn : 4), bar);
+      if (tiles.InStages(stage, bytes) &&
+          (lane == 0 ? tiles.InTensor(from, bytes, 16) : tiles.InSlots(kPush ? tiles.me : i < tiles.me ? i : i + 1, from, bytes, 16)))
+        BulkLoad(stage, from, bytes, bar);
     }
     __syncwarp();
   }
@@ -277,7 +336,10 @@ __device__ __forceinline__ void QuantLoader(const Tiles<ELEM, MODE_QUANT, kPush,
     if (c0 + kOneChunk <= tiles.Len(k)) {
       const char* smem = held + k % kOneLoadStages * kOneStageBytes;
 #pragma unroll
-      for (int u = 0; u < 8; u++) x[u] = LoadGroupAsFloat<ELEM>(smem, u * 32 + lane);
+      for (int u = 0; u < 8; u++) {
+        x[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (tiles.InStage(k % kOneLoadStages, smem + (u * 32 + lane) * 4 * kIn, 4 * kIn)) x[u] = LoadGroupAsFloat<ELEM>(smem, u * 32 + lane);
+      }
     } else {  // the job's end: from the tensor
       const char* in = tiles.In(k);
       const unsigned len = tiles.Len(k);
@@ -285,6 +347,7 @@ __device__ __forceinline__ void QuantLoader(const Tiles<ELEM, MODE_QUANT, kPush,
       for (int u = 0; u < 8; u++) {
         const unsigned e = c0 + u * 128 + lane * 4;
         x[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (e < len && !tiles.InTensor(in + e * kIn, min(4u, len - e) * kIn, min(4u, len - e) == 4 ? 4 * kIn : kIn)) continue;
         if (e + 4 <= len) {
           x[u] = LoadGroupAsFloat<ELEM>(in, e / 4);
         } else {
@@ -304,9 +367,10 @@ __device__ __forceinline__ void QuantLoader(const Tiles<ELEM, MODE_QUANT, kPush,
       const size_t exp_off = exp0 + (k % kExpRing) * exp_bytes + me * 4;
       const unsigned tag = static_cast<unsigned>(base + k + 1) << 8;
       PublishRows8(ctx.block_numel, lane, x, 0, [&](size_t block, int exponent) {
-        for (int p = 0; p < n; p++)
-          asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(ctx.stage_peer[p] + exp_off + block * plan.block_words * 4),
-                       "r"(tag | (exponent + 128)) : "memory");
+        for (int p = 0; p < n; p++) {
+          char* const to = ctx.stage_peer[p] + exp_off + block * plan.block_words * 4;
+          if (tiles.InWords(p, to, 4)) asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(to), "r"(tag | (exponent + 128)) : "memory");
+        }
       });
     }
     ++published;
@@ -317,6 +381,7 @@ __device__ __forceinline__ void QuantLoader(const Tiles<ELEM, MODE_QUANT, kPush,
   auto fetch_words = [&](unsigned k) {
     if (static_cast<unsigned>(lane) >= blocks || c0 + (lane << shift) >= tiles.Len(k)) return;
     const char* from = ctx.stage_peer[me] + exp0 + (k % kExpRing) * exp_bytes + lane * plan.block_words * 4;
+    if (!tiles.InWords(me, from, kWords == 2 ? 8 : 16)) return;
     if constexpr (kWords == 2) {
       asm volatile("ld.relaxed.gpu.global.v2.u32 {%0, %1}, [%2];" : "=r"(word[0]), "=r"(word[1]) : "l"(from) : "memory");
     } else {
@@ -353,7 +418,7 @@ __device__ __forceinline__ void QuantLoader(const Tiles<ELEM, MODE_QUANT, kPush,
 #pragma unroll
       for (int i = 0; i < kWords; i++)
         if (i < n) m = max(m, word[i] & 0xff);
-      sf[lane] = quant::ScaleFactorFromBase(static_cast<int>(m) - 128, ctx.quant_base);
+      if (tiles.InScales(s_sf, sf + lane)) sf[lane] = quant::ScaleFactorFromBase(static_cast<int>(m) - 128, ctx.quant_base);
     }
     __syncwarp();
     return true;
@@ -373,8 +438,10 @@ __device__ __forceinline__ void QuantLoader(const Tiles<ELEM, MODE_QUANT, kPush,
       if (!plain || !own) {
         float4 x[8];
         rows(k, x);
-        auto quantise = [&](int u, char* to) {
-          const float f = sf[(u * 128 + lane * 4) >> shift];
+        auto quantise = [&](int u, int d, char* to) {
+          const float* const scale = sf + ((u * 128 + lane * 4) >> shift);
+          if (!tiles.InScales(s_sf, scale) || !tiles.InSlots(kPush ? d : me, to, 16, 16)) return;
+          const float f = *scale;
           int4 q;
           q.x = quant::Quantize(x[u].x, f);
           q.y = quant::Quantize(x[u].y, f);
@@ -385,13 +452,13 @@ __device__ __forceinline__ void QuantLoader(const Tiles<ELEM, MODE_QUANT, kPush,
         if (plain) {
           char* to = to0 + tiles.SlotOff(k);
 #pragma unroll
-          for (int u = 0; u < 8; u++) quantise(u, to + u * 512);
+          for (int u = 0; u < 8; u++) quantise(u, d0, to + u * 512);
         } else {
           const unsigned per = tiles.Per(k), len = tiles.Len(k);
 #pragma unroll
           for (int u = 0; u < 8; u++) {
             const unsigned row = c0 + u * 128, e = row + lane * 4, d = row / per;
-            if (static_cast<int>(d) != me && e < len) quantise(u, tiles.Slot(d, d * per, e) + tiles.SlotOff(k));
+            if (static_cast<int>(d) != me && e < len) quantise(u, d, tiles.Slot(d, d * per, e) + tiles.SlotOff(k));
           }
         }
       }
@@ -426,8 +493,9 @@ __device__ __forceinline__ void CopyLoader(const Tiles<ELEM, MODE_SUM, kPush, kR
       const unsigned bytes = (e - b) * kEsz & ~15u;
       if (load_i < pieces && load_off < bytes) {
         const unsigned size = min(bytes - load_off, kOneCopyBytes), s = loads % kOneCopyStages;
+        const char* const from = tiles.In(load_k) + static_cast<size_t>(b) * kEsz + load_off;
         ExpectBytes(full + s, size);
-        BulkLoad(ring + s * kOneCopyBytes, tiles.In(load_k) + static_cast<size_t>(b) * kEsz + load_off, size, full + s);
+        if (tiles.InTensor(from, size, 16) && tiles.InStages(ring + s * kOneCopyBytes, size)) BulkLoad(ring + s * kOneCopyBytes, from, size, full + s);
         ++loads;
         load_off += size;
         return;
@@ -460,9 +528,11 @@ __device__ __forceinline__ void CopyLoader(const Tiles<ELEM, MODE_SUM, kPush, kR
           if (!WaitForBytes(ctx, tiles.channel, full + s, (stores / kOneCopyStages) & 1, sh)) return;
           ++stores;
           if (lane == 0) {
-            asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;"
-                         ::"l"(tiles.Slot(d, b, b) + slot_off + off), "r"(BulkSmemAddr(ring + s * kOneCopyBytes)), "r"(min(bytes - off, kOneCopyBytes))
-                         : "memory");
+            char* const to = tiles.Slot(d, b, b) + slot_off + off;
+            const unsigned size = min(bytes - off, kOneCopyBytes);
+            if (tiles.InSlots(kPush ? d : me, to, size, 16) && tiles.InStages(ring + s * kOneCopyBytes, size))
+              asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;"
+                           ::"l"(to), "r"(BulkSmemAddr(ring + s * kOneCopyBytes)), "r"(size) : "memory");
             asm volatile("cp.async.bulk.commit_group;" ::: "memory");
             asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");  // the buffer of the store before this one is free
             load_next();
@@ -473,6 +543,7 @@ __device__ __forceinline__ void CopyLoader(const Tiles<ELEM, MODE_SUM, kPush, kR
         for (unsigned j = b + bytes / kEsz + lane; j < e; j += 32) {
           char* to = tiles.Slot(d, b, j) + slot_off;
           const char* from = tiles.In(k) + static_cast<size_t>(j) * kEsz;
+          if (!tiles.InSlots(kPush ? d : me, to, kEsz, kEsz) || !tiles.InTensor(from, kEsz, kEsz)) continue;
           if (kEsz == 4) *reinterpret_cast<unsigned*>(to) = *reinterpret_cast<const unsigned*>(from);
           else *reinterpret_cast<unsigned short*>(to) = *reinterpret_cast<const unsigned short*>(from);
         }
@@ -498,6 +569,7 @@ struct ShardView {
   size_t apart;
   unsigned long long at;    // the shard's first element in the outputs
   const float* sf;          // scale factors of the tile
+  const float* scales;      // ... of all slots
   unsigned sb;              // the shard's first element in the tile
   int shift;
 };
@@ -514,7 +586,11 @@ __device__ __forceinline__ void SumVectors(const T& tiles, const ShardView& s, u
     const char* src = s.others + static_cast<size_t>(kPush ? i - 1 : i) * s.apart;
     if (i == (kPush ? 0 : me)) src = s.own;
 #pragma unroll
-    for (int u = 0; u < U; u++) x[i][u] = __ldcg(reinterpret_cast<const uint4*>(src) + v + u * stride);
+    for (int u = 0; u < U; u++) {
+      const uint4* const from = reinterpret_cast<const uint4*>(src) + v + u * stride;
+      x[i][u] = make_uint4(0, 0, 0, 0);
+      if (i == (kPush ? 0 : me) ? tiles.InTensor(from, 16, 16) : tiles.InSlots(kPush ? me : i, from, 16, 16)) x[i][u] = __ldcg(from);
+    }
   }
   // In rank order from zero (staged), or the own shard first (push): the order of the streaming kernels.
   VecAcc<ELEM> acc[U];
@@ -534,7 +610,8 @@ __device__ __forceinline__ void SumVectors(const T& tiles, const ShardView& s, u
   for (int p = 0; p < n; p++) {
     uint4* out = reinterpret_cast<uint4*>(tiles.Out(p, s.at));
 #pragma unroll
-    for (int u = 0; u < U; u++) __stcs(out + v + u * stride, x[0][u]);  // leaves L2 to the slots: 4 x 2^24 119 -> 113 us
+    for (int u = 0; u < U; u++)
+      if (tiles.InOut(p, out + v + u * stride, 16)) __stcs(out + v + u * stride, x[0][u]);  // leaves L2 to the slots: 4 x 2^24 119 -> 113 us
   }
 }
 
@@ -549,7 +626,12 @@ __device__ __forceinline__ void QuantGroups(const T& tiles, const ShardView& s, 
   float4 y[U];
 #pragma unroll
   for (int u = 0; u < U; u++) {
-    const float f = s.sf[(s.sb + (g + u * kStride) * 4) >> s.shift];
+    const float* const scale = s.sf + ((s.sb + (g + u * kStride) * 4) >> s.shift);
+    y[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (!tiles.InScales(s.scales, scale) || !tiles.InStages(held + (g + u * kStride) * 4 * T::kIn, 4 * T::kIn, 4 * T::kIn) ||
+        (n > 1 && !tiles.InStages(others + (n - 2) * area + (g + u * kStride) * 16, 16)))
+      continue;
+    const float f = *scale;
     const float4 x = LoadGroupAsFloat<ELEM>(held, g + u * kStride);
     int4 a = make_int4(quant::Quantize(x.x, f), quant::Quantize(x.y, f), quant::Quantize(x.z, f), quant::Quantize(x.w, f));
     const int4* from = reinterpret_cast<const int4*>(others) + g + u * kStride;
@@ -566,6 +648,7 @@ __device__ __forceinline__ void QuantGroups(const T& tiles, const ShardView& s, 
     char* out = tiles.Out(p, s.at);
 #pragma unroll
     for (int u = 0; u < U; u++) {
+      if (!tiles.InOut(p, out + (g + u * kStride) * 4 * T::kIn, 4 * T::kIn)) continue;
       if (ELEM == ELEM_BF16)
         reinterpret_cast<uint2*>(out)[g + u * kStride] = make_uint2(Float2ToBf16x2(y[u].x, y[u].y), Float2ToBf16x2(y[u].z, y[u].w));
       else
@@ -578,8 +661,15 @@ __device__ __forceinline__ void QuantGroups(const T& tiles, const ShardView& s, 
 template <int ELEM, int MODE, bool kPush, typename T>
 __device__ __forceinline__ void ReduceElement(const T& tiles, const ShardView& s, unsigned i) {
   const int n = tiles.n, me = tiles.me;
+  for (int j = 0; j < n; j++) {
+    const int r = kPush ? (j + me) % n : j;  // (push: the areas of the others, in any order)
+    if (r == me ? !tiles.InTensor(s.own + i * T::kIn, T::kIn, T::kIn)
+                : !tiles.InSlots(kPush ? me : r, s.others + static_cast<size_t>(kPush ? j - 1 : j) * s.apart + i * T::kSlot, T::kSlot, T::kSlot))
+      return;
+  }
   unsigned bits;
   if (MODE == MODE_QUANT) {
+    if (!tiles.InScales(s.scales, s.sf + ((s.sb + i) >> s.shift))) return;
     const float f = s.sf[(s.sb + i) >> s.shift];
     unsigned a = static_cast<unsigned>(quant::Quantize(TileLoadAsFloat(s.own, i, ELEM), f));
     for (int j = 0; j < n - 1; j++) a += __ldcg(reinterpret_cast<const unsigned*>(s.others + (kPush || j < me ? j : j + 1) * s.apart) + i);
@@ -602,6 +692,7 @@ __device__ __forceinline__ void ReduceElement(const T& tiles, const ShardView& s
   }
   for (int p = 0; p < n; p++) {
     char* out = tiles.Out(p, s.at + i);
+    if (!tiles.InOut(p, out, T::kIn)) continue;
     if (ELEM == ELEM_BF16) *reinterpret_cast<unsigned short*>(out) = FloatToBf16(__uint_as_float(bits));
     else *reinterpret_cast<unsigned*>(out) = bits;
   }
@@ -618,6 +709,7 @@ __device__ __forceinline__ void Reducer(const Tiles<ELEM, MODE, kPush, R>& tiles
   ShardView s;
   s.shift = 31 - __clz(ctx.block_numel);
   s.apart = tiles.Apart();
+  s.scales = s_sf;
   const unsigned tile_blocks = tiles.size >> s.shift;
   Seen loaded;
   for (unsigned k = 0; k < tiles.ntiles; k++) {
@@ -685,9 +777,9 @@ AllReduceOneGpuKernel(const __grid_constant__ EmuArgs args, const __grid_constan
   __syncthreads();
   const int channel = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const Epoch base = ctx.epoch_words[channel];
-  const Tiles<ELEM, MODE, kPush, R> tiles(ctx, job, plan, channel);
+  char* const ring = reinterpret_cast<char*>(s_ring);
+  const Tiles<ELEM, MODE, kPush, R> tiles(ctx, job, plan, channel, &sh, ring);
   if (tiles.ntiles > 0) {
-    char* const ring = reinterpret_cast<char*>(s_ring);
     if (warp < kLoad) {
       if constexpr (MODE == MODE_QUANT) QuantLoader<ELEM, kPush, R>(tiles, plan, warp, lane, base, &sh, ring, s_sf);
       else CopyLoader<ELEM, kPush, R>(tiles, warp, lane, &sh, ring);

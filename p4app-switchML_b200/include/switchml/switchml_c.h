@@ -86,9 +86,11 @@ int sml_emu_allreduce(int nranks, void* const* in_ptrs, void* const* out_ptrs, u
                       int slots_per_channel, int channels, float post_scale, int repeats,
                       int exponent_lookahead);
 /* The same for tests, with what they ask of it (zero: nothing of the kind):
+ * kernels: of algorithms 0 and 3: 1 the streaming kernels, 2 those of ranks that share a GPU (or an error);
  * present: only the first `present` ranks come, and the waits for the others run out;
  * timeout_ns: of every wait. */
 typedef struct sml_emu_options {
+  int kernels;
   int present;
   uint64_t timeout_ns;
 } sml_emu_options;

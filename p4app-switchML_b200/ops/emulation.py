@@ -40,14 +40,18 @@ def emulated_allreduce(inputs, mode="quant", algo="staged", block_numel=256, slo
 
 
 class _Options(ctypes.Structure):
-    _fields_ = [("present", ctypes.c_int), ("timeout_ns", ctypes.c_uint64)]
+    _fields_ = [("kernels", ctypes.c_int), ("present", ctypes.c_int), ("timeout_ns", ctypes.c_uint64)]
 
 
-def emulated_allreduce_with(inputs, present=0, timeout=0.0, mode="quant", algo="staged", block_numel=256, slot_bytes=131072,
+_KERNELS = {None: 0, "streaming": 1, "one_gpu": 2}
+
+
+def emulated_allreduce_with(inputs, kernels=None, present=0, timeout=0.0, mode="quant", algo="staged", block_numel=256, slot_bytes=131072,
                             slots_per_channel=2, channels=0, post_scale=1.0, repeats=1, outputs=None, exponent_lookahead=-1):
-    """The same for tests. `present`: only the first `present` ranks come, so that the others' waits for the rest run out;
+    """The same for tests. `kernels`: "streaming" or "one_gpu", for "staged" and "push" of any size and in any build of the library
+    (an error where those of ranks that share a GPU cannot). `present`: only the first `present` ranks come, so that the others' waits for the rest run out;
     `timeout`: seconds until any wait does (0: the library's 2 s)."""
-    options = _Options(present, int(timeout * 1e9))
+    options = _Options(_KERNELS[kernels], present, int(timeout * 1e9))
     return _through_ctypes(options, inputs, mode, algo, block_numel, slot_bytes, slots_per_channel, channels, post_scale, repeats, outputs,
                            exponent_lookahead)
 
@@ -70,7 +74,7 @@ def _through_ctypes(options, inputs, mode, algo, block_numel, slot_bytes, slots_
     array = _ARRAYS.get(n) or _ARRAYS.setdefault(n, ctypes.c_void_p * n)
     ins = array(*[x.data_ptr() for x in inputs])
     outs = array(*[o.data_ptr() for o in outputs])
-    rc = lib().sml_emu_allreduce_with(ctypes.byref(options or _Options()), n, ins, outs, numel, elem, MODE[mode], ALGO[algo], block_numel,
+    rc = lib().sml_emu_allreduce_with(ctypes.byref(_Options() if options is None else options), n, ins, outs, numel, elem, MODE[mode], ALGO[algo], block_numel,
                                       slot_bytes, slots_per_channel, channels, float(post_scale), repeats,
                                       int(exponent_lookahead))
     if rc != 0:

@@ -20,7 +20,7 @@ import sys
 sys.path.insert(0, %r)
 import numpy as np, torch
 from switchml_b200._native import lib, NativeError
-from switchml_b200.ops.emulation import emulated_allreduce
+from switchml_b200.ops.emulation import emulated_allreduce, emulated_allreduce_with
 from switchml_b200.ops.oracle import quant_allreduce_oracle, int_allreduce_oracle
 assert lib().sml_checked_build() == 1, "not the checked build"
 """ % ROOT
@@ -114,3 +114,54 @@ def test_code_for_ranks_on_gpus_of_their_own(algo):
         print("as on several GPUs")
     """ % algo)
     assert "as on several GPUs" in out
+
+
+@pytest.mark.parametrize("algo", ["staged", "push"])
+def test_every_access_of_ranks_that_share_a_gpu(algo):
+    """The kernels for ranks that share a GPU look at each address here: none is out of place, whatever the geometry."""
+    out = _child("""
+        algo = %r
+        cases = ((1, 256, 32768, 2), (2, 32, 131072, 1), (3, 1024, 12288, 3), (4, 64, 16384, 4), (5, 256, 65536, 5),
+                 (7, 64, 32768, 2), (8, 1024, 32768, 1), (8, 256, 262144, 4))
+        for n, block, slot_bytes, slots in cases[algo == "push":]:
+            for numel, channels in ((1, 0), (1023, 3), (8192 * 40 - 1, 1), ((1 << 18) + 9 * 1024 + 5, 3), ((1 << 18) + 1, 0)):
+                opts = dict(kernels="one_gpu", algo=algo, block_numel=block, slot_bytes=slot_bytes, slots_per_channel=slots, channels=channels)
+                g = torch.Generator().manual_seed(numel + n)
+                xs = [torch.randn(numel, generator=g) * 10.0 ** (r %% 3) for r in range(n)]
+                for dtype in (torch.float32, torch.bfloat16):
+                    ys = [x.to(dtype) for x in xs]
+                    want = torch.from_numpy(quant_allreduce_oracle([y.float().numpy() for y in ys], block)).to(dtype)
+                    for o in emulated_allreduce_with([y.cuda() for y in ys], mode="quant", **opts):
+                        assert torch.equal(o.cpu(), want), (n, numel, dtype, "quant")
+                    # n float32 additions and at most one rounding to bf16: 2^-24 and 2^-8 of what is added
+                    want = sum(y.double() for y in ys)
+                    bound = n * 2.0 ** -24 * sum(y.double().abs() for y in ys) + (2.0 ** -8 * want.abs() if dtype == torch.bfloat16 else 0)
+                    for o in emulated_allreduce_with([y.cuda() for y in ys], mode="sum", **opts):
+                        assert bool(((o.cpu().double() - want).abs() <= bound).all()), (n, numel, dtype, "sum")
+                xi = [torch.randint(-2 ** 30, 2 ** 30, (numel,), generator=g, dtype=torch.int32) for r in range(n)]
+                want = int_allreduce_oracle([x.numpy() for x in xi])
+                for o in emulated_allreduce_with([x.cuda() for x in xi], mode="sum", **opts):
+                    assert np.array_equal(o.cpu().numpy(), want), (n, numel, "int")
+        print("all in place")
+    """ % algo)
+    assert "all in place" in out
+
+
+@pytest.mark.parametrize("mode", ["quant", "sum"])
+@pytest.mark.parametrize("algo", ["staged", "push"])
+def test_outputs_that_are_too_small_are_reported_not_written(algo, mode):
+    """The kernels are told that the outputs hold 4096 elements: no channel that goes beyond is written, status 3."""
+    out = _child("""
+        xs = [torch.ones(300000, device="cuda") * (r + 1) for r in range(4)]
+        outs = [torch.full((300000,), -7.0, device="cuda") for _ in range(4)]
+        try:
+            emulated_allreduce_with(xs, kernels="one_gpu", mode=%r, algo=%r, block_numel=64, outputs=outs)
+            raise SystemExit("no check fired")
+        except NativeError as e:
+            msg = str(e)
+        torch.cuda.synchronize()
+        assert all(bool((o[4096:] == -7.0).all()) for o in outs), "written beyond the end"
+        print("refused:", msg)
+    """ % (mode, algo), SWITCHML_CHECKED_PRETEND_OUTPUT_BYTES=str(4096 * 4))
+    assert "refused:" in out and "kernel status" in out
+    assert int(out.split("kernel status")[1].split()[0]) & 0xf == 3

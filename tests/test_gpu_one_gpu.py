@@ -66,6 +66,27 @@ def test_plain_sums(algo, n, slot_bytes, slots, numel, channels):
             assert torch.equal(o, outs[0]), "all ranks hold the same bits"
 
 
+@pytest.mark.parametrize("algo", ["staged", "push"])
+@pytest.mark.parametrize("n", [2, 3, 8])
+def test_nothing_beside_the_outputs_is_written(n, algo):
+    """Outputs in frames: aligned, with elements before and behind that stay as they are; the inputs stay, too."""
+    for numel in (1, 5, 1023, 20 * 1024 + 9, SMALLEST + 4097):
+        for mode, dtype in (("quant", torch.float32), ("quant", torch.bfloat16), ("sum", torch.float32), ("sum", torch.bfloat16), ("sum", torch.int32)):
+            xs = _inputs(n, numel, dtype, numel + n)
+            ins = [x.cuda() for x in xs]
+            frames = [torch.full((numel + 48,), 7, dtype=dtype, device="cuda") for _ in range(n)]
+            outs = [f[16:16 + numel] for f in frames]
+            emulated_allreduce_with(ins, kernels="one_gpu", mode=mode, algo=algo, block_numel=64, slot_bytes=16384, channels=5, outputs=outs)
+            for x, i, f, o in zip(xs, ins, frames, outs):
+                assert bool((f[:16] == 7).all()) and bool((f[16 + numel:] == 7).all()), (numel, mode, dtype)
+                assert torch.equal(i.cpu().view(torch.int16 if dtype == torch.bfloat16 else torch.int32), x.view(torch.int16 if dtype == torch.bfloat16 else torch.int32))
+                assert torch.equal(o, outs[0])
+            if mode == "quant":
+                assert torch.equal(outs[0].cpu(), torch.from_numpy(quant_allreduce_oracle([x.float().numpy() for x in xs], 64)).to(dtype))
+            elif dtype == torch.int32:
+                assert np.array_equal(outs[0].cpu().numpy(), int_allreduce_oracle([x.numpy() for x in xs]))
+
+
 def test_values_that_are_not_finite():
     """Infinities and NaN come out as between GPUs: as the same job in pieces below 2^18 elements gives them."""
     n, numel, block = 2, SMALLEST, 64

@@ -153,8 +153,23 @@ int EmulatedAllReduce(int nranks, void* const* in_ptrs, void* const* out_ptrs,
   if (options.present < 0 || options.present > nranks) return fail("more ranks come than there are", -1);
   if (block_numel < 1) return fail("block_numel out of range", -1);
   if (algo == ALGO_ZEROCOPY) return fail("zero-copy needs real symmetric memory", -1);
+  const bool exact = mode == MODE_QUANT && elem_type != ELEM_I32;
+  if (algo != ALGO_ONESHOT) {
+    // The streaming kernels and those of one_gpu_allreduce.cu know blocks as a context has them (the words and scale factors
+    // of others would lie beyond their arrays); for plain sums a block is nothing but a unit of the geometry. A slot is whole
+    // units, or whole blocks where it has no room for one per rank.
+    const bool known = block_numel >= 32 && block_numel <= 1024 && (block_numel & (block_numel - 1)) == 0;
+    if (exact && !known) return fail("block_numel must be a power of two from 32 to 1024", -1);
+    if (!known) block_numel = 128;
+    const size_t block = static_cast<size_t>(block_numel > 128 ? block_numel : 128) * 4, unit = nranks * block;
+    slot_bytes = slot_bytes >= unit ? slot_bytes / unit * unit : slot_bytes / block * block;
+    if (slots_per_channel < 1 || slot_bytes < (exact && elem_type == ELEM_BF16 ? unit : block))
+      return fail("no room in the slots for max(block, 128) * 4 bytes, times nranks for bfloat16 in the exact mode", -1);
+  }
   if (slot_bytes / 4 / block_numel * slots_per_channel > 8192)
     return fail("slots_per_channel * slot_bytes / (4 * block_numel) exceeds 8192", -1);
+  for (int r = 0; r < nranks; r++)
+    if (numel > 0 && (!in_ptrs[r] || !out_ptrs[r])) return fail("a rank has no tensor", -1);
   int dev = 0;
   cudaGetDevice(&dev);
   const int sms = SmCount(dev);

@@ -156,7 +156,10 @@ py::object Emulate(const py::object& inputs, const py::object& outputs, int mode
       made.append(py::cast(out[r]));
     } else {
       out[r] = THPVariable_Unpack(PyList_GET_ITEM(outputs.ptr(), r));
-      if (out[r].layout() != at::kStrided) return py::none();
+      // (Python says what is wrong with another one.)
+      if (out[r].layout() != at::kStrided || !out[r].is_contiguous() || out[r].device() != in[r].device() ||
+          out[r].scalar_type() != in[0].scalar_type() || out[r].numel() < in[0].numel())
+        return py::none();
     }
     ins[r] = in[r].data_ptr();
     outs[r] = out[r].data_ptr();

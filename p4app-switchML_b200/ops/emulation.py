@@ -67,6 +67,11 @@ def _through_ctypes(options, inputs, mode, algo, block_numel, slot_bytes, slots_
         assert x.is_cuda and x.is_contiguous() and x.dtype == dtype and x.numel() == numel
     if outputs is None:
         outputs = [torch.empty_like(x) for x in inputs]
+    if len(outputs) != n:
+        raise ValueError("%d outputs for %d inputs" % (len(outputs), n))
+    for o in outputs:
+        if torch.is_tensor(o) and (not o.is_contiguous() or o.dtype != dtype or o.numel() < numel or not (o.is_cuda or o.is_pinned())):
+            raise ValueError("an output must be contiguous device (or pinned) memory of the inputs' type, with room for the result")
     esz_unit = n * max(block_numel, 128) * 4
     slot_bytes = max(esz_unit, slot_bytes // esz_unit * esz_unit)
     if algo == "push":  # a slot holds n-1 receive areas and n-1 result areas of one shard each

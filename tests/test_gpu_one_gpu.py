@@ -194,6 +194,24 @@ def test_waits_that_run_out_at_once(n, mode):
             assert all(np.array_equal(o.cpu().numpy(), want) for o in outs), (algo, timeout)
 
 
+@pytest.mark.parametrize("numel", [1000, SMALLEST])
+def test_outputs_without_room_for_the_result(numel):
+    xs = [torch.ones(numel, device="cuda") * r for r in range(2)]
+    good = torch.empty(numel, device="cuda")
+    for bad in (torch.empty(numel - 1, device="cuda"), torch.empty(2 * numel, device="cuda")[::2], torch.empty(numel, device="cuda", dtype=torch.bfloat16),
+                torch.empty(numel, device="cuda", dtype=torch.float64), torch.empty(numel)):
+        for outs in ([good, bad], (bad, good)):
+            with pytest.raises(ValueError):
+                emulated_allreduce(xs, mode="sum", outputs=outs)
+    for outs in ([], [good], [good] * 3):
+        with pytest.raises(ValueError):
+            emulated_allreduce(xs, mode="sum", outputs=outs)
+    # What has more room than that, and pinned memory.
+    for outs in ([torch.zeros(numel + 5, device="cuda") for _ in xs], [torch.zeros(numel, pin_memory=True) for _ in xs]):
+        for o in emulated_allreduce(xs, mode="sum", outputs=outs):
+            assert bool((o[:numel] == 1).all()) and bool((o[numel:] == 0).all())
+
+
 def test_arguments_that_python_looks_at():
     xs = [torch.ones(5000, device="cuda") * r for r in range(3)]
     for seq in (xs, tuple(xs)):  # with and without the native call

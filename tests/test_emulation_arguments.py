@@ -47,3 +47,13 @@ def test_slots_without_room():
     assert _call(elem=BF16, slot_bytes=1024)[0] == -1 and _looked_for_tensors(*_call(elem=BF16, slot_bytes=2048))
     assert _looked_for_tensors(*_call(slot_bytes=1024)) and _looked_for_tensors(*_call(slot_bytes=100001))
     assert _looked_for_tensors(*_call(algo=ONESHOT, slots=0, slot_bytes=0))
+
+
+def test_numbers_of_other_types():
+    """Python converts what the native call would not take."""
+    import torch
+    from switchml_b200.ops.emulation import emulated_allreduce
+    xs = [torch.ones(4) for _ in range(2)]
+    for options in ({"exponent_lookahead": 2.0}, {"exponent_lookahead": "2"}, {"post_scale": "0.5"}, {"post_scale": 1}):
+        with pytest.raises(AssertionError):  # the tensors are not on a GPU: nothing else is wrong
+            emulated_allreduce(xs, mode="sum", **options)

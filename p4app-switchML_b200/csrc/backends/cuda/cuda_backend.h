@@ -55,6 +55,7 @@ struct EmulationOptions {
   int kernels = kAny;                 // for ALGO_STAGED and ALGO_PUSH: those between GPUs, or those of one_gpu_allreduce.cu
   int present = 0;                    // only the first `present` ranks come; what the others wait for runs out
   unsigned long long timeout_ns = 0;  // of every wait
+  unsigned long long epoch_limit = 0; // beyond which a workspace's flags and words are cleared
 };
 
 // Stand-alone multi-rank emulation on one GPU (no Context needed): `nranks` virtual

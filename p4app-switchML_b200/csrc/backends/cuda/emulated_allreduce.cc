@@ -237,8 +237,9 @@ int EmulatedAllReduce(int nranks, void* const* in_ptrs, void* const* out_ptrs,
     return fail("ALGO_PUSH needs at least two ranks and slots of about twice nranks * max(block, 128) * 4 bytes", -1);
 
   // Flags and exponent words of another layout are noise in this one, so they are cleared (with
-  // the epochs, which start over) when the layout changes, and only then; or when the epochs outgrow the tags of
-  // one_gpu_allreduce.cu, after hours.
+  // the epochs, which start over) when the layout changes, and only then; or before the epochs outgrow the 24 bits of the tags of
+  // one_gpu_allreduce.cu: half a minute of calls back to back (2 ranks x 2^25 exact: 56 epochs in 0.15 ms) to some
+  // minutes (calls of one epoch).
   char layout[128];
   snprintf(layout, sizeof(layout), "%d/%d/%zu/%d/%d/%d/%zu", direct, nranks, slot_bytes, slots_per_channel, block_numel, max_channels, bytes);
   const size_t need = kHeadBytes + bytes * nranks;
@@ -247,7 +248,7 @@ int EmulatedAllReduce(int nranks, void* const* in_ptrs, void* const* out_ptrs,
   if (!ws) ws = NewWorkspace(dev, need, &e);
   if (!ws) return fail(std::string("allocation failed: ") + cudaGetErrorString(e), -3);
   char* const stage0 = ws->memory + kHeadBytes;
-  if (ws->layout != layout || ws->epochs > (1u << 23)) {
+  if (ws->layout != layout || ws->epochs > (options.epoch_limit ? options.epoch_limit : 1ull << 23)) {
     ws->layout.clear();
     ws->epochs = 0;
     e = cudaMemsetAsync(ws->memory, 0, kHeadBytes, 0);

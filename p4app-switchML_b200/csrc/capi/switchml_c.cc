@@ -270,6 +270,7 @@ int sml_emu_allreduce_with(const sml_emu_options* options, int nranks, void* con
   o.kernels = options->kernels;
   o.present = options->present;
   o.timeout_ns = options->timeout_ns;
+  o.epoch_limit = options->epoch_limit;
   int r = EmulatedAllReduce(nranks, in_ptrs, out_ptrs, numel, elem_type, mode, algo, block_numel,
                             slot_bytes, slots_per_channel, channels, post_scale, repeats,
                             exponent_lookahead, o, &err);

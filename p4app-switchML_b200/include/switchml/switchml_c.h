@@ -88,11 +88,13 @@ int sml_emu_allreduce(int nranks, void* const* in_ptrs, void* const* out_ptrs, u
 /* The same for tests, with what they ask of it (zero: nothing of the kind):
  * kernels: of algorithms 0 and 3: 1 the streaming kernels, 2 those of ranks that share a GPU (or an error);
  * present: only the first `present` ranks come, and the waits for the others run out;
- * timeout_ns: of every wait. */
+ * timeout_ns: of every wait;
+ * epoch_limit: epochs that flags and words may have counted before they are cleared. */
 typedef struct sml_emu_options {
   int kernels;
   int present;
   uint64_t timeout_ns;
+  uint64_t epoch_limit;
 } sml_emu_options;
 int sml_emu_allreduce_with(const sml_emu_options* options, int nranks, void* const* in_ptrs, void* const* out_ptrs,
                            uint64_t numel, int elem_type, int mode, int algo, int block_numel, uint64_t slot_bytes,

@@ -40,18 +40,19 @@ def emulated_allreduce(inputs, mode="quant", algo="staged", block_numel=256, slo
 
 
 class _Options(ctypes.Structure):
-    _fields_ = [("kernels", ctypes.c_int), ("present", ctypes.c_int), ("timeout_ns", ctypes.c_uint64)]
+    _fields_ = [("kernels", ctypes.c_int), ("present", ctypes.c_int), ("timeout_ns", ctypes.c_uint64), ("epoch_limit", ctypes.c_uint64)]
 
 
 _KERNELS = {None: 0, "streaming": 1, "one_gpu": 2}
 
 
-def emulated_allreduce_with(inputs, kernels=None, present=0, timeout=0.0, mode="quant", algo="staged", block_numel=256, slot_bytes=131072,
-                            slots_per_channel=2, channels=0, post_scale=1.0, repeats=1, outputs=None, exponent_lookahead=-1):
+def emulated_allreduce_with(inputs, kernels=None, present=0, timeout=0.0, epoch_limit=0, mode="quant", algo="staged", block_numel=256,
+                            slot_bytes=131072, slots_per_channel=2, channels=0, post_scale=1.0, repeats=1, outputs=None, exponent_lookahead=-1):
     """The same for tests. `kernels`: "streaming" or "one_gpu", for "staged" and "push" of any size and in any build of the library
     (an error where those of ranks that share a GPU cannot). `present`: only the first `present` ranks come, so that the others' waits for the rest run out;
-    `timeout`: seconds until any wait does (0: the library's 2 s)."""
-    options = _Options(_KERNELS[kernels], present, int(timeout * 1e9))
+    `timeout`: seconds until any wait does (0: the library's 2 s). `epoch_limit`: epochs after which the flags and exponent words of
+    the staging memory are cleared (0: 2^23)."""
+    options = _Options(_KERNELS[kernels], present, int(timeout * 1e9), epoch_limit)
     return _through_ctypes(options, inputs, mode, algo, block_numel, slot_bytes, slots_per_channel, channels, post_scale, repeats, outputs,
                            exponent_lookahead)
 

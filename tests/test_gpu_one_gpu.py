@@ -194,6 +194,22 @@ def test_waits_that_run_out_at_once(n, mode):
             assert all(np.array_equal(o.cpu().numpy(), want) for o in outs), (algo, timeout)
 
 
+@pytest.mark.parametrize("kernels", ["one_gpu", "streaming"])
+@pytest.mark.parametrize("algo", ["staged", "push"])
+def test_epochs_that_start_over(algo, kernels):
+    """The tags of exponent words have 24 bits: before they come round, words and flags are cleared and epochs start at 0
+    again. Jobs of other lengths before and behind that, in the same staging memory, never take a word for another's."""
+    rng = np.random.default_rng(7)
+    for n in (2, 3, 8):
+        for case in range(14):
+            numel = int(rng.integers(1, 3 * SMALLEST if case % 2 else 5000))
+            xs = _inputs(n, max(numel, 3), torch.float32, case)
+            want = quant_allreduce_oracle([x.numpy() for x in xs], 64)
+            outs = emulated_allreduce_with([x.cuda() for x in xs], kernels=kernels, epoch_limit=(1, 9, 30)[case % 3], mode="quant", algo=algo,
+                                           block_numel=64, slot_bytes=16384, channels=3, repeats=1 + case % 3)
+            assert all(np.array_equal(o.cpu().numpy(), want) for o in outs), (n, case)
+
+
 @pytest.mark.parametrize("numel", [1000, SMALLEST])
 def test_outputs_without_room_for_the_result(numel):
     xs = [torch.ones(numel, device="cuda") * r for r in range(2)]

@@ -784,11 +784,15 @@ extern "C" int switchml_wgrad_gemm_2cta(const void* dy, const void* x, float* dw
 //   Fewer: one, for its smaller tiles and open epilogue (512 x 8192 x 8192: 92 and 95, 256 x 4096 x 4096: 18.0 and 20.8,
 //   512 x 4096 x 1024: 8.2 and 8.6), but
 //   - few tiles are split over pairs that add up in shared memory (512 x 512 x 512 7.6 and 6.2, 256 x 1024 x 1024: 6.4 and 6.2,
-//     192 x 1024 x 1024: 5.9 and 6.1);
+//     192 x 1024 x 1024: 5.9 and 6.1, 196 x 1000 x 1000: 6.9 and 6.5);
 //   - rows that are not whole lines of 128 bytes make loads cost half as much again, and the pairs load less: with more tiles than
-//     pairs from K = 384 on (448 x 3000 x 3000: 16.8 and 15.3, 512 x 6000 x 2000: 22.5 and 20.9, 384 x 6000 x 2000: 18.7 and 19.0), with
+//     pairs beyond K = 384 (448 x 3000 x 3000: 16.8 and 15.3, 512 x 6000 x 2000: 22.5 and 20.9, 384 x 6000 x 2000: 18.7 and 19.0), with
 //     at most half as many, where a tile's epilogue is hidden by nothing in either kernel, as with few tiles (384 x 1200 x
-//     1000: 8.3 and 7.6). Between them the one-CTA kernel keeps ahead (512 x 2000 x 2000: 8.6 and 9.0).
+//     1000: 8.3 and 7.6, 196 x 72 x 7000: 6.6 and 6.4, 196 x 8200 x 200: 7.5 and 7.0; with 1000 x 1400 the two cross at K = 240: 196
+//     6.94 and 7.08, 256 7.32 and 7.21, 384 8.43 and 8.08; where the second row of tiles is mostly padding, of which one CTA has
+//     less, they cross at K = 384: 264 x 4000 at K = 196 6.5 and 6.9). Between them the one-CTA kernel keeps ahead
+//     (512 x 2000 x 2000: 8.6 and 9.0).
+// The numbers of tiles are those of 148 SMs: 74 pairs, 33 clusters of two, about half as many of four.
 extern "C" int switchml_wgrad_gemm_auto(const void* dy, const void* x, float* dw, int M, int N, int K, int* error_flag,
                                         void* stream) {
   const long long tiles = static_cast<long long>((M + 255) / 256) * ((N + 255) / 256);

@@ -633,14 +633,18 @@ __device__ __forceinline__ void QuantGroups(const T& tiles, const ShardView& s, 
       continue;
     const float f = *scale;
     const float4 x = LoadGroupAsFloat<ELEM>(held, g + u * kStride);
-    int4 a = make_int4(quant::Quantize(x.x, f), quant::Quantize(x.y, f), quant::Quantize(x.z, f), quant::Quantize(x.w, f));
-    const int4* from = reinterpret_cast<const int4*>(others) + g + u * kStride;
-    for (int i = 0; i < n - 1; i++, from = reinterpret_cast<const int4*>(reinterpret_cast<const char*>(from) + area)) {
-      const int4 v = *from;
+    auto own = [&](float v) { return static_cast<unsigned>(quant::Quantize(v, f)); };
+    uint4 a = make_uint4(own(x.x), own(x.y), own(x.z), own(x.w));  // (sums that wrap: values that saturate)
+    const uint4* from = reinterpret_cast<const uint4*>(others) + g + u * kStride;
+    for (int i = 0; i < n - 1; i++, from = reinterpret_cast<const uint4*>(reinterpret_cast<const char*>(from) + area)) {
+      const uint4 v = *from;
       a.x += v.x; a.y += v.y; a.z += v.z; a.w += v.w;
     }
     const float inv = __uint_as_float(0x7f000000u - __float_as_uint(f));
-    auto back = [&](int q) { return R ? __int2float_rn(q) * inv : __fdiv_rn(__int2float_rn(q), f); };
+    auto back = [&](unsigned sum) {
+      const int q = static_cast<int>(sum);
+      return R ? __int2float_rn(q) * inv : __fdiv_rn(__int2float_rn(q), f);
+    };
     y[u] = make_float4(back(a.x), back(a.y), back(a.z), back(a.w));
     if (post_scale != 1.0f) { y[u].x *= post_scale; y[u].y *= post_scale; y[u].z *= post_scale; y[u].w *= post_scale; }
   }

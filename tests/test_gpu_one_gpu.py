@@ -103,6 +103,20 @@ def test_values_that_are_not_finite():
                 assert torch.equal(o[at:at + numel // 4].view(torch.int32), p.view(torch.int32)), (algo, at)
 
 
+@pytest.mark.parametrize("n", [2, 3, 4, 8])
+def test_sums_that_wrap(n):
+    """Values that are not finite saturate, and sums of those wrap, as the oracle's do."""
+    xs = _inputs(n, SMALLEST, torch.float32, n)
+    for r, x in enumerate(xs):
+        x[::64] = float("inf")
+        x[1::64] = -float("inf") if r else 3e38
+        x[2::64] = 3.4e38
+    want = quant_allreduce_oracle([x.numpy() for x in xs], 64)
+    for algo in ("staged", "push"):
+        for o in emulated_allreduce([x.cuda() for x in xs], mode="quant", algo=algo, block_numel=64):
+            assert np.array_equal(o.cpu().numpy().view(np.int32), want.view(np.int32)), algo
+
+
 @pytest.mark.parametrize("block", [64, 128, 256, 512, 1024])
 def test_the_largest_of_a_block_wherever_it_lies(block):
     """... with both signs, beside NaN, which never wins, and in blocks of nothing else than zeros of both signs."""

@@ -778,9 +778,11 @@ namespace {
 
 // ------------------------------------------------------------------------------------
 // Exact mode of RunOneShot for blocks that its rows do not hold: a warp per block, element by element. `src` + r * apart is
-// rank r's copy. Only ops/emulation.py comes here: a context's blocks are powers of two from 32 to 1024.
+// rank r's copy. Only ops/emulation.py comes here, with a kernel of its own (the call cost the others registers): a
+// context's blocks are powers of two from 32 to 1024.
+bool RowsHoldBlocks(int block) { return block >= 4 && (block <= 256 ? (block & (block - 1)) == 0 : block % 256 == 0); }
 template <int ELEM>
-__device__ __noinline__ void ReduceBlocksOfAnySize(int nranks, size_t B, float quant_base, const char* src, size_t apart, char* out,
+__device__ __forceinline__ void ReduceBlocksOfAnySize(int nranks, size_t B, float quant_base, const char* src, size_t apart, char* out,
                                                    size_t len, float post_scale) {
   const int lane = threadIdx.x & 31;
   for (size_t base = (threadIdx.x >> 5) * B; base < len; base += (blockDim.x >> 5) * B) {
@@ -805,7 +807,7 @@ __device__ __noinline__ void ReduceBlocksOfAnySize(int nranks, size_t B, float q
 // kOneGpu: all ranks live on this GPU. A rank then parks its input in its own buffer only, and the others read it there:
 // posted stores to everybody spare a trip back over a link that is not there, and cost the stores (8 ranks x 262143, whole
 // calls: plain sums 38 -> 28 us, exact 47 -> 38; 4 x 65536 24.4 -> 22.7).
-template <int ELEM, int MODE, bool kOneGpu>
+template <int ELEM, int MODE, bool kOneGpu, bool kAnyBlock>
 __device__ void RunOneShot(const RankCtx& ctx, const JobArgs& job, int channel,
                            unsigned long long elems_per_channel, Epoch base, int* s_failed) {
   const int esz = ELEM == ELEM_BF16 ? 2 : 4;
@@ -990,7 +992,7 @@ __device__ void RunOneShot(const RankCtx& ctx, const JobArgs& job, int channel,
         if (s < ctx.nranks) add4(acc, x[s], sf);
       if (i < len) finish(i, acc, sf);
     };
-    if (B < 4 || (B <= kRows * 128 ? (B & (B - 1)) != 0 : B % (kRows * 128) != 0)) {
+    if (kAnyBlock) {
       ReduceBlocksOfAnySize<ELEM>(ctx.nranks, B, ctx.quant_base, src0, src_step, out, len, job.post_scale);
     } else if (B <= kRows * 128) {
       // A warp takes two rows, whatever blocks they consist of: with a warp per block, blocks of 64 left three quarters of
@@ -1177,7 +1179,7 @@ __device__ void RunZeroCopy(const RankCtx& ctx, const JobArgs& job, int channel,
 }
 
 // ------------------------------------------------------------------------------------
-template <int ELEM, int MODE, int ALGO, bool kOneGpu>
+template <int ELEM, int MODE, int ALGO, bool kOneGpu, bool kAnyBlock = false>
 __device__ __forceinline__ void RunJob(const RankCtx& ctx, const JobArgs& job, int channel,
                                        unsigned long long epc, Epoch base, int* s_failed, float* s_sf) {
   // The quantising loader reads its input twice and meets its peers once more per tile,
@@ -1189,7 +1191,7 @@ __device__ __forceinline__ void RunJob(const RankCtx& ctx, const JobArgs& job, i
     RunStaged<ELEM, MODE, kOneGpu>(ctx, job, channel, epc, base, reinterpret_cast<StagedShared*>(s_failed), s_sf);
   else if (ALGO == ALGO_PUSH)
     RunPush<ELEM, MODE, kOneGpu>(ctx, job, channel, epc, base, reinterpret_cast<StagedShared*>(s_failed), s_sf);
-  else if (ALGO == ALGO_ONESHOT) RunOneShot<ELEM, MODE, kOneGpu>(ctx, job, channel, epc, base, s_failed);
+  else if (ALGO == ALGO_ONESHOT) RunOneShot<ELEM, MODE, kOneGpu, kAnyBlock>(ctx, job, channel, epc, base, s_failed);
   else if (ctx.use_multimem) RunZeroCopy<ELEM, kZeroCopyUnrollLink>(ctx, job, channel, epc, base, s_failed);
   else RunZeroCopy<ELEM, kZeroCopyUnrollPeer>(ctx, job, channel, epc, base, s_failed);
 }
@@ -1244,7 +1246,7 @@ static constexpr bool kEmuOneGpu = true;
 #endif
 
 // All ranks in one grid: blockIdx.y selects the rank whose role this CTA plays.
-template <int ELEM, int MODE, int ALGO>
+template <int ELEM, int MODE, int ALGO, bool kAnyBlock>
 __global__ void __launch_bounds__(kThreads, 1)
 AllReduceEmuKernel(const __grid_constant__ EmuArgs args, unsigned long long epc) {
   __shared__ StagedShared s_state;
@@ -1260,7 +1262,7 @@ AllReduceEmuKernel(const __grid_constant__ EmuArgs args, unsigned long long epc)
   for (unsigned i = threadIdx.x; i < sizeof(JobArgs) / 4; i += blockDim.x) reinterpret_cast<unsigned*>(&s_job)[i] = from_job[i];
   __syncthreads();
   SML_EPOCH_PROLOGUE(s_ctx, s_job, blockIdx.x, ALGO)
-  RunJob<ELEM, MODE, ALGO, kEmuOneGpu>(s_ctx, s_job, blockIdx.x, epc, s_base, &s_state.failed, s_sf);
+  RunJob<ELEM, MODE, ALGO, kEmuOneGpu, kAnyBlock>(s_ctx, s_job, blockIdx.x, epc, s_base, &s_state.failed, s_sf);
   SML_EPOCH_EPILOGUE(s_ctx, s_job, blockIdx.x)
 }
 
@@ -1339,7 +1341,7 @@ cudaError_t LaunchOne(const RankCtx& ctx, const JobArgs& job, const LaunchPlan& 
   return cudaGetLastError();
 }
 
-template <int ELEM, int MODE, int ALGO>
+template <int ELEM, int MODE, int ALGO, bool kAnyBlock = false>
 cudaError_t LaunchOneEmu(const EmuArgs& emu, int present, const LaunchPlan& plan, cudaStream_t stream) {
   unsigned long long epc = plan.elems_per_channel;
   void* args[] = {const_cast<EmuArgs*>(&emu), &epc};
@@ -1348,9 +1350,9 @@ cudaError_t LaunchOneEmu(const EmuArgs& emu, int present, const LaunchPlan& plan
   // together, which the cross-"rank" barriers need.
   constexpr size_t dyn = DynamicSmemBytes<ALGO>();
   static std::atomic<unsigned long long> allowed{0};
-  const cudaError_t e = AllowDynamicSmem(reinterpret_cast<const void*>(AllReduceEmuKernel<ELEM, MODE, ALGO>), dyn, &allowed);
+  const cudaError_t e = AllowDynamicSmem(reinterpret_cast<const void*>(AllReduceEmuKernel<ELEM, MODE, ALGO, kAnyBlock>), dyn, &allowed);
   if (e != cudaSuccess) return e;
-  return cudaLaunchCooperativeKernel(reinterpret_cast<void*>(AllReduceEmuKernel<ELEM, MODE, ALGO>),
+  return cudaLaunchCooperativeKernel(reinterpret_cast<void*>(AllReduceEmuKernel<ELEM, MODE, ALGO, kAnyBlock>),
                                      grid, dim3(kThreads), args, dyn, stream);
 }
 
@@ -1557,6 +1559,10 @@ cudaError_t LaunchAllReduceEmulated(const EmuArgs& args, int nranks, int present
                                     cudaStream_t stream) {
   if (nranks < 1 || nranks > kMaxRanks || present < 1 || present > nranks || plan.channels > kMaxChannels) return cudaErrorInvalidValue;
   if (args.job[0].out_zero_copy) return LaunchOneGpuAllReduce(args, nranks, present, plan, stream);
+  if (args.job[0].algo == ALGO_ONESHOT && args.job[0].mode == MODE_QUANT && args.job[0].elem_type != ELEM_I32 &&
+      !RowsHoldBlocks(args.ctx[0].block_numel))
+    return (args.job[0].elem_type == ELEM_F32 ? LaunchOneEmu<ELEM_F32, MODE_QUANT, ALGO_ONESHOT, true>
+                                              : LaunchOneEmu<ELEM_BF16, MODE_QUANT, ALGO_ONESHOT, true>)(args, present, plan, stream);
   SML_DISPATCH(LaunchOneEmu, args.job[0].elem_type, args.job[0].mode, args.job[0].algo, args, present, plan, stream);
 }
 

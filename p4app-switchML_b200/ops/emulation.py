@@ -31,8 +31,11 @@ def emulated_allreduce(inputs, mode="quant", algo="staged", block_numel=256, slo
     they are upper bounds: tiles and rings are cut to what stays in L2 and in shared memory. The results do not depend on either, but
     for the order in which plain sums add ("push": the owner of a shard first)."""
     if _emulate is not None and mode in MODE and algo in ALGO:
-        done = _emulate(inputs, outputs, MODE[mode], ALGO[algo], block_numel, slot_bytes, slots_per_channel, channels,
-                        float(post_scale), repeats, int(exponent_lookahead))
+        try:
+            done = _emulate(inputs, outputs, MODE[mode], ALGO[algo], block_numel, slot_bytes, slots_per_channel, channels, post_scale,
+                            repeats, exponent_lookahead)
+        except TypeError:  # a number of another type: below it is converted, or refused
+            done = None
         if done is not None:
             return done
     return _through_ctypes(None, inputs, mode, algo, block_numel, slot_bytes, slots_per_channel, channels, post_scale, repeats, outputs,

@@ -1487,13 +1487,13 @@ LaunchPlan PlanLaunch(const RankCtx& ctx, const JobArgs& job, int requested_chan
                               (ctx.block_numel > 128 ? ctx.block_numel : 128);
     unsigned long long tile = (numel + 4ull * ch - 1) / (4ull * ch);
     if (ctx.one_gpu) {
-      // (Short messages and tensors off their boundaries; the others: one_gpu_allreduce.cu.)
-      // Meeting costs little on one GPU, an idle SM as much as anywhere: one to four tiles of 4 Ki to 14 Ki
-      // elements for every channel before they grow (2^18 elements were 16 tiles for 74 channels). Whole calls, this rule,
-      // always four tiles, and tiles of at least 16 Ki as between GPUs: 2 ranks x 2^18 push exact 39 / 39 / 44 us, 2 x 2^20
-      // 42 / 54 / 44, 4 x 2^19 staged exact 44 / 55 / 45, 8 x 2^18 staged sum 36 / 49 / 37; the same from 2^22 elements
-      // on 4 ranks. A second tile from 28 Ki elements per channel on, not 14 Ki, measured no slower and up to 10 %
-      // faster between (2 x 2^22 push exact 63 us instead of 70, 8 x 2^20 75 instead of 91).
+      // (Messages below 2^18 elements, and of any length in pinned memory or off their boundaries: the others go to
+      // one_gpu_allreduce.cu.) Meeting costs little on one GPU, an idle SM as much as anywhere: one to four tiles of 4 Ki to 14 Ki
+      // elements for every channel before they grow (2^18 elements were 16 tiles for 74 channels). Measured when aligned messages
+      // of these lengths still came here; whole calls, this rule, always four tiles, and tiles of at least 16 Ki as between
+      // GPUs: 2 ranks x 2^18 push exact 39 / 39 / 44 us, 2 x 2^20 42 / 54 / 44, 4 x 2^19 staged exact 44 / 55 / 45, 8 x 2^18
+      // staged sum 36 / 49 / 37; the same from 2^22 elements on 4 ranks. A second tile from 28 Ki elements per channel on, not
+      // 14 Ki, measured no slower and up to 10 % faster between (2 x 2^22 push exact 63 us instead of 70, 8 x 2^20 75 instead of 91).
       const unsigned long long per_channel = (numel + ch - 1) / ch;
       unsigned long long count = (per_channel + 7168) / 14336;
       count = count < 1 ? 1 : count > 4 ? 4 : count;

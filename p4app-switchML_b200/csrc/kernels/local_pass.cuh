@@ -349,7 +349,7 @@ __device__ __noinline__ void LocalQuantSlow(const char* in, char* out, int lane,
 
 // One chunk per warp; the last warp takes what is left over (fewer than kQuantChunk elements).
 // Three blocks per SM (float32, 80 registers) and four (bfloat16, 64) keep 96 and 64 KB in flight. With two and three, the
-// slow way inlined, and maxima by shuffles in all of these: 25 MB float32 7.5 us instead of 6.7, bfloat16 8.5 instead of 8.1, 2^27 elements 168 instead of 155
+// slow way inlined, and maxima by shuffles in all of these: 25 MB float32 7.5 us instead of 6.7, bfloat16 8.5 instead of 7.7, 2^27 elements 168 instead of 155
 // and 96 instead of 84 (blocks of 256, in place), bfloat16 one element off 133 instead of 98. One block more
 // costs registers that the fast way needs (bfloat16 25 MB 10.6). With WarpLargest() instead of shuffles 25 MB take 6.2 and
 // 7.0 us, 2^27 elements of bfloat16 78.7 instead of 81.7, one element off 87.5 instead of 91.7.

@@ -79,8 +79,9 @@ int sml_convert_u8(int widen, const void* in, void* out, uint64_t numel, void* s
 
 /* `nranks` virtual ranks on the current CUDA device in one cooperative kernel.
  * elem_type 0 f32 / 1 i32 / 2 bf16; mode 0 sum / 1 quant; algo 0 staged / 1 one-shot / 3 push;
- * slot_bytes and slots_per_channel are upper bounds for plain sums of more than 44 MB through the slots;
- * exponent_lookahead: tiles by which the exponents run ahead of the data (< 0: the default). */
+ * block_numel: with 0 and 3 a power of two from 32 to 1024 in the exact mode;
+ * slot_bytes and slots_per_channel are upper bounds from 2^18 elements on;
+ * exponent_lookahead: tiles by which the exponents run ahead of the data (< 0: the default), below 2^18 elements. */
 int sml_emu_allreduce(int nranks, void* const* in_ptrs, void* const* out_ptrs, uint64_t numel,
                       int elem_type, int mode, int algo, int block_numel, uint64_t slot_bytes,
                       int slots_per_channel, int channels, float post_scale, int repeats,

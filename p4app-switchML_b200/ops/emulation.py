@@ -2,12 +2,15 @@
 
 Kernels of different ranks wait for each other, so they cannot be tested as separate
 launches on a single device. Instead one cooperative launch plays all ranks: its
-``blockIdx.y`` is the rank, every rank's staging memory lives on the same device and the
-peer-memory code path runs unchanged (csrc/kernels/allreduce_kernels.cu,
-``AllReduceEmuKernel``). Messages of 2^18 elements per rank and more ("staged" and "push") take
-pipelines made for ranks that share a GPU instead, whose results go straight into all outputs
-(csrc/kernels/one_gpu_allreduce.cu); the checked build of the library keeps to the kernels between
-GPUs at every size. Used by the GPU tests and for kernel profiling on one device.
+``blockIdx.y`` is the rank and every rank's staging memory lives on the same device
+(csrc/kernels/allreduce_kernels.cu, ``AllReduceEmuKernel``). The code is that of ranks on GPUs of
+their own, but for what only links ask for: the one-barrier kernel parks an input once and has
+the others read it there, reducers keep more loads in flight, flags have GPU scope. The checked
+build of the library runs the code between GPUs as it is. Messages of 2^18 elements per rank and
+more ("staged" and "push") take pipelines made for ranks that share a GPU instead, whose results go
+straight into all outputs (csrc/kernels/one_gpu_allreduce.cu), unless a tensor is off its 16-byte
+boundary or in pinned memory; the checked build does not, unless it is asked to
+(``emulated_allreduce_with``). Used by the GPU tests and for kernel profiling on one device.
 """
 import ctypes
 
@@ -24,8 +27,9 @@ def emulated_allreduce(inputs, mode="quant", algo="staged", block_numel=256, slo
                        slots_per_channel=2, channels=0, post_scale=1.0, repeats=1, outputs=None,
                        exponent_lookahead=-1):
     """Allreduce `inputs` (a list of equally sized 1-D CUDA tensors, one per virtual rank,
-    all on the current device). Returns the list of per-rank outputs. `exponent_lookahead`:
-    tiles by which the exact mode's exponents run ahead of their data (-1: the library's default).
+    all on the current device). Returns the list of per-rank outputs. `block_numel`: with "staged" and "push" a power of two
+    from 32 to 1024 in the exact mode. `exponent_lookahead`: tiles by which the exact mode's exponents run ahead of their data
+    (-1: the library's default) below 2^18 elements per rank; the pipelines above always run two ahead.
 
     `slot_bytes` and `slots_per_channel` are taken as they are (rounded to whole units of a tile) below 2^18 elements per rank. Above
     they are upper bounds: tiles and rings are cut to what stays in L2 and in shared memory. The results do not depend on either, but

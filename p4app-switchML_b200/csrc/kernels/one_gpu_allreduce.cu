@@ -309,7 +309,6 @@ __device__ __forceinline__ void FeedReducer(const Tiles<ELEM, MODE_QUANT, kPush,
           (lane == 0 ? tiles.InTensor(from, bytes, 16) : tiles.InSlots(kPush ? tiles.me : i < tiles.me ? i : i + 1, from, bytes, 16)))
         BulkLoad(stage, from, bytes, bar);
     }
-    __syncwarp();
   }
   for (unsigned t = k > kOneReduceStages ? k - kOneReduceStages : 0; t < k; t++)  // as above
     Drain(&sh->full[kOneLoadStages + t % kOneReduceStages], (t / kOneReduceStages) & 1);
